@@ -1,153 +1,500 @@
-// Paged attention, general kernel: any head size up to 256, any head counts, any mix of
+// Paged attention, general kernels: any head size up to 256, any head counts, any mix of
 // prompt portions and decode tokens, optional sliding window (with an optional number of first
-// positions that stay visible behind it), float or bf16 storage.
+// positions that stay visible behind it), float or bf16 storage.  The attention of the 32-bit
+// path; the bf16 path uses it for shapes its faster kernels refuse.
 //
-// One warp owns one (token, query head) row and walks the request's keys (the kept first positions
-// that lie behind the window, then from the first position inside the window to the token's own) in
-// steps of 32 keys: each lane scores one key
-// (a full dot product over the head, in ascending order), the warp keeps a running maximum
-// and sum (online softmax, 32-bit), and every lane accumulates its own slice of the output
-// over the 32 values.  The walk depends only on the token's position, never on how the
-// step was cut or batched, so a row's result is bit-identical under any cutting.  This is
-// the kernel of the 32-bit path; the bf16 path uses it for shapes its faster kernels refuse.
+// A row is a (token, query head) pair.  What is computed for it depends on its position alone, never
+// on how the step was cut or batched, so that a row has the same bits under any cutting:
+//   * the cached positions fall into segments of 256 and chunks of 64 (both from position 0 on);
+//   * a score is one accumulator in ascending d, times the scale; a chunk's maximum and its sum of
+//     exponentials (lanes hold keys n and n + 32, then a butterfly) update a running maximum and sum
+//     that start anew with every segment; an output entry is one accumulator over the segment's keys
+//     in ascending order, scaled down when the maximum grows;
+//   * segments are added to the row's result one after the other (`Folded`).
+// A key the row does not see has probability zero, and a chunk without visible keys changes nothing.
+//
+// Two kernels do exactly that:
+//   attention_tile: 64 rows of one request and kv head a block (portions of prompts).  Keys and values
+//     of a chunk lie in shared memory and serve all rows, 4 x 4 scores and 4 x 4 NJ outputs a thread.
+//     Bound by the FMA units and the shared-memory reads that feed them.
+//   attention_few: at most 8 rows (decoded tokens), a warp a row; the segments of a request go to
+//     different blocks and a third kernel folds them.  Bound by the reading of keys and values.
+// Which one takes a request follows its rows (new tokens times query heads a kv head): a tile of 64 rows
+// costs its 64 rows' arithmetic however few there are.  24 heads of 128 over 8 kv heads, a portion of 250
+// tokens beside 6 decoded ones behind 750 to 1,000 cached: 82 us (tiles) and 61 us (few and folding); a warp
+// a row walking its keys alone, which these kernels took the place of, needed 926 us.
 //
 // Cache layout: [pages, KVH, page_size, D]; page ids come from table[req, pos / page_size].
 #include "common.cuh"
 
 #define ATT_MAX_D 256
-#define ATT_WARPS 4
+#define ATT_THREADS 256
+#define ATT_CHUNK 64
+#define ATT_SEGMENT 256
+#define ATT_ROWS 64
+#define ATT_FEW 8
+#define ATT_LS (ATT_ROWS + 4)
 
 template <typename T>
-__device__ __forceinline__ float dot_row(const T* __restrict__ k, const float* __restrict__ q, int D,
-                                         bool vec) {
-  float acc = 0.0f;
+struct AttParams {
+  T* out; const T* q; const T* k_cache; const T* v_cache;
+  const int* table; const int* positions; const int* query_start;
+  int out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages, window, keep_first, vec, segments;
+  float scale;
+  float* partial;            // [reqs, KVH, segments, ATT_FEW, D + 2]: accumulators, maximum, sum
+  int* status;
+};
+
+// A row's result over the segments so far: maximum M, sum L; each of its accumulators a becomes a_factor * a +
+// s_factor * (the segment's accumulator).
+struct Folded {
+  float M, L;
+  float a_factor, s_factor;
+  __device__ __forceinline__ void fold(float m, float l) {           // m is finite: the segment holds a visible key
+    const float top = fmaxf(M, m);
+    a_factor = M == -INFINITY ? 0.0f : expf(M - top);
+    s_factor = expf(m - top);
+    L = fmaf(l, s_factor, __fmul_rn(L, a_factor));
+    M = top;
+  }
+};
+
+// One chunk's scores of a row, keys `lane` and `lane + 32` (-INFINITY: not seen), become probabilities; the row's
+// running maximum and sum move on.  Returns the factor its accumulators take.
+__device__ __forceinline__ float att_softmax(float& s0, float& s1, float& m, float& l) {
+  const float top = fmaxf(m, warp_max(fmaxf(s0, s1)));
+  const float factor = m == -INFINITY ? 0.0f : expf(m - top);
+  s0 = s0 == -INFINITY ? 0.0f : expf(s0 - top);
+  s1 = s1 == -INFINITY ? 0.0f : expf(s1 - top);
+  l = fmaf(l, factor, warp_sum(s0 + s1));
+  m = top;
+  return factor;
+}
+
+__device__ __forceinline__ float4 att_load4(const float* p, int valid, int vec) {
+  if (vec) return *reinterpret_cast<const float4*>(p);
+  return make_float4(p[0], valid > 1 ? p[1] : 0.0f, valid > 2 ? p[2] : 0.0f, valid > 3 ? p[3] : 0.0f);
+}
+__device__ __forceinline__ float4 att_load4(const bf16* p, int valid, int vec) {
   if (vec) {
-    constexpr int N = Vec16<T>::N;
-    for (int d = 0; d < D; d += N) {
-      Vec16<T> kv;
-      kv.load(k + d);
-#pragma unroll
-      for (int j = 0; j < N; ++j) acc = fmaf(kv.get(j), q[d + j], acc);
-    }
-  } else {
-    for (int d = 0; d < D; ++d) acc = fmaf(to_float(k[d]), q[d], acc);
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                       __uint_as_float(raw.y & 0xffff0000u));
   }
-  return acc;
+  return make_float4(to_float(p[0]), valid > 1 ? to_float(p[1]) : 0.0f, valid > 2 ? to_float(p[2]) : 0.0f,
+                     valid > 3 ? to_float(p[3]) : 0.0f);
+}
+
+// What both kernels share: the rows' positions, which keys any of them sees, and the chunk in shared memory.
+template <typename T>
+struct AttBlock {
+  const AttParams<T>& p;
+  int req, kvh, G, begin, rows, row0;      // rows of this block: row0 .. row0 + rows - 1 of the request's
+  int lo, hi, kept;                        // keys some row sees: [0, kept) and [lo, hi)
+  long long head_off, page_elems;
+
+  __device__ __forceinline__ int position(int r) const { return p.positions[begin + (row0 + r) / G]; }
+  __device__ __forceinline__ int first_of(int pos) const { return p.window > 0 ? max(0, pos - p.window + 1) : 0; }
+  // all threads; `pos` [rows] in shared memory is filled, barrier included
+  __device__ __forceinline__ void look(int* pos, int* ends) {
+    if (threadIdx.x == 0) { ends[0] = 0x7fffffff; ends[1] = 0; ends[2] = 0; }
+    __syncthreads();
+    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+      const int at = position(r), first = first_of(at);
+      pos[r] = at;
+      atomicMin(&ends[0], first);
+      atomicMax(&ends[1], at + 1);
+      atomicMax(&ends[2], min(p.keep_first, first));
+    }
+    __syncthreads();
+    lo = ends[0]; hi = ends[1]; kept = ends[2];
+  }
+  __device__ __forceinline__ bool wanted(int key) const { return (key >= lo && key < hi) || key < kept; }
+  __device__ __forceinline__ bool chunk_wanted(int base) const {
+    return (base + ATT_CHUNK > lo && base < hi) || base < kept;
+  }
+  __device__ __forceinline__ bool seen(int key, int pos) const {
+    const int first = first_of(pos);
+    return key <= pos && (key >= first || key < min(p.keep_first, first));
+  }
+  // Offsets of the chunk's keys in the cache (-1: nobody's, or a bad page, which is reported); barrier included.
+  __device__ __forceinline__ void find(int base, long long* offset) {
+    if (threadIdx.x < ATT_CHUNK) {
+      const int key = base + threadIdx.x;
+      long long at = -1;
+      if (wanted(key)) {
+        const int page = p.table[(size_t)req * p.table_stride + key / p.page_size];
+        if (page <= 0 || page >= p.num_pages) atomicOr(p.status, KVB_STATUS_BAD_PAGE);
+        else at = (long long)page * page_elems + head_off + (long long)(key % p.page_size) * p.D;
+      }
+      offset[threadIdx.x] = at;
+    }
+    __syncthreads();
+  }
+  // Rows of a plane's chunk into shared memory as floats, `width` (a multiple of four) a row, zeros behind D.
+  __device__ __forceinline__ void fetch(float* dst, int stride, int width, const T* plane, const long long* offset) {
+    const int pieces = width >> 2;
+#pragma unroll 8
+    for (int e = threadIdx.x; e < ATT_CHUNK * pieces; e += ATT_THREADS) {
+      const int key = e / pieces, d = (e - key * pieces) << 2;
+      const long long at = offset[key];
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (at >= 0 && d < p.D) v = att_load4(plane + at + d, p.D - d, p.vec);
+      *reinterpret_cast<float4*>(dst + key * stride + d) = v;
+    }
+  }
+  __device__ __forceinline__ void fetch_queries(float* dst, int stride, int width) {
+    const int pieces = width >> 2;
+    for (int e = threadIdx.x; e < rows * pieces; e += ATT_THREADS) {
+      const int r = e / pieces, d = (e - r * pieces) << 2, row = row0 + r;
+      const T* src = p.q + (size_t)(begin + row / G) * p.q_stride + (size_t)(kvh * G + row % G) * p.D;
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (d < p.D) {                       // rows of q lie anywhere: entry by entry
+        v.x = to_float(src[d]);
+        if (d + 1 < p.D) v.y = to_float(src[d + 1]);
+        if (d + 2 < p.D) v.z = to_float(src[d + 2]);
+        if (d + 3 < p.D) v.w = to_float(src[d + 3]);
+      }
+      *reinterpret_cast<float4*>(dst + r * stride + d) = v;
+    }
+  }
+  __device__ __forceinline__ T* out_row(int r) const {
+    const int row = row0 + r;
+    return p.out + (size_t)(begin + row / G) * p.out_stride + (size_t)(kvh * G + row % G) * p.D;
+  }
+};
+
+template <typename T, int NJ>              // NJ: output columns in runs of 64
+__global__ void __launch_bounds__(ATT_THREADS)
+attention_tile_kernel(AttParams<T> p) {
+  KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
+  const int req = blockIdx.x / p.KVH, kvh = blockIdx.x % p.KVH, G = p.H / p.KVH;
+  const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
+  const int row0 = (gridDim.y - 1 - blockIdx.y) * ATT_ROWS;          // the tiles with the most keys first
+  if (all_rows <= ATT_FEW || row0 >= all_rows) return;
+  extern __shared__ __align__(16) float smem[];
+  const int DK = (p.D + 3) & ~3, LK = DK + 4;
+  constexpr int DV = 64 * NJ;
+  float* const qs = smem;                                            // [ATT_ROWS][LK]
+  float* const ks = qs + ATT_ROWS * LK;                              // [ATT_CHUNK][LK]
+  float* const vs = ks + ATT_CHUNK * LK;                             // [ATT_CHUNK][DV]
+  float* const ss = vs + ATT_CHUNK * DV;                             // [ATT_CHUNK][ATT_LS]: scores, then probabilities
+  __shared__ long long offset[ATT_CHUNK];
+  __shared__ int pos[ATT_ROWS], ends[3];
+  __shared__ float factor[ATT_ROWS], run_m[ATT_ROWS], run_l[ATT_ROWS];
+  AttBlock<T> b{p, req, kvh, G, begin, min(ATT_ROWS, all_rows - row0), row0, 0, 0, 0,
+                (long long)kvh * p.page_size * p.D, (long long)p.KVH * p.page_size * p.D};
+  b.look(pos, ends);
+  b.fetch_queries(qs, LK, DK);
+  // lanes of a warp: 4 x 8 threads, neighbours sharing a row, so that a warp's 16-byte reads are few distinct lines
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ty = (warp >> 1) * 4 + (lane & 1) + 2 * (lane >> 4), tx = (warp & 1) * 8 + ((lane >> 1) & 7);
+  float acc[4][4 * NJ], sum[4][4 * NJ];
+  Folded total[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    total[i] = Folded{-INFINITY, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int j = 0; j < 4 * NJ; ++j) sum[i][j] = 0.0f;
+  }
+
+  for (int segment = 0; segment < b.hi; segment += ATT_SEGMENT) {
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4 * NJ; ++j) acc[i][j] = 0.0f;
+    for (int base = segment; base < segment + ATT_SEGMENT; base += ATT_CHUNK) {
+      if (!b.chunk_wanted(base)) continue;
+      __syncthreads();                                               // the chunk in front has been read
+      if (!any)
+        for (int r = threadIdx.x; r < ATT_ROWS; r += ATT_THREADS) { run_m[r] = -INFINITY; run_l[r] = 0.0f; }
+      any = true;
+      b.find(base, offset);
+      b.fetch(ks, LK, DK, p.k_cache, offset);
+      b.fetch(vs, DV, DV, p.v_cache, offset);
+      __syncthreads();
+      float s[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+#pragma unroll 2
+      for (int d = 0; d < DK; d += 4) {
+        float4 qv[4], kv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const float4*>(qs + (ty + 16 * i) * LK + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * LK + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            s[i][j] = fmaf(kv[j].x, qv[i].x, s[i][j]);
+            s[i][j] = fmaf(kv[j].y, qv[i].y, s[i][j]);
+            s[i][j] = fmaf(kv[j].z, qv[i].z, s[i][j]);
+            s[i][j] = fmaf(kv[j].w, qv[i].w, s[i][j]);
+          }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = tx + 16 * j;
+        const bool there = offset[key] >= 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = ty + 16 * i;
+          ss[key * ATT_LS + r] = there && r < b.rows && b.seen(base + key, pos[r]) ? __fmul_rn(s[i][j], p.scale) : -INFINITY;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int n = 0; n < ATT_ROWS / 8; ++n) {
+        const int r = warp * (ATT_ROWS / 8) + n;
+        float s0 = ss[lane * ATT_LS + r], s1 = ss[(lane + 32) * ATT_LS + r], m = run_m[r], l = run_l[r];
+        const float f = att_softmax(s0, s1, m, l);
+        ss[lane * ATT_LS + r] = s0;
+        ss[(lane + 32) * ATT_LS + r] = s1;
+        __syncwarp();
+        if (lane == 0) { run_m[r] = m; run_l[r] = l; factor[r] = f; }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float f = factor[ty * 4 + i];
+#pragma unroll
+        for (int j = 0; j < 4 * NJ; ++j) acc[i][j] *= f;
+      }
+#pragma unroll 4
+      for (int key = 0; key < ATT_CHUNK; ++key) {
+        const float4 pr = *reinterpret_cast<const float4*>(ss + key * ATT_LS + ty * 4);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const float4 v = *reinterpret_cast<const float4*>(vs + key * DV + j * 64 + tx * 4);
+          const float w[4] = {pr.x, pr.y, pr.z, pr.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            acc[i][4 * j] = fmaf(w[i], v.x, acc[i][4 * j]);
+            acc[i][4 * j + 1] = fmaf(w[i], v.y, acc[i][4 * j + 1]);
+            acc[i][4 * j + 2] = fmaf(w[i], v.z, acc[i][4 * j + 2]);
+            acc[i][4 * j + 3] = fmaf(w[i], v.w, acc[i][4 * j + 3]);
+          }
+        }
+      }
+    }
+    if (!any) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float m = run_m[ty * 4 + i];
+      if (m == -INFINITY) continue;
+      total[i].fold(m, run_l[ty * 4 + i]);
+#pragma unroll
+      for (int j = 0; j < 4 * NJ; ++j)
+        sum[i][j] = fmaf(acc[i][j], total[i].s_factor, __fmul_rn(sum[i][j], total[i].a_factor));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = ty * 4 + i;
+    if (r >= b.rows) continue;
+    const float inv = total[i].L > 0.0f ? 1.0f / total[i].L : 0.0f;
+    T* to = b.out_row(r);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int d = j * 64 + tx * 4 + c;
+        if (d < p.D) to[d] = from_float<T>(sum[i][4 * j + c] * inv);
+      }
+  }
+}
+
+template <typename T, int NJ>              // NJ: output columns in runs of 64
+__global__ void __launch_bounds__(ATT_THREADS)
+attention_few_kernel(AttParams<T> p) {
+  KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
+  const int req = blockIdx.x / p.KVH, kvh = blockIdx.x % p.KVH, G = p.H / p.KVH;
+  const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
+  if (all_rows > ATT_FEW || all_rows == 0) return;
+  extern __shared__ __align__(16) float smem[];
+  const int DK = (p.D + 3) & ~3, LK = DK + 4;
+  constexpr int DV = 64 * NJ, RUNS = (NJ + 1) / 2;                   // a lane's quads of output columns: 128 apart
+  float* const qs = smem;                                            // [ATT_FEW][LK]
+  float* const ks = qs + ATT_FEW * LK;                               // [ATT_CHUNK][LK]
+  float* const vs = ks + ATT_CHUNK * LK;                             // [ATT_CHUNK][DV]
+  __shared__ long long offset[ATT_CHUNK];
+  __shared__ int pos[ATT_FEW], ends[3];
+  __shared__ float probability[ATT_FEW][ATT_CHUNK];
+  AttBlock<T> b{p, req, kvh, G, begin, all_rows, 0, 0, 0, 0,
+                (long long)kvh * p.page_size * p.D, (long long)p.KVH * p.page_size * p.D};
+  b.look(pos, ends);
+  b.fetch_queries(qs, LK, DK);
+  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;           // a warp a row
+  const bool live = r < all_rows;
+  const int segment = blockIdx.y * ATT_SEGMENT;
+  float acc[RUNS][4], m = -INFINITY, l = 0.0f;
+#pragma unroll
+  for (int j = 0; j < RUNS; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+  for (int base = segment; base < segment + ATT_SEGMENT; base += ATT_CHUNK) {
+    if (!b.chunk_wanted(base)) continue;
+    __syncthreads();                                                 // the chunk in front has been read
+    b.find(base, offset);
+    b.fetch(ks, LK, DK, p.k_cache, offset);
+    b.fetch(vs, DV, DV, p.v_cache, offset);
+    __syncthreads();
+    if (!live) continue;
+    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll 4
+    for (int d = 0; d < DK; d += 4) {
+      const float4 q = *reinterpret_cast<const float4*>(qs + r * LK + d);
+      const float4 a = *reinterpret_cast<const float4*>(ks + lane * LK + d);
+      const float4 c = *reinterpret_cast<const float4*>(ks + (lane + 32) * LK + d);
+      s0 = fmaf(a.x, q.x, s0); s0 = fmaf(a.y, q.y, s0); s0 = fmaf(a.z, q.z, s0); s0 = fmaf(a.w, q.w, s0);
+      s1 = fmaf(c.x, q.x, s1); s1 = fmaf(c.y, q.y, s1); s1 = fmaf(c.z, q.z, s1); s1 = fmaf(c.w, q.w, s1);
+    }
+    s0 = offset[lane] >= 0 && b.seen(base + lane, pos[r]) ? __fmul_rn(s0, p.scale) : -INFINITY;
+    s1 = offset[lane + 32] >= 0 && b.seen(base + lane + 32, pos[r]) ? __fmul_rn(s1, p.scale) : -INFINITY;
+    const float f = att_softmax(s0, s1, m, l);
+    probability[r][lane] = s0;
+    probability[r][lane + 32] = s1;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < RUNS; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[j][c] *= f;
+#pragma unroll 8
+    for (int key = 0; key < ATT_CHUNK; ++key) {
+      const float w = probability[r][key];
+#pragma unroll
+      for (int j = 0; j < RUNS; ++j) {
+        const int d = j * 128 + lane * 4;
+        if (d < DV) {
+          const float4 v = *reinterpret_cast<const float4*>(vs + key * DV + d);
+          acc[j][0] = fmaf(w, v.x, acc[j][0]);
+          acc[j][1] = fmaf(w, v.y, acc[j][1]);
+          acc[j][2] = fmaf(w, v.z, acc[j][2]);
+          acc[j][3] = fmaf(w, v.w, acc[j][3]);
+        }
+      }
+    }
+    __syncwarp();                                                    // the probabilities have been read
+  }
+  if (!live) return;
+  if (p.segments > 1) {
+    float* part = p.partial + (((size_t)blockIdx.x * p.segments + blockIdx.y) * ATT_FEW + r) * (p.D + 2);
+#pragma unroll
+    for (int j = 0; j < RUNS; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int d = j * 128 + lane * 4 + c;
+        if (d < p.D && m != -INFINITY) part[d] = acc[j][c];
+      }
+    if (lane == 0) { part[p.D] = m; part[p.D + 1] = l; }
+    return;
+  }
+  const float inv = l > 0.0f ? 1.0f / l : 0.0f;                      // one segment: folding it changes nothing
+  T* to = b.out_row(r);
+#pragma unroll
+  for (int j = 0; j < RUNS; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int d = j * 128 + lane * 4 + c;
+      if (d < p.D) to[d] = from_float<T>(acc[j][c] * inv);
+    }
+}
+
+// Folds the segments of the requests that attention_few took: a block a (request, kv head), a warp a row.
+template <typename T>
+__global__ void __launch_bounds__(ATT_THREADS)
+attention_fold_kernel(AttParams<T> p) {
+  KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
+  const int req = blockIdx.x / p.KVH, kvh = blockIdx.x % p.KVH, G = p.H / p.KVH;
+  const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
+  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (all_rows > ATT_FEW || r >= all_rows) return;
+  constexpr int MOST = ATT_MAX_D / 32;
+  float sum[MOST];
+#pragma unroll
+  for (int j = 0; j < MOST; ++j) sum[j] = 0.0f;
+  Folded total{-INFINITY, 0.0f, 0.0f, 0.0f};
+  const int last = min(p.segments - 1, p.positions[begin + r / G] / ATT_SEGMENT);
+  for (int s = 0; s <= last; ++s) {
+    const float* part = p.partial + (((size_t)blockIdx.x * p.segments + s) * ATT_FEW + r) * (p.D + 2);
+    const float m = part[p.D];
+    if (m == -INFINITY) continue;
+    total.fold(m, part[p.D + 1]);
+#pragma unroll
+    for (int j = 0; j < MOST; ++j)
+      if (lane + 32 * j < p.D) sum[j] = fmaf(part[lane + 32 * j], total.s_factor, __fmul_rn(sum[j], total.a_factor));
+  }
+  const float inv = total.L > 0.0f ? 1.0f / total.L : 0.0f;
+  T* to = p.out + (size_t)(begin + r / G) * p.out_stride + (size_t)(kvh * G + r % G) * p.D;
+#pragma unroll
+  for (int j = 0; j < MOST; ++j)
+    if (lane + 32 * j < p.D) to[lane + 32 * j] = from_float<T>(sum[j] * inv);
+}
+
+template <typename T, int NJ>
+static int launch_attention(AttParams<T> p, int tokens, int reqs, int max_query_len, cudaStream_t stream) {
+  const int G = p.H / p.KVH, most = max_query_len * G, LK = ((p.D + 3) & ~3) + 4, DV = 64 * NJ;
+  // a batch of equal portions has only one kind of request
+  const bool equal = (long long)max_query_len * reqs == tokens;
+  if (most > ATT_FEW) {
+    const int smem = (int)sizeof(float) * (ATT_ROWS * LK + ATT_CHUNK * (LK + DV + ATT_LS));
+    KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_tile_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KVB_CHECK_CUDA(kvb_launch((attention_tile_kernel<T, NJ>), dim3(reqs * p.KVH, (most + ATT_ROWS - 1) / ATT_ROWS),
+                              dim3(ATT_THREADS), smem, stream, true, p));
+  }
+  if (G <= ATT_FEW && (most <= ATT_FEW || !equal)) {
+    const int smem = (int)sizeof(float) * (ATT_FEW * LK + ATT_CHUNK * (LK + DV));
+    KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_few_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3(reqs * p.KVH, p.segments), dim3(ATT_THREADS), smem, stream,
+                              true, p));
+    if (p.segments > 1)
+      KVB_CHECK_CUDA(kvb_launch((attention_fold_kernel<T>), dim3(reqs * p.KVH), dim3(ATT_THREADS), 0, stream, true, p));
+  }
+  KVB_CHECK_LAUNCH();
+  return 0;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
-paged_attention_rows_kernel(T* __restrict__ out, int out_stride, const T* __restrict__ q,
-                            int q_stride, const T* __restrict__ k_cache,
-                            const T* __restrict__ v_cache, const int* __restrict__ table,
-                            int table_stride, const int* __restrict__ positions,
-                            const int* __restrict__ req_index, int num_rows, int H, int KVH, int D,
-                            int page_size, int num_pages, float scale, int window, int keep_first,
-                            int vec, int* status) {
-  KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
-  __shared__ float q_smem[ATT_WARPS][ATT_MAX_D];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * ATT_WARPS + warp;
-  if (row >= num_rows) return;
-  const int token = row / H, head = row % H;
-  const int kvh = head / (H / KVH);
-  const int pos = positions[token];
-  const int* pages = table + (size_t)req_index[token] * table_stride;
-
-  const T* qrow = q + (size_t)token * q_stride + (size_t)head * D;
-  for (int d = lane; d < D; d += 32) q_smem[warp][d] = to_float(qrow[d]);
-  __syncwarp();
-
-  constexpr int SLICES = ATT_MAX_D / 32;
-  float acc[SLICES];
-#pragma unroll
-  for (int i = 0; i < SLICES; ++i) acc[i] = 0.0f;
-  float running_max = -INFINITY, running_sum = 0.0f;
-  const size_t head_off = (size_t)kvh * page_size * D;
-  const size_t page_elems = (size_t)KVH * page_size * D;
-  const int first = window > 0 ? max(0, pos - window + 1) : 0;
-
-  // two runs of keys: [0, kept) behind the window, then [first, pos]
-  const int kept = min(keep_first, first);
-  for (int run = kept > 0 ? 0 : 1; run < 2; ++run) {
-  const int run_lo = run == 0 ? 0 : first, run_hi = run == 0 ? kept : pos + 1;
-  for (int base = run_lo; base < run_hi; base += 32) {
-    const int key = base + lane;
-    const bool valid = key < run_hi;
-    float score = -INFINITY;
-    int page = 0;
-    if (valid) {
-      page = pages[key / page_size];
-      if (page <= 0 || page >= num_pages) {
-        atomicOr(status, KVB_STATUS_BAD_PAGE);
-        page = 0;
-      } else {
-        const T* krow = k_cache + (size_t)page * page_elems + head_off + (size_t)(key % page_size) * D;
-        score = dot_row<T>(krow, q_smem[warp], D, vec) * scale;
-      }
-    }
-    const float chunk_max = warp_max(score);
-    const float new_max = fmaxf(running_max, chunk_max);
-    // new_max is finite whenever the chunk holds one readable key; key `base` always is
-    const float p = (score == -INFINITY) ? 0.0f : expf(score - new_max);
-    const float correction = (running_max == -INFINITY) ? 0.0f : expf(running_max - new_max);
-    running_sum = running_sum * correction + warp_sum(p);
-    running_max = new_max;
-#pragma unroll
-    for (int i = 0; i < SLICES; ++i) acc[i] *= correction;
-    const int count = min(32, run_hi - base);
-    for (int kk = 0; kk < count; ++kk) {
-      const float pk = __shfl_sync(0xffffffffu, p, kk);
-      const int pg = __shfl_sync(0xffffffffu, page, kk);
-      if (pg == 0) continue;  // uniform across the warp
-      const T* vrow = v_cache + (size_t)pg * page_elems + head_off + (size_t)((base + kk) % page_size) * D;
-#pragma unroll
-      for (int i = 0; i < SLICES; ++i) {
-        const int d = lane + 32 * i;
-        if (d < D) acc[i] = fmaf(pk, to_float(vrow[d]), acc[i]);
-      }
-    }
-  }
-  }
-  const float inv = running_sum > 0.0f ? 1.0f / running_sum : 0.0f;
-  T* orow = out + (size_t)token * out_stride + (size_t)head * D;
-#pragma unroll
-  for (int i = 0; i < SLICES; ++i) {
-    const int d = lane + 32 * i;
-    if (d < D) orow[d] = from_float<T>(acc[i] * inv);
-  }
+static int attention_of(const AttParams<T>& p, int tokens, int reqs, int max_query_len, cudaStream_t stream) {
+  if (p.D <= 64) return launch_attention<T, 1>(p, tokens, reqs, max_query_len, stream);
+  if (p.D <= 128) return launch_attention<T, 2>(p, tokens, reqs, max_query_len, stream);
+  return launch_attention<T, 4>(p, tokens, reqs, max_query_len, stream);
 }
 
+// Floats of the scratch that a batch takes whose longest request has `segments` segments of cached tokens.
+extern "C" long long kvb_paged_attention_scratch(int num_reqs, int KVH, int D, int segments) {
+  return segments > 1 ? (long long)num_reqs * KVH * segments * ATT_FEW * (D + 2) : 0;
+}
+extern "C" int kvb_paged_attention_segment() { return ATT_SEGMENT; }
+
+// `segments`: segments of cached tokens that the longest request of at most ATT_FEW rows may have.
 extern "C" int kvb_paged_attention_rows(void* out, int out_stride, const void* q, int q_stride,
                                         const void* k_cache, const void* v_cache, const int* table,
-                                        int table_stride, const int* positions, const int* req_index,
-                                        int tokens, int H, int KVH, int D, int page_size,
-                                        int num_pages, float scale, int window, int keep_first,
+                                        int table_stride, const int* positions, const int* query_start, int num_reqs,
+                                        int max_query_len, int tokens, int H, int KVH, int D, int page_size,
+                                        int num_pages, float scale, int window, int keep_first, int segments, float* partial,
                                         int dtype, cudaStream_t stream) {
-  if (tokens == 0) return 0;
+  if (tokens == 0 || num_reqs == 0) return 0;
   KVB_REQUIRE(D > 0 && D <= ATT_MAX_D, "paged_attention: head_dim must be in [1, 256]");
   KVB_REQUIRE(H > 0 && KVH > 0 && H % KVH == 0, "paged_attention: H must be a multiple of KVH");
   KVB_REQUIRE(page_size > 0 && num_pages > 1, "paged_attention: empty cache");
   KVB_REQUIRE(keep_first >= 0 && (keep_first == 0 || window > 0), "paged_attention: kept first positions need a window");
+  KVB_REQUIRE((long long)num_reqs * KVH < (1ll << 31), "paged_attention: too many requests");
+  KVB_REQUIRE(max_query_len > 0 && (long long)max_query_len * (H / KVH) <= 65535LL * ATT_ROWS, "paged_attention: too many rows");
+  KVB_REQUIRE(segments >= 1 && segments <= 65535 && (segments == 1 || partial != nullptr), "paged_attention: no scratch");
   int* status = kvb_status_word();
   KVB_REQUIRE(status != nullptr, "paged_attention: no status word");
   const int esize = dtype == KVB_F32 ? 4 : 2;
-  const int vec = ((size_t)D * esize) % 16 == 0 && aligned16(k_cache);
-  const long long rows = (long long)tokens * H;
-  KVB_REQUIRE(rows < (1ll << 31), "paged_attention: too many rows");
-  const int blocks = (int)((rows + ATT_WARPS - 1) / ATT_WARPS);
-  if (dtype == KVB_F32)
-    KVB_CHECK_CUDA(kvb_launch((paged_attention_rows_kernel<float>), dim3(blocks), dim3(ATT_WARPS * 32), 0, stream, true, 
-        (float*)out, out_stride, (const float*)q, q_stride, (const float*)k_cache,
-        (const float*)v_cache, table, table_stride, positions, req_index, (int)rows, H, KVH, D,
-        page_size, num_pages, scale, window, keep_first, vec, status));
-  else
-    KVB_CHECK_CUDA(kvb_launch((paged_attention_rows_kernel<bf16>), dim3(blocks), dim3(ATT_WARPS * 32), 0, stream, true, 
-        (bf16*)out, out_stride, (const bf16*)q, q_stride, (const bf16*)k_cache,
-        (const bf16*)v_cache, table, table_stride, positions, req_index, (int)rows, H, KVH, D,
-        page_size, num_pages, scale, window, keep_first, vec, status));
-  KVB_CHECK_LAUNCH();
-  return 0;
+  const int vec = D % 4 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % (4 * esize) == 0;
+#define KVB_ATT(T_)                                                                                                    \
+  attention_of<T_>(AttParams<T_>{(T_*)out, (const T_*)q, (const T_*)k_cache, (const T_*)v_cache, table, positions,     \
+                                 query_start, out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages,     \
+                                 window, keep_first, vec, segments, scale, partial, status},                           \
+                   tokens, num_reqs, max_query_len, stream)
+  return dtype == KVB_F32 ? KVB_ATT(float) : KVB_ATT(bf16);
+#undef KVB_ATT
 }
 
 KVB_TRACE_TU(attention_generic)

@@ -1,10 +1,11 @@
-"""The 32-bit path's product: every kernel a batch may go to gives a row the same bits."""
+"""The 32-bit path's product and attention: every kernel a batch may go to gives a row the same bits."""
 from __future__ import annotations
 
 import pytest
 import torch
 
-from test_kernels_gpu import DEV, K, randn
+import plain_kernels as P
+from test_kernels_gpu import DEV, K, _cache_case, _Ctx, randn
 
 pytestmark = pytest.mark.gpu
 
@@ -23,3 +24,33 @@ def test_product_rows_have_the_same_bits_in_every_kernel(n, k):
     wide = torch.zeros(20, k + 3, dtype=torch.float32, device=DEV)          # rows that start off 16-byte boundaries
     wide[:, 3:] = x[:20]
     assert torch.equal(K().linear(wide[:, 3:], w, bias), full[:20])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv_heads,dim,page,window,keep", [
+    (6, 2, 128, 16, None, 0), (4, 2, 16, 16, None, 0), (3, 1, 72, 8, None, 0), (4, 4, 256, 32, None, 0), (4, 1, 130, 4, None, 0),
+    (6, 2, 64, 16, 100, 0), (6, 2, 128, 16, 300, 0), (4, 1, 64, 16, 70, 65), (24, 2, 32, 16, 33, 5)])
+def test_attention_rows_have_the_same_bits_in_every_kernel(dtype, heads, kv_heads, dim, page, window, keep):
+    """A prompt in tiles of 64 rows against its last tokens alone, whose segments are read by different blocks; lengths
+    around segments (256) and chunks (64)."""
+    for total in (1, 63, 257, 513, 700):
+        case = _cache_case(dtype, heads, kv_heads, dim, page, [(0, total)], seed=total)
+
+        def run(first, count, reserved):
+            part = dict(case, positions=case["positions"][first:first + count], lens=[(first, count)],
+                        req_index=case["req_index"][first:first + count],
+                        query_start=torch.tensor([0, count], dtype=torch.int32, device=DEV),
+                        context_lens=torch.tensor([first], dtype=torch.int32, device=DEV))
+            ctx = _Ctx(part)
+            ctx.max_seq_len_bound = first + count + reserved
+            return K().paged_attention(case["qkv"][first:first + count], case["k_cache"], case["v_cache"], case["table"], ctx,
+                                       heads, kv_heads, dim, dim ** -0.5, window, keep_first=keep, force_general=True)
+        whole = run(0, total, 0)
+        for count in (1, 2, 8, 40):
+            if count <= total:
+                assert torch.equal(run(total - count, count, 600), whole[total - count:]), (total, count)
+        want = P.paged_attention_plain(case["qkv"], case["k_cache"], case["v_cache"], case["table"], case["positions"],
+                                       case["req_index"], heads, kv_heads, dim, dim ** -0.5, window, keep)
+        torch.testing.assert_close(whole, want, **(dict(rtol=2e-5, atol=2e-5) if dtype == torch.float32
+                                                   else dict(rtol=2e-2, atol=2e-2)))
+    assert K().read_status() == 0
