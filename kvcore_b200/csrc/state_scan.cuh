@@ -33,6 +33,7 @@
 #include "common.cuh"
 
 #define SCAN_THREADS 128
+#define SCAN_SM_BYTES (228 * 1024)     // shared memory of an SM; a block's share comes with 1 KB on top
 
 __device__ __forceinline__ void scan_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
@@ -41,6 +42,27 @@ __device__ __forceinline__ void scan_copy4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
 __device__ __forceinline__ void scan_copies_done() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// Two neighbouring rows of a column (or the same number twice) in one register pair; an instruction rounds each half as
+// the plain one does, so the state has the same bits, and takes one issue slot for both.
+typedef unsigned long long ScanPair;
+__device__ __forceinline__ ScanPair scan_pair(float lo, float hi) {
+  ScanPair d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+  return d;
+}
+__device__ __forceinline__ float scan_lo(ScanPair a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float scan_hi(ScanPair a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ ScanPair scan_mul(ScanPair a, ScanPair b) {
+  ScanPair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ ScanPair scan_fma(ScanPair a, ScanPair b, ScanPair c) {
+  ScanPair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
 
 struct ScanParams {
   // 32-bit vectors per token: q and k [D] of head h / kv_share, and (decay per key channel) the decays a [D]
@@ -65,7 +87,7 @@ struct ScanParams {
 // holds those rows of CPT neighbouring columns (one load of q, k and the decays then serves CPT columns, and the
 // columns' chains of dependent instructions run interleaved); BATCH tokens a stage of shared memory.
 template <typename TV, int MODE, int DREG, int RSPLIT, int CPT, int BATCH>
-__global__ void __launch_bounds__(SCAN_THREADS)
+__global__ void __launch_bounds__(SCAN_THREADS, BATCH <= 2 ? 5 : 1)     // brief: every block's state in flight counts
 state_scan_kernel(ScanParams p) {
   KVB_KERNEL_PROLOGUE(MODE == 0 ? KVB_TAG_GLA_SCAN : MODE == 1 ? KVB_TAG_DELTA_SCAN
                                                    : MODE == 2 ? KVB_TAG_LIGHTNING_SCAN : KVB_TAG_SSM_SCAN);
@@ -80,10 +102,13 @@ state_scan_kernel(ScanParams p) {
   constexpr int J = DREG / 4;
   constexpr int GROUP = BATCH < 8 ? BATCH : 8;      // tokens whose read-outs are summed over the threads together
   float* const vectors = smem;                      // [2][BATCH][TOKEN]
-  float* const values = smem + 2 * STAGE;           // [2][BATCH][COLS]
+  float* const values = smem + 2 * STAGE;           // [2][BATCH][COLS][2]: every value twice, the halves of a pair
 
   const int req = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-  const int part = tid % RSPLIT, c = tid / RSPLIT * CPT;
+  // neighbouring lanes hold the same rows of different columns: what they read of q and k is then the same word, which
+  // the shared memory serves them at once
+  constexpr int BESIDE = 32 / RSPLIT;               // columns (times CPT) a warp holds side by side
+  const int part = (tid & 31) / BESIDE, c = ((tid >> 5) * BESIDE + (tid & 31) % BESIDE) * CPT;
   const int col = blockIdx.z * COLS + c;            // the first of this thread's columns
   const int begin = p.query_start[req], end = p.query_start[req + 1];
   const int D = p.D, V = p.V;
@@ -94,7 +119,7 @@ state_scan_kernel(ScanParams p) {
   // In shared memory a vector's piece n lies at place (n % J) * RSPLIT + n / J, so that for one j the parts of a
   // column read neighbouring pieces.
   float* const S_head = p.state + (size_t)p.state_slots[req] * p.state_stride + p.state_offset + (size_t)h * V * D;
-  float S[CPT][DREG];
+  float4 held_state[CPT][J];                        // all of it on its way before any of it is looked at
 #pragma unroll
   for (int cc = 0; cc < CPT; ++cc) {
     const float* S_column = S_head + (size_t)(col + cc < V ? col + cc : 0) * D;
@@ -112,9 +137,10 @@ state_scan_kernel(ScanParams p) {
           if (row + 3 < D) s4.w = S_column[row + 3];
         }
       }
-      S[cc][4 * j] = s4.x; S[cc][4 * j + 1] = s4.y; S[cc][4 * j + 2] = s4.z; S[cc][4 * j + 3] = s4.w;
+      held_state[cc][j] = s4;
     }
   }
+  ScanPair S[CPT][DREG / 2];
   auto place = [](int row) { return (((row >> 2) % J) * RSPLIT + (row >> 2) / J) * 4 + (row & 3); };
   if (D < DP)                                       // rows beyond D read zeros whatever the stage holds
     for (int e = tid; e < 2 * BATCH * NVEC * (DP - D); e += SCAN_THREADS) {
@@ -174,10 +200,11 @@ state_scan_kernel(ScanParams p) {
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       const int e = tid + j * SCAN_THREADS, tt = e / COLS, cc = blockIdx.z * COLS + e % COLS;
-      if (e < BATCH * COLS) values[stage * BATCH * COLS + e] = (tt < nb && cc < V) ? to_float(held[j]) : 0.0f;
+      const float v = (tt < nb && cc < V) ? to_float(held[j]) : 0.0f;
+      if (e < BATCH * COLS) *reinterpret_cast<ScanPair*>(values + 2 * (stage * BATCH * COLS + e)) = scan_pair(v, v);
     }
   };
-  const float head_decay = MODE == 2 ? p.a[h] : 0.0f;
+  const ScanPair head_decay = MODE == 2 ? scan_pair(p.a[h], p.a[h]) : 0;
   const float head_skip = MODE == 3 ? p.skip[h] : 0.0f;
   // One token: the state's step and this thread's part of the read-out of each of its columns.  A sum over a
   // column's rows is taken piece by piece (four rows, in order), and the pieces are added as a tree over their
@@ -192,95 +219,91 @@ state_scan_kernel(ScanParams p) {
   };
   // The sums over the column's threads of the read-out are left to the caller, who takes them for all tokens of
   // a stage at once: those shuffles do not wait for one another, and the state's step does not wait for them.
-  auto token = [&](const float* q, const float* vs, float (&o_own)[CPT]) {
+  struct Vectors {                                    // what a token brings: its columns' values (twice), q, k, decays
+    ScanPair v[CPT];
+    ulonglong2 k4[J], a4[J];
+    float4 q4[J];
+    float first, second;                              // beta and g, or dt and g
+  };
+  auto take = [&](Vectors& n, const float* q, const float* vs) {
     const float* k = q + DP;
-    float v[CPT];
     if constexpr (CPT == 4) {
-      const float4 v4 = *reinterpret_cast<const float4*>(vs);
-      v[0] = v4.x; v[1] = v4.y; v[2] = v4.z; v[3] = v4.w;
+      const ulonglong2 v01 = *reinterpret_cast<const ulonglong2*>(vs), v23 = *reinterpret_cast<const ulonglong2*>(vs + 4);
+      n.v[0] = v01.x; n.v[1] = v01.y; n.v[2] = v23.x; n.v[3] = v23.y;
     } else {
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) v[cc] = vs[cc];
+      for (int cc = 0; cc < CPT; ++cc) n.v[cc] = *reinterpret_cast<const ScanPair*>(vs + 2 * cc);
     }
-    float4 k4[J], q4[J];
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-      k4[j] = *reinterpret_cast<const float4*>(k + (j * RSPLIT + part) * 4);
-      q4[j] = *reinterpret_cast<const float4*>(q + (j * RSPLIT + part) * 4);
+      n.k4[j] = *reinterpret_cast<const ulonglong2*>(k + (j * RSPLIT + part) * 4);
+      n.q4[j] = *reinterpret_cast<const float4*>(q + (j * RSPLIT + part) * 4);
+      if (MODE == 0) n.a4[j] = *reinterpret_cast<const ulonglong2*>(k + DP + (j * RSPLIT + part) * 4);
     }
+    if (MODE == 1 || MODE == 3) {
+      const float2 two = *reinterpret_cast<const float2*>(q + NVEC * DP);
+      n.first = two.x;
+      n.second = two.y;
+    }
+  };
+  auto token = [&](Vectors& n, float (&o_own)[CPT]) {
+    ScanPair (&v)[CPT] = n.v;
+    const ulonglong2 (&k4)[J] = n.k4;
+    const float4 (&q4)[J] = n.q4;
     float o[CPT][J];
-    if (MODE == 0) {
-      const float* a = k + DP;
+    auto dot4 = [](const ScanPair* s, const float4& w) {
+      return fmaf(scan_hi(s[1]), w.w, fmaf(scan_lo(s[1]), w.z, fmaf(scan_hi(s[0]), w.y, scan_lo(s[0]) * w.x)));
+    };
+    if (MODE != 1) {
+      ScanPair decay = MODE == 2 ? head_decay : 0;
+      if (MODE == 3) {
+        const float dt = n.first, g = n.second;
+        decay = scan_pair(g, g);
+#pragma unroll
+        for (int cc = 0; cc < CPT; ++cc) v[cc] = scan_mul(scan_pair(dt, dt), v[cc]);
+      }
 #pragma unroll
       for (int j = 0; j < J; ++j) {
-        const float4 a4 = *reinterpret_cast<const float4*>(a + (j * RSPLIT + part) * 4);
+        ulonglong2 a4 = make_ulonglong2(decay, decay);
+        if (MODE == 0) a4 = n.a4[j];
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
-          float* s = &S[cc][4 * j];
-          s[0] = fmaf(k4[j].x, v[cc], a4.x * s[0]);
-          s[1] = fmaf(k4[j].y, v[cc], a4.y * s[1]);
-          s[2] = fmaf(k4[j].z, v[cc], a4.z * s[2]);
-          s[3] = fmaf(k4[j].w, v[cc], a4.w * s[3]);
-          o[cc][j] = fmaf(s[3], q4[j].w, fmaf(s[2], q4[j].z, fmaf(s[1], q4[j].y, s[0] * q4[j].x)));
-        }
-      }
-    } else if (MODE == 2) {
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-#pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) {
-          float* s = &S[cc][4 * j];
-          s[0] = fmaf(k4[j].x, v[cc], head_decay * s[0]);
-          s[1] = fmaf(k4[j].y, v[cc], head_decay * s[1]);
-          s[2] = fmaf(k4[j].z, v[cc], head_decay * s[2]);
-          s[3] = fmaf(k4[j].w, v[cc], head_decay * s[3]);
-          o[cc][j] = fmaf(s[3], q4[j].w, fmaf(s[2], q4[j].z, fmaf(s[1], q4[j].y, s[0] * q4[j].x)));
-        }
-      }
-    } else if (MODE == 3) {
-      const float dt = q[NVEC * DP], g = q[NVEC * DP + 1];
-#pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) {
-        const float u = dt * v[cc];
-#pragma unroll
-        for (int j = 0; j < J; ++j) {
-          float* s = &S[cc][4 * j];
-          s[0] = fmaf(k4[j].x, u, g * s[0]);
-          s[1] = fmaf(k4[j].y, u, g * s[1]);
-          s[2] = fmaf(k4[j].z, u, g * s[2]);
-          s[3] = fmaf(k4[j].w, u, g * s[3]);
-          o[cc][j] = fmaf(s[3], q4[j].w, fmaf(s[2], q4[j].z, fmaf(s[1], q4[j].y, s[0] * q4[j].x)));
+          ScanPair* s = &S[cc][2 * j];
+          s[0] = scan_fma(k4[j].x, v[cc], scan_mul(a4.x, s[0]));
+          s[1] = scan_fma(k4[j].y, v[cc], scan_mul(a4.y, s[1]));
+          o[cc][j] = dot4(s, q4[j]);
         }
       }
     } else {
-      const float beta = q[NVEC * DP], g = q[NVEC * DP + 1];
+      const float beta = n.first, g = n.second;
+      const ScanPair decay = scan_pair(g, g);
       float dot[CPT];
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) {
         float d[J];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-          float* s = &S[cc][4 * j];
-          s[0] *= g; s[1] *= g; s[2] *= g; s[3] *= g;
-          d[j] = fmaf(s[3], k4[j].w, fmaf(s[2], k4[j].z, fmaf(s[1], k4[j].y, s[0] * k4[j].x)));
+          ScanPair* s = &S[cc][2 * j];
+          s[0] = scan_mul(decay, s[0]);
+          s[1] = scan_mul(decay, s[1]);
+          d[j] = dot4(s, make_float4(scan_lo(k4[j].x), scan_hi(k4[j].x), scan_lo(k4[j].y), scan_hi(k4[j].y)));
         }
         dot[cc] = own(d);
       }
 #pragma unroll
       for (int m = 1; m < RSPLIT; m <<= 1)
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) dot[cc] += __shfl_xor_sync(0xffffffffu, dot[cc], m);
+        for (int cc = 0; cc < CPT; ++cc) dot[cc] += __shfl_xor_sync(0xffffffffu, dot[cc], m * BESIDE);
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) {
-        const float u = beta * (v[cc] - dot[cc]);
+        const float u1 = beta * (scan_lo(v[cc]) - dot[cc]);
+        const ScanPair u = scan_pair(u1, u1);
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-          float* s = &S[cc][4 * j];
-          s[0] = fmaf(k4[j].x, u, s[0]);
-          s[1] = fmaf(k4[j].y, u, s[1]);
-          s[2] = fmaf(k4[j].z, u, s[2]);
-          s[3] = fmaf(k4[j].w, u, s[3]);
-          o[cc][j] = fmaf(s[3], q4[j].w, fmaf(s[2], q4[j].z, fmaf(s[1], q4[j].y, s[0] * q4[j].x)));
+          ScanPair* s = &S[cc][2 * j];
+          s[0] = scan_fma(k4[j].x, u, s[0]);
+          s[1] = scan_fma(k4[j].y, u, s[1]);
+          o[cc][j] = dot4(s, q4[j]);
         }
       }
     }
@@ -293,7 +316,7 @@ state_scan_kernel(ScanParams p) {
     if (part != 0) return;
     if (MODE == 3)
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) sum[cc] = fmaf(head_skip, vs[cc], sum[cc]);
+      for (int cc = 0; cc < CPT; ++cc) sum[cc] = fmaf(head_skip, vs[2 * cc], sum[cc]);
     if (CPT == 4 && out16 && col < V) {
       *reinterpret_cast<float4*>(at) = make_float4(sum[0], sum[1], sum[2], sum[3]);
       return;
@@ -310,6 +333,13 @@ state_scan_kernel(ScanParams p) {
   }
   scan_copies_done();
   __syncthreads();
+#pragma unroll
+  for (int cc = 0; cc < CPT; ++cc)
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      S[cc][2 * j] = scan_pair(held_state[cc][j].x, held_state[cc][j].y);
+      S[cc][2 * j + 1] = scan_pair(held_state[cc][j].z, held_state[cc][j].w);
+    }
   int stage = 0;
   const size_t out_token = (size_t)p.heads * V;
   for (int t0 = begin; t0 < end; t0 += BATCH, stage ^= 1) {
@@ -320,32 +350,63 @@ state_scan_kernel(ScanParams p) {
       load_values(next, next_nb);
     }
     const float* st = vectors + stage * STAGE;
-    const float* vs = values + stage * BATCH * COLS + c;
+    const float* vs = values + 2 * (stage * BATCH * COLS + c);
     float* out_at = p.out + ((size_t)t0 * p.heads + h) * V + (col < V ? col : 0);
-    if (nb == BATCH) {                                // a full stage: nothing to ask between its tokens
+    if (BATCH > 2 && nb == BATCH) {                   // a full stage: nothing to ask between its tokens
+      Vectors now;                                    // a token's vectors are read while the one in front is computed
+      take(now, st, vs);
 #pragma unroll
       for (int g = 0; g < BATCH; g += GROUP) {
-        float sums[GROUP][CPT];
+        float sums[GROUP * CPT];                      // entry tt * CPT + cc
 #pragma unroll
-        for (int tt = 0; tt < GROUP; ++tt) token(st + (g + tt) * TOKEN, vs + (g + tt) * COLS, sums[tt]);
+        for (int tt = 0; tt < GROUP; ++tt) {
+          float own_part[CPT];
+          Vectors next_one;
+          if (g + tt + 1 < BATCH) take(next_one, st + (g + tt + 1) * TOKEN, vs + 2 * (g + tt + 1) * COLS);
+          token(now, own_part);
+          now = next_one;
 #pragma unroll
-        for (int m = 1; m < RSPLIT; m <<= 1)
+          for (int cc = 0; cc < CPT; ++cc) sums[tt * CPT + cc] = own_part[cc];
+        }
+        // The same tree as above, but a pair of threads shares the work of a level: either keeps half of the entries,
+        // hands the other half over and adds what it is handed (31 exchanges for 32 entries of 32 threads, not 160).
+        // At the end a thread holds LEFT entries, from `entry` on.
+        constexpr int N = GROUP * CPT, LEFT = N > RSPLIT ? N / RSPLIT : 1;
+        int entry = 0;
 #pragma unroll
-          for (int tt = 0; tt < GROUP; ++tt)
+        for (int m = 1, half = N / 2; m < RSPLIT; m <<= 1, half >>= 1) {
+          if (half > 0) {
+            const bool upper = (part & m) != 0;
+            if (upper) entry += half;
 #pragma unroll
-            for (int cc = 0; cc < CPT; ++cc) sums[tt][cc] += __shfl_xor_sync(0xffffffffu, sums[tt][cc], m);
+            for (int i = 0; i < half; ++i) {
+              const float keep = upper ? sums[i + half] : sums[i], give = upper ? sums[i] : sums[i + half];
+              sums[i] = keep + __shfl_xor_sync(0xffffffffu, give, m * BESIDE);
+            }
+          } else {
+            sums[0] += __shfl_xor_sync(0xffffffffu, sums[0], m * BESIDE);
+          }
+        }
+        if (part < N) {                               // with more threads than entries, several hold the same
 #pragma unroll
-        for (int tt = 0; tt < GROUP; ++tt) write_out(out_at + (g + tt) * out_token, sums[tt], vs + (g + tt) * COLS);
+          for (int i = 0; i < LEFT; ++i) {
+            const int tt = g + (entry + i) / CPT, cc = (entry + i) % CPT;
+            if (MODE == 3) sums[i] = fmaf(head_skip, vs[2 * (tt * COLS + cc)], sums[i]);
+            if (col + cc < V) out_at[tt * out_token + cc] = sums[i];
+          }
+        }
       }
     } else {
       for (int tt = 0; tt < nb; ++tt) {
         float sum[CPT];
-        token(st + tt * TOKEN, vs + tt * COLS, sum);
+        Vectors now;
+        take(now, st + tt * TOKEN, vs + 2 * tt * COLS);
+        token(now, sum);
 #pragma unroll
         for (int m = 1; m < RSPLIT; m <<= 1)
 #pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) sum[cc] += __shfl_xor_sync(0xffffffffu, sum[cc], m);
-        write_out(out_at + tt * out_token, sum, vs + tt * COLS);
+          for (int cc = 0; cc < CPT; ++cc) sum[cc] += __shfl_xor_sync(0xffffffffu, sum[cc], m * BESIDE);
+        write_out(out_at + tt * out_token, sum, vs + 2 * tt * COLS);
       }
     }
     if (next < end) store_values(stage ^ 1, next_nb);
@@ -362,12 +423,12 @@ state_scan_kernel(ScanParams p) {
       if (row < D) {
         if (p.state16) {
           *reinterpret_cast<float4*>(S_column + row) =
-              make_float4(S[cc][4 * j], S[cc][4 * j + 1], S[cc][4 * j + 2], S[cc][4 * j + 3]);
+              make_float4(scan_lo(S[cc][2 * j]), scan_hi(S[cc][2 * j]), scan_lo(S[cc][2 * j + 1]), scan_hi(S[cc][2 * j + 1]));
         } else {
-          S_column[row] = S[cc][4 * j];
-          if (row + 1 < D) S_column[row + 1] = S[cc][4 * j + 1];
-          if (row + 2 < D) S_column[row + 2] = S[cc][4 * j + 2];
-          if (row + 3 < D) S_column[row + 3] = S[cc][4 * j + 3];
+          S_column[row] = scan_lo(S[cc][2 * j]);
+          if (row + 1 < D) S_column[row + 1] = scan_hi(S[cc][2 * j]);
+          if (row + 2 < D) S_column[row + 2] = scan_lo(S[cc][2 * j + 1]);
+          if (row + 3 < D) S_column[row + 3] = scan_hi(S[cc][2 * j + 1]);
         }
       }
     }
@@ -379,10 +440,13 @@ state_scan_kernel(ScanParams p) {
 // 4,096 columns a request).  A step of single tokens moves every state once and does little else: 8 rows of four
 // columns, stages of two tokens (6 KB a block, so that many blocks share an SM).  A step with prompts in it is a
 // chain of dependent instructions per token, and the stages' hand-overs cost as much as their tokens: stages of
-// 16 tokens; the delta rule, whose chain passes through a sum over the column's threads, 16 rows of one column
-// (three shuffles in the chain, not five); the decay per channel, whose chain stays inside a thread, 8 or 4 rows
-// of four columns (one load of q, k and the decays serves four columns) while that still fills the SMs, else 4
-// rows of one column, which gives four times the warps.
+// 16 tokens; 8 rows of four columns (one load of q, k and the decays serves four columns, the least work a row) once
+// they give the SMs two blocks each (one for the delta rule), else 4 rows of four columns; for the delta rule, whose
+// chain passes through a sum over the column's threads, 16 rows of one column (three shuffles in the chain, not five).
+// Microseconds, preparation included (B200, keys of 128): fixed decay, one prompt of 2,048, 16 heads of 256 values: 8 x 4
+// 310, 4 x 4 286, 16 x 1 362, 4 x 1 710 (before two rows of the state shared an instruction and threads shared the sums'
+// exchanges: 4 x 4 726); 8 heads: 298, 203, 231, 489; state space, 4 prompts of 400, 32 heads of 64: 118, 126, 154, 267;
+// delta rule, one prompt of 2,048, 16 heads of 128: 658, 462, 318, 670; 4 prompts of 512: 201, 279, 237, 597.
 struct ScanShape { int rows, cols; bool brief; };
 static long long scan_blocks(int D, long long heads_of_all, int V, int rows, int cols) {
   int rsplit = 1;
@@ -402,9 +466,9 @@ static ScanShape scan_shape(int mode, int D, long long heads_of_all, int V, bool
   if (c == 4) return {least, least <= 8 ? 4 : 1, brief && least == 8};
   if (c == 1) return {least, 1, false};
   if (brief) return least <= 8 ? ScanShape{8, 4, true} : ScanShape{16, 1, true};
+  if (least <= 8 && scan_blocks(D, heads_of_all, V, 8, 4) >= (mode == 1 ? 1 : 2) * sms) return {8, 4, false};
   if (mode == 1) return {16, 1, false};
-  if (least <= 8 && scan_blocks(D, heads_of_all, V, 8, 4) >= 2 * sms) return {8, 4, false};
-  if (least <= 4 && scan_blocks(D, heads_of_all, V, 4, 4) >= sms) return {4, 4, false};
+  if (least <= 4) return {4, 4, false};
   return {least, 1, false};
 }
 
@@ -422,16 +486,20 @@ static int launch_state_scan(const ScanParams& p_in, int num_reqs, long long tok
   const int cols = SCAN_THREADS / rsplit * cpt;
   const dim3 grid(num_reqs, p.heads, (p.V + cols - 1) / cols), block(SCAN_THREADS);
   cudaError_t err = cudaErrorInvalidValue;
+  // A launch with prompts in it lasts as long as its fullest SM.  Its blocks may come in while the kernel in front
+  // still holds some SMs (dependent launch) and would then crowd on the others: each asks for so much shared memory
+  // that no SM holds more of them than its share.
+  const long long sms = kvb_sm_count() > 0 ? kvb_sm_count() : 148;
+  const long long blocks = (long long)grid.x * grid.y * grid.z, share = (blocks + sms - 1) / sms;
+  const size_t alone = !shape.brief && share <= 8 ? SCAN_SM_BYTES / (size_t)(share + 1) : 0;
 #define SCAN_CASE(DR, RS, CP, BRIEF)                                                                          \
   if (dreg == DR && rsplit == RS && cpt == CP && shape.brief == BRIEF) {                                      \
     constexpr int B = BRIEF ? 2 : DR * RS <= 128 ? 16 : 2048 / (DR * RS);                                     \
-    const size_t smem = 2 * (size_t)B * ((MODE == 0 ? 3 : 2) * DR * RS + 4 + SCAN_THREADS / RS * CP) * sizeof(float); \
-    static bool allowed = false;                      /* more than 48 KB a block is asked for once */         \
-    if (smem > 48 * 1024 && !allowed) {                                                                       \
+    size_t smem = 2 * (size_t)B * ((MODE == 0 ? 3 : 2) * DR * RS + 4 + 2 * (SCAN_THREADS / RS * CP)) * sizeof(float); \
+    if (smem < alone) smem = alone;                                                                           \
+    if (smem > 48 * 1024)                                                                                     \
       KVB_CHECK_CUDA(cudaFuncSetAttribute(state_scan_kernel<TV, MODE, DR, RS, CP, B>,                         \
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));           \
-      allowed = true;                                                                                         \
-    }                                                                                                         \
     err = kvb_launch((state_scan_kernel<TV, MODE, DR, RS, CP, B>), grid, block, smem, stream, true, p);       \
   }
 #define SCAN_ROWS(DR, CP, BRIEF)                                                                              \
