@@ -1,7 +1,7 @@
 // Mixture of experts: router, grouping of (token, chosen expert) pairs by expert, the experts' two
 // matrix products as grouped products over that order, and the weighted sum back per token.
 //
-//   route:   z = W_router x in 32-bit (one warp per expert row, lane-strided k in a fixed order, butterfly sum);
+//   route:   z = W_router x in 32-bit (lane-strided k in a fixed order, butterfly sum);
 //            scores = sigmoid(z) or softmax(z); the `top` largest (lowest index among equals); weights are
 //            the chosen scores, optionally divided by their sum.  A third way scores with z itself and weights the
 //            chosen experts by the softmax over their logits alone.  Optionally z has a bias, the choice goes by
@@ -32,68 +32,150 @@
 #define MOE_BM 16
 #define MOE_BN 64
 #define MOE_BK 16
-#define MOE_ROUTE_THREADS 512
 
-// TPB tokens a block share every pass over a router row (a prompt's tokens would otherwise each pull the
-// whole router through the L2 cache); a token's sums are formed in the same order whatever TPB is: lane l
-// adds the products k = l, l + 32, ... into four partial sums by (k / 32) % 4, then ((p0 + p1) + (p2 + p3)),
-// then the butterfly over the lanes.
-template <typename T, int TPB>
-__global__ void __launch_bounds__(MOE_ROUTE_THREADS)
-moe_route_kernel(int* __restrict__ ids_out, float* __restrict__ weights_out, float* __restrict__ gate_out,
-                 const T* __restrict__ x, long long x_stride, const float* __restrict__ router,
-                 const float* __restrict__ gate_rows, int tokens, int E, int R, int K, int top, int score_mode,
-                 int renormalize, const float* __restrict__ correction, int groups, int keep, float weight_scale,
-                 const float* __restrict__ bias) {
+// The logits, [tokens, E + R] 32-bit, and the choice are two kernels, so that a step of few tokens spreads the router's
+// rows over many blocks.  A logit is formed in the same order whichever kernel takes it: lane l adds the products
+// k = l, l + 32, ... into four partial sums by (k / 32) % 4, then ((p0 + p1) + (p2 + p3)), then the butterfly over the
+// lanes.  2,048 tokens, 32 experts, rows of 4,096 (B200, cold caches): 55 us and 10 for the choice; one kernel that read
+// x entry by entry from shared memory for each expert apart took 88.
+template <typename T>
+struct RouteParams {
+  float* logits; const T* x; long long x_stride;
+  const float* router; const float* gate_rows;
+  int tokens, E, R, K;
+  __device__ __forceinline__ const float* row(int e) const {
+    return e < E ? router + (size_t)e * K : gate_rows + (size_t)(e - E) * K;
+  }
+};
+
+// Few tokens: a block takes one expert and ROUTE_FEW tokens, its four warps a partial sum each, everything straight from
+// memory.  Bound by the latency of the reads.
+#define ROUTE_FEW 4
+#define ROUTE_AHEAD 16
+template <typename T>
+__global__ void __launch_bounds__(128)
+moe_logits_few_kernel(RouteParams<T> p) {
+  KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ROUTE);
+  __shared__ float parts[4][ROUTE_FEW][32];
+  const int lane = threadIdx.x & 31, j = threadIdx.x >> 5, e = blockIdx.y, token0 = blockIdx.x * ROUTE_FEW;
+  const float* w = p.row(e);
+  const T* x[ROUTE_FEW];
+#pragma unroll
+  for (int t = 0; t < ROUTE_FEW; ++t) x[t] = p.x + (size_t)min(token0 + t, p.tokens - 1) * p.x_stride;
+  float part[ROUTE_FEW];
+#pragma unroll
+  for (int t = 0; t < ROUTE_FEW; ++t) part[t] = 0.0f;
+  for (int k0 = 32 * j + lane; k0 < p.K; k0 += ROUTE_AHEAD * 128) {
+    float wv[ROUTE_AHEAD];
+    T xv[ROUTE_FEW][ROUTE_AHEAD];
+#pragma unroll
+    for (int i = 0; i < ROUTE_AHEAD; ++i) {
+      const int k = k0 + 128 * i;
+      wv[i] = k < p.K ? w[k] : 0.0f;                  // zeros add nothing
+#pragma unroll
+      for (int t = 0; t < ROUTE_FEW; ++t) xv[t][i] = k < p.K ? x[t][k] : from_float<T>(0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < ROUTE_AHEAD; ++i)
+#pragma unroll
+      for (int t = 0; t < ROUTE_FEW; ++t) part[t] = fmaf(wv[i], to_float(xv[t][i]), part[t]);
+  }
+#pragma unroll
+  for (int t = 0; t < ROUTE_FEW; ++t) parts[j][t][lane] = part[t];
+  __syncthreads();
+  const float acc = warp_sum((parts[0][j][lane] + parts[1][j][lane]) + (parts[2][j][lane] + parts[3][j][lane]));
+  if (lane == 0 && token0 + j < p.tokens) p.logits[(size_t)(token0 + j) * (p.E + p.R) + e] = acc;   // warp t: token t
+}
+
+// Many tokens: a block holds TOKENS (8 or 16) rows of x in shared memory, a lane's four entries of 128 lying together, and
+// a warp forms the logits of four experts for eight of them at once: an entry of x read once serves four experts, one of
+// the router eight tokens.  Bound by the latency of the router's entries, which come from the L2 cache a run of 128 ahead.
+#define ROUTE_TOKENS 8
+#define ROUTE_EXPERTS 4
+template <typename T>
+struct __align__(4 * sizeof(T)) RouteQuad { T v[4]; };
+template <typename T, int TOKENS>
+__global__ void __launch_bounds__(TOKENS * 16)
+moe_logits_kernel(RouteParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ROUTE);
   extern __shared__ __align__(16) unsigned char route_smem[];
-  T* xs = reinterpret_cast<T*>(route_smem);                                   // [TPB][K]
-  float* scores = reinterpret_cast<float*>(route_smem + (size_t)TPB * K * sizeof(T));   // [TPB][E + R]
-  float* choices = scores + (size_t)TPB * (E + R);                                      // [TPB][E + 2 * groups]
-  const int token0 = blockIdx.x * TPB;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = MOE_ROUTE_THREADS / 32;
-  for (int i = threadIdx.x; i < TPB * K; i += MOE_ROUTE_THREADS) {
-    const int t = i / K, k = i % K;
-    xs[i] = token0 + t < tokens ? x[(size_t)(token0 + t) * x_stride + k] : from_float<T>(0.0f);
+  RouteQuad<T>* xs = reinterpret_cast<RouteQuad<T>*>(route_smem);             // [TOKENS][runs of 128][32 lanes]
+  const int runs = (p.K + 127) / 128;
+  int token0 = blockIdx.x * TOKENS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll 8
+  for (int i = warp; i < TOKENS * runs; i += TOKENS / 2) {
+    const int t = i / runs, k = (i - t * runs) * 128 + lane;
+    const T* row = p.x + (size_t)(token0 + t) * p.x_stride;
+    RouteQuad<T> q;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      q.v[j] = token0 + t < p.tokens && k + 32 * j < p.K ? row[k + 32 * j] : from_float<T>(0.0f);
+    xs[i * 32 + lane] = q;
   }
   __syncthreads();
-  for (int e = warp; e < E + R; e += nwarps) {
-    const float* w = e < E ? router + (size_t)e * K : gate_rows + (size_t)(e - E) * K;
-    float part[TPB][4];
+  const int all = p.E + p.R;
+  token0 += warp / 4 * ROUTE_TOKENS;                  // four warps share eight tokens
+  xs += (size_t)(warp / 4) * ROUTE_TOKENS * runs * 32;
+  for (int e0 = warp % 4 * ROUTE_EXPERTS; e0 < all; e0 += 4 * ROUTE_EXPERTS) {
+    const float* w[ROUTE_EXPERTS];
 #pragma unroll
-    for (int t = 0; t < TPB; ++t) part[t][0] = part[t][1] = part[t][2] = part[t][3] = 0.0f;
-    int k = lane;
-    for (; k + 96 < K; k += 128) {
-      const float w0 = w[k], w1 = w[k + 32], w2 = w[k + 64], w3 = w[k + 96];
+    for (int n = 0; n < ROUTE_EXPERTS; ++n) w[n] = p.row(min(e0 + n, all - 1));
+    float part[ROUTE_EXPERTS][ROUTE_TOKENS][4];
 #pragma unroll
-      for (int t = 0; t < TPB; ++t) {
-        const T* xt = xs + (size_t)t * K;
-        part[t][0] = fmaf(w0, to_float(xt[k]), part[t][0]);
-        part[t][1] = fmaf(w1, to_float(xt[k + 32]), part[t][1]);
-        part[t][2] = fmaf(w2, to_float(xt[k + 64]), part[t][2]);
-        part[t][3] = fmaf(w3, to_float(xt[k + 96]), part[t][3]);
+    for (int n = 0; n < ROUTE_EXPERTS; ++n)
+#pragma unroll
+      for (int t = 0; t < ROUTE_TOKENS; ++t) part[n][t][0] = part[n][t][1] = part[n][t][2] = part[n][t][3] = 0.0f;
+    float wv[ROUTE_EXPERTS][4], next[ROUTE_EXPERTS][4];
+    auto fetch = [&](int run) {                       // the next run's router entries are on their way meanwhile
+      const int k = run * 128 + lane;
+#pragma unroll
+      for (int n = 0; n < ROUTE_EXPERTS; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) next[n][j] = k + 32 * j < p.K ? w[n][k + 32 * j] : 0.0f;   // zeros add nothing
+    };
+    fetch(0);
+    for (int run = 0; run < runs; ++run) {
+#pragma unroll
+      for (int n = 0; n < ROUTE_EXPERTS; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wv[n][j] = next[n][j];
+      if (run + 1 < runs) fetch(run + 1);
+#pragma unroll
+      for (int t = 0; t < ROUTE_TOKENS; ++t) {
+        const RouteQuad<T> q = xs[(t * runs + run) * 32 + lane];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float xv = to_float(q.v[j]);
+#pragma unroll
+          for (int n = 0; n < ROUTE_EXPERTS; ++n) part[n][t][j] = fmaf(wv[n][j], xv, part[n][t][j]);
+        }
       }
     }
-    for (int j = 0; k < K; k += 32, ++j) {
-      const float wk = w[k];
 #pragma unroll
-      for (int t = 0; t < TPB; ++t) {
-        const float prod_x = to_float(xs[(size_t)t * K + k]);
-        if (j == 0) part[t][0] = fmaf(wk, prod_x, part[t][0]);
-        else if (j == 1) part[t][1] = fmaf(wk, prod_x, part[t][1]);
-        else part[t][2] = fmaf(wk, prod_x, part[t][2]);
+    for (int n = 0; n < ROUTE_EXPERTS; ++n)
+#pragma unroll
+      for (int t = 0; t < ROUTE_TOKENS; ++t) {
+        const float acc = warp_sum((part[n][t][0] + part[n][t][1]) + (part[n][t][2] + part[n][t][3]));
+        if (lane == 0 && e0 + n < all && token0 + t < p.tokens) p.logits[(size_t)(token0 + t) * all + e0 + n] = acc;
       }
-    }
-#pragma unroll
-    for (int t = 0; t < TPB; ++t) {
-      const float acc = warp_sum((part[t][0] + part[t][1]) + (part[t][2] + part[t][3]));
-      if (lane == 0) scores[t * (E + R) + e] = acc;
-    }
   }
-  __syncthreads();
-  if (warp >= TPB || token0 + warp >= tokens) return;
-  const int token = token0 + warp;                    // warp t finishes token t of the block
-  float* sc = scores + warp * (E + R);
+}
+
+// From the logits to the chosen experts and their weights: a warp a token.
+#define CHOOSE_THREADS 128
+__global__ void __launch_bounds__(CHOOSE_THREADS)
+moe_choose_kernel(int* __restrict__ ids_out, float* __restrict__ weights_out, float* __restrict__ gate_out,
+                  const float* __restrict__ logits, int tokens, int E, int R, int top, int score_mode, int renormalize,
+                  const float* __restrict__ correction, int groups, int keep, float weight_scale,
+                  const float* __restrict__ bias) {
+  KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ROUTE);
+  extern __shared__ __align__(16) float choose_smem[];                         // a warp: [E + R] and [E + 2 * groups]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, token = blockIdx.x * (blockDim.x / 32) + warp;
+  if (token >= tokens) return;
+  float* sc = choose_smem + (size_t)warp * (2 * E + R + 2 * groups);
+  for (int e = lane; e < E + R; e += 32) sc[e] = logits[(size_t)token * (E + R) + e];
+  __syncwarp();
   for (int r = lane; r < R; r += 32) gate_out[(size_t)token * R + r] = 1.0f / (1.0f + expf(-sc[E + r]));
   if (bias != nullptr)
     for (int e = lane; e < E; e += 32) sc[e] += bias[e];
@@ -110,7 +192,7 @@ moe_route_kernel(int* __restrict__ ids_out, float* __restrict__ weights_out, flo
   }
   __syncwarp();
   // what the choice goes by: the scores, with the correction when there is one
-  float* ch = choices + warp * (E + 2 * groups);
+  float* ch = sc + E + R;
   for (int e = lane; e < E; e += 32) ch[e] = correction != nullptr ? sc[e] + correction[e] : sc[e];
   __syncwarp();
   auto arg_max = [&](const float* values, int count, float& best, int& best_i) {
@@ -175,25 +257,31 @@ moe_route_kernel(int* __restrict__ ids_out, float* __restrict__ weights_out, flo
     }
 }
 
-template <typename T, int TPB>
-static int launch_moe_route(int* ids_out, float* weights_out, float* gate_out, const void* x, long long x_stride,
-                            const float* router, const float* gate_rows, int tokens, int E, int R, int K, int top,
-                            int score_mode, int renormalize, const float* correction, int groups, int keep,
-                            float weight_scale, const float* bias, cudaStream_t stream) {
-  const size_t smem = (size_t)TPB * K * sizeof(T) + (size_t)TPB * (2 * E + R + 2 * groups) * sizeof(float);
-  KVB_REQUIRE(smem <= 200 * 1024, "moe_route: the tokens' rows and scores do not fit in shared memory");
-  if (smem > 48 * 1024)
-    KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_route_kernel<T, TPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  KVB_CHECK_CUDA(kvb_launch((moe_route_kernel<T, TPB>), dim3((tokens + TPB - 1) / TPB), dim3(MOE_ROUTE_THREADS), smem,
-                            stream, true, ids_out, weights_out, gate_out, (const T*)x, x_stride, router, gate_rows,
-                            tokens, E, R, K, top, score_mode, renormalize, correction, groups, keep, weight_scale,
-                            bias));
+template <typename T>
+static int launch_moe_logits(const RouteParams<T>& p, cudaStream_t stream) {
+  // From 128 tokens on the blocks of eight tokens fill enough SMs that reading x and the router less often pays, and
+  // blocks of sixteen once they do; rows too long for shared memory take the other kernel at any number.
+  const long long sms = kvb_sm_count() > 0 ? kvb_sm_count() : 148;
+  const size_t smem = (size_t)ROUTE_TOKENS * ((p.K + 127) / 128) * 128 * sizeof(T);
+  if (p.tokens >= 16 * sms * 2 / 3 && 2 * smem <= 200 * 1024) {
+    KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * smem)));
+    KVB_CHECK_CUDA(kvb_launch((moe_logits_kernel<T, 16>), dim3((p.tokens + 15) / 16), dim3(256), 2 * smem, stream, true, p));
+    return 0;
+  }
+  if (p.tokens >= 128 && smem <= 200 * 1024) {
+    KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T, 8>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KVB_CHECK_CUDA(kvb_launch((moe_logits_kernel<T, 8>), dim3((p.tokens + 7) / 8), dim3(128), smem, stream, true, p));
+    return 0;
+  }
+  KVB_CHECK_CUDA(kvb_launch((moe_logits_few_kernel<T>), dim3((p.tokens + ROUTE_FEW - 1) / ROUTE_FEW, p.E + p.R), dim3(128), 0,
+                            stream, true, p));
   return 0;
 }
 
-extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, const void* x, long long x_stride,
-                             const float* router, const float* gate_rows, int tokens, int E, int R, int K, int top,
-                             int score_mode, int renormalize, const float* correction, int groups, int keep,
+// logits: scratch, [tokens, E + R].
+extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, float* logits, const void* x,
+                             long long x_stride, const float* router, const float* gate_rows, int tokens, int E, int R, int K,
+                             int top, int score_mode, int renormalize, const float* correction, int groups, int keep,
                              float weight_scale, const float* bias, int dtype, cudaStream_t stream) {
   if (tokens == 0) return 0;
   KVB_REQUIRE(E > 0 && K > 0 && top > 0 && top <= E, "moe_route: need 0 < top <= experts");
@@ -202,16 +290,22 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
   KVB_REQUIRE(R >= 0 && (R == 0 || (gate_rows != nullptr && gate_out != nullptr)), "moe_route: gate rows need their weights and output");
   KVB_REQUIRE(score_mode >= 0 && score_mode <= 2, "moe_route: unknown score function");
   if (score_mode == 2) renormalize = 1;
-  // a prompt's tokens go eight a block; a few tokens one a block, for the parallelism
-  const bool many = tokens >= 256 && (size_t)8 * K * (dtype == KVB_F32 ? 4 : 2) <= 96 * 1024;
-  int rc;
-  if (dtype == KVB_F32)
-    rc = many ? launch_moe_route<float, 8>(ids_out, weights_out, gate_out, x, x_stride, router, gate_rows, tokens, E, R, K, top, score_mode, renormalize, correction, groups, keep, weight_scale, bias, stream)
-              : launch_moe_route<float, 1>(ids_out, weights_out, gate_out, x, x_stride, router, gate_rows, tokens, E, R, K, top, score_mode, renormalize, correction, groups, keep, weight_scale, bias, stream);
-  else
-    rc = many ? launch_moe_route<bf16, 8>(ids_out, weights_out, gate_out, x, x_stride, router, gate_rows, tokens, E, R, K, top, score_mode, renormalize, correction, groups, keep, weight_scale, bias, stream)
-              : launch_moe_route<bf16, 1>(ids_out, weights_out, gate_out, x, x_stride, router, gate_rows, tokens, E, R, K, top, score_mode, renormalize, correction, groups, keep, weight_scale, bias, stream);
+  KVB_REQUIRE((long long)E + R <= 65535, "moe_route: too many experts");
+  size_t smem = (size_t)(2 * E + R + 2 * groups) * sizeof(float);
+  KVB_REQUIRE((size_t)K * (dtype == KVB_F32 ? sizeof(float) : sizeof(bf16)) + smem <= 200 * 1024,
+              "moe_route: a token's row and scores do not fit in shared memory");
+  const int rc = dtype == KVB_F32
+      ? launch_moe_logits(RouteParams<float>{logits, (const float*)x, x_stride, router, gate_rows, tokens, E, R, K}, stream)
+      : launch_moe_logits(RouteParams<bf16>{logits, (const bf16*)x, x_stride, router, gate_rows, tokens, E, R, K}, stream);
   if (rc) return rc;
+  int warps = CHOOSE_THREADS / 32;
+  while (warps > 1 && warps * smem > 48 * 1024) warps /= 2;
+  smem *= warps;
+  if (smem > 48 * 1024)
+    KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_choose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  KVB_CHECK_CUDA(kvb_launch((moe_choose_kernel), dim3((tokens + warps - 1) / warps), dim3(32 * warps), smem, stream, true,
+                            ids_out, weights_out, gate_out, (const float*)logits, tokens, E, R, top, score_mode, renormalize,
+                            correction, groups, keep, weight_scale, bias));
   KVB_CHECK_LAUNCH();
   return 0;
 }
@@ -393,73 +487,117 @@ extern "C" int kvb_moe_gemm(void* out, const void* a, long long a_stride, int a_
   return 0;
 }
 
-// Decode-sized batches in bf16: one pass over each chosen expert's matrices.  grid (N / 32, pairs): a block
-// holds the pair's input row (weighted and rounded) in shared memory; each of its 8 warps owns 4 output
-// columns (GATED: the 4 gate rows and the 4 up rows) and walks K in 16-byte loads, lane-strided, the four
-// rows' loads in flight together; a butterfly sums the lanes.  No tile is padded with rows that are not
-// there, so the kernel is bound by the weights it reads.
+// Decode-sized batches in bf16: one pass over each chosen expert's matrices.  grid (N / 32, pairs): the block of the
+// first pair that chose an expert works for all that did, two at a time (the others' blocks leave).  It holds the pairs'
+// input rows (weighted and rounded) in shared memory; each of its 8 warps owns 4 output columns (GATED: the 4 gate rows
+// and the 4 up rows) and walks K in 16-byte loads, lane-strided, two rounds of 256 columns in flight; a butterfly sums
+// the lanes.  No tile is padded with rows that are not there, so the kernel is bound by the weights it reads.
+// 16 experts of 2 x 4,096 x 2,048 and 2,048 x 4,096, 8 tokens of 2 (16 pairs, about 10 experts), the layer around them
+// included: 123 us; a pass for every pair, a round in flight: 138.
 #define MOE_GEMV_COLS 32
+#define MOE_GEMV_PAIRS 2
 template <bool GATED>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, GATED ? 2 : 3)
 moe_gemv_kernel(bf16* __restrict__ out, const bf16* __restrict__ a, long long a_stride, int a_row_div,
                 const float* __restrict__ pair_weight, const bf16* __restrict__ w, const int* __restrict__ ids,
-                int E, int known, int N, int K, int* status, MoeJoin join) {
+                int pairs, int hold, int E, int known, int N, int K, int* status, MoeJoin join) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_GEMM);
   extern __shared__ __align__(16) unsigned char gemv_smem[];
-  bf16* xs = reinterpret_cast<bf16*>(gemv_smem);
-  const int pair = blockIdx.y;
+  bf16* xs = reinterpret_cast<bf16*>(gemv_smem);      // [hold][K], hold <= MOE_GEMV_PAIRS
+  __shared__ int mates[MOE_GEMV_PAIRS];
+  const int pair = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int expert = ids[pair];
   if (expert < 0 || expert >= E) {                   // none, or one without tensors
     if (threadIdx.x == 0 && (expert < 0 || expert >= known)) atomicOr(status, KVB_STATUS_BAD_TOKEN);
     return;
   }
-  const bf16* row = a + (size_t)(pair / a_row_div) * a_stride;
-  const float scale = pair_weight != nullptr ? pair_weight[pair] : 1.0f;
-  for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {
-    Vec16<bf16> v;
-    v.load(row + k);
-    if (pair_weight != nullptr) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v.set(j, v.get(j) * scale);
-    }
-    v.store(xs + k);
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = 0; i < pair; i += 32)                  // every warp sees the same
+    if (__any_sync(0xffffffffu, i + lane < pair && ids[i + lane] == expert)) return;
   const int n0 = blockIdx.x * MOE_GEMV_COLS + warp * 4;
   const bf16* we = w + (size_t)expert * (GATED ? 2 : 1) * N * K;
   constexpr int ROWS = GATED ? 8 : 4;
-  const bf16* rows[ROWS];
-  float acc[ROWS];
+  const bf16* rows[4];                                // (the up rows lie N rows behind the gate rows)
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r) {
-    const int n = min(n0 + (r & 3), N - 1) + (r >= 4 ? N : 0);
-    rows[r] = we + (size_t)n * K;
-    acc[r] = 0.0f;
-  }
-  for (int k = lane * 8; k < K; k += 32 * 8) {
-    Vec16<bf16> x, wv[ROWS];
+  for (int r = 0; r < 4; ++r) rows[r] = we + (size_t)min(n0 + r, N - 1) * K;
+  Vec16<bf16> wv[2][ROWS];                            // this round's 256 columns of K and the next's
+  auto fetch = [&](Vec16<bf16> (&to)[ROWS], int k) {
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) wv[r].load(rows[r] + k);
-    x.load(xs + k);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float xv = x.get(j);
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) acc[r] = fmaf(wv[r].get(j), xv, acc[r]);
+    for (int r = 0; r < ROWS; ++r)
+      if (k < K) to[r].load(rows[r & 3] + (r >= 4 ? (size_t)N * K : 0) + k);
+  };
+  for (int next = pair;;) {
+    int count = 0;                                    // the next pairs of this expert
+    for (int i = next; i < pairs && count < hold; i += 32) {
+      unsigned found = __ballot_sync(0xffffffffu, i + lane < pairs && ids[i + lane] == expert);
+      for (; found != 0 && count < hold; found &= found - 1) {
+        const int mate = i + __ffs(found) - 1;
+        if (threadIdx.x == 0) mates[count] = mate;
+        next = mate + 1;
+        ++count;
+      }
     }
-  }
+    if (count == 0) return;
+    fetch(wv[0], lane * 8);                           // on its way while the rows are staged
+    fetch(wv[1], lane * 8 + 256);
+    __syncthreads();
+    for (int p = 0; p < count; ++p) {
+      const bf16* row = a + (size_t)(mates[p] / a_row_div) * a_stride;
+      const float scale = pair_weight != nullptr ? pair_weight[mates[p]] : 1.0f;
+      for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {
+        Vec16<bf16> v;
+        v.load(row + k);
+        if (pair_weight != nullptr) {
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r) acc[r] = warp_sum(acc[r]);
-  if (lane < 4 && n0 + lane < N) {
-    float v = lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3];
-    if (GATED) {
-      const float u = lane == 0 ? acc[4 % ROWS] : lane == 1 ? acc[5 % ROWS] : lane == 2 ? acc[6 % ROWS] : acc[7 % ROWS];
-      v = moe_join<bf16>(v, u, join);
-    } else {
-      v = moe_plain(v, join);
+          for (int j = 0; j < 8; ++j) v.set(j, v.get(j) * scale);
+        }
+        v.store(xs + (size_t)p * K + k);
+      }
     }
-    out[(size_t)pair * N + n0 + lane] = from_float<bf16>(v);
+    __syncthreads();
+    float acc[MOE_GEMV_PAIRS][ROWS];
+#pragma unroll
+    for (int p = 0; p < MOE_GEMV_PAIRS; ++p)
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) acc[p][r] = 0.0f;
+    auto multiply = [&](const Vec16<bf16> (&from)[ROWS], int k) {
+      if (k >= K) return;
+#pragma unroll
+      for (int p = 0; p < MOE_GEMV_PAIRS; ++p) {
+        if (p < count) {
+          Vec16<bf16> x;
+          x.load(xs + (size_t)p * K + k);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float xv = x.get(j);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) acc[p][r] = fmaf(from[r].get(j), xv, acc[p][r]);
+          }
+        }
+      }
+    };
+    for (int k = lane * 8; k < K; k += 512) {
+      multiply(wv[0], k);
+      fetch(wv[0], k + 512);
+      multiply(wv[1], k + 256);
+      fetch(wv[1], k + 768);
+    }
+#pragma unroll
+    for (int p = 0; p < MOE_GEMV_PAIRS; ++p) {
+      if (p >= count) continue;
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) acc[p][r] = warp_sum(acc[p][r]);
+      if (lane < 4 && n0 + lane < N) {
+        float v = lane == 0 ? acc[p][0] : lane == 1 ? acc[p][1] : lane == 2 ? acc[p][2] : acc[p][3];
+        if (GATED) {
+          const float u = lane == 0 ? acc[p][4 % ROWS] : lane == 1 ? acc[p][5 % ROWS] : lane == 2 ? acc[p][6 % ROWS] : acc[p][7 % ROWS];
+          v = moe_join<bf16>(v, u, join);
+        } else {
+          v = moe_plain(v, join);
+        }
+        out[(size_t)mates[p] * N + n0 + lane] = from_float<bf16>(v);
+      }
+    }
+    __syncthreads();                                  // the rows and their numbers have been read
   }
 }
 
@@ -471,7 +609,10 @@ extern "C" int kvb_moe_gemv(void* out, const void* a, long long a_stride, int a_
   KVB_REQUIRE(N > 0 && K > 0 && K % 8 == 0 && a_stride % 8 == 0 && a_row_div > 0, "moe_gemv: K and the row stride must be multiples of 8");
   KVB_REQUIRE(aligned16(a) && aligned16(w), "moe_gemv: operands must be 16-byte aligned");
   KVB_REQUIRE(pairs <= 65535, "moe_gemv: too many pairs for one launch");
-  const size_t smem = (size_t)K * sizeof(bf16);
+  // as many rows as leave room for several blocks an SM
+  const size_t row_bytes = (size_t)K * sizeof(bf16), fit = 48 * 1024 / row_bytes;
+  const int hold = fit < 1 ? 1 : fit > MOE_GEMV_PAIRS ? MOE_GEMV_PAIRS : (int)fit;
+  const size_t smem = hold * row_bytes;
   KVB_REQUIRE(smem <= 200 * 1024, "moe_gemv: an input row does not fit in shared memory");
   int* status = kvb_status_word();
   KVB_REQUIRE(status != nullptr, "moe_gemv: no status word");
@@ -481,7 +622,7 @@ extern "C" int kvb_moe_gemv(void* out, const void* a, long long a_stride, int a_
     if (smem > 48 * 1024)                                                                                      \
       KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_gemv_kernel<G_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
     KVB_CHECK_CUDA(kvb_launch((moe_gemv_kernel<G_>), grid, dim3(256), smem, stream, true, (bf16*)out, (const bf16*)a, \
-                              a_stride, a_row_div, pair_weight, (const bf16*)w, ids, E, known, N, K, status, join));  \
+                              a_stride, a_row_div, pair_weight, (const bf16*)w, ids, pairs, hold, E, known, N, K, status, join)); \
   } while (0)
   if (gated == 1) KVB_MOE_GEMV(true); else KVB_MOE_GEMV(false);
 #undef KVB_MOE_GEMV

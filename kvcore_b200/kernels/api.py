@@ -51,7 +51,7 @@ def ensure_built(verbose: bool = False) -> str:
         "kvb_qk_prepare": [_vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _int, _vp, _vp, _int, _int, _int, _int, _int,
                            _int, _int, _float, _int, _int, _int, _int, _vp],
         "kvb_glu_clamped": [_vp, _vp, _int, _int, _float, _float, _float, _int, _vp],
-        "kvb_moe_route": [_vp, _vp, _vp, _vp, _ll, _vp, _vp, _int, _int, _int, _int, _int, _int, _int, _vp, _int, _int,
+        "kvb_moe_route": [_vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _int, _int, _int, _int, _int, _int, _int, _vp, _int, _int,
                           _float, _vp, _int, _vp],
         "kvb_moe_align": [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _vp],
         "kvb_moe_gemv": [_vp, _vp, _ll, _int, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _float, _float, _float, _vp],
@@ -2101,11 +2101,12 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, top: int, *, score: str = "
     if (group_count <= 0 or experts % group_count or not 0 < group_keep <= group_count
             or group_keep * (experts // group_count) < top):
         raise KernelError(f"moe_route: {group_keep} of {group_count} groups of {experts} experts must hold {top} experts")
+    logits = torch.empty((tokens, experts + extra), dtype=torch.float32, device=x.device)
     _call("kvb_moe_route", ids.data_ptr(), weights.data_ptr(), None if gates is None else gates.data_ptr(),
-          x.data_ptr(), x.stride(0), router.data_ptr(), None if gate_rows is None else gate_rows.data_ptr(),
+          logits.data_ptr(), x.data_ptr(), x.stride(0), router.data_ptr(), None if gate_rows is None else gate_rows.data_ptr(),
           tokens, experts, extra, k, int(top), MOE_SCORE_MODES[score], int(bool(renormalize)),
           None if correction is None else correction.data_ptr(), int(group_count), int(group_keep), float(weight_scale),
-          None if bias is None else bias.data_ptr(), _dtype_code(x), _stream())
+          None if bias is None else bias.data_ptr(), _dtype_code(x), _stream(), kernels=2)
     return ids, weights, gates
 
 
