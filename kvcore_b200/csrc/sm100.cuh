@@ -153,6 +153,22 @@ __device__ __forceinline__ void kvb_tc5_mma8_ss(unsigned tmem_d, unsigned long l
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate),
         "n"(A_STEP), "n"(A_JUMP), "n"(B_STEP), "n"(B_JUMP) : "memory");
 }
+// Four more products of the same accumulator, both operands from shared memory.
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void kvb_tc5_mma4_ss(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
+                                                unsigned idesc) {
+  asm volatile(
+      "{\n.reg .pred q;\n.reg .b64 a, b;\n"
+      "setp.eq.b32 q, 0, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q;\n"
+      "add.u64 a, %1, %4;\nadd.u64 b, %2, %5;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n"
+      "add.u64 a, a, %4;\nadd.u64 b, b, %5;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n"
+      "add.u64 a, a, %4;\nadd.u64 b, b, %5;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "n"(A_STEP), "n"(B_STEP) : "memory");
+}
 // The same with A in tensor memory: its address advances by A_COLS columns a step, B's descriptor by B_STEP.
 template <int A_COLS, int B_STEP>
 __device__ __forceinline__ void kvb_tc5_mma8_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc,

@@ -80,6 +80,8 @@ def ensure_built(verbose: bool = False) -> str:
         "kvb_flash_dims_attention": [_vp, _ll, _ll, _int, _vp, _ll, _ll, _vp, _ll, _ll, _ll, _vp, _ll, _ll, _ll, _vp,
                                      _int, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _int, _int, _int,
                                      _float, _float, _int, _int, _vp, _vp],
+        "kvb_flash_rows_tc5": [_vp, _ll, _ll, _int, _vp, _ll, _ll, _vp, _vp, _ll, _int, _int, _vp, _int, _vp, _vp, _vp, _vp,
+                               _int, _int, _int, _int, _int, _int, _int, _int, _int, _int, _float, _int, _int, _vp],
         "kvb_latent_prepare": [_vp, _ll, _vp, _float, _vp, _int, _vp, _vp, _vp, _int, _vp, _int, _int, _int, _vp,
                                _ll, _ll, _int, _vp, _ll, _ll, _vp, _int, _int, _int, _int, _int, _int, _vp],
         "kvb_gather_cached_rows": [_vp, _ll, _ll, _int, _vp, _int, _int, _int, _vp, _vp, _int, _vp, _int, _int,
@@ -746,7 +748,7 @@ TRACE_TAGS = {27: "rms_norm_shift", 28: "stream_add_norm", 29: "attention_dims_r
               7: "flash_paged", 8: "flash_combine", 9: "flash_decode_tma", 10: "flash_decode_combine",
               11: "flash_prefill_tc5", 12: "gemm_f32", 13: "gemm_stream", 14: "sample", 16: "feed_tokens"}
 _TRACE_UNITS = ("elementwise", "attention_decode_tma", "attention_flash", "attention_generic",
-                "attention_prefill_tc5", "gemm_f32", "sampling", "gemm_stream", "layer_norm", "qk_prepare", "moe", "attention_kept_first",
+                "attention_prefill_tc5", "attention_rows_tc5", "gemm_f32", "sampling", "gemm_stream", "layer_norm", "qk_prepare", "moe", "attention_kept_first",
                 "stream_norm", "attention_dims", "mixer_prepare", "attention_flash_dims", "recurrence", "turn_norm",
                 "state_space", "stream_rows", "fixed_decay", "attention_prepare")
 _trace_buffer: torch.Tensor | None = None
@@ -1221,7 +1223,8 @@ def attention_dims(q: torch.Tensor, keys: torch.Tensor, values: torch.Tensor, ta
                    sink: torch.Tensor | None = None, window: int | None = None,
                    out: torch.Tensor | None = None, out_dtype: torch.dtype | None = None,
                    force_general: bool = False, num_splits: int | None = None,
-                   slopes: torch.Tensor | None = None, softcap: float | None = None) -> torch.Tensor:
+                   slopes: torch.Tensor | None = None, softcap: float | None = None,
+                   rows_in_order: bool = False) -> torch.Tensor:
     """Paged attention with a key width and a value width of their own.
 
     ``q [T, HQ, key_width]`` (a view; last stride 1) with ``HQ = value_heads * group * maps``: query head
@@ -1233,8 +1236,9 @@ def attention_dims(q: torch.Tensor, keys: torch.Tensor, values: torch.Tensor, ta
     score of the key at position ``j`` for the query at position ``i`` is lowered by ``slopes[hq] * (i - j)``.
     ``softcap``: the scaled score first becomes ``softcap * tanh(score / softcap)``.  Returns ``[T, HQ, value_width]`` in
     ``out_dtype`` (32-bit or the cache's type; default the cache's) or fills ``out`` (a view with last
-    stride 1).  bfloat16 shapes the tensor-core kernel takes run there; everything else, and all of float32,
-    on the general kernel."""
+    stride 1).  ``rows_in_order``: the pages hold one row, and the table's entries of a request's visible positions are
+    neighbours in ascending order (a hint that lets whole tiles be copied).  bfloat16 shapes the tensor-core kernels
+    take run there; everything else, and all of float32, on the general kernel."""
     _check(q, "q", contiguous=False)
     _check(keys, "keys", dtype=q.dtype, contiguous=False)
     _check(values, "values", dtype=q.dtype, contiguous=False)
@@ -1262,7 +1266,8 @@ def attention_dims(q: torch.Tensor, keys: torch.Tensor, values: torch.Tensor, ta
     if (not force_general and flash_dims_supported(q, out, key_width, value_width, page_size, key_strides,
                                                     value_strides, keys, values, maps)):
         _flash_dims(out, q, keys, values, table, ctx, value_heads, group, maps, key_width, value_width, page_size,
-                    num_pages, key_strides, value_strides, scale, sink, window, num_splits, slopes, softcap)
+                    num_pages, key_strides, value_strides, scale, sink, window, num_splits, slopes, softcap,
+                    rows_in_order)
         return out
     _call("kvb_attention_dims_rows", out.data_ptr(), out.stride(0), out.stride(1), int(out.dtype == torch.float32),
           q.data_ptr(), q.stride(0), q.stride(1), keys.data_ptr(), *key_strides, values.data_ptr(), *value_strides,
@@ -1315,9 +1320,27 @@ def flash_dims_supported(q, out, key_width, value_width, page_size, key_strides,
     return all(_flash_dims_geometry(key_width, value_width, rows, alias) is not None for rows in (64, 32, 16))
 
 
+def _rows_tc5_takes(out, key_width, value_width, page_size, key_strides, value_strides, softcap, rows_in_order) -> bool:
+    """Whether the tcgen05 kernel for prompt portions takes this call (of those that ``flash_dims_supported``): keys of 128
+    or 192 entries, values of a multiple of 128, both in rows that lie one behind the other, no cap on the scores."""
+    pitch = key_strides[0] if rows_in_order else key_strides[2]
+    if key_width not in (128, 192) or value_width % 128 or softcap is not None or not pitch:
+        return False
+    if rows_in_order:
+        if page_size != 1 or value_strides[0] != pitch:
+            return False
+    elif (page_size not in (8, 16, 32, 64) or value_strides[2] != pitch
+          or key_strides[0] != page_size * pitch or value_strides[0] != page_size * pitch):
+        return False
+    wide = 4 if out.dtype == torch.float32 else 8
+    return (max(key_strides[1], value_strides[1]) < 1 << 31 and out.data_ptr() % 16 == 0
+            and out.stride(0) % wide == 0 and out.stride(1) % wide == 0)
+
+
 def _flash_dims(out, q, keys, values, table, ctx, value_heads, group, maps, key_width, value_width, page_size,
-                num_pages, key_strides, value_strides, scale, sink, window, num_splits, slopes=None, softcap=None) -> None:
-    """The tensor-core kernel on the step's batch.  A mixed step (portions of prompts beside single decoded
+                num_pages, key_strides, value_strides, scale, sink, window, num_splits, slopes=None, softcap=None,
+                rows_in_order=False) -> None:
+    """The tensor-core kernels on the step's batch.  A mixed step (portions of prompts beside single decoded
     tokens, longest first as the step function packs them) goes as two runs of requests, so that the
     decoded tokens take the shape made for few rows and have their keys cut into chunks."""
     lens = getattr(ctx, "host_query_lens", None)
@@ -1328,8 +1351,19 @@ def _flash_dims(out, q, keys, values, table, ctx, value_heads, group, maps, key_
         if 0 < long_count < ctx.num_reqs and all(n * group > 32 for n in lens[:long_count]):
             runs = [(_RequestRun(ctx, begin, end), table[begin:end])
                     for begin, end in ((0, long_count), (long_count, ctx.num_reqs))]
+    tc5 = num_splits is None and _rows_tc5_takes(out, key_width, value_width, page_size, key_strides, value_strides, softcap,
+                                                 rows_in_order)
     for run, run_table in runs:
         max_rows = run.max_query_len * group
+        if tc5 and max_rows > 32:            # beyond the few-row form, at any length (from 40 rows behind 2,000 keys: 79 us, 188)
+            _call("kvb_flash_rows_tc5", out.data_ptr(), out.stride(0), out.stride(1), int(out.dtype == torch.float32),
+                  q.data_ptr(), q.stride(0), q.stride(1), keys.data_ptr(), values.data_ptr(),
+                  key_strides[0] if rows_in_order else key_strides[2], key_strides[1], value_strides[1],
+                  run_table.data_ptr(), run_table.stride(0), run.query_start.data_ptr(), run.context_lens.data_ptr(),
+                  None if sink is None else sink.data_ptr(), None if slopes is None else slopes.data_ptr(),
+                  run.num_reqs, run.max_query_len, q.shape[0], value_heads, group, maps, key_width, value_width, page_size,
+                  num_pages, float(scale), int(window or 0), int(rows_in_order), _stream())
+            continue
         split_mode = max_rows <= 32                 # the few-row form: 16 or 32 rows a key head
         tile_m = 16 if max_rows <= 16 else 32 if split_mode else 64
         alias = keys.data_ptr() == values.data_ptr() and tuple(key_strides) == tuple(value_strides) and maps == 1

@@ -260,7 +260,7 @@ class LatentAttention(Mixer):
         K.attention_dims(queries, carried, carried.view(-1)[d + r:], row_table, K.api._RequestRun(ctx, 0, count),
                          value_heads=heads, group=1, maps=1, key_width=d + r, value_width=v, page_size=1,
                          num_pages=rows_needed + 1, key_strides=strides, value_strides=strides, scale=self.scale,
-                         sink=self.sink_f32, window=self.window, out=out[:tokens])
+                         sink=self.sink_f32, window=self.window, out=out[:tokens], rows_in_order=True)
 
     def _turned_queries(self, rows, q, kv_rows, ctx, table, plane, cache, first: int, latent_q: torch.Tensor):
         """Every token's latent row into the cache; the queries of the first ``first`` tokens (long portions) as heads

@@ -108,3 +108,94 @@ def test_few_pairs_share_an_experts_pass(width, ff):
         want = P.moe_experts(x, ids.clamp(max=experts - 1), weights, gate_up, down, weight_on_input=True).view(-1, top, width)
         torch.testing.assert_close(rows[real], want[real], rtol=3e-2, atol=0.02 * float(want[real].float().abs().max()))
     assert K().read_status() == 0
+
+
+def _attend(q, keys, values, lens, how):
+    """Plain attention in 64 bits: q [T, HQ, DK], keys [N, KH, DK] and values [N, VH, DV] of each request."""
+    out, at, group = [], 0, how["group"] * how["maps"]
+    for (cached, n), k, v in zip(lens, keys, values):
+        i, j = torch.arange(cached, cached + n, device=DEV)[:, None], torch.arange(cached + n, device=DEV)[None]
+        rows = []
+        for h in range(q.shape[1]):
+            s = q[at:at + n, h].double() @ k[:, h // group * how["maps"] + h % how["maps"]].double().T * how["scale"]
+            if how["slopes"] is not None:
+                s = s - how["slopes"][h].double() * (i - j)
+            hidden = j > i if how["window"] is None else (j > i) | (j <= i - how["window"])
+            s = s.masked_fill(hidden, float("-inf"))
+            if how["sink"] is not None:
+                s = torch.cat([s, how["sink"][h].double().expand(n, 1)], 1)
+            rows.append(torch.softmax(s, 1)[:, :cached + n] @ v[:, h // group].double())
+        out.append(torch.stack(rows, 1))
+        at += n
+    return torch.cat(out)
+
+
+def _compare(got, other, want, values):
+    """Not further from the values in 64 bits than the kernel of the other shapes (5 % for the sums' order), and nowhere
+    more than the rounding of probabilities and of the result to bfloat16 (2^-9 each) allows, twice."""
+    error = [float((t.double() - want).norm() / want.norm()) for t in (got, other)]
+    assert error[0] <= 1.05 * error[1] and K().read_status() == 0, error
+    assert (got.double() - want).abs().max() <= 2.0 ** -7 * max(float(v.float().abs().max()) for v in values)
+
+
+ROWS_LENS = [[(0, 128)], [(0, 257), (130, 129), (0, 40)], [(300, 33)], [(127, 300), (1, 64)]]
+
+
+@pytest.mark.parametrize("lens", ROWS_LENS)
+@pytest.mark.parametrize("kv_heads,group,maps,vdim,page,window,extra,f32", [
+    (2, 4, 1, 128, 16, None, False, True), (2, 3, 1, 128, 8, 100, True, False), (1, 16, 2, 256, 64, None, False, True),
+    (3, 1, 1, 384, 32, 33, True, True)])
+def test_prompt_attention_over_rows_of_a_plane(lens, kv_heads, group, maps, vdim, page, window, extra, f32):
+    """Keys of 128 and values of multiples of 128 in the rows of a page: tiles that are not full, groups that do and do
+    not divide a tile, several score maps, windows, sinks and slopes."""
+    hq, totals = kv_heads * group * maps, [c + n for c, n in lens]
+    tokens, k_cols = sum(n for _, n in lens), kv_heads * maps * 128
+    width = k_cols + kv_heads * vdim
+    pages = [-(-t // page) for t in totals]
+    order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(1)) + 1
+    table, at = torch.zeros(len(lens), max(pages), dtype=torch.int32), 0
+    for row, count in enumerate(pages):
+        table[row, :count] = order[at:at + count]
+        at += count
+    table = table.to(DEV)
+    plane = randn(sum(pages) + 1, 1, page, width, dtype=torch.bfloat16, seed=2)
+    seen = [plane[table[r, :count].long()].reshape(-1, width)[:t] for r, (count, t) in enumerate(zip(pages, totals))]
+    keys = [s[:, :k_cols].unflatten(1, (kv_heads * maps, 128)) for s in seen]
+    values = [s[:, k_cols:].unflatten(1, (kv_heads, vdim)) for s in seen]
+    q = randn(tokens, hq, 128, dtype=torch.bfloat16, seed=3)
+    how = dict(group=group, maps=maps, scale=128 ** -0.5, window=window,
+               sink=randn(hq, dtype=torch.float32, seed=4) if extra else None,
+               slopes=randn(hq, dtype=torch.float32, seed=5).abs() * 0.05 if extra else None)
+    call = dict(how, value_heads=kv_heads, key_width=128, value_width=vdim, page_size=page, num_pages=plane.shape[0],
+                key_strides=(page * width, 128, width), value_strides=(page * width, vdim, width),
+                out_dtype=torch.float32 if f32 else torch.bfloat16)
+    got = K().attention_dims(q, plane, plane.view(-1)[k_cols:], table, _Batch(lens), **call)
+    other = K().attention_dims(q, plane, plane.view(-1)[k_cols:], table, _Batch(lens), num_splits=1, **call)
+    _compare(got, other, _attend(q, keys, values, lens, how), values)
+
+
+@pytest.mark.parametrize("lens", ROWS_LENS + [[(1500, 200), (900, 40)]])
+@pytest.mark.parametrize("heads,turned,window", [(3, 64, None), (2, 0, None), (2, 0, 150), (2, 64, 40)])
+def test_prompt_attention_over_rows_in_order(lens, heads, turned, window):
+    """Keys of 128 or 192 entries and values of 128 carried up for the positions that are seen, one row a position: tiles
+    that begin in front of a request's first row and end behind the last one."""
+    dk, per, totals = 128 + turned, 256 + turned, [c + n for c, n in lens]
+    starts = [0 if window is None else max(0, c - window + 1) for c, _ in lens]
+    count, tokens = sum(t - s for t, s in zip(totals, starts)), sum(n for _, n in lens)
+    carried = randn(count + 1, heads * per, dtype=torch.bfloat16, seed=1)
+    table, at, keys, values = torch.zeros(len(lens), max(totals), dtype=torch.int32, device=DEV), 1, [], []
+    for row, (start, total) in enumerate(zip(starts, totals)):
+        table[row, start:total] = torch.arange(at, at + total - start, dtype=torch.int32, device=DEV)
+        rows = torch.zeros(total, heads, per, dtype=torch.bfloat16, device=DEV)
+        rows[start:] = carried[at:at + total - start].unflatten(1, (heads, per))
+        at += total - start
+        keys.append(rows[..., :dk])
+        values.append(rows[..., dk:])
+    q = randn(tokens, heads, dk, dtype=torch.bfloat16, seed=2)
+    how = dict(group=1, maps=1, scale=dk ** -0.5, window=window, sink=randn(heads, dtype=torch.float32, seed=3), slopes=None)
+    call = dict(how, value_heads=heads, key_width=dk, value_width=128, page_size=1, num_pages=count + 1,
+                key_strides=(heads * per, per, 0), value_strides=(heads * per, per, 0))
+    flat = carried.view(-1)
+    got = K().attention_dims(q, carried, flat[dk:], table, _Batch(lens), rows_in_order=True, **call)
+    other = K().attention_dims(q, carried, flat[dk:], table, _Batch(lens), **call)
+    _compare(got, other, _attend(q, keys, values, lens, how), values)
