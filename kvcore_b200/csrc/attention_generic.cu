@@ -39,9 +39,9 @@ template <typename T>
 struct AttParams {
   T* out; const T* q; const T* k_cache; const T* v_cache;
   const int* table; const int* positions; const int* query_start;
-  int out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages, window, keep_first, vec, segments;
+  int out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages, window, keep_first, vec, segments, reqs, part_rows;
   float scale;
-  float* partial;            // [reqs, KVH, segments, ATT_FEW, D + 2]: accumulators, maximum, sum
+  float* partial;            // [reqs, KVH, segments, part_rows, D + 2]: accumulators, maximum, sum
   int* status;
 };
 
@@ -168,9 +168,10 @@ template <typename T, int NJ>              // NJ: output columns in runs of 64
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_tile_kernel(AttParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
-  const int req = blockIdx.x / p.KVH, kvh = blockIdx.x % p.KVH, G = p.H / p.KVH;
+  // blocks: (request, kv head) fastest, then the tiles, those with the most keys first
+  const int heads = p.reqs * p.KVH, head = blockIdx.x % heads, req = head / p.KVH, kvh = head % p.KVH, G = p.H / p.KVH;
   const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
-  const int row0 = (gridDim.y - 1 - blockIdx.y) * ATT_ROWS;          // the tiles with the most keys first
+  const int row0 = (gridDim.x / heads - 1 - blockIdx.x / heads) * ATT_ROWS;
   if (all_rows <= ATT_FEW || row0 >= all_rows) return;
   extern __shared__ __align__(16) float smem[];
   const int DK = (p.D + 3) & ~3, LK = DK + 4;
@@ -312,7 +313,9 @@ template <typename T, int NJ>              // NJ: output columns in runs of 64
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_few_kernel(AttParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
-  const int req = blockIdx.x / p.KVH, kvh = blockIdx.x % p.KVH, G = p.H / p.KVH;
+  // blocks: the segments of a (request, kv head) next to one another
+  const int head = blockIdx.x / p.segments, part_no = blockIdx.x % p.segments;
+  const int req = head / p.KVH, kvh = head % p.KVH, G = p.H / p.KVH;
   const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
   if (all_rows > ATT_FEW || all_rows == 0) return;
   extern __shared__ __align__(16) float smem[];
@@ -330,7 +333,7 @@ attention_few_kernel(AttParams<T> p) {
   b.fetch_queries(qs, LK, DK);
   const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;           // a warp a row
   const bool live = r < all_rows;
-  const int segment = blockIdx.y * ATT_SEGMENT;
+  const int segment = part_no * ATT_SEGMENT;
   float acc[RUNS][4], m = -INFINITY, l = 0.0f;
 #pragma unroll
   for (int j = 0; j < RUNS; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
@@ -380,7 +383,7 @@ attention_few_kernel(AttParams<T> p) {
   }
   if (!live) return;
   if (p.segments > 1) {
-    float* part = p.partial + (((size_t)blockIdx.x * p.segments + blockIdx.y) * ATT_FEW + r) * (p.D + 2);
+    float* part = p.partial + ((size_t)blockIdx.x * p.part_rows + r) * (p.D + 2);
 #pragma unroll
     for (int j = 0; j < RUNS; ++j)
 #pragma unroll
@@ -418,7 +421,7 @@ attention_fold_kernel(AttParams<T> p) {
   Folded total{-INFINITY, 0.0f, 0.0f, 0.0f};
   const int last = min(p.segments - 1, p.positions[begin + r / G] / ATT_SEGMENT);
   for (int s = 0; s <= last; ++s) {
-    const float* part = p.partial + (((size_t)blockIdx.x * p.segments + s) * ATT_FEW + r) * (p.D + 2);
+    const float* part = p.partial + (((size_t)blockIdx.x * p.segments + s) * p.part_rows + r) * (p.D + 2);
     const float m = part[p.D];
     if (m == -INFINITY) continue;
     total.fold(m, part[p.D + 1]);
@@ -441,13 +444,13 @@ static int launch_attention(AttParams<T> p, int tokens, int reqs, int max_query_
   if (most > ATT_FEW) {
     const int smem = (int)sizeof(float) * (ATT_ROWS * LK + ATT_CHUNK * (LK + DV + ATT_LS));
     KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_tile_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    KVB_CHECK_CUDA(kvb_launch((attention_tile_kernel<T, NJ>), dim3(reqs * p.KVH, (most + ATT_ROWS - 1) / ATT_ROWS),
+    KVB_CHECK_CUDA(kvb_launch((attention_tile_kernel<T, NJ>), dim3((unsigned)((long long)reqs * p.KVH * ((most + ATT_ROWS - 1) / ATT_ROWS))),
                               dim3(ATT_THREADS), smem, stream, true, p));
   }
   if (G <= ATT_FEW && (most <= ATT_FEW || !equal)) {
     const int smem = (int)sizeof(float) * (ATT_FEW * LK + ATT_CHUNK * (LK + DV));
     KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_few_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3(reqs * p.KVH, p.segments), dim3(ATT_THREADS), smem, stream,
+    KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3((unsigned)((long long)reqs * p.KVH * p.segments)), dim3(ATT_THREADS), smem, stream,
                               true, p));
     if (p.segments > 1)
       KVB_CHECK_CUDA(kvb_launch((attention_fold_kernel<T>), dim3(reqs * p.KVH), dim3(ATT_THREADS), 0, stream, true, p));
@@ -463,9 +466,14 @@ static int attention_of(const AttParams<T>& p, int tokens, int reqs, int max_que
   return launch_attention<T, 4>(p, tokens, reqs, max_query_len, stream);
 }
 
-// Floats of the scratch that a batch takes whose longest request has `segments` segments of cached tokens.
-extern "C" long long kvb_paged_attention_scratch(int num_reqs, int KVH, int D, int segments) {
-  return segments > 1 ? (long long)num_reqs * KVH * segments * ATT_FEW * (D + 2) : 0;
+// Floats of the scratch that a batch takes whose longest request has `segments` segments of cached tokens: a row of it
+// for each row that a segment's block can have (one for decoded tokens of ungrouped heads).
+static int part_rows_of(int H, int KVH, int max_query_len) {
+  const long long most = (long long)max_query_len * (H / KVH);
+  return most < ATT_FEW ? (int)most : ATT_FEW;
+}
+extern "C" long long kvb_paged_attention_scratch(int num_reqs, int H, int KVH, int D, int max_query_len, int segments) {
+  return segments > 1 ? (long long)num_reqs * KVH * segments * part_rows_of(H, KVH, max_query_len) * (D + 2) : 0;
 }
 extern "C" int kvb_paged_attention_segment() { return ATT_SEGMENT; }
 
@@ -481,9 +489,10 @@ extern "C" int kvb_paged_attention_rows(void* out, int out_stride, const void* q
   KVB_REQUIRE(H > 0 && KVH > 0 && H % KVH == 0, "paged_attention: H must be a multiple of KVH");
   KVB_REQUIRE(page_size > 0 && num_pages > 1, "paged_attention: empty cache");
   KVB_REQUIRE(keep_first >= 0 && (keep_first == 0 || window > 0), "paged_attention: kept first positions need a window");
-  KVB_REQUIRE((long long)num_reqs * KVH < (1ll << 31), "paged_attention: too many requests");
-  KVB_REQUIRE(max_query_len > 0 && (long long)max_query_len * (H / KVH) <= 65535LL * ATT_ROWS, "paged_attention: too many rows");
-  KVB_REQUIRE(segments >= 1 && segments <= 65535 && (segments == 1 || partial != nullptr), "paged_attention: no scratch");
+  KVB_REQUIRE((long long)tokens * H < (1ll << 31) && max_query_len > 0 && max_query_len <= tokens, "paged_attention: too many rows");
+  KVB_REQUIRE((long long)num_reqs * KVH * (((long long)max_query_len * (H / KVH) + ATT_ROWS - 1) / ATT_ROWS) < (1ll << 31) &&
+              (long long)num_reqs * KVH * segments < (1ll << 31), "paged_attention: too many blocks for one launch");
+  KVB_REQUIRE(segments >= 1 && (segments == 1 || partial != nullptr), "paged_attention: no scratch");
   int* status = kvb_status_word();
   KVB_REQUIRE(status != nullptr, "paged_attention: no status word");
   const int esize = dtype == KVB_F32 ? 4 : 2;
@@ -491,7 +500,8 @@ extern "C" int kvb_paged_attention_rows(void* out, int out_stride, const void* q
 #define KVB_ATT(T_)                                                                                                    \
   attention_of<T_>(AttParams<T_>{(T_*)out, (const T_*)q, (const T_*)k_cache, (const T_*)v_cache, table, positions,     \
                                  query_start, out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages,     \
-                                 window, keep_first, vec, segments, scale, partial, status},                           \
+                                 window, keep_first, vec, segments, num_reqs, part_rows_of(H, KVH, max_query_len),     \
+                                 scale, partial, status},                                                              \
                    tokens, num_reqs, max_query_len, stream)
   return dtype == KVB_F32 ? KVB_ATT(float) : KVB_ATT(bf16);
 #undef KVB_ATT

@@ -140,7 +140,7 @@ def ensure_built(verbose: bool = False) -> str:
     lib.kvb_gemm_stream_norm_max_k.restype = _int
     lib.kvb_gemm_stream_scratch_marker.argtypes = []
     lib.kvb_gemm_stream_scratch_marker.restype = ctypes.c_uint
-    lib.kvb_paged_attention_scratch.argtypes = [_int, _int, _int, _int]
+    lib.kvb_paged_attention_scratch.argtypes = [_int] * 6
     lib.kvb_paged_attention_scratch.restype = _ll
     lib.kvb_paged_attention_segment.argtypes = []
     lib.kvb_paged_attention_segment.restype = _int
@@ -646,7 +646,8 @@ def paged_attention(
         segments = -(-max(1, bound) // _lib.kvb_paged_attention_segment())
     partial = None
     if segments > 1:
-        partial = torch.empty(_lib.kvb_paged_attention_scratch(ctx.num_reqs, num_kv_heads, head_dim, segments),
+        partial = torch.empty(_lib.kvb_paged_attention_scratch(ctx.num_reqs, num_heads, num_kv_heads, head_dim,
+                                                               ctx.max_query_len, segments),
                               dtype=torch.float32, device=qkv.device)
     _call("kvb_paged_attention_rows", out.data_ptr(), out.stride(0), qkv.data_ptr(), qkv.stride(0),
           k_cache.data_ptr(), v_cache.data_ptr(), table.data_ptr(), table.stride(0),
