@@ -1,7 +1,8 @@
 // Paged flash attention for prompt portions on the 5th-generation tensor cores (sm_100a):
 // tcgen05.mma with accumulators in tensor memory, operands staged by TMA.  bf16, head size 128.
 //
-// A block owns TWO tiles of 128 query rows of one (request, kv head), A and B, one behind the other;
+// A block owns TWO tiles of 128 query rows of one (request, kv head), A and B, one behind the other (A alone in launches
+// of few blocks: kvb_tc5_query_tiles);
 // a row is a (token, query head of the group) pair, so the G heads that share a kv head reuse every
 // K/V tile, and every K/V tile that TMA brings is used by both query tiles.  The block walks the
 // keys in tiles of 128.  Eleven warps:
@@ -65,6 +66,7 @@ struct Tc5Params {
   int* status;
   float* lse;                // optional [tokens, H]: log2 of the sum of 2^(scaled score) over the keys seen (-inf: none)
   int q_by_tma;                // the query tiles are brought by TMA (q_map is valid)
+  int tiles;                   // query tiles of a block: two, or A alone (kvb_tc5_query_tiles)
 };
 
 // Byte offset of the 16-byte chunk `chunk16` (0..15 across the 128 columns) of row `r` in a
@@ -149,7 +151,7 @@ flash_prefill_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid
   const int q_len = p.query_start[req + 1] - q_begin;
   const int context = p.context_lens[req];
   const int rows_total = q_len * p.G;
-  const int row0 = pair * 2 * T5_BM;
+  const int row0 = pair * p.tiles * T5_BM;
   if (row0 >= rows_total) return;  // whole block, before any barrier or allocation
   if (kvb_smem(base) & 1023u) {     // cannot happen with the alignment asked for; never run misaligned
     if (threadIdx.x == 0) atomicOr(p.status, KVB_STATUS_WAIT_TIMEOUT);
@@ -158,7 +160,7 @@ flash_prefill_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid
 
   // keys of the two tiles: tile X sees [lo_X, hi_X); both walk the key tiles from tile_begin (the
   // first tile of A, whose rows come first), tile X through n_X of them
-  const bool has_b = row0 + T5_BM < rows_total;
+  const bool has_b = p.tiles == 2 && row0 + T5_BM < rows_total;
   const int last_row_a = min(row0 + T5_BM, rows_total) - 1;
   const int last_row_b = min(row0 + 2 * T5_BM, rows_total) - 1;
   const int first_pos_a = context + row0 / p.G;
@@ -186,7 +188,7 @@ flash_prefill_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid
   if (warp < 8 && !p.q_by_tma) {
     const int r = threadIdx.x & 127, x = threadIdx.x >> 7;
     const int flat = row0 + x * T5_BM + r;
-    const bool valid = flat < rows_total;
+    const bool valid = flat < rows_total && x < p.tiles;
     const bf16* src = p.q + (size_t)(q_begin + (valid ? flat / p.G : 0)) * p.q_stride +
                       (size_t)(kvh * p.G + (valid ? flat % p.G : 0)) * T5_D;
     unsigned char* dst = q_smem + x * T5_TILE_BYTES;
@@ -624,7 +626,8 @@ extern "C" int kvb_flash_prefill_tc5(void* out, long long out_stride, const void
     configured = true;
   }
   const int max_rows = max_query_len * p.G;
-  const int pairs = (max_rows + 2 * T5_BM - 1) / (2 * T5_BM);            // a block takes two query tiles
+  p.tiles = kvb_tc5_query_tiles((long long)KVH * num_reqs * ((max_rows + 2 * T5_BM - 1) / (2 * T5_BM)));
+  const int pairs = (max_rows + p.tiles * T5_BM - 1) / (p.tiles * T5_BM);
   KVB_REQUIRE(pairs <= 65535, "prefill attention (tcgen05): portion too long for one launch");
   dim3 grid(KVH, num_reqs, pairs);
   if (cap > 0.0f)

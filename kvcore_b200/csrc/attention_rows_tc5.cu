@@ -3,7 +3,8 @@
 // attention_flash_dims.cu (several score maps a value head, 32-bit results, a sink per query head, a slope per query head
 // times the distance taken off the score).  bf16 operands, 32-bit scores, softmax and accumulation.
 //
-// A block owns two tiles of 128 query rows of one (request, key head, slice of 128 value columns), A and B; a row is a
+// A block owns two tiles of 128 query rows of one (request, key head, slice of 128 value columns), A and B (A alone in
+// launches of few blocks: kvb_tc5_query_tiles); a row is a
 // (token, query head of the key head's group) pair.  It walks the keys in tiles of 128; eleven warps as there: two softmax
 // warpgroups (a thread a row), a producer warp for keys and one for values, one thread that issues the products
 //     S_A(0), S_B(0); per key tile j:  O_A += P_A(j).V(j), S_A(j+1), O_B += P_B(j).V(j), S_B(j+1).
@@ -46,6 +47,7 @@ struct RowsTc5Params {
   const float* sink; const float* slopes;
   int* status;
   int q_by_tma;
+  int tiles;                              // query tiles of a block (kvb_tc5_query_tiles)
 };
 
 // Byte offset of the 16-byte piece `piece` of row `r` in an operand tile stored as swizzled parts of 64 columns.
@@ -112,13 +114,13 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
   const int q_len = p.query_start[req + 1] - q_begin;
   const int context = p.context_lens[req];
   const int rows_total = q_len * p.G;
-  const int row0 = pair * 2 * RT_BM;
+  const int row0 = pair * p.tiles * RT_BM;
   if (row0 >= rows_total) return;           // whole block, before any barrier or allocation
   if (kvb_smem(rt_dyn) & 1023u) {            // cannot happen with the alignment asked for; never run misaligned
     if (threadIdx.x == 0) atomicOr(p.status, KVB_STATUS_WAIT_TIMEOUT);
     return;
   }
-  const bool has_b = row0 + RT_BM < rows_total;
+  const bool has_b = p.tiles == 2 && row0 + RT_BM < rows_total;
   const int last_row_a = min(row0 + RT_BM, rows_total) - 1;
   const int last_row_b = min(row0 + 2 * RT_BM, rows_total) - 1;
   const int first_pos_a = context + row0 / p.G;
@@ -144,7 +146,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
   if (warp < 8 && !p.q_by_tma) {             // thread t of warpgroup X: row t of tile X
     const int r = threadIdx.x & 127, x = threadIdx.x >> 7;
     const int flat = row0 + x * RT_BM + r;
-    const bool valid = flat < rows_total;
+    const bool valid = flat < rows_total && x < p.tiles;
     const bf16* src = p.q + (size_t)(q_begin + (valid ? flat / p.G : 0)) * p.q_token + (size_t)query_head(valid ? flat : 0) * p.q_head;
     unsigned char* dst = q_smem + x * K_BYTES;
 #pragma unroll
@@ -515,7 +517,9 @@ extern "C" int kvb_flash_rows_tc5(void* out, long long out_token, long long out_
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS, "rows attention (tcgen05): no tensor map for the queries");
     p.q_by_tma = 1;
   }
-  const long long pairs = ((long long)max_query_len * group + 2 * RT_BM - 1) / (2 * RT_BM);
+  const long long all_rows = (long long)max_query_len * group, heads = (long long)value_heads * maps * p.slices;
+  p.tiles = kvb_tc5_query_tiles(heads * num_reqs * ((all_rows + 2 * RT_BM - 1) / (2 * RT_BM)));
+  const long long pairs = (all_rows + p.tiles * RT_BM - 1) / (p.tiles * RT_BM);
   KVB_REQUIRE(pairs <= 65535, "rows attention (tcgen05): portion too long for one launch");
   const dim3 grid(value_heads * maps * p.slices, num_reqs, (unsigned)pairs);
   cudaError_t err;

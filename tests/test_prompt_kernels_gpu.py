@@ -199,3 +199,21 @@ def test_prompt_attention_over_rows_in_order(lens, heads, turned, window):
     got = K().attention_dims(q, carried, flat[dk:], table, _Batch(lens), rows_in_order=True, **call)
     other = K().attention_dims(q, carried, flat[dk:], table, _Batch(lens), **call)
     _compare(got, other, _attend(q, keys, values, lens, how), values)
+
+
+@pytest.mark.parametrize("group,window,cached,new", [(4, None, 0, 700), (3, None, 130, 129), (1, 90, 257, 300), (8, None, 1000, 33)])
+def test_blocks_of_one_query_tile_give_the_bits_of_two(group, window, cached, new):
+    """A request alone takes blocks of one query tile; beside twenty of its like they take two.  (A window's first key
+    tile depends on the block's rows; the tiles in front of a row's window add nothing.)"""
+    kv_heads, page = 2, 16
+    heads, pages, copies = kv_heads * group, -(-(cached + new) // 16), 21
+    k_cache = randn(pages + 1, kv_heads, page, 128, dtype=torch.bfloat16, seed=1)
+    v_cache = randn(pages + 1, kv_heads, page, 128, dtype=torch.bfloat16, seed=2)
+    row = (torch.randperm(pages, generator=torch.Generator().manual_seed(3)) + 1).to(DEV, torch.int32)[None]
+    qkv = randn(new, (heads + 2 * kv_heads) * 128, dtype=torch.bfloat16, seed=4)
+
+    def attend(count):
+        return K().paged_attention(qkv.repeat(count, 1), k_cache, v_cache, row.repeat(count, 1).contiguous(),
+                                   _Batch([(cached, new)] * count), heads, kv_heads, 128, 128 ** -0.5, window)
+    one, many = attend(1), attend(copies)
+    assert all(torch.equal(part, one) for part in many.split(new)) and K().read_status() == 0
