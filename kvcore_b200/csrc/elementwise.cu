@@ -91,8 +91,12 @@ extern "C" int kvb_feed_tokens(int* token_ids, const int* source, const int* sam
 //   ADD: s = h + residual (rounded to T, stored back as the new residual), else s = h
 //   out = T( w * (s * rsqrt(mean(s^2) + eps)) ), everything between in 32-bit.
 // ------------------------------------------------------------------------------------------
-template <typename T, typename W, bool ADD, bool VEC>
-__global__ void __launch_bounds__(256)
+// SLOTS: 16-byte pieces of a row that a thread keeps in registers (rows of up to 256 SLOTS pieces); 0: none, each thread
+// re-reads what it wrote.  Bound by the bytes: the row, the residual and the weight are all asked for before anything
+// waits.  2,048 rows of 4,096 (B200, cold caches, call by call): 14.3 us, with the sum 18.5; 18.4 and 20.5 with the pieces
+// asked for one after the other and the weight behind the sum.
+template <typename T, typename W, bool ADD, bool VEC, int SLOTS>
+__global__ void __launch_bounds__(256, SLOTS == 4 ? 4 : 1)
 rmsnorm_kernel(T* __restrict__ out, T* __restrict__ residual, const T* __restrict__ h,
                const W* __restrict__ weight, int width, float eps) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_RMSNORM);
@@ -102,13 +106,49 @@ rmsnorm_kernel(T* __restrict__ out, T* __restrict__ residual, const T* __restric
   T* rr = ADD ? residual + base : nullptr;
   T* orow = out + base;
   float sq = 0.0f;
-  if (VEC) {
+  if (VEC && SLOTS > 0) {
+    constexpr int N = Vec16<T>::N, KEEP = SLOTS > 0 ? SLOTS : 1;
+    constexpr bool SAME = sizeof(W) == sizeof(T), EARLY = SAME && SLOTS <= 2;   // (four pieces of each are too many registers)
+    Vec16<T> mine[KEEP], other[KEEP];
+    Vec16<W> g[KEEP];
+#pragma unroll
+    for (int s = 0; s < KEEP; ++s) {
+      const int i = (threadIdx.x + s * 256) * N;
+      if (i < width) {
+        mine[s].load(hr + i);
+        if (ADD) other[s].load(rr + i);
+        if (EARLY) g[s].load(weight + i);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < KEEP; ++s) {
+      const int i = (threadIdx.x + s * 256) * N;
+      if (i < width) {
+        if (ADD) {
+#pragma unroll
+          for (int j = 0; j < N; ++j) mine[s].set(j, mine[s].get(j) + other[s].get(j));
+          mine[s].store(rr + i);
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) { const float x = mine[s].get(j); sq += x * x; }
+      }
+    }
+    const float total = block_sum(sq, scratch);
+    const float inv = 1.0f / sqrtf(total / (float)width + eps);
+#pragma unroll
+    for (int s = 0; s < KEEP; ++s) {
+      const int i = (threadIdx.x + s * 256) * N;
+      if (i < width) {
+        if (SAME && !EARLY) g[s].load(weight + i);
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+          mine[s].set(j, (SAME ? g[s].get(j % Vec16<W>::N) : to_float(weight[i + j])) * (mine[s].get(j) * inv));
+        mine[s].store(orow + i);
+      }
+    }
+  } else if (VEC) {
     constexpr int N = Vec16<T>::N;
-    constexpr int KEEP = 4;                       // vectors a thread keeps in registers between the passes
-    const bool kept = width <= 256 * N * KEEP;    // rows up to 8,192 bf16 (4,096 float) values wide
-    Vec16<T> mine[KEEP];
-    int slot = 0;
-    for (int i = threadIdx.x * N; i < width; i += 256 * N, ++slot) {
+    for (int i = threadIdx.x * N; i < width; i += 256 * N) {
       Vec16<T> a;
       a.load(hr + i);
       if (ADD) {
@@ -120,23 +160,13 @@ rmsnorm_kernel(T* __restrict__ out, T* __restrict__ residual, const T* __restric
       }
 #pragma unroll
       for (int j = 0; j < N; ++j) { const float x = a.get(j); sq += x * x; }
-      if (kept) {
-#pragma unroll
-        for (int s = 0; s < KEEP; ++s) if (s == slot) mine[s] = a;
-      }
     }
     const float total = block_sum(sq, scratch);
     const float inv = 1.0f / sqrtf(total / (float)width + eps);
     const T* src = ADD ? rr : hr;  // each thread re-reads exactly what it wrote itself
-    slot = 0;
-    for (int i = threadIdx.x * N; i < width; i += 256 * N, ++slot) {
+    for (int i = threadIdx.x * N; i < width; i += 256 * N) {
       Vec16<T> a, o;
-      if (kept) {
-#pragma unroll
-        for (int s = 0; s < KEEP; ++s) if (s == slot) a = mine[s];
-      } else {
-        a.load(src + i);
-      }
+      a.load(src + i);
       if (sizeof(W) == sizeof(T)) {
         Vec16<W> g;
         g.load(weight + i);
@@ -169,11 +199,17 @@ rmsnorm_kernel(T* __restrict__ out, T* __restrict__ residual, const T* __restric
 template <typename T, typename W>
 static int launch_rmsnorm(void* out, void* residual, const void* h, const void* w, int rows,
                           int width, float eps, bool add, bool vec, cudaStream_t stream) {
-#define KVB_RMS(ADD_, VEC_)                                                                       \
-  KVB_CHECK_CUDA(kvb_launch((rmsnorm_kernel<T, W, ADD_, VEC_>), dim3(rows), dim3(256), 0, stream, true, \
+  const int pieces = width / Vec16<T>::N;
+#define KVB_RMS(ADD_, VEC_, SLOTS_)                                                                       \
+  KVB_CHECK_CUDA(kvb_launch((rmsnorm_kernel<T, W, ADD_, VEC_, SLOTS_>), dim3(rows), dim3(256), 0, stream, true, \
                             (T*)out, (T*)residual, (const T*)h, (const W*)w, width, eps))
-  if (add) { if (vec) KVB_RMS(true, true); else KVB_RMS(true, false); }
-  else { if (vec) KVB_RMS(false, true); else KVB_RMS(false, false); }
+#define KVB_RMS_ADD(VEC_, SLOTS_) if (add) KVB_RMS(true, VEC_, SLOTS_); else KVB_RMS(false, VEC_, SLOTS_)
+  if (!vec) { KVB_RMS_ADD(false, 0); }
+  else if (pieces <= 256) { KVB_RMS_ADD(true, 1); }
+  else if (pieces <= 512) { KVB_RMS_ADD(true, 2); }
+  else if (pieces <= 1024) { KVB_RMS_ADD(true, 4); }
+  else { KVB_RMS_ADD(true, 0); }
+#undef KVB_RMS_ADD
 #undef KVB_RMS
   return 0;
 }

@@ -217,3 +217,21 @@ def test_blocks_of_one_query_tile_give_the_bits_of_two(group, window, cached, ne
                                    _Batch([(cached, new)] * count), heads, kv_heads, 128, 128 ** -0.5, window)
     one, many = attend(1), attend(copies)
     assert all(torch.equal(part, one) for part in many.split(new)) and K().read_status() == 0
+
+
+@pytest.mark.parametrize("dtype,weights", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("pieces", [1, 255, 256, 257, 512, 513, 1024, 1025])
+def test_norms_around_the_pieces_a_thread_keeps(dtype, weights, pieces):
+    width = pieces * 16 // dtype.itemsize
+    h, residual = randn(3, width, dtype=dtype, seed=1, scale=3.0), randn(3, width, dtype=dtype, seed=2)
+    weight = randn(width, dtype=weights, seed=3)
+    # 32-bit sums in another order (2^-20 at these widths): a bfloat16 result may be the neighbouring number, at most 2^-7 off
+    close = F32 if dtype == torch.float32 else dict(rtol=2.0 ** -7, atol=1e-6)
+
+    def plain(x):
+        x = x.double()
+        return (weight.double() * x / (x.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()).to(dtype)
+    torch.testing.assert_close(K().rmsnorm(h, weight, 1e-5), plain(h), **close)
+    total = h + residual
+    torch.testing.assert_close(K().add_rmsnorm(h, residual, weight, 1e-5), plain(total), **close)
+    assert torch.equal(residual, total)
