@@ -33,11 +33,11 @@
 #define MOE_BN 64
 #define MOE_BK 16
 
-// The logits, [tokens, E + R] 32-bit, and the choice are two kernels, so that a step of few tokens spreads the router's
-// rows over many blocks.  A logit is formed in the same order whichever kernel takes it: lane l adds the products
+// Routing: a token's logits, then its choice.  Up to a token an SM one kernel does both; beyond, the logits [tokens, E + R]
+// go through memory, so that tokens share the router's rows (four tokens a block up to ROUTE_FEW_MAX, then eight) and a
+// warp a token chooses.  A logit is formed in the same order whichever kernel takes it: lane l adds the products
 // k = l, l + 32, ... into four partial sums by (k / 32) % 4, then ((p0 + p1) + (p2 + p3)), then the butterfly over the
-// lanes.  2,048 tokens, 32 experts, rows of 4,096 (B200, cold caches): 55 us and 10 for the choice; one kernel that read
-// x entry by entry from shared memory for each expert apart took 88.
+// lanes.
 template <typename T>
 struct RouteParams {
   float* logits; const T* x; long long x_stride;
@@ -48,8 +48,8 @@ struct RouteParams {
   }
 };
 
-// Few tokens: a block takes one expert and ROUTE_FEW tokens, its four warps a partial sum each, everything straight from
-// memory.  Bound by the latency of the reads.
+// A block takes one expert and ROUTE_FEW tokens, its four warps a partial sum each, everything straight from memory.
+// Bound by the latency of the reads.
 #define ROUTE_FEW 4
 #define ROUTE_AHEAD 16
 template <typename T>
@@ -87,24 +87,25 @@ moe_logits_few_kernel(RouteParams<T> p) {
   if (lane == 0 && token0 + j < p.tokens) p.logits[(size_t)(token0 + j) * (p.E + p.R) + e] = acc;   // warp t: token t
 }
 
-// Many tokens: a block holds TOKENS (8 or 16) rows of x in shared memory, a lane's four entries of 128 lying together, and
-// a warp forms the logits of four experts for eight of them at once: an entry of x read once serves four experts, one of
-// the router eight tokens.  Bound by the latency of the router's entries, which come from the L2 cache a run of 128 ahead.
+// Many tokens: a block holds eight rows of x in shared memory, a lane's four entries of 128 lying together, and a warp forms
+// the logits of four experts for all of them at once: an entry of x read once serves four experts, one of the router eight
+// tokens.  Bound by the latency of the router's entries, which come from the L2 cache two runs of 128 ahead (2,048 tokens,
+// with the choice: 58 us; blocks of sixteen tokens 67).
 #define ROUTE_TOKENS 8
 #define ROUTE_EXPERTS 4
 template <typename T>
 struct __align__(4 * sizeof(T)) RouteQuad { T v[4]; };
-template <typename T, int TOKENS>
-__global__ void __launch_bounds__(TOKENS * 16)
+template <typename T>
+__global__ void __launch_bounds__(128)
 moe_logits_kernel(RouteParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ROUTE);
   extern __shared__ __align__(16) unsigned char route_smem[];
-  RouteQuad<T>* xs = reinterpret_cast<RouteQuad<T>*>(route_smem);             // [TOKENS][runs of 128][32 lanes]
+  RouteQuad<T>* xs = reinterpret_cast<RouteQuad<T>*>(route_smem);             // [ROUTE_TOKENS][runs of 128][32 lanes]
   const int runs = (p.K + 127) / 128;
-  int token0 = blockIdx.x * TOKENS;
+  const int token0 = blockIdx.x * ROUTE_TOKENS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 8
-  for (int i = warp; i < TOKENS * runs; i += TOKENS / 2) {
+  for (int i = warp; i < ROUTE_TOKENS * runs; i += 4) {
     const int t = i / runs, k = (i - t * runs) * 128 + lane;
     const T* row = p.x + (size_t)(token0 + t) * p.x_stride;
     RouteQuad<T> q;
@@ -115,9 +116,7 @@ moe_logits_kernel(RouteParams<T> p) {
   }
   __syncthreads();
   const int all = p.E + p.R;
-  token0 += warp / 4 * ROUTE_TOKENS;                  // four warps share eight tokens
-  xs += (size_t)(warp / 4) * ROUTE_TOKENS * runs * 32;
-  for (int e0 = warp % 4 * ROUTE_EXPERTS; e0 < all; e0 += 4 * ROUTE_EXPERTS) {
+  for (int e0 = warp * ROUTE_EXPERTS; e0 < all; e0 += 4 * ROUTE_EXPERTS) {
     const float* w[ROUTE_EXPERTS];
 #pragma unroll
     for (int n = 0; n < ROUTE_EXPERTS; ++n) w[n] = p.row(min(e0 + n, all - 1));
@@ -126,29 +125,31 @@ moe_logits_kernel(RouteParams<T> p) {
     for (int n = 0; n < ROUTE_EXPERTS; ++n)
 #pragma unroll
       for (int t = 0; t < ROUTE_TOKENS; ++t) part[n][t][0] = part[n][t][1] = part[n][t][2] = part[n][t][3] = 0.0f;
-    float wv[ROUTE_EXPERTS][4], next[ROUTE_EXPERTS][4];
-    auto fetch = [&](int run) {                       // the next run's router entries are on their way meanwhile
+    float wv[3][ROUTE_EXPERTS][4];                    // the router's entries of this run and of the next two, on their way
+    auto fetch = [&](float (&to)[ROUTE_EXPERTS][4], int run) {
       const int k = run * 128 + lane;
 #pragma unroll
       for (int n = 0; n < ROUTE_EXPERTS; ++n)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) next[n][j] = k + 32 * j < p.K ? w[n][k + 32 * j] : 0.0f;   // zeros add nothing
+        for (int j = 0; j < 4; ++j) to[n][j] = k + 32 * j < p.K ? w[n][k + 32 * j] : 0.0f;     // zeros add nothing
     };
-    fetch(0);
-    for (int run = 0; run < runs; ++run) {
+    fetch(wv[0], 0);
+    fetch(wv[1], 1);
+    for (int run0 = 0; run0 < runs; run0 += 3) {
 #pragma unroll
-      for (int n = 0; n < ROUTE_EXPERTS; ++n)
+      for (int u = 0; u < 3; ++u) {
+        const int run = run0 + u;
+        if (run >= runs) break;
+        fetch(wv[(u + 2) % 3], run + 2);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) wv[n][j] = next[n][j];
-      if (run + 1 < runs) fetch(run + 1);
+        for (int t = 0; t < ROUTE_TOKENS; ++t) {
+          const RouteQuad<T> q = xs[(t * runs + run) * 32 + lane];
 #pragma unroll
-      for (int t = 0; t < ROUTE_TOKENS; ++t) {
-        const RouteQuad<T> q = xs[(t * runs + run) * 32 + lane];
+          for (int j = 0; j < 4; ++j) {
+            const float xv = to_float(q.v[j]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float xv = to_float(q.v[j]);
-#pragma unroll
-          for (int n = 0; n < ROUTE_EXPERTS; ++n) part[n][t][j] = fmaf(wv[n][j], xv, part[n][t][j]);
+            for (int n = 0; n < ROUTE_EXPERTS; ++n) part[n][t][j] = fmaf(wv[u][n][j], xv, part[n][t][j]);
+          }
         }
       }
     }
@@ -162,20 +163,23 @@ moe_logits_kernel(RouteParams<T> p) {
   }
 }
 
-// From the logits to the chosen experts and their weights: a warp a token.
-#define CHOOSE_THREADS 128
-__global__ void __launch_bounds__(CHOOSE_THREADS)
-moe_choose_kernel(int* __restrict__ ids_out, float* __restrict__ weights_out, float* __restrict__ gate_out,
-                  const float* __restrict__ logits, int tokens, int E, int R, int top, int score_mode, int renormalize,
-                  const float* __restrict__ correction, int groups, int keep, float weight_scale,
-                  const float* __restrict__ bias) {
-  KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ROUTE);
-  extern __shared__ __align__(16) float choose_smem[];                         // a warp: [E + R] and [E + 2 * groups]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, token = blockIdx.x * (blockDim.x / 32) + warp;
-  if (token >= tokens) return;
-  float* sc = choose_smem + (size_t)warp * (2 * E + R + 2 * groups);
-  for (int e = lane; e < E + R; e += 32) sc[e] = logits[(size_t)token * (E + R) + e];
-  __syncwarp();
+// From a token's logits sc [E + R] to its chosen experts and their weights, by one warp; sc goes on with room for
+// E + 2 * groups more.
+struct ChooseParams {
+  int* ids_out; float* weights_out; float* gate_out;
+  int E, R, top, score_mode, renormalize;
+  const float* correction;
+  int groups, keep;
+  float weight_scale;
+  const float* bias;
+};
+__device__ __forceinline__ void moe_choose(const ChooseParams& c, int token, float* sc, int lane) {
+  const int E = c.E, R = c.R, top = c.top, score_mode = c.score_mode, groups = c.groups, keep = c.keep;
+  const float* correction = c.correction;
+  const float* bias = c.bias;
+  int* ids_out = c.ids_out;
+  float* weights_out = c.weights_out;
+  float* gate_out = c.gate_out;
   for (int r = lane; r < R; r += 32) gate_out[(size_t)token * R + r] = 1.0f / (1.0f + expf(-sc[E + r]));
   if (bias != nullptr)
     for (int e = lane; e < E; e += 32) sc[e] += bias[e];
@@ -249,28 +253,75 @@ moe_choose_kernel(int* __restrict__ ids_out, float* __restrict__ weights_out, fl
     chosen_sum += weight;
     __syncwarp();
   }
-  if (lane == 0 && (renormalize || weight_scale != 1.0f))
+  if (lane == 0 && (c.renormalize || c.weight_scale != 1.0f))
     for (int slot = 0; slot < top; ++slot) {
       float w = weights_out[(size_t)token * top + slot];
-      if (renormalize) w /= chosen_sum;
-      weights_out[(size_t)token * top + slot] = w * weight_scale;
+      if (c.renormalize) w /= chosen_sum;
+      weights_out[(size_t)token * top + slot] = w * c.weight_scale;
     }
 }
 
+// A warp a token, from the logits in memory.
+#define CHOOSE_THREADS 128
+__global__ void __launch_bounds__(CHOOSE_THREADS)
+moe_choose_kernel(const float* __restrict__ logits, int tokens, ChooseParams c) {
+  KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ROUTE);
+  extern __shared__ __align__(16) float choose_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, token = blockIdx.x * (blockDim.x / 32) + warp, all = c.E + c.R;
+  if (token >= tokens) return;
+  float* sc = choose_smem + (size_t)warp * (all + c.E + 2 * c.groups);
+  for (int e = lane; e < all; e += 32) sc[e] = logits[(size_t)token * all + e];
+  __syncwarp();
+  moe_choose(c, token, sc, lane);
+}
+
+// Up to a token an SM: a block a token, a warp an expert's row, and the choice behind them in the same launch.
+template <typename T>
+__global__ void __launch_bounds__(1024)
+moe_route_token_kernel(RouteParams<T> p, ChooseParams c) {
+  KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ROUTE);
+  extern __shared__ __align__(16) float choose_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, token = blockIdx.x;
+  const T* x = p.x + (size_t)token * p.x_stride;
+  for (int e = warp; e < p.E + p.R; e += 32) {
+    const float* w = p.row(e);
+    float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int k0 = lane; k0 < p.K; k0 += ROUTE_AHEAD * 32) {
+      float wv[ROUTE_AHEAD];
+      T xv[ROUTE_AHEAD];
+#pragma unroll
+      for (int i = 0; i < ROUTE_AHEAD; ++i) {
+        const int k = k0 + 32 * i;
+        wv[i] = k < p.K ? w[k] : 0.0f;                // zeros add nothing
+        xv[i] = k < p.K ? x[k] : from_float<T>(0.0f);
+      }
+#pragma unroll
+      for (int i = 0; i < ROUTE_AHEAD; ++i) part[i & 3] = fmaf(wv[i], to_float(xv[i]), part[i & 3]);
+    }
+    const float acc = warp_sum((part[0] + part[1]) + (part[2] + part[3]));
+    if (lane == 0) choose_smem[e] = acc;
+  }
+  __syncthreads();
+  if (warp == 0) moe_choose(c, token, choose_smem, lane);
+}
+
+// Where the kernels change, measured with 32 experts of 4,096 in bf16 (the whole routing, cold caches; before these: a
+// block of one token, then of eight, that read x from shared memory for each expert apart): 8 tokens 18.6 us by a block a
+// token, 25.6 and 44 by the others (34.8 before); 96: 19.5, 27.6, 46 (31.7); 150: 29.6, 27.6, 44 (31.7); 256: 30.8, 27.7,
+// 44 (91); 400: 41, 42, 44 (91); 600: 61, 50, 46 (91); 2,048: 161, 114, 58 (94).  64 experts of 2,048, 16 of 1,024 and 32-bit
+// rows change at the same places.
+#define ROUTE_FEW_MAX 400
+// Batches of up to so many tokens are routed by one kernel (and need no logits in memory), others by two.
+extern "C" int kvb_moe_route_alone() { return kvb_sm_count() > 0 ? kvb_sm_count() : 148; }
+
 template <typename T>
 static int launch_moe_logits(const RouteParams<T>& p, cudaStream_t stream) {
-  // From 128 tokens on the blocks of eight tokens fill enough SMs that reading x and the router less often pays, and
-  // blocks of sixteen once they do; rows too long for shared memory take the other kernel at any number.
-  const long long sms = kvb_sm_count() > 0 ? kvb_sm_count() : 148;
+  // rows too long for shared memory take the few tokens' kernel at any number
   const size_t smem = (size_t)ROUTE_TOKENS * ((p.K + 127) / 128) * 128 * sizeof(T);
-  if (p.tokens >= 16 * sms * 2 / 3 && 2 * smem <= 200 * 1024) {
-    KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * smem)));
-    KVB_CHECK_CUDA(kvb_launch((moe_logits_kernel<T, 16>), dim3((p.tokens + 15) / 16), dim3(256), 2 * smem, stream, true, p));
-    return 0;
-  }
-  if (p.tokens >= 128 && smem <= 200 * 1024) {
-    KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T, 8>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    KVB_CHECK_CUDA(kvb_launch((moe_logits_kernel<T, 8>), dim3((p.tokens + 7) / 8), dim3(128), smem, stream, true, p));
+  if (p.tokens > ROUTE_FEW_MAX && smem <= 200 * 1024) {
+    KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KVB_CHECK_CUDA(kvb_launch((moe_logits_kernel<T>), dim3((p.tokens + ROUTE_TOKENS - 1) / ROUTE_TOKENS), dim3(128), smem, stream,
+                              true, p));
     return 0;
   }
   KVB_CHECK_CUDA(kvb_launch((moe_logits_few_kernel<T>), dim3((p.tokens + ROUTE_FEW - 1) / ROUTE_FEW, p.E + p.R), dim3(128), 0,
@@ -278,7 +329,7 @@ static int launch_moe_logits(const RouteParams<T>& p, cudaStream_t stream) {
   return 0;
 }
 
-// logits: scratch, [tokens, E + R].
+// logits: scratch, [tokens, E + R]; none for up to kvb_moe_route_alone() tokens.
 extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, float* logits, const void* x,
                              long long x_stride, const float* router, const float* gate_rows, int tokens, int E, int R, int K,
                              int top, int score_mode, int renormalize, const float* correction, int groups, int keep,
@@ -294,9 +345,21 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
   size_t smem = (size_t)(2 * E + R + 2 * groups) * sizeof(float);
   KVB_REQUIRE((size_t)K * (dtype == KVB_F32 ? sizeof(float) : sizeof(bf16)) + smem <= 200 * 1024,
               "moe_route: a token's row and scores do not fit in shared memory");
-  const int rc = dtype == KVB_F32
-      ? launch_moe_logits(RouteParams<float>{logits, (const float*)x, x_stride, router, gate_rows, tokens, E, R, K}, stream)
-      : launch_moe_logits(RouteParams<bf16>{logits, (const bf16*)x, x_stride, router, gate_rows, tokens, E, R, K}, stream);
+  const ChooseParams c = {ids_out, weights_out, gate_out, E, R, top, score_mode, renormalize, correction, groups, keep,
+                          weight_scale, bias};
+  const RouteParams<float> in32 = {logits, (const float*)x, x_stride, router, gate_rows, tokens, E, R, K};
+  const RouteParams<bf16> in16 = {logits, (const bf16*)x, x_stride, router, gate_rows, tokens, E, R, K};
+  if (tokens <= kvb_moe_route_alone()) {
+#define KVB_ROUTE_TOKEN(T_, P_)                                                                                        \
+    if (smem > 48 * 1024)                                                                                             \
+      KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_route_token_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    KVB_CHECK_CUDA(kvb_launch((moe_route_token_kernel<T_>), dim3(tokens), dim3(1024), smem, stream, true, P_, c))
+    if (dtype == KVB_F32) { KVB_ROUTE_TOKEN(float, in32); } else { KVB_ROUTE_TOKEN(bf16, in16); }
+#undef KVB_ROUTE_TOKEN
+    KVB_CHECK_LAUNCH();
+    return 0;
+  }
+  const int rc = dtype == KVB_F32 ? launch_moe_logits(in32, stream) : launch_moe_logits(in16, stream);
   if (rc) return rc;
   int warps = CHOOSE_THREADS / 32;
   while (warps > 1 && warps * smem > 48 * 1024) warps /= 2;
@@ -304,8 +367,7 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
   if (smem > 48 * 1024)
     KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_choose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   KVB_CHECK_CUDA(kvb_launch((moe_choose_kernel), dim3((tokens + warps - 1) / warps), dim3(32 * warps), smem, stream, true,
-                            ids_out, weights_out, gate_out, (const float*)logits, tokens, E, R, top, score_mode, renormalize,
-                            correction, groups, keep, weight_scale, bias));
+                            (const float*)logits, tokens, c));
   KVB_CHECK_LAUNCH();
   return 0;
 }

@@ -146,6 +146,8 @@ def ensure_built(verbose: bool = False) -> str:
     lib.kvb_paged_attention_segment.restype = _int
     lib.kvb_moe_tile_rows.argtypes = []
     lib.kvb_moe_tile_rows.restype = _int
+    lib.kvb_moe_route_alone.argtypes = []
+    lib.kvb_moe_route_alone.restype = _int
     _lib = lib
     return str(path)
 
@@ -2138,12 +2140,14 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, top: int, *, score: str = "
     if (group_count <= 0 or experts % group_count or not 0 < group_keep <= group_count
             or group_keep * (experts // group_count) < top):
         raise KernelError(f"moe_route: {group_keep} of {group_count} groups of {experts} experts must hold {top} experts")
-    logits = torch.empty((tokens, experts + extra), dtype=torch.float32, device=x.device)
+    ensure_built()
+    alone = tokens <= _lib.kvb_moe_route_alone()
+    logits = None if alone else torch.empty((tokens, experts + extra), dtype=torch.float32, device=x.device)
     _call("kvb_moe_route", ids.data_ptr(), weights.data_ptr(), None if gates is None else gates.data_ptr(),
-          logits.data_ptr(), x.data_ptr(), x.stride(0), router.data_ptr(), None if gate_rows is None else gate_rows.data_ptr(),
+          None if alone else logits.data_ptr(), x.data_ptr(), x.stride(0), router.data_ptr(), None if gate_rows is None else gate_rows.data_ptr(),
           tokens, experts, extra, k, int(top), MOE_SCORE_MODES[score], int(bool(renormalize)),
           None if correction is None else correction.data_ptr(), int(group_count), int(group_keep), float(weight_scale),
-          None if bias is None else bias.data_ptr(), _dtype_code(x), _stream(), kernels=2)
+          None if bias is None else bias.data_ptr(), _dtype_code(x), _stream(), kernels=1 if alone else 2)
     return ids, weights, gates
 
 

@@ -63,7 +63,7 @@ def test_norm_and_gate_in_pieces(dtype, heads, vdim, act, weighted):
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("experts,gates,width", [(32, 1, 384), (5, 0, 1000), (70, 3, 129), (16, 0, 4096)])
 def test_router_logits_have_the_same_bits_in_every_kernel(dtype, experts, gates, width):
-    """Few tokens (four a block), many (eight or sixteen a block), and rows that no piece fits."""
+    """A block a token, four tokens a block, eight, and rows that no piece fits."""
     tokens, top = 1700, min(4, experts)
     x = randn(tokens, width, dtype=dtype, seed=1)
     router = randn(experts, width, dtype=torch.float32, seed=2, scale=0.1)
@@ -79,7 +79,7 @@ def test_router_logits_have_the_same_bits_in_every_kernel(dtype, experts, gates,
     bound = (x.double().abs() @ router.double().abs().T).amax() * width * 2.0 ** -24 + 1e-6
     assert ((z.gather(1, ids.long()) - best).abs() <= 2 * bound).all()
     torch.testing.assert_close(weights.double(), torch.softmax(z.gather(1, ids.long()), -1), rtol=0, atol=float(2 * bound) + 1e-6)
-    for rows in (slice(0, 1), slice(3, 8), slice(100, 227), slice(100, 228), slice(0, 600)):
+    for rows in (slice(0, 1), slice(3, 8), slice(100, 248), slice(100, 249), slice(7, 407), slice(7, 408)):
         some = route(x[rows])
         assert torch.equal(some[0], ids[rows]) and torch.equal(some[1], weights[rows])
         assert g is None or torch.equal(some[2], g[rows])
@@ -235,3 +235,26 @@ def test_norms_around_the_pieces_a_thread_keeps(dtype, weights, pieces):
     total = h + residual
     torch.testing.assert_close(K().add_rmsnorm(h, residual, weight, 1e-5), plain(total), **close)
     assert torch.equal(residual, total)
+
+
+@pytest.mark.parametrize("experts,identity,tokens,top", [(1, 0, 1, 1), (33, 2, 700, 3), (70, 0, 1024, 8), (32, 0, 2049, 4), (64, 1, 2731, 6)])
+def test_grouping_of_many_pairs(experts, identity, tokens, top):
+    """One thread's choices in one lot and in several, experts in one warp's worth and in several."""
+    ids = torch.randint(0, experts + identity, (tokens, top), generator=torch.Generator().manual_seed(1)).to(DEV, torch.int32)
+    g = K().moe_group(ids, experts, for_library=True, identity=identity)
+    flat, rows, sorted_pairs, begins = ids.flatten().cpu(), g.row_of_pair.cpu().long(), g.sorted_pairs.cpu(), g.begins()
+    tile = g.capacity // g.max_tiles
+    counts = torch.bincount(flat.long(), minlength=experts + identity)[:experts]
+    want, at = [0], 0
+    for count in counts.tolist():
+        at += -(-count // tile) * tile
+        want.append(at)
+    assert begins == want and int(g.meta[0]) == at // tile
+    own = flat < experts
+    assert (rows[~own] == -1).all() and rows[own].unique().numel() == int(own.sum())
+    assert torch.equal(sorted_pairs[rows[own]].long(), own.nonzero().flatten())
+    begin = torch.tensor(begins)[flat[own].long()]
+    assert ((rows[own] >= begin) & (rows[own] < begin + counts[flat[own].long()])).all()
+    assert int((sorted_pairs >= 0).sum()) == int(own.sum())
+    assert g.tile_expert[:at // tile].tolist() == [e for e, c in enumerate(counts.tolist()) for _ in range(-(-c // tile))]
+    assert K().read_status() == 0
