@@ -12,8 +12,10 @@
 // of 128, in one beside keys of 192 (the shared memory is then full: 96 KB of queries, 96 of keys, 32 of values; the next
 // values are asked for when B's product with the last ones has been taken, half a key tile's time ahead of A's).
 // Rows come by TMA, a box a page; or, when the rows of a request's positions lie one behind the other (keys carried up
-// from cached latents), a box of 128 rows that may begin in front of the request's first row (masked like every row
-// nobody sees).
+// from cached latents), a box of 128 rows that may begin in front of the request's first row and end behind its last.
+// Rows that nobody in the block sees are another request's, or what a page's former owner left there: their scores are
+// masked, and their values, which a probability of zero would not undo if they were no numbers, are cleared in shared
+// memory ahead of the product (pages that hold nothing but such rows are not read at all).
 // What bounds it is the chain of products and softmax of each query tile (see attention_prefill_tc5.cu), not a unit.
 // One prompt of 2,048 tokens, call by call (B200; mma.sync tiles of attention_flash_dims.cu before): carried-up latents,
 // 32 heads of 192 / 128: 96 us (394); 16 heads of two maps, 128 / 256: 150 us (432); 32 heads over 8, 128 / 128, window
@@ -48,6 +50,7 @@ struct RowsTc5Params {
   int* status;
   int q_by_tma;
   int tiles;                              // query tiles of a block (kvb_tc5_query_tiles)
+  int no_row;                             // behind the last row of the planes: a box there is all zeros
 };
 
 // Byte offset of the 16-byte piece `piece` of row `r` in an operand tile stored as swizzled parts of 64 columns.
@@ -162,25 +165,22 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
   const int ppt = RT_BN / p.page_rows;       // copies a tile (and part): 1 or 2..16
   const int total_entries = num_tiles * ppt;
   auto fetch = [&](int entry) -> int {
-    if (entry >= total_entries) return 0;
+    if (entry >= total_entries) return p.no_row;
     if (p.in_order) {                        // an entry is a tile: its first row, counted back from the first that is seen
       const int key0 = (tile_begin + entry) * RT_BN, key = max(key0, key_lo);
-      if (key >= key_hi || key >= p.table_stride) return 0;
+      if (key >= key_hi || key >= p.table_stride) return p.no_row;
       const int row = entries[key];
       if (row <= 0 || row >= p.num_pages) {
         atomicOr(p.status, KVB_STATUS_BAD_PAGE);
-        return 0;
+        return p.no_row;
       }
       return row - (key - key0);
     }
     const int index = tile_begin * ppt + entry;
-    if (index >= p.table_stride || index * p.page_rows >= key_hi) return 0;
+    if (index >= p.table_stride || index * p.page_rows >= key_hi || (index + 1) * p.page_rows <= key_lo) return p.no_row;
     const int page = entries[index];
-    if (page < 0 || page >= p.num_pages) {
-      atomicOr(p.status, KVB_STATUS_BAD_PAGE);
-      return 0;
-    }
-    return page * p.page_rows;
+    if (page < 0 || page >= p.num_pages) atomicOr(p.status, KVB_STATUS_BAD_PAGE);
+    return page > 0 && page < p.num_pages ? page * p.page_rows : p.no_row;      // page 0 is nobody's
   };
   int cur = 0, nxt = 0;
   if (warp == 8 || warp == 9) {
@@ -395,6 +395,21 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
           kvb_tc5_st32(o_addr + c * 32, o);
         }
       }
+      // Values of rows outside [key_lo, key_hi): thread r clears row r, in the first tile that reads this key tile's
+      // values (A where it sees the tile), whose product waits for all its threads and is issued ahead of the other's.
+      if (key0 + r < key_lo || key0 + r >= key_hi) {
+        const int vs = j % VS;
+        if ((j < n_a) == (x == 0)) {
+          if (!RT_WAIT(&v_full[vs], (j / VS) & 1)) { ok = false; break; }
+          unsigned char* row = v_smem + vs * V_BYTES + r * 128;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {              // (lanes start at different pieces: no bank conflicts)
+            *reinterpret_cast<uint4*>(row + ((c ^ (r & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(row + RT_PART_BYTES + ((c ^ (r & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+          }
+          kvb_fence_async_shared();                  // generic writes -> visible to the product's reads
+        }
+      }
       kvb_tc5_wait_st();
       kvb_tc5_fence_before();
       kvb_mbar_arrive(&p_ready[x]);
@@ -499,6 +514,7 @@ extern "C" int kvb_flash_rows_tc5(void* out, long long out_token, long long out_
   p.sink = sink; p.slopes = slopes; p.status = kvb_status_word();
   KVB_REQUIRE(p.status != nullptr, "rows attention (tcgen05): no status word");
   const long long rows = (long long)num_pages * page_size;
+  p.no_row = (int)rows;
   alignas(64) CUtensorMap k_map, v_map, q_map;
   memset(&q_map, 0, sizeof(q_map));
   KVB_REQUIRE(rt_rows_map(&k_map, keys, (long long)(value_heads * maps - 1) * k_head + DK, rows, pitch, p.page_rows) &&

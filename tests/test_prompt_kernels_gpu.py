@@ -258,3 +258,91 @@ def test_grouping_of_many_pairs(experts, identity, tokens, top):
     assert int((sorted_pairs >= 0).sum()) == int(own.sum())
     assert g.tile_expert[:at // tile].tolist() == [e for e, c in enumerate(counts.tolist()) for _ in range(-(-c // tile))]
     assert K().read_status() == 0
+
+
+def _two_tiles(requests, heads_and_slices, rows):
+    """Whether a launch of the tcgen05 prompt kernels over so many requests of at most ``rows`` query rows takes blocks of
+    two query tiles (of 128 rows each)."""
+    return 2 * requests * heads_and_slices * -(-rows // 256) > K().api.sm_count(torch.device(DEV))
+
+
+def _paged_rows(lens, kv_heads, group, maps, vdim, page, window, copies=1):
+    """A call of attention_dims on keys (128) and values in the rows of a plane, and which slots of the plane are seen;
+    ``copies`` of the requests, which share their pages."""
+    tokens, width = sum(n for _, n in lens), kv_heads * (maps * 128 + vdim)
+    count = [-(-(c + n) // page) for c, n in lens]
+    order = torch.randperm(sum(count), generator=torch.Generator().manual_seed(1)) + 1
+    table, seen, at = torch.zeros(len(lens), max(count), dtype=torch.int32), torch.zeros(sum(count) + 1, page, dtype=torch.bool), 0
+    for row, ((c, n), pages) in enumerate(zip(lens, count)):
+        first = 0 if window is None else max(0, c - window + 1)
+        table[row, first // page:pages] = order[at + first // page:at + pages]          # pages behind the window are gone
+        for pos in range(first, c + n):
+            seen[order[at + pos // page], pos % page] = True
+        at += pages
+    plane = randn(sum(count) + 1, 1, page, width, dtype=torch.bfloat16, seed=2)
+    q = randn(tokens, kv_heads * group * maps, 128, dtype=torch.bfloat16, seed=3)
+    how = dict(value_heads=kv_heads, group=group, maps=maps, key_width=128, value_width=vdim, page_size=page,
+               num_pages=plane.shape[0], key_strides=(page * width, 128, width), value_strides=(page * width, vdim, width),
+               scale=128 ** -0.5, window=window)
+    table, q = table.repeat(copies, 1).to(DEV), q.repeat(copies, 1, 1)
+
+    def attend(plane, **more):
+        return K().attention_dims(q, plane, plane.view(-1)[kv_heads * maps * 128:], table, _Batch(lens * copies), **dict(how, **more))
+    return attend, plane, seen.to(DEV)
+
+
+def _rows_in_order(lens, heads, turned, window, copies=1):
+    """A call of attention_dims on keys of 128 + ``turned`` entries and values of 128 carried up for the positions that are
+    seen, one row a position; the rows that each request has.  ``copies`` of the requests, which share their rows."""
+    dk, per, totals = 128 + turned, 256 + turned, [c + n for c, n in lens]
+    starts = [0 if window is None else max(0, c - window + 1) for c, _ in lens]
+    rows = sum(t - s for t, s in zip(totals, starts)) + 1
+    carried = randn(rows, heads * per, dtype=torch.bfloat16, seed=1)
+    table, at, own = torch.zeros(len(lens), max(totals), dtype=torch.int32, device=DEV), 1, []
+    for row, (start, total) in enumerate(zip(starts, totals)):
+        table[row, start:total] = torch.arange(at, at + total - start, dtype=torch.int32, device=DEV)
+        own.append(slice(at, at + total - start))
+        at += total - start
+    q = randn(sum(n for _, n in lens), heads, dk, dtype=torch.bfloat16, seed=2).repeat(copies, 1, 1)
+    table, strides = table.repeat(copies, 1), (heads * per, per, 0)
+
+    def attend(carried, **more):
+        return K().attention_dims(q, carried, carried.view(-1)[dk:], table, _Batch(lens * copies), **dict(dict(
+            value_heads=heads, group=1, maps=1, key_width=dk, value_width=128, page_size=1, num_pages=rows,
+            key_strides=strides, value_strides=strides, scale=dk ** -0.5, window=window, rows_in_order=True), **more))
+    return attend, carried, own
+
+
+NAN = float("nan")
+
+
+@pytest.mark.parametrize("kv_heads,two", [(2, False), (40, True)])
+@pytest.mark.parametrize("group,page,window", [(1, 16, None), (3, 64, 100), (4, 8, 300)])
+def test_rows_of_a_plane_that_nobody_sees_do_not_count(kv_heads, two, group, page, window):
+    """The unwritten end of a request's last page, page 0 and what lies in front of a window hold NaN: the same bits as
+    with zeros there."""
+    lens = [(300, 201), (0, 77), (600, 129)]
+    assert _two_tiles(len(lens), kv_heads, 201 * group) == two
+    attend, plane, seen = _paged_rows(lens, kv_heads, group, 1, 128, page, window)
+    hidden = ~seen[:, None, :, None]
+    want = attend(plane.masked_fill(hidden, 0.0))
+    assert torch.isfinite(want.float()).all()
+    assert torch.equal(attend(plane.masked_fill(hidden, NAN)), want) and K().read_status() == 0
+
+
+@pytest.mark.parametrize("heads,two", [(2, False), (40, True)])
+@pytest.mark.parametrize("turned,window", [(64, None), (0, None), (0, 90), (64, 200)])
+def test_rows_of_other_requests_do_not_count(heads, two, turned, window):
+    """Carried-up rows lie one behind the other, and boxes of 128 run on into the next request's: NaN in the rows of all
+    others leaves a request's bits as they are."""
+    lens = [(300, 201), (0, 77), (600, 129)]
+    assert _two_tiles(len(lens), heads, 201) == two
+    attend, carried, own = _rows_in_order(lens, heads, turned, window)
+    want, at = attend(carried), 0
+    assert torch.isfinite(want.float()).all()
+    for (_, n), rows in zip(lens, own):
+        others = torch.full_like(carried, NAN)
+        others[rows] = carried[rows]
+        assert torch.equal(attend(others)[at:at + n], want[at:at + n])
+        at += n
+    assert K().read_status() == 0
