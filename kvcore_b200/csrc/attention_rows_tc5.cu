@@ -8,6 +8,8 @@
 // (token, query head of the key head's group) pair.  It walks the keys in tiles of 128; eleven warps as there: two softmax
 // warpgroups (a thread a row), a producer warp for keys and one for values, one thread that issues the products
 //     S_A(0), S_B(0); per key tile j:  O_A += P_A(j).V(j), S_A(j+1), O_B += P_B(j).V(j), S_B(j+1).
+// Behind a window B begins with the first key tile that it sees itself, so that a row's result has the same bits in blocks
+// of one and of two query tiles.
 // Keys are staged as KH parts of 64 columns (128-byte swizzle), two stages; values as two parts, in two stages beside keys
 // of 128, in one beside keys of 192 (the shared memory is then full: 96 KB of queries, 96 of keys, 32 of values; the next
 // values are asked for when B's product with the last ones has been taken, half a key tile's time ahead of A's).
@@ -132,6 +134,8 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
   const int n_a = (context + last_row_a / p.G + RT_BN) / RT_BN - tile_begin;              // >= 1
   const int n_b = has_b ? (context + last_row_b / p.G + RT_BN) / RT_BN - tile_begin : 0;  // >= n_a when tile B exists
   const int num_tiles = max(n_a, n_b);
+  // the first key tile that B sees (A's is 0); its own tiles are counted from there
+  const int b_begin = has_b && p.window > 0 ? max(0, context + (row0 + RT_BM) / p.G - p.window + 1) / RT_BN - tile_begin : 0;
   const int key_hi = context + (has_b ? last_row_b : last_row_a) / p.G + 1;
   auto query_head = [&](int flat) { return (vh * p.G + flat % p.G) * p.maps + map; };
 
@@ -268,7 +272,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
       if (ok) {
         kvb_tc5_fence_after();
         issue_s(0, 0);
-        if (has_b) issue_s(1, 0);
+        if (has_b && b_begin == 0) issue_s(1, 0);
         kvb_tc5_commit(&k_empty[0]);
       }
       for (int j = 0; j < num_tiles && ok; ++j) {
@@ -285,14 +289,14 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
           kvb_tc5_fence_after();
           if (j + 1 < n_a) issue_s(0, ks);
         }
-        if (j < n_b) {
-          if (!RT_WAIT(&p_ready[1], j & 1)) { ok = false; break; }
+        if (j >= b_begin && j < n_b) {
+          if (!RT_WAIT(&p_ready[1], (j - b_begin) & 1)) { ok = false; break; }
           kvb_tc5_fence_after();
-          issue_pv(1, vs, j > 0);
+          issue_pv(1, vs, j > b_begin);
         }
         kvb_tc5_commit(&v_empty[vs]);
         if (more) {
-          if (j + 1 < n_b) issue_s(1, ks);
+          if (j + 1 >= b_begin && j + 1 < n_b) issue_s(1, ks);
           kvb_tc5_commit(&k_empty[ks]);
         }
       }
@@ -304,7 +308,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
   } else {
     // ================= softmax: thread r of warpgroup x owns row r of tile x =================
     const int r = threadIdx.x & 127, x = threadIdx.x >> 7;
-    const int n_mine = x == 0 ? n_a : n_b;
+    const int begin = x == 0 ? 0 : b_begin, n_mine = (x == 0 ? n_a : n_b) - begin;     // this tile's key tiles
     const int flat = row0 + x * RT_BM + r;
     const bool row_valid = flat < rows_total;
     const int pos = context + (row_valid ? flat / p.G : 0), hq = query_head(row_valid ? flat : 0);
@@ -318,10 +322,10 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
     const float slope = SLOPE ? p.slopes[hq] * 1.4426950408889634f : 0.0f;
     const float scale_log2 = SLOPE ? 1.0f : p.scale_log2; // with slopes the scores are brought into the log2 domain first
     bool ok = true;
-    for (int j = 0; j < n_mine; ++j) {
-      if (!RT_WAIT(&s_full[x], j & 1)) { ok = false; break; }
+    for (int turn = 0; turn < n_mine; ++turn) {
+      if (!RT_WAIT(&s_full[x], turn & 1)) { ok = false; break; }
       kvb_tc5_fence_after();
-      const int key0 = (tile_begin + j) * RT_BN;
+      const int j = begin + turn, key0 = (tile_begin + j) * RT_BN;
       const bool need_mask = ragged || p.window > 0 || key0 + RT_BN - 1 > first_pos;
       float s[4][32];
 #pragma unroll
@@ -357,10 +361,10 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
         for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = rt_max3(mx[(i >> 1) & 3], s[c][i], s[c][i + 1]);
       const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;   // scale > 0; -inf stays -inf
       const float new_max = fmaxf(row_max, tile_max);
-      // The maximum is moved (and O rescaled) only when it would grow by more than 2^8; but always within the first 512
-      // keys: a row's largest probability is then exactly one, which counts while it is a large part of the row (33
+      // The maximum is moved (and O rescaled) only when it would grow by more than 2^8; but always within the first four
+      // key tiles that the query tile sees: a row's largest probability is then exactly one, which counts while it is a large part of the row (33
       // tokens behind 300 are 11 % further from their values in 64 bits without).
-      const bool grows = new_max > row_max + (j < 4 ? 0.0f : 8.0f);       // from -inf too
+      const bool grows = new_max > row_max + (turn < 4 ? 0.0f : 8.0f);       // from -inf too
       const bool move = __any_sync(0xffffffffu, grows);
       float correction = 1.0f;
       if (move) {
@@ -384,7 +388,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
         kvb_tc5_st16(s_addr + c * 16, packed);       // over S(j); S(j+1) comes after the tensor pipe has taken P(j)
       }
       row_sum = row_sum * correction + ((sm[0] + sm[1]) + (sm[2] + sm[3]));
-      if (move && j > 0) {                           // P(j-1).V(j-1) has landed: it was issued before S(j)
+      if (move && turn > 0) {                        // P(j-1).V(j-1) has landed: it was issued before S(j)
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           float o[32];

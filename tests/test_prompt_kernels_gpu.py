@@ -346,3 +346,19 @@ def test_rows_of_other_requests_do_not_count(heads, two, turned, window):
         assert torch.equal(attend(others)[at:at + n], want[at:at + n])
         at += n
     assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("cached,new,window", [(257, 300, 90), (0, 700, None), (1000, 385, 200), (1000, 385, 1000)])
+@pytest.mark.parametrize("turned", [None, 0, 64])
+def test_rows_have_the_same_bits_in_blocks_of_one_and_two_query_tiles(cached, new, window, turned):
+    """A request alone (one tile a block), and beside forty of its like (two); over pages, and over rows in order."""
+    heads, copies = 2, 41
+    assert not _two_tiles(1, heads, new) and _two_tiles(copies, heads, new)
+
+    def run(copies):
+        lens = [(cached, new)]
+        made = (_paged_rows(lens, heads, 1, 1, 128, 16, window, copies) if turned is None
+                else _rows_in_order(lens, heads, turned, window, copies))
+        return made[0](made[1])
+    alone, beside = run(1), run(copies)
+    assert all(torch.equal(part, alone) for part in beside.split(new)) and K().read_status() == 0
