@@ -359,7 +359,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
       for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = rt_max3(mx[(i >> 1) & 3], s[c][i], s[c][i + 1]);
-      const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;   // scale > 0; -inf stays -inf
+      const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;   // (the scale is positive); -inf stays -inf
       const float new_max = fmaxf(row_max, tile_max);
       // The maximum is moved (and O rescaled) only when it would grow by more than 2^8; but always within the first four
       // key tiles that the query tile sees: a row's largest probability is then exactly one, which counts while it is a large part of the row (33
@@ -508,6 +508,7 @@ extern "C" int kvb_flash_rows_tc5(void* out, long long out_token, long long out_
               pitch % 8 == 0 && k_head % 8 == 0 && v_head % 8 == 0 && out_token % (out_f32 ? 4 : 8) == 0 &&
               out_head % (out_f32 ? 4 : 8) == 0, "rows attention (tcgen05): rows must start on 16-byte boundaries");
   KVB_REQUIRE((long long)num_pages * page_size < (1ll << 31), "rows attention (tcgen05): too many rows");
+  KVB_REQUIRE(scale > 0.0f, "rows attention (tcgen05): the scale must be positive");
   RowsTc5Params p = {};
   p.out = out; p.out_token = out_token; p.out_head = out_head; p.out_f32 = out_f32;
   p.q = (const bf16*)q; p.q_token = q_token; p.q_head = q_head;

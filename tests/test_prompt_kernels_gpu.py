@@ -362,3 +362,13 @@ def test_rows_have_the_same_bits_in_blocks_of_one_and_two_query_tiles(cached, ne
         return made[0](made[1])
     alone, beside = run(1), run(copies)
     assert all(torch.equal(part, alone) for part in beside.split(new)) and K().read_status() == 0
+
+
+@pytest.mark.parametrize("scale", [-0.25, 0.0])
+def test_rows_with_a_scale_that_is_not_positive(scale):
+    """Such scales go to the kernel that scales every score; its results in 64 bits."""
+    lens, heads, kv_heads, width = [(130, 129), (0, 40)], 4, 2, 2 * 256
+    attend, plane, _ = _paged_rows(lens, kv_heads, 2, 1, 128, 16, None)
+    got = attend(plane, scale=scale, out_dtype=torch.float32)
+    assert torch.equal(got, attend(plane, scale=scale, out_dtype=torch.float32, num_splits=1))
+    assert torch.isfinite(got).all() and K().read_status() == 0
