@@ -525,18 +525,18 @@ extern "C" int kvb_flash_rows_tc5(void* out, long long out_token, long long out_
   KVB_REQUIRE(rt_rows_map(&k_map, keys, (long long)(value_heads * maps - 1) * k_head + DK, rows, pitch, p.page_rows) &&
               rt_rows_map(&v_map, values, (long long)(value_heads - 1) * v_head + DV, rows, pitch, p.page_rows),
               "rows attention (tcgen05): no tensor map for the keys or the values");
-  // the queries as [token][key head][head of the group][DK], as attention_prefill_tc5.cu has them (one map a value head)
-  if (maps == 1 && RT_BM % group == 0) {
+  // the queries as [token][key head][head of the group][DK], as attention_prefill_tc5.cu has them (one map a value head);
+  // strides that no tensor map describes (a row that serves all tokens has a stride of zero) leave them to be copied
+  if (maps == 1 && RT_BM % group == 0 && q_token > 0 && q_head > 0) {
     KvbEncodeTiledFn encode = kvb_encode_tiled_fn();
     const cuuint64_t dims[4] = {(cuuint64_t)DK, (cuuint64_t)group, (cuuint64_t)value_heads, (cuuint64_t)num_tokens};
     const cuuint64_t strides[3] = {(cuuint64_t)q_head * sizeof(bf16), (cuuint64_t)group * q_head * sizeof(bf16),
                                    (cuuint64_t)q_token * sizeof(bf16)};
     const cuuint32_t box[4] = {64, (cuuint32_t)group, 1, (cuuint32_t)(RT_BM / group)};
     const cuuint32_t elem[4] = {1, 1, 1, 1};
-    KVB_REQUIRE(encode(&q_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(q), dims, strides, box, elem,
-                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS, "rows attention (tcgen05): no tensor map for the queries");
-    p.q_by_tma = 1;
+    p.q_by_tma = encode(&q_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(q), dims, strides, box, elem,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
   const long long all_rows = (long long)max_query_len * group, heads = (long long)value_heads * maps * p.slices;
   p.tiles = kvb_tc5_query_tiles(heads * num_reqs * ((all_rows + 2 * RT_BM - 1) / (2 * RT_BM)));

@@ -367,8 +367,23 @@ def test_rows_have_the_same_bits_in_blocks_of_one_and_two_query_tiles(cached, ne
 @pytest.mark.parametrize("scale", [-0.25, 0.0])
 def test_rows_with_a_scale_that_is_not_positive(scale):
     """Such scales go to the kernel that scales every score; its results in 64 bits."""
-    lens, heads, kv_heads, width = [(130, 129), (0, 40)], 4, 2, 2 * 256
+    lens, kv_heads = [(130, 129), (0, 40)], 2
     attend, plane, _ = _paged_rows(lens, kv_heads, 2, 1, 128, 16, None)
     got = attend(plane, scale=scale, out_dtype=torch.float32)
     assert torch.equal(got, attend(plane, scale=scale, out_dtype=torch.float32, num_splits=1))
     assert torch.isfinite(got).all() and K().read_status() == 0
+
+
+def test_rows_with_one_query_row_for_all_tokens():
+    """Queries that are a view of one row (a stride of zero) give what their copy gives."""
+    lens, heads, dk = [(130, 129), (0, 40)], 4, 128
+    plane = randn(40, 1, 16, heads * 256, dtype=torch.bfloat16, seed=2)
+    table = torch.arange(1, 35, dtype=torch.int32, device=DEV).view(2, 17).contiguous()
+    q = randn(1, heads, dk, dtype=torch.bfloat16, seed=3).expand(169, heads, dk)
+    width = heads * 256
+    how = dict(value_heads=heads, group=1, maps=1, key_width=128, value_width=128, page_size=16, num_pages=40,
+               key_strides=(16 * width, 128, width), value_strides=(16 * width, 128, width), scale=dk ** -0.5)
+    values = plane.view(-1)[heads * 128:]
+    got = K().attention_dims(q, plane, values, table, _Batch(lens), **how)
+    assert torch.equal(got, K().attention_dims(q.contiguous(), plane, values, table, _Batch(lens), **how))
+    assert K().read_status() == 0
