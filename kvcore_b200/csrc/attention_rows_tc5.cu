@@ -422,7 +422,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
     if (ok && n_mine > 0) {
       kvb_tc5_fence_after();
       if (p.sink != nullptr && row_sum > 0.0f) row_sum += exp2f(p.sink[hq] * 1.4426950408889634f - row_max);   // counts once
-      const float inv = row_sum > 0.0f ? 1.0f / row_sum : 0.0f;
+      const float inv = row_sum == 0.0f ? 0.0f : 1.0f / row_sum;     // a sink that is no number leaves none
       float o[4][32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) kvb_tc5_ld32(o_addr + c * 32, o[c]);

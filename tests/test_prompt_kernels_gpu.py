@@ -387,3 +387,11 @@ def test_rows_with_one_query_row_for_all_tokens():
     got = K().attention_dims(q, plane, values, table, _Batch(lens), **how)
     assert torch.equal(got, K().attention_dims(q.contiguous(), plane, values, table, _Batch(lens), **how))
     assert K().read_status() == 0
+
+
+def test_rows_with_a_sink_that_is_no_number():
+    lens, heads = [(130, 129), (0, 40)], 4
+    sink = torch.tensor([0.5, NAN, -float("inf"), 1.0], device=DEV)
+    attend, plane, _ = _paged_rows(lens, heads, 1, 1, 128, 16, None)
+    got, other = attend(plane, sink=sink), attend(plane, sink=sink, num_splits=1)
+    assert got[:, 1].isnan().all() and other[:, 1].isnan().all() and torch.isfinite(got[:, [0, 2, 3]].float()).all()
