@@ -7,7 +7,7 @@ import torch
 
 import plain_kernels as P
 from test_dutivik_kernels_gpu import F32, _HostBatch, _states
-from test_kernels_gpu import DEV, DTYPES, K, randn
+from test_kernels_gpu import DEV, DTYPES, K, _cache_case, randn
 from test_pipesun_kernels_gpu import _Batch
 
 pytestmark = pytest.mark.gpu
@@ -395,3 +395,56 @@ def test_rows_with_a_sink_that_is_no_number():
     attend, plane, _ = _paged_rows(lens, heads, 1, 1, 128, 16, None)
     got, other = attend(plane, sink=sink), attend(plane, sink=sink, num_splits=1)
     assert got[:, 1].isnan().all() and other[:, 1].isnan().all() and torch.isfinite(got[:, [0, 2, 3]].float()).all()
+
+
+@pytest.mark.parametrize("lens,kv_heads,group,maps,vdim,page,window,extra,f32", [
+    ([(0, 257), (130, 129), (0, 40)], 40, 1, 1, 128, 16, None, True, False),
+    ([(0, 700), (300, 385), (127, 64)], 20, 2, 1, 128, 8, 100, True, True),
+    ([(1500, 257), (0, 128)], 16, 3, 1, 256, 64, 1000, True, False),
+    ([(300, 333)], 6, 4, 2, 256, 32, None, False, True)])
+def test_two_query_tiles_over_rows_of_a_plane(lens, kv_heads, group, maps, vdim, page, window, extra, f32):
+    """The same as above in launches that take two query tiles a block: B partly filled, missing, a key tile behind A."""
+    assert _two_tiles(len(lens), kv_heads * maps * vdim // 128, max(n for _, n in lens) * group)
+    test_prompt_attention_over_rows_of_a_plane(lens, kv_heads, group, maps, vdim, page, window, extra, f32)
+
+
+@pytest.mark.parametrize("lens", [[(0, 2047)], [(100, 700), (0, 129), (33, 64)]])
+@pytest.mark.parametrize("turned,window", [(64, None), (64, 150), (0, None), (0, 600)])
+def test_two_query_tiles_over_rows_in_order(lens, turned, window):
+    """What a latent prompt of 32 heads runs: values in one stage beside keys of 192 entries, queries by TMA."""
+    assert _two_tiles(len(lens), 32, max(n for _, n in lens))
+    test_prompt_attention_over_rows_in_order(lens, 32, turned, window)
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_batches_in_two_query_tiles_give_the_bits_of_their_requests_alone(seed):
+    """Batches drawn at random for the paged prompt kernel, with windows, or sinks and capped scores; every request and a
+    kv head of it once more alone, in blocks of one query tile."""
+    import random
+
+    rng = random.Random(seed)
+    group, page = rng.choice([1, 2, 4, 8, 3]), rng.choice([8, 16, 32, 64])
+    lens = [(rng.choice([0, rng.randint(1, 700), 128 * rng.randint(0, 3), 127, 129]),
+             rng.choice([rng.randint(17, 400), 64, 65, 128 // group + 1, 256 // group])) for _ in range(rng.randint(2, 4))]
+    longest = max(n for _, n in lens)
+    kv_heads = -(-80 // (len(lens) * -(-longest * group // 256)))
+    heads, form = kv_heads * group, seed % 3
+    window = rng.randint(20, 300) if form == 1 else None
+    sink = randn(heads, dtype=torch.float32, seed=5) if form == 2 else None
+    softcap = 3.0 if form == 2 else None
+    assert _two_tiles(len(lens), kv_heads, longest * group) and not _two_tiles(1, 1, longest * group)
+    case = _cache_case(torch.bfloat16, heads, kv_heads, 128, page, lens, seed=seed)
+    got = K().paged_attention(case["qkv"], case["k_cache"], case["v_cache"], case["table"], _Batch(lens, host=False), heads,
+                              kv_heads, 128, 128 ** -0.5, window, sink=sink, softcap=softcap)
+    at = 0
+    for row, (cached, new) in enumerate(lens):
+        for h in (0, kv_heads - 1):
+            cols = slice(h * group * 128, (h + 1) * group * 128)
+            part = torch.cat([case["qkv"][at:at + new, cols], case["qkv"][at:at + new, heads * 128:heads * 128 + 256]], 1)
+            alone = K().paged_attention(part, case["k_cache"][:, h:h + 1].contiguous(), case["v_cache"][:, h:h + 1].contiguous(),
+                                        case["table"][row:row + 1], _Batch([(cached, new)], host=False), group, 1, 128, 128 ** -0.5, window,
+                                        sink=None if sink is None else sink[h * group:(h + 1) * group].clone(), softcap=softcap)
+            if new * group > 16:                  # shorter ones take the decode kernel when they are alone
+                assert torch.equal(got[at:at + new, cols], alone), (lens, group, page, window, form)
+        at += new
+    assert K().read_status() == 0
