@@ -1323,7 +1323,8 @@ def flash_dims_supported(q, out, key_width, value_width, page_size, key_strides,
     return all(_flash_dims_geometry(key_width, value_width, rows, alias) is not None for rows in (64, 32, 16))
 
 
-def _rows_tc5_takes(out, key_width, value_width, page_size, key_strides, value_strides, scale, softcap, rows_in_order) -> bool:
+def _rows_tc5_takes(out, value_heads, maps, key_width, value_width, page_size, key_strides, value_strides, scale, softcap,
+                    rows_in_order) -> bool:
     """Whether the tcgen05 kernel for prompt portions takes this call (of those that ``flash_dims_supported``): keys of 128
     or 192 entries, values of a multiple of 128, both in rows that lie one behind the other, no cap on the scores, a
     positive scale (it takes the largest score ahead of scaling)."""
@@ -1337,7 +1338,8 @@ def _rows_tc5_takes(out, key_width, value_width, page_size, key_strides, value_s
           or key_strides[0] != page_size * pitch or value_strides[0] != page_size * pitch):
         return False
     wide = 4 if out.dtype == torch.float32 else 8
-    return (max(key_strides[1], value_strides[1]) < 1 << 31 and out.data_ptr() % 16 == 0
+    # a head's first column is a coordinate of the copy: 31 bits
+    return (max(value_heads * maps * key_strides[1], value_heads * value_strides[1]) < 1 << 31 and out.data_ptr() % 16 == 0
             and out.stride(0) % wide == 0 and out.stride(1) % wide == 0)
 
 
@@ -1355,8 +1357,8 @@ def _flash_dims(out, q, keys, values, table, ctx, value_heads, group, maps, key_
         if 0 < long_count < ctx.num_reqs and all(n * group > 32 for n in lens[:long_count]):
             runs = [(_RequestRun(ctx, begin, end), table[begin:end])
                     for begin, end in ((0, long_count), (long_count, ctx.num_reqs))]
-    tc5 = num_splits is None and _rows_tc5_takes(out, key_width, value_width, page_size, key_strides, value_strides, scale,
-                                                 softcap, rows_in_order)
+    tc5 = num_splits is None and _rows_tc5_takes(out, value_heads, maps, key_width, value_width, page_size, key_strides,
+                                                 value_strides, scale, softcap, rows_in_order)
     for run, run_table in runs:
         max_rows = run.max_query_len * group
         if tc5 and max_rows > 32:            # beyond the few-row form, at any length (from 40 rows behind 2,000 keys: 79 us, 188)

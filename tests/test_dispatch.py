@@ -1,0 +1,32 @@
+"""Rules that send a call to one kernel or another, checked without a GPU."""
+from __future__ import annotations
+
+import torch
+
+from kvcore_b200.kernels import api
+
+
+def test_which_calls_the_tcgen05_kernel_over_rows_takes():
+    """Keys and values in rows one behind the other, a positive scale, no cap, columns within 31 bits; everything else is left
+    to the kernel that took it before."""
+    width, page = 8 * 256, 16
+    strides = (page * width, 128, width)
+
+    def takes(dtype=torch.bfloat16, offset=0, **change):
+        out = torch.empty(10 * 8 * 128 + 8, dtype=dtype)[offset:offset + 10 * 8 * 128].view(10, 8, 128)
+        call = dict(value_heads=8, maps=1, key_width=128, value_width=128, page_size=page, key_strides=strides,
+                    value_strides=strides, scale=0.1, softcap=None, rows_in_order=False)
+        return api._rows_tc5_takes(out, **dict(call, **change))
+    in_order = dict(page_size=1, key_strides=(width, 128, 0), value_strides=(width, 128, 0), rows_in_order=True)
+    assert takes() and takes(torch.float32) and takes(**in_order) and takes(key_width=192)
+    for scale in (0.0, -0.1, float("nan")):
+        assert not takes(scale=scale)
+    assert not takes(softcap=5.0) and not takes(offset=1)
+    for change in (dict(key_width=64), dict(key_width=256), dict(value_width=192), dict(page_size=4), dict(page_size=128),
+                   dict(value_strides=(page * width, 128, width + 8)), dict(key_strides=(page * width + 8, 128, width)),
+                   dict(key_strides=(page * width, 128, 0)), dict(key_strides=(page * width, 1 << 28, width)),
+                   dict(value_strides=(page * width, 1 << 28, width)), dict(maps=2, key_strides=(page * width, 1 << 27, width))):
+        assert not takes(**change), change
+    for change in (dict(page_size=16), dict(value_strides=(width + 8, 128, 0)), dict(key_strides=(0, 128, 0), value_strides=(0, 128, 0))):
+        assert not takes(**dict(in_order, **change)), change
+    assert takes(key_strides=(page * width, (1 << 28) - 8, width))
