@@ -11,7 +11,8 @@
 //     that start anew with every segment; an output entry is one accumulator over the segment's keys
 //     in ascending order, scaled down when the maximum grows;
 //   * segments are added to the row's result one after the other (`Folded`).
-// A key the row does not see has probability zero, and a chunk without visible keys changes nothing.
+// A key the row does not see has no part in any of it, whatever its value holds (a later token's may be no number): in
+// chunks that not every row sees whole, an entry's sum passes over the keys that its row does not see.
 //
 // Two kernels do exactly that:
 //   attention_tile: 64 rows of one request and kv head a block (portions of prompts).  Keys and values
@@ -85,19 +86,23 @@ __device__ __forceinline__ float4 att_load4(const bf16* p, int valid, int vec) {
                      valid > 3 ? to_float(p[3]) : 0.0f);
 }
 
+// Where some row of a block does not see a whole chunk, this stands for the probability of a key that its row does not see.
+#define ATT_UNSEEN -1.0f
+
 // What both kernels share: the rows' positions, which keys any of them sees, and the chunk in shared memory.
 template <typename T>
 struct AttBlock {
   const AttParams<T>& p;
   int req, kvh, G, begin, rows, row0;      // rows of this block: row0 .. row0 + rows - 1 of the request's
   int lo, hi, kept;                        // keys some row sees: [0, kept) and [lo, hi)
+  int all_lo, all_hi;                      // keys every row sees: [all_lo, all_hi)
   long long head_off, page_elems;
 
   __device__ __forceinline__ int position(int r) const { return p.positions[begin + (row0 + r) / G]; }
   __device__ __forceinline__ int first_of(int pos) const { return p.window > 0 ? max(0, pos - p.window + 1) : 0; }
   // all threads; `pos` [rows] in shared memory is filled, barrier included
   __device__ __forceinline__ void look(int* pos, int* ends) {
-    if (threadIdx.x == 0) { ends[0] = 0x7fffffff; ends[1] = 0; ends[2] = 0; }
+    if (threadIdx.x == 0) { ends[0] = ends[4] = 0x7fffffff; ends[1] = ends[2] = ends[3] = 0; }
     __syncthreads();
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
       const int at = position(r), first = first_of(at);
@@ -105,10 +110,13 @@ struct AttBlock {
       atomicMin(&ends[0], first);
       atomicMax(&ends[1], at + 1);
       atomicMax(&ends[2], min(p.keep_first, first));
+      atomicMax(&ends[3], first);
+      atomicMin(&ends[4], at + 1);
     }
     __syncthreads();
-    lo = ends[0]; hi = ends[1]; kept = ends[2];
+    lo = ends[0]; hi = ends[1]; kept = ends[2]; all_lo = ends[3]; all_hi = ends[4];
   }
+  __device__ __forceinline__ bool ragged(int base) const { return base < all_lo || base + ATT_CHUNK > all_hi; }
   __device__ __forceinline__ bool wanted(int key) const { return (key >= lo && key < hi) || key < kept; }
   __device__ __forceinline__ bool chunk_wanted(int base) const {
     return (base + ATT_CHUNK > lo && base < hi) || base < kept;
@@ -181,9 +189,9 @@ attention_tile_kernel(AttParams<T> p) {
   float* const vs = ks + ATT_CHUNK * LK;                             // [ATT_CHUNK][DV]
   float* const ss = vs + ATT_CHUNK * DV;                             // [ATT_CHUNK][ATT_LS]: scores, then probabilities
   __shared__ long long offset[ATT_CHUNK];
-  __shared__ int pos[ATT_ROWS], ends[3];
+  __shared__ int pos[ATT_ROWS], ends[5];
   __shared__ float factor[ATT_ROWS], run_m[ATT_ROWS], run_l[ATT_ROWS];
-  AttBlock<T> b{p, req, kvh, G, begin, min(ATT_ROWS, all_rows - row0), row0, 0, 0, 0,
+  AttBlock<T> b{p, req, kvh, G, begin, min(ATT_ROWS, all_rows - row0), row0, 0, 0, 0, 0, 0,
                 (long long)kvh * p.page_size * p.D, (long long)p.KVH * p.page_size * p.D};
   b.look(pos, ends);
   b.fetch_queries(qs, LK, DK);
@@ -258,6 +266,13 @@ attention_tile_kernel(AttParams<T> p) {
         __syncwarp();
         if (lane == 0) { run_m[r] = m; run_l[r] = l; factor[r] = f; }
       }
+      const bool ragged = b.ragged(base);
+      if (ragged)
+        for (int n = 0; n < ATT_ROWS / 8; ++n) {
+          const int r = warp * (ATT_ROWS / 8) + n;
+          if (!b.seen(base + lane, pos[r])) ss[lane * ATT_LS + r] = ATT_UNSEEN;
+          if (!b.seen(base + lane + 32, pos[r])) ss[(lane + 32) * ATT_LS + r] = ATT_UNSEEN;
+        }
       __syncthreads();
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -265,8 +280,7 @@ attention_tile_kernel(AttParams<T> p) {
 #pragma unroll
         for (int j = 0; j < 4 * NJ; ++j) acc[i][j] *= f;
       }
-#pragma unroll 4
-      for (int key = 0; key < ATT_CHUNK; ++key) {
+      auto add_key = [&](int key, bool some) {                       // `some`: only to the rows that see the key
         const float4 pr = *reinterpret_cast<const float4*>(ss + key * ATT_LS + ty * 4);
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
@@ -274,12 +288,21 @@ attention_tile_kernel(AttParams<T> p) {
           const float w[4] = {pr.x, pr.y, pr.z, pr.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
+            if (some && w[i] == ATT_UNSEEN) continue;
             acc[i][4 * j] = fmaf(w[i], v.x, acc[i][4 * j]);
             acc[i][4 * j + 1] = fmaf(w[i], v.y, acc[i][4 * j + 1]);
             acc[i][4 * j + 2] = fmaf(w[i], v.z, acc[i][4 * j + 2]);
             acc[i][4 * j + 3] = fmaf(w[i], v.w, acc[i][4 * j + 3]);
           }
         }
+      };
+      if (ragged) {
+        const int keys = min(ATT_CHUNK, max(b.hi, b.kept) - base);
+#pragma unroll 4
+        for (int key = 0; key < keys; ++key) add_key(key, true);
+      } else {
+#pragma unroll 4
+        for (int key = 0; key < ATT_CHUNK; ++key) add_key(key, false);
       }
     }
     if (!any) continue;
@@ -325,9 +348,9 @@ attention_few_kernel(AttParams<T> p) {
   float* const ks = qs + ATT_FEW * LK;                               // [ATT_CHUNK][LK]
   float* const vs = ks + ATT_CHUNK * LK;                             // [ATT_CHUNK][DV]
   __shared__ long long offset[ATT_CHUNK];
-  __shared__ int pos[ATT_FEW], ends[3];
+  __shared__ int pos[ATT_FEW], ends[5];
   __shared__ float probability[ATT_FEW][ATT_CHUNK];
-  AttBlock<T> b{p, req, kvh, G, begin, all_rows, 0, 0, 0, 0,
+  AttBlock<T> b{p, req, kvh, G, begin, all_rows, 0, 0, 0, 0, 0, 0,
                 (long long)kvh * p.page_size * p.D, (long long)p.KVH * p.page_size * p.D};
   b.look(pos, ends);
   b.fetch_queries(qs, LK, DK);
@@ -356,7 +379,12 @@ attention_few_kernel(AttParams<T> p) {
     }
     s0 = offset[lane] >= 0 && b.seen(base + lane, pos[r]) ? __fmul_rn(s0, p.scale) : -INFINITY;
     s1 = offset[lane + 32] >= 0 && b.seen(base + lane + 32, pos[r]) ? __fmul_rn(s1, p.scale) : -INFINITY;
+    const bool ragged = b.ragged(base);
     const float f = att_softmax(s0, s1, m, l);
+    if (ragged) {
+      if (!b.seen(base + lane, pos[r])) s0 = ATT_UNSEEN;
+      if (!b.seen(base + lane + 32, pos[r])) s1 = ATT_UNSEEN;
+    }
     probability[r][lane] = s0;
     probability[r][lane + 32] = s1;
     __syncwarp();
@@ -367,6 +395,7 @@ attention_few_kernel(AttParams<T> p) {
 #pragma unroll 8
     for (int key = 0; key < ATT_CHUNK; ++key) {
       const float w = probability[r][key];
+      if (ragged && w == ATT_UNSEEN) continue;                       // the whole warp: a row
 #pragma unroll
       for (int j = 0; j < RUNS; ++j) {
         const int d = j * 128 + lane * 4;

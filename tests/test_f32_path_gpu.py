@@ -54,3 +54,38 @@ def test_attention_rows_have_the_same_bits_in_every_kernel(dtype, heads, kv_head
         torch.testing.assert_close(whole, want, **(dict(rtol=2e-5, atol=2e-5) if dtype == torch.float32
                                                    else dict(rtol=2e-2, atol=2e-2)))
     assert K().read_status() == 0
+
+
+def _attention(dtype, heads, kv_heads, dim, page, lens, window=None, keep=0, seed=1):
+    """A batch for the general attention kernels, and the call on caches of the caller's."""
+    case = _cache_case(dtype, heads, kv_heads, dim, page, lens, seed=seed)
+
+    def attend(k_cache, v_cache, qkv=case["qkv"]):
+        return K().paged_attention(qkv, k_cache, v_cache, case["table"], _Ctx(case), heads, kv_heads, dim, dim ** -0.5, window,
+                                   keep_first=keep, force_general=True)
+    return case, attend
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("window,keep", [(None, 0), (40, 0), (70, 9)])
+def test_values_a_row_does_not_see_do_not_count(dtype, value, window, keep):
+    """Keys and values of one position hold no number: rows in front of it, and rows whose window lies behind it, keep their
+    bits, rows that see it do not hide it.  A prompt (tiles of 64 rows), its last 2 tokens (a block a segment), and
+    what the pages hold behind the last position."""
+    heads, kv_heads, dim, page, total = 6, 2, 40, 16, 333
+    for first, count in ((0, total), (total - 2, 2)):
+        case, attend = _attention(dtype, heads, kv_heads, dim, page, [(first, count)], window, keep)
+        want = attend(case["k_cache"], case["v_cache"])
+        position = torch.arange(first, first + count, device=DEV)
+        for at in (0, 7, 100, 255, 256, 300, total - 2, total - 1, total + 1):
+            planes = [case["k_cache"].clone(), case["v_cache"].clone()]
+            for plane in planes[1:] if value == float("inf") else planes:
+                plane[int(case["table"][0, at // page]), :, at % page] = value
+            got = attend(*planes)
+            sees = position >= at
+            if window is not None:
+                sees &= (position - window < at) | (at < keep)
+            assert torch.equal(got[~sees], want[~sees]), at
+            assert (~torch.isfinite(got[sees].float())).all(), at
+    assert K().read_status() == 0
