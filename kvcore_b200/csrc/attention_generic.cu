@@ -51,7 +51,9 @@ struct AttParams {
 struct Folded {
   float M, L;
   float a_factor, s_factor;
-  __device__ __forceinline__ void fold(float m, float l) {           // m is finite: the segment holds a visible key
+  // l is not zero: the segment holds a visible key.  (Where every score is NaN, m is still -INFINITY, l is NaN, and so
+  // are the factors and the result.)
+  __device__ __forceinline__ void fold(float m, float l) {
     const float top = fmaxf(M, m);
     a_factor = M == -INFINITY ? 0.0f : expf(M - top);
     s_factor = expf(m - top);
@@ -308,9 +310,9 @@ attention_tile_kernel(AttParams<T> p) {
     if (!any) continue;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float m = run_m[ty * 4 + i];
-      if (m == -INFINITY) continue;
-      total[i].fold(m, run_l[ty * 4 + i]);
+      const float l = run_l[ty * 4 + i];
+      if (l == 0.0f) continue;
+      total[i].fold(run_m[ty * 4 + i], l);
 #pragma unroll
       for (int j = 0; j < 4 * NJ; ++j)
         sum[i][j] = fmaf(acc[i][j], total[i].s_factor, __fmul_rn(sum[i][j], total[i].a_factor));
@@ -418,7 +420,7 @@ attention_few_kernel(AttParams<T> p) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int d = j * 128 + lane * 4 + c;
-        if (d < p.D && m != -INFINITY) part[d] = acc[j][c];
+        if (d < p.D && l != 0.0f) part[d] = acc[j][c];
       }
     if (lane == 0) { part[p.D] = m; part[p.D + 1] = l; }
     return;
@@ -451,9 +453,9 @@ attention_fold_kernel(AttParams<T> p) {
   const int last = min(p.segments - 1, p.positions[begin + r / G] / ATT_SEGMENT);
   for (int s = 0; s <= last; ++s) {
     const float* part = p.partial + (((size_t)blockIdx.x * p.segments + s) * p.part_rows + r) * (p.D + 2);
-    const float m = part[p.D];
-    if (m == -INFINITY) continue;
-    total.fold(m, part[p.D + 1]);
+    const float l = part[p.D + 1];
+    if (l == 0.0f) continue;
+    total.fold(part[p.D], l);
 #pragma unroll
     for (int j = 0; j < MOST; ++j)
       if (lane + 32 * j < p.D) sum[j] = fmaf(part[lane + 32 * j], total.s_factor, __fmul_rn(sum[j], total.a_factor));

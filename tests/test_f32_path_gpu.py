@@ -89,3 +89,16 @@ def test_values_a_row_does_not_see_do_not_count(dtype, value, window, keep):
             assert torch.equal(got[~sees], want[~sees]), at
             assert (~torch.isfinite(got[sees].float())).all(), at
     assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_query_that_is_no_number_is_not_hidden(dtype):
+    """All of a row's scores are NaN, in one segment or several: so is its result, as that of plain attention."""
+    for lens in ([(0, 70)], [(0, 300)], [(700, 1)], [(100, 1)]):
+        case, attend = _attention(dtype, 4, 2, 64, 16, lens)
+        qkv = case["qkv"].clone()
+        qkv[-1, 64:128] = float("nan")                # the last token's second head
+        got, want = attend(case["k_cache"], case["v_cache"], qkv), attend(case["k_cache"], case["v_cache"])
+        assert got[-1, 64:128].isnan().all()
+        got[-1, 64:128] = want[-1, 64:128]
+        assert torch.equal(got, want)
