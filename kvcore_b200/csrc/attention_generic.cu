@@ -41,8 +41,9 @@ struct AttParams {
   T* out; const T* q; const T* k_cache; const T* v_cache;
   const int* table; const int* positions; const int* query_start;
   int out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages, window, keep_first, vec, segments, reqs, part_rows;
+  int head0;                 // the first (request, kv head) of this launch of attention_few and of the fold behind it
   float scale;
-  float* partial;            // [reqs, KVH, segments, part_rows, D + 2]: accumulators, maximum, sum
+  float* partial;            // [(request, kv head) of a launch, segments, part_rows, D + 2]: accumulators, maximum, sum
   int* status;
 };
 
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(ATT_THREADS)
 attention_few_kernel(AttParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
   // blocks: the segments of a (request, kv head) next to one another
-  const int head = blockIdx.x / p.segments, part_no = blockIdx.x % p.segments;
+  const int head = p.head0 + blockIdx.x / p.segments, part_no = blockIdx.x % p.segments;
   const int req = head / p.KVH, kvh = head % p.KVH, G = p.H / p.KVH;
   const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
   if (all_rows > ATT_FEW || all_rows == 0) return;
@@ -441,7 +442,7 @@ template <typename T>
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_fold_kernel(AttParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
-  const int req = blockIdx.x / p.KVH, kvh = blockIdx.x % p.KVH, G = p.H / p.KVH;
+  const int head = p.head0 + blockIdx.x, req = head / p.KVH, kvh = head % p.KVH, G = p.H / p.KVH;
   const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
   const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (all_rows > ATT_FEW || r >= all_rows) return;
@@ -467,6 +468,21 @@ attention_fold_kernel(AttParams<T> p) {
     if (lane + 32 * j < p.D) to[lane + 32 * j] = from_float<T>(sum[j] * inv);
 }
 
+// A row of the scratch for each row that a segment's block can have (one for decoded tokens of ungrouped heads).
+static int part_rows_of(int H, int KVH, int max_query_len) {
+  const long long most = (long long)max_query_len * (H / KVH);
+  return most < ATT_FEW ? (int)most : ATT_FEW;
+}
+// (Request, kv head) pairs that attention_few takes a launch: all of them, or as many as the scratch's bound has room for
+// (the blocks of one launch fill the GPU many times over by then; one long context beside many short ones asks for as much
+// as if all were long).
+#define ATT_SCRATCH_FLOATS (16 << 20)
+static long long heads_a_launch(long long heads, int D, int part_rows, int segments) {
+  if (segments <= 1 || part_rows <= 0) return heads;
+  const long long fit = ATT_SCRATCH_FLOATS / ((long long)segments * part_rows * (D + 2));
+  return heads <= fit ? heads : fit < 1 ? 1 : fit;
+}
+
 template <typename T, int NJ>
 static int launch_attention(AttParams<T> p, int tokens, int reqs, int max_query_len, cudaStream_t stream) {
   const int G = p.H / p.KVH, most = max_query_len * G, LK = ((p.D + 3) & ~3) + 4, DV = 64 * NJ;
@@ -481,10 +497,14 @@ static int launch_attention(AttParams<T> p, int tokens, int reqs, int max_query_
   if (G <= ATT_FEW && (most <= ATT_FEW || !equal)) {
     const int smem = (int)sizeof(float) * (ATT_FEW * LK + ATT_CHUNK * (LK + DV));
     KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_few_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3((unsigned)((long long)reqs * p.KVH * p.segments)), dim3(ATT_THREADS), smem, stream,
-                              true, p));
-    if (p.segments > 1)
-      KVB_CHECK_CUDA(kvb_launch((attention_fold_kernel<T>), dim3(reqs * p.KVH), dim3(ATT_THREADS), 0, stream, true, p));
+    const long long heads = (long long)reqs * p.KVH, lot = heads_a_launch(heads, p.D, p.part_rows, p.segments);
+    for (long long head0 = 0; head0 < heads; head0 += lot) {         // one behind the other: the scratch is the same
+      const unsigned here = (unsigned)(heads - head0 < lot ? heads - head0 : lot);
+      p.head0 = (int)head0;
+      KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3(here * p.segments), dim3(ATT_THREADS), smem, stream, true, p));
+      if (p.segments > 1)
+        KVB_CHECK_CUDA(kvb_launch((attention_fold_kernel<T>), dim3(here), dim3(ATT_THREADS), 0, stream, true, p));
+    }
   }
   KVB_CHECK_LAUNCH();
   return 0;
@@ -497,14 +517,15 @@ static int attention_of(const AttParams<T>& p, int tokens, int reqs, int max_que
   return launch_attention<T, 4>(p, tokens, reqs, max_query_len, stream);
 }
 
-// Floats of the scratch that a batch takes whose longest request has `segments` segments of cached tokens: a row of it
-// for each row that a segment's block can have (one for decoded tokens of ungrouped heads).
-static int part_rows_of(int H, int KVH, int max_query_len) {
-  const long long most = (long long)max_query_len * (H / KVH);
-  return most < ATT_FEW ? (int)most : ATT_FEW;
-}
+// Floats of the scratch that a batch takes whose longest request has `segments` segments of cached tokens, and how many
+// times attention_few is launched for it.
 extern "C" long long kvb_paged_attention_scratch(int num_reqs, int H, int KVH, int D, int max_query_len, int segments) {
-  return segments > 1 ? (long long)num_reqs * KVH * segments * part_rows_of(H, KVH, max_query_len) * (D + 2) : 0;
+  const int rows = part_rows_of(H, KVH, max_query_len);
+  return segments > 1 ? heads_a_launch((long long)num_reqs * KVH, D, rows, segments) * segments * rows * (D + 2) : 0;
+}
+extern "C" int kvb_paged_attention_lots(int num_reqs, int H, int KVH, int D, int max_query_len, int segments) {
+  const long long heads = (long long)num_reqs * KVH, lot = heads_a_launch(heads, D, part_rows_of(H, KVH, max_query_len), segments);
+  return lot > 0 ? (int)((heads + lot - 1) / lot) : 0;
 }
 extern "C" int kvb_paged_attention_segment() { return ATT_SEGMENT; }
 
@@ -531,7 +552,7 @@ extern "C" int kvb_paged_attention_rows(void* out, int out_stride, const void* q
 #define KVB_ATT(T_)                                                                                                    \
   attention_of<T_>(AttParams<T_>{(T_*)out, (const T_*)q, (const T_*)k_cache, (const T_*)v_cache, table, positions,     \
                                  query_start, out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages,     \
-                                 window, keep_first, vec, segments, num_reqs, part_rows_of(H, KVH, max_query_len),     \
+                                 window, keep_first, vec, segments, num_reqs, part_rows_of(H, KVH, max_query_len), 0,  \
                                  scale, partial, status},                                                              \
                    tokens, num_reqs, max_query_len, stream)
   return dtype == KVB_F32 ? KVB_ATT(float) : KVB_ATT(bf16);

@@ -102,3 +102,25 @@ def test_a_query_that_is_no_number_is_not_hidden(dtype):
         assert got[-1, 64:128].isnan().all()
         got[-1, 64:128] = want[-1, 64:128]
         assert torch.equal(got, want)
+
+
+def test_scratch_of_few_rows_is_bounded():
+    """One long context beside many short ones: the scratch is bounded, whatever the longest asks for, and requests that are
+    taken in several lots have the bits they have alone."""
+    heads, kv_heads, dim, page = 16, 8, 64, 16
+    lens = [(60000, 1)] + [(50 + 7 * i, 1) for i in range(99)]
+    case, attend = _attention(torch.float32, heads, kv_heads, dim, page, lens)
+    attend(case["k_cache"], case["v_cache"])
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got = attend(case["k_cache"], case["v_cache"])
+    assert torch.cuda.max_memory_allocated() - before <= (64 << 20) + 2 * got.nbytes
+    for row in (0, 1, 37, 99):
+        part = dict(case, positions=case["positions"][row:row + 1], lens=[lens[row]], req_index=case["req_index"][:1],
+                    query_start=case["query_start"][:2], context_lens=case["context_lens"][row:row + 1])
+        alone = K().paged_attention(case["qkv"][row:row + 1], case["k_cache"], case["v_cache"], case["table"][row:row + 1],
+                                    _Ctx(part), heads, kv_heads, dim, dim ** -0.5, None)
+        assert torch.equal(alone, got[row:row + 1])
+    assert K().read_status() == 0
