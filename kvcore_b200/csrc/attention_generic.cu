@@ -92,7 +92,7 @@ __device__ __forceinline__ float4 att_load4(const bf16* p, int valid, int vec) {
 // Where some row of a block does not see a whole chunk, this stands for the probability of a key that its row does not see.
 #define ATT_UNSEEN -1.0f
 
-// What both kernels share: the rows' positions, which keys any of them sees, and the chunk in shared memory.
+// What both kernels share: which keys the rows see, and the chunk in shared memory.
 template <typename T>
 struct AttBlock {
   const AttParams<T>& p;
@@ -128,25 +128,21 @@ struct AttBlock {
     const int first = first_of(pos);
     return key <= pos && (key >= first || key < min(p.keep_first, first));
   }
-  // Offsets of the chunk's keys in the cache (-1: nobody's, or a bad page, which is reported); barrier included.
-  __device__ __forceinline__ void find(int base, long long* offset) {
-    if (threadIdx.x < ATT_CHUNK) {
-      const int key = base + threadIdx.x;
-      long long at = -1;
-      if (wanted(key)) {
-        const int page = p.table[(size_t)req * p.table_stride + key / p.page_size];
-        if (page <= 0 || page >= p.num_pages) atomicOr(p.status, KVB_STATUS_BAD_PAGE);
-        else at = (long long)page * page_elems + head_off + (long long)(key % p.page_size) * p.D;
-      }
-      offset[threadIdx.x] = at;
-    }
-    __syncthreads();
+  // Offset of a key in the cache (-1: nobody's, or a bad page, which is reported).
+  __device__ __forceinline__ long long find(int key) const {
+    if (!wanted(key)) return -1;
+    const int page = p.table[(size_t)req * p.table_stride + key / p.page_size];
+    if (page > 0 && page < p.num_pages) return (long long)page * page_elems + head_off + (long long)(key % p.page_size) * p.D;
+    atomicOr(p.status, KVB_STATUS_BAD_PAGE);
+    return -1;
   }
-  // Rows of a plane's chunk into shared memory as floats, `width` (a multiple of four) a row, zeros behind D.
-  __device__ __forceinline__ void fetch(float* dst, int stride, int width, const T* plane, const long long* offset) {
+  // Keys of a chunk up to the last that somebody sees (what shared memory holds behind them counts for nothing).
+  __device__ __forceinline__ int keys_of(int base) const { return min(ATT_CHUNK, max(hi, kept) - base); }
+  // `keys` rows of a plane's chunk into shared memory as floats, `width` (a multiple of four) a row, zeros behind D.
+  __device__ __forceinline__ void fetch(float* dst, int stride, int width, const T* plane, const long long* offset, int keys) {
     const int pieces = width >> 2;
 #pragma unroll 8
-    for (int e = threadIdx.x; e < ATT_CHUNK * pieces; e += ATT_THREADS) {
+    for (int e = threadIdx.x; e < keys * pieces; e += ATT_THREADS) {
       const int key = e / pieces, d = (e - key * pieces) << 2;
       const long long at = offset[key];
       float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -222,9 +218,11 @@ attention_tile_kernel(AttParams<T> p) {
       if (!any)
         for (int r = threadIdx.x; r < ATT_ROWS; r += ATT_THREADS) { run_m[r] = -INFINITY; run_l[r] = 0.0f; }
       any = true;
-      b.find(base, offset);
-      b.fetch(ks, LK, DK, p.k_cache, offset);
-      b.fetch(vs, DV, DV, p.v_cache, offset);
+      if (threadIdx.x < ATT_CHUNK) offset[threadIdx.x] = b.find(base + threadIdx.x);
+      __syncthreads();
+      const int keys = b.keys_of(base);
+      b.fetch(ks, LK, DK, p.k_cache, offset, keys);
+      b.fetch(vs, DV, DV, p.v_cache, offset, keys);
       __syncthreads();
       float s[4][4];
 #pragma unroll
@@ -300,7 +298,6 @@ attention_tile_kernel(AttParams<T> p) {
         }
       };
       if (ragged) {
-        const int keys = min(ATT_CHUNK, max(b.hi, b.kept) - base);
 #pragma unroll 4
         for (int key = 0; key < keys; ++key) add_key(key, true);
       } else {
@@ -344,6 +341,13 @@ attention_few_kernel(AttParams<T> p) {
   const int req = head / p.KVH, kvh = head % p.KVH, G = p.H / p.KVH;
   const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
   if (all_rows > ATT_FEW || all_rows == 0) return;
+  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;           // a warp a row
+  const bool live = r < all_rows;
+  const int segment = part_no * ATT_SEGMENT;
+  // every warp looks the rows up for itself, a lane a row
+  const int at = lane < all_rows ? p.positions[begin + lane / G] : -1, mine = __shfl_sync(0xffffffffu, at, live ? r : 0);
+  const int last = __reduce_max_sync(0xffffffffu, at);
+  if (segment > last) return;              // a longer request's segment (the fold does not read what was not written)
   extern __shared__ __align__(16) float smem[];
   const int DK = (p.D + 3) & ~3, LK = DK + 4;
   constexpr int DV = 64 * NJ, RUNS = (NJ + 1) / 2;                   // a lane's quads of output columns: 128 apart
@@ -351,24 +355,32 @@ attention_few_kernel(AttParams<T> p) {
   float* const ks = qs + ATT_FEW * LK;                               // [ATT_CHUNK][LK]
   float* const vs = ks + ATT_CHUNK * LK;                             // [ATT_CHUNK][DV]
   __shared__ long long offset[ATT_CHUNK];
-  __shared__ int pos[ATT_FEW], ends[5];
   __shared__ float probability[ATT_FEW][ATT_CHUNK];
   AttBlock<T> b{p, req, kvh, G, begin, all_rows, 0, 0, 0, 0, 0, 0,
                 (long long)kvh * p.page_size * p.D, (long long)p.KVH * p.page_size * p.D};
-  b.look(pos, ends);
-  b.fetch_queries(qs, LK, DK);
-  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;           // a warp a row
-  const bool live = r < all_rows;
-  const int segment = part_no * ATT_SEGMENT;
+  {
+    const int first = b.first_of(at);
+    b.lo = __reduce_min_sync(0xffffffffu, at < 0 ? 0x7fffffff : first);
+    b.hi = last + 1;
+    b.kept = __reduce_max_sync(0xffffffffu, at < 0 ? 0 : min(p.keep_first, first));
+    b.all_lo = b.first_of(mine);           // all the rows of a warp: one
+    b.all_hi = mine + 1;
+  }
+  bool any = false;
   float acc[RUNS][4], m = -INFINITY, l = 0.0f;
 #pragma unroll
   for (int j = 0; j < RUNS; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
   for (int base = segment; base < segment + ATT_SEGMENT; base += ATT_CHUNK) {
     if (!b.chunk_wanted(base)) continue;
-    __syncthreads();                                                 // the chunk in front has been read
-    b.find(base, offset);
-    b.fetch(ks, LK, DK, p.k_cache, offset);
-    b.fetch(vs, DV, DV, p.v_cache, offset);
+    const long long found = threadIdx.x < ATT_CHUNK ? b.find(base + threadIdx.x) : -1;
+    if (any) __syncthreads();                                        // the chunk in front has been read
+    else b.fetch_queries(qs, LK, DK);
+    any = true;
+    if (threadIdx.x < ATT_CHUNK) offset[threadIdx.x] = found;
+    __syncthreads();
+    const int keys = b.keys_of(base);
+    b.fetch(ks, LK, DK, p.k_cache, offset, keys);
+    b.fetch(vs, DV, DV, p.v_cache, offset, keys);
     __syncthreads();
     if (!live) continue;
     float s0 = 0.0f, s1 = 0.0f;
@@ -380,14 +392,12 @@ attention_few_kernel(AttParams<T> p) {
       s0 = fmaf(a.x, q.x, s0); s0 = fmaf(a.y, q.y, s0); s0 = fmaf(a.z, q.z, s0); s0 = fmaf(a.w, q.w, s0);
       s1 = fmaf(c.x, q.x, s1); s1 = fmaf(c.y, q.y, s1); s1 = fmaf(c.z, q.z, s1); s1 = fmaf(c.w, q.w, s1);
     }
-    s0 = offset[lane] >= 0 && b.seen(base + lane, pos[r]) ? __fmul_rn(s0, p.scale) : -INFINITY;
-    s1 = offset[lane + 32] >= 0 && b.seen(base + lane + 32, pos[r]) ? __fmul_rn(s1, p.scale) : -INFINITY;
-    const bool ragged = b.ragged(base);
+    const bool sees0 = b.seen(base + lane, mine), sees1 = b.seen(base + lane + 32, mine);
+    s0 = offset[lane] >= 0 && sees0 ? __fmul_rn(s0, p.scale) : -INFINITY;
+    s1 = offset[lane + 32] >= 0 && sees1 ? __fmul_rn(s1, p.scale) : -INFINITY;
     const float f = att_softmax(s0, s1, m, l);
-    if (ragged) {
-      if (!b.seen(base + lane, pos[r])) s0 = ATT_UNSEEN;
-      if (!b.seen(base + lane + 32, pos[r])) s1 = ATT_UNSEEN;
-    }
+    if (!sees0) s0 = ATT_UNSEEN;
+    if (!sees1) s1 = ATT_UNSEEN;
     probability[r][lane] = s0;
     probability[r][lane + 32] = s1;
     __syncwarp();
@@ -395,10 +405,9 @@ attention_few_kernel(AttParams<T> p) {
     for (int j = 0; j < RUNS; ++j)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[j][c] *= f;
-#pragma unroll 8
-    for (int key = 0; key < ATT_CHUNK; ++key) {
+    auto add_key = [&](int key, bool some) {                         // `some`: not if the row does not see the key
       const float w = probability[r][key];
-      if (ragged && w == ATT_UNSEEN) continue;                       // the whole warp: a row
+      if (some && w == ATT_UNSEEN) return;
 #pragma unroll
       for (int j = 0; j < RUNS; ++j) {
         const int d = j * 128 + lane * 4;
@@ -410,6 +419,12 @@ attention_few_kernel(AttParams<T> p) {
           acc[j][3] = fmaf(w, v.w, acc[j][3]);
         }
       }
+    };
+    if (b.ragged(base)) {
+      for (int key = 0; key < keys; ++key) add_key(key, true);
+    } else {
+#pragma unroll 8
+      for (int key = 0; key < ATT_CHUNK; ++key) add_key(key, false);
     }
     __syncwarp();                                                    // the probabilities have been read
   }
