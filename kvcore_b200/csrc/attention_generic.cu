@@ -18,9 +18,10 @@
 //   attention_tile: 64 rows of one request and kv head a block (portions of prompts).  Keys and values
 //     of a chunk lie in shared memory and serve all rows, 4 x 4 scores and 4 x 4 NJ outputs a thread.
 //     Bound by the FMA units and the shared-memory reads that feed them.
-//   attention_few: at most 8 rows (decoded tokens), a warp a row; the segments of a request go to
-//     different blocks and a third kernel folds them.  Bound by the reading of keys and values.
-// Which one takes a request follows its rows (new tokens times query heads a kv head): a tile of 64 rows
+//   attention_few: 8 rows a block, a warp a row.  At most 8 rows (decoded tokens): the segments of a request go to
+//     different blocks and a third kernel folds them; bound by the reading of keys and values.  A short portion of a
+//     prompt within the first segment: its rows go to different blocks; bound by the latency of its few loads.
+// Which one takes a request (att_request) follows its rows (new tokens times query heads a kv head): a tile of 64 rows
 // costs its 64 rows' arithmetic however few there are.  24 heads of 128 over 8 kv heads, a portion of 250
 // tokens beside 6 decoded ones behind 750 to 1,000 cached: 82 us (tiles) and 61 us (few and folding); a warp
 // a row walking its keys alone, which these kernels took the place of, needed 926 us.
@@ -34,6 +35,7 @@
 #define ATT_SEGMENT 256
 #define ATT_ROWS 64
 #define ATT_FEW 8
+#define ATT_FEW_TOKENS 32      // of a short portion: one lane each
 #define ATT_LS (ATT_ROWS + 4)
 
 template <typename T>
@@ -41,6 +43,7 @@ struct AttParams {
   T* out; const T* q; const T* k_cache; const T* v_cache;
   const int* table; const int* positions; const int* query_start;
   int out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages, window, keep_first, vec, segments, reqs, part_rows;
+  int parts;                 // blocks of attention_few a (request, kv head)
   int head0;                 // the first (request, kv head) of this launch of attention_few and of the fold behind it
   float scale;
   float* partial;            // [(request, kv head) of a launch, segments, part_rows, D + 2]: accumulators, maximum, sum
@@ -91,6 +94,22 @@ __device__ __forceinline__ float4 att_load4(const bf16* p, int valid, int vec) {
 
 // Where some row of a block does not see a whole chunk, this stands for the probability of a key that its row does not see.
 #define ATT_UNSEEN -1.0f
+
+// A request's new tokens, rows a kv head and last position, and which kernel takes it.  By all threads of a warp.
+// A portion of 3, 9, 16 and 32 tokens without cached ones, 24 heads of 128 over 8 (B200, call by call): 5.5, 5.6, 6.2 and
+// 7.6 us by eights of rows, 15.4, 16.5, 17.6 and 18.8 in tiles; 64 tokens 22 in tiles.  16 tokens behind 100: 16 and 34.
+struct AttRequest { int begin, rows, last; bool few, portion; };
+template <typename T>
+__device__ __forceinline__ AttRequest att_request(const AttParams<T>& p, int req) {
+  const int begin = p.query_start[req], tokens = p.query_start[req + 1] - begin, lane = threadIdx.x & 31;
+  AttRequest a = {begin, tokens * (p.H / p.KVH), 0, false, false};
+  if (tokens <= ATT_FEW_TOKENS) {
+    a.last = __reduce_max_sync(0xffffffffu, lane < tokens ? p.positions[begin + lane] : -1);
+    a.few = a.rows <= ATT_FEW;
+    a.portion = !a.few && a.last < ATT_SEGMENT;
+  }
+  return a;
+}
 
 // What both kernels share: which keys the rows see, and the chunk in shared memory.
 template <typename T>
@@ -177,9 +196,10 @@ attention_tile_kernel(AttParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
   // blocks: (request, kv head) fastest, then the tiles, those with the most keys first
   const int heads = p.reqs * p.KVH, head = blockIdx.x % heads, req = head / p.KVH, kvh = head % p.KVH, G = p.H / p.KVH;
-  const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
+  const AttRequest a = att_request(p, req);
+  const int begin = a.begin, all_rows = a.rows;
   const int row0 = (gridDim.x / heads - 1 - blockIdx.x / heads) * ATT_ROWS;
-  if (all_rows <= ATT_FEW || row0 >= all_rows) return;
+  if (a.few || a.portion || row0 >= all_rows) return;
   extern __shared__ __align__(16) float smem[];
   const int DK = (p.D + 3) & ~3, LK = DK + 4;
   constexpr int DV = 64 * NJ;
@@ -333,21 +353,20 @@ attention_tile_kernel(AttParams<T> p) {
 }
 
 template <typename T, int NJ>              // NJ: output columns in runs of 64
-__global__ void __launch_bounds__(ATT_THREADS)
+__global__ void __launch_bounds__(ATT_THREADS, NJ == 1 ? 4 : 3)
 attention_few_kernel(AttParams<T> p) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_ATTN_ROWS);
-  // blocks: the segments of a (request, kv head) next to one another
-  const int head = p.head0 + blockIdx.x / p.segments, part_no = blockIdx.x % p.segments;
+  // blocks: the segments of a (request, kv head), or its rows eight by eight, next to one another
+  const int head = p.head0 + blockIdx.x / p.parts, part_no = blockIdx.x % p.parts;
   const int req = head / p.KVH, kvh = head % p.KVH, G = p.H / p.KVH;
-  const int begin = p.query_start[req], all_rows = (p.query_start[req + 1] - begin) * G;
-  if (all_rows > ATT_FEW || all_rows == 0) return;
-  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;           // a warp a row
-  const bool live = r < all_rows;
-  const int segment = part_no * ATT_SEGMENT;
+  const AttRequest a = att_request(p, req);
+  const int segment = a.few ? part_no * ATT_SEGMENT : 0, row0 = a.few ? 0 : part_no * ATT_FEW, begin = a.begin;
+  if (!(a.few || a.portion) || row0 >= a.rows) return;
+  if (segment > a.last) return;            // a longer request's segment (the fold does not read what was not written)
+  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31, rows = min(ATT_FEW, a.rows - row0);     // a warp a row
+  const bool live = r < rows;
   // every warp looks the rows up for itself, a lane a row
-  const int at = lane < all_rows ? p.positions[begin + lane / G] : -1, mine = __shfl_sync(0xffffffffu, at, live ? r : 0);
-  const int last = __reduce_max_sync(0xffffffffu, at);
-  if (segment > last) return;              // a longer request's segment (the fold does not read what was not written)
+  const int at = lane < rows ? p.positions[begin + (row0 + lane) / G] : -1, mine = __shfl_sync(0xffffffffu, at, live ? r : 0);
   extern __shared__ __align__(16) float smem[];
   const int DK = (p.D + 3) & ~3, LK = DK + 4;
   constexpr int DV = 64 * NJ, RUNS = (NJ + 1) / 2;                   // a lane's quads of output columns: 128 apart
@@ -356,12 +375,12 @@ attention_few_kernel(AttParams<T> p) {
   float* const vs = ks + ATT_CHUNK * LK;                             // [ATT_CHUNK][DV]
   __shared__ long long offset[ATT_CHUNK];
   __shared__ float probability[ATT_FEW][ATT_CHUNK];
-  AttBlock<T> b{p, req, kvh, G, begin, all_rows, 0, 0, 0, 0, 0, 0,
+  AttBlock<T> b{p, req, kvh, G, begin, rows, row0, 0, 0, 0, 0, 0,
                 (long long)kvh * p.page_size * p.D, (long long)p.KVH * p.page_size * p.D};
   {
     const int first = b.first_of(at);
     b.lo = __reduce_min_sync(0xffffffffu, at < 0 ? 0x7fffffff : first);
-    b.hi = last + 1;
+    b.hi = __reduce_max_sync(0xffffffffu, at) + 1;
     b.kept = __reduce_max_sync(0xffffffffu, at < 0 ? 0 : min(p.keep_first, first));
     b.all_lo = b.first_of(mine);           // all the rows of a warp: one
     b.all_hi = mine + 1;
@@ -429,8 +448,8 @@ attention_few_kernel(AttParams<T> p) {
     __syncwarp();                                                    // the probabilities have been read
   }
   if (!live) return;
-  if (p.segments > 1) {
-    float* part = p.partial + ((size_t)blockIdx.x * p.part_rows + r) * (p.D + 2);
+  if (a.few && p.segments > 1) {
+    float* part = p.partial + (((size_t)(blockIdx.x / p.parts) * p.segments + part_no) * p.part_rows + r) * (p.D + 2);
 #pragma unroll
     for (int j = 0; j < RUNS; ++j)
 #pragma unroll
@@ -483,41 +502,56 @@ attention_fold_kernel(AttParams<T> p) {
     if (lane + 32 * j < p.D) to[lane + 32 * j] = from_float<T>(sum[j] * inv);
 }
 
-// A row of the scratch for each row that a segment's block can have (one for decoded tokens of ungrouped heads).
-static int part_rows_of(int H, int KVH, int max_query_len) {
-  const long long most = (long long)max_query_len * (H / KVH);
-  return most < ATT_FEW ? (int)most : ATT_FEW;
-}
-// (Request, kv head) pairs that attention_few takes a launch: all of them, or as many as the scratch's bound has room for
-// (the blocks of one launch fill the GPU many times over by then; one long context beside many short ones asks for as much
-// as if all were long).
+// What a batch launches, from its shape and a bound on its positions.
+struct AttPlan {
+  bool tile, few, fold;
+  int segments, part_rows, parts;      // of attention_few: see AttParams
+  long long lot;                       // (request, kv head) pairs a launch of attention_few takes
+  long long scratch;                   // floats
+};
+// One long context beside many short ones asks for as much as if all were long: pairs are taken in lots for which this
+// many floats are enough (their blocks fill the GPU many times over by then).
 #define ATT_SCRATCH_FLOATS (16 << 20)
-static long long heads_a_launch(long long heads, int D, int part_rows, int segments) {
-  if (segments <= 1 || part_rows <= 0) return heads;
-  const long long fit = ATT_SCRATCH_FLOATS / ((long long)segments * part_rows * (D + 2));
-  return heads <= fit ? heads : fit < 1 ? 1 : fit;
+static AttPlan att_plan(int reqs, int H, int KVH, int D, int max_query_len, int tokens, int bound) {
+  AttPlan a = {false, false, false, 1, 1, 1, 1, 0};
+  if (reqs <= 0 || KVH <= 0 || H < KVH || D <= 0 || max_query_len <= 0) return a;      // nothing to do, or refused below
+  const long long G = H / KVH, most = max_query_len * G;
+  const bool equal = (long long)max_query_len * reqs == tokens;      // only one kind of request
+  const bool eight = G <= ATT_FEW && (most <= ATT_FEW || !equal);    // some may have at most 8 rows
+  const bool portions = most > ATT_FEW && (max_query_len <= ATT_FEW_TOKENS || !equal);
+  const int all = bound > ATT_SEGMENT ? (bound + ATT_SEGMENT - 1) / ATT_SEGMENT : 1;
+  a.tile = most > ATT_FEW && (max_query_len > ATT_FEW_TOKENS || all > 1);
+  a.few = eight || portions;
+  a.segments = eight ? all : 1;
+  a.fold = a.segments > 1;
+  a.part_rows = (int)(most < ATT_FEW ? most : ATT_FEW);
+  const long long groups = ((max_query_len < ATT_FEW_TOKENS ? max_query_len : ATT_FEW_TOKENS) * G + ATT_FEW - 1) / ATT_FEW;
+  a.parts = portions && groups > a.segments ? (int)groups : a.segments;
+  const long long heads = (long long)reqs * KVH, each = (long long)a.segments * a.part_rows * (D + 2);
+  const long long fit = ATT_SCRATCH_FLOATS / each;
+  a.lot = !a.fold || heads <= fit ? heads : fit < 1 ? 1 : fit;
+  a.scratch = a.fold ? a.lot * each : 0;
+  return a;
 }
 
 template <typename T, int NJ>
-static int launch_attention(AttParams<T> p, int tokens, int reqs, int max_query_len, cudaStream_t stream) {
-  const int G = p.H / p.KVH, most = max_query_len * G, LK = ((p.D + 3) & ~3) + 4, DV = 64 * NJ;
-  // a batch of equal portions has only one kind of request
-  const bool equal = (long long)max_query_len * reqs == tokens;
-  if (most > ATT_FEW) {
+static int launch_attention(AttParams<T> p, const AttPlan& plan, int max_query_len, cudaStream_t stream) {
+  const int LK = ((p.D + 3) & ~3) + 4, DV = 64 * NJ;
+  const long long heads = (long long)p.reqs * p.KVH, most = (long long)max_query_len * (p.H / p.KVH);
+  if (plan.tile) {
     const int smem = (int)sizeof(float) * (ATT_ROWS * LK + ATT_CHUNK * (LK + DV + ATT_LS));
     KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_tile_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    KVB_CHECK_CUDA(kvb_launch((attention_tile_kernel<T, NJ>), dim3((unsigned)((long long)reqs * p.KVH * ((most + ATT_ROWS - 1) / ATT_ROWS))),
+    KVB_CHECK_CUDA(kvb_launch((attention_tile_kernel<T, NJ>), dim3((unsigned)(heads * ((most + ATT_ROWS - 1) / ATT_ROWS))),
                               dim3(ATT_THREADS), smem, stream, true, p));
   }
-  if (G <= ATT_FEW && (most <= ATT_FEW || !equal)) {
+  if (plan.few) {
     const int smem = (int)sizeof(float) * (ATT_FEW * LK + ATT_CHUNK * (LK + DV));
     KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_few_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const long long heads = (long long)reqs * p.KVH, lot = heads_a_launch(heads, p.D, p.part_rows, p.segments);
-    for (long long head0 = 0; head0 < heads; head0 += lot) {         // one behind the other: the scratch is the same
-      const unsigned here = (unsigned)(heads - head0 < lot ? heads - head0 : lot);
+    for (long long head0 = 0; head0 < heads; head0 += plan.lot) {    // one behind the other: the scratch is the same
+      const unsigned here = (unsigned)(heads - head0 < plan.lot ? heads - head0 : plan.lot);
       p.head0 = (int)head0;
-      KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3(here * p.segments), dim3(ATT_THREADS), smem, stream, true, p));
-      if (p.segments > 1)
+      KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3(here * p.parts), dim3(ATT_THREADS), smem, stream, true, p));
+      if (plan.fold)
         KVB_CHECK_CUDA(kvb_launch((attention_fold_kernel<T>), dim3(here), dim3(ATT_THREADS), 0, stream, true, p));
     }
   }
@@ -526,30 +560,27 @@ static int launch_attention(AttParams<T> p, int tokens, int reqs, int max_query_
 }
 
 template <typename T>
-static int attention_of(const AttParams<T>& p, int tokens, int reqs, int max_query_len, cudaStream_t stream) {
-  if (p.D <= 64) return launch_attention<T, 1>(p, tokens, reqs, max_query_len, stream);
-  if (p.D <= 128) return launch_attention<T, 2>(p, tokens, reqs, max_query_len, stream);
-  return launch_attention<T, 4>(p, tokens, reqs, max_query_len, stream);
+static int attention_of(const AttParams<T>& p, const AttPlan& plan, int max_query_len, cudaStream_t stream) {
+  if (p.D <= 64) return launch_attention<T, 1>(p, plan, max_query_len, stream);
+  if (p.D <= 128) return launch_attention<T, 2>(p, plan, max_query_len, stream);
+  return launch_attention<T, 4>(p, plan, max_query_len, stream);
 }
 
-// Floats of the scratch that a batch takes whose longest request has `segments` segments of cached tokens, and how many
-// times attention_few is launched for it.
-extern "C" long long kvb_paged_attention_scratch(int num_reqs, int H, int KVH, int D, int max_query_len, int segments) {
-  const int rows = part_rows_of(H, KVH, max_query_len);
-  return segments > 1 ? heads_a_launch((long long)num_reqs * KVH, D, rows, segments) * segments * rows * (D + 2) : 0;
+// Floats of the scratch, and the kernels that are launched.  `bound`: no request has more positions, cached and new.
+extern "C" long long kvb_paged_attention_scratch(int num_reqs, int H, int KVH, int D, int max_query_len, int tokens, int bound) {
+  return att_plan(num_reqs, H, KVH, D, max_query_len, tokens, bound).scratch;
 }
-extern "C" int kvb_paged_attention_lots(int num_reqs, int H, int KVH, int D, int max_query_len, int segments) {
-  const long long heads = (long long)num_reqs * KVH, lot = heads_a_launch(heads, D, part_rows_of(H, KVH, max_query_len), segments);
-  return lot > 0 ? (int)((heads + lot - 1) / lot) : 0;
+extern "C" int kvb_paged_attention_launches(int num_reqs, int H, int KVH, int D, int max_query_len, int tokens, int bound) {
+  const AttPlan a = att_plan(num_reqs, H, KVH, D, max_query_len, tokens, bound);
+  const long long heads = (long long)num_reqs * KVH;
+  return (a.tile ? 1 : 0) + (a.few ? (int)((heads + a.lot - 1) / a.lot) * (a.fold ? 2 : 1) : 0);
 }
-extern "C" int kvb_paged_attention_segment() { return ATT_SEGMENT; }
 
-// `segments`: segments of cached tokens that the longest request of at most ATT_FEW rows may have.
 extern "C" int kvb_paged_attention_rows(void* out, int out_stride, const void* q, int q_stride,
                                         const void* k_cache, const void* v_cache, const int* table,
                                         int table_stride, const int* positions, const int* query_start, int num_reqs,
                                         int max_query_len, int tokens, int H, int KVH, int D, int page_size,
-                                        int num_pages, float scale, int window, int keep_first, int segments, float* partial,
+                                        int num_pages, float scale, int window, int keep_first, int bound, float* partial,
                                         int dtype, cudaStream_t stream) {
   if (tokens == 0 || num_reqs == 0) return 0;
   KVB_REQUIRE(D > 0 && D <= ATT_MAX_D, "paged_attention: head_dim must be in [1, 256]");
@@ -557,9 +588,10 @@ extern "C" int kvb_paged_attention_rows(void* out, int out_stride, const void* q
   KVB_REQUIRE(page_size > 0 && num_pages > 1, "paged_attention: empty cache");
   KVB_REQUIRE(keep_first >= 0 && (keep_first == 0 || window > 0), "paged_attention: kept first positions need a window");
   KVB_REQUIRE((long long)tokens * H < (1ll << 31) && max_query_len > 0 && max_query_len <= tokens, "paged_attention: too many rows");
+  const AttPlan plan = att_plan(num_reqs, H, KVH, D, max_query_len, tokens, bound);
   KVB_REQUIRE((long long)num_reqs * KVH * (((long long)max_query_len * (H / KVH) + ATT_ROWS - 1) / ATT_ROWS) < (1ll << 31) &&
-              (long long)num_reqs * KVH * segments < (1ll << 31), "paged_attention: too many blocks for one launch");
-  KVB_REQUIRE(segments >= 1 && (segments == 1 || partial != nullptr), "paged_attention: no scratch");
+              plan.lot * plan.parts < (1ll << 31), "paged_attention: too many blocks for one launch");
+  KVB_REQUIRE(plan.scratch == 0 || partial != nullptr, "paged_attention: no scratch");
   int* status = kvb_status_word();
   KVB_REQUIRE(status != nullptr, "paged_attention: no status word");
   const int esize = dtype == KVB_F32 ? 4 : 2;
@@ -567,9 +599,9 @@ extern "C" int kvb_paged_attention_rows(void* out, int out_stride, const void* q
 #define KVB_ATT(T_)                                                                                                    \
   attention_of<T_>(AttParams<T_>{(T_*)out, (const T_*)q, (const T_*)k_cache, (const T_*)v_cache, table, positions,     \
                                  query_start, out_stride, q_stride, table_stride, H, KVH, D, page_size, num_pages,     \
-                                 window, keep_first, vec, segments, num_reqs, part_rows_of(H, KVH, max_query_len), 0,  \
+                                 window, keep_first, vec, plan.segments, num_reqs, plan.part_rows, plan.parts, 0,      \
                                  scale, partial, status},                                                              \
-                   tokens, num_reqs, max_query_len, stream)
+                   plan, max_query_len, stream)
   return dtype == KVB_F32 ? KVB_ATT(float) : KVB_ATT(bf16);
 #undef KVB_ATT
 }

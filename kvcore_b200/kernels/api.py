@@ -140,12 +140,9 @@ def ensure_built(verbose: bool = False) -> str:
     lib.kvb_gemm_stream_norm_max_k.restype = _int
     lib.kvb_gemm_stream_scratch_marker.argtypes = []
     lib.kvb_gemm_stream_scratch_marker.restype = ctypes.c_uint
-    lib.kvb_paged_attention_scratch.argtypes = [_int] * 6
+    lib.kvb_paged_attention_scratch.argtypes = lib.kvb_paged_attention_launches.argtypes = [_int] * 7
     lib.kvb_paged_attention_scratch.restype = _ll
-    lib.kvb_paged_attention_lots.argtypes = [_int] * 6
-    lib.kvb_paged_attention_lots.restype = _int
-    lib.kvb_paged_attention_segment.argtypes = []
-    lib.kvb_paged_attention_segment.restype = _int
+    lib.kvb_paged_attention_launches.restype = _int
     lib.kvb_moe_tile_rows.argtypes = []
     lib.kvb_moe_tile_rows.restype = _int
     lib.kvb_moe_route_alone.argtypes = []
@@ -642,24 +639,17 @@ def paged_attention(
     # Requests of at most 8 rows a kv head (decoded tokens) have the segments of their cached tokens read by different
     # blocks and folded behind them (sized by the bound that the batch's shape gives, which a captured step keeps), in lots
     # whose scratch stays below 64 MB.
-    group = num_heads // num_kv_heads
-    few = group <= 8 and (ctx.max_query_len * group <= 8 or ctx.max_query_len * ctx.num_reqs != tokens)
-    segments = 1
-    if few:
-        ensure_built()
-        bound = getattr(ctx, "max_seq_len_bound", 0) or ctx.max_seq_len
-        segments = -(-max(1, bound) // _lib.kvb_paged_attention_segment())
-    partial, lots = None, 1
-    if segments > 1:
-        sizes = (ctx.num_reqs, num_heads, num_kv_heads, head_dim, ctx.max_query_len, segments)
-        partial = torch.empty(_lib.kvb_paged_attention_scratch(*sizes), dtype=torch.float32, device=qkv.device)
-        lots = _lib.kvb_paged_attention_lots(*sizes)
+    ensure_built()
+    bound = getattr(ctx, "max_seq_len_bound", 0) or getattr(ctx, "max_seq_len", 0) or table.shape[1] * page_size
+    sizes = (ctx.num_reqs, num_heads, num_kv_heads, head_dim, ctx.max_query_len, tokens, bound)
+    floats = _lib.kvb_paged_attention_scratch(*sizes)
+    partial = torch.empty(floats, dtype=torch.float32, device=qkv.device) if floats else None
     _call("kvb_paged_attention_rows", out.data_ptr(), out.stride(0), qkv.data_ptr(), qkv.stride(0),
           k_cache.data_ptr(), v_cache.data_ptr(), table.data_ptr(), table.stride(0),
           ctx.positions.data_ptr(), ctx.query_start.data_ptr(), ctx.num_reqs, ctx.max_query_len, tokens, num_heads,
-          num_kv_heads, head_dim, page_size, num_pages, float(scale), int(window or 0), int(keep_first), segments,
+          num_kv_heads, head_dim, page_size, num_pages, float(scale), int(window or 0), int(keep_first), bound,
           None if partial is None else partial.data_ptr(), _dtype_code(qkv), _stream(),
-          kernels=int(ctx.max_query_len * group > 8) + int(few) * (1 if partial is None else 2 * lots))
+          kernels=_lib.kvb_paged_attention_launches(*sizes))
     return out
 
 

@@ -124,3 +124,24 @@ def test_scratch_of_few_rows_is_bounded():
                                     _Ctx(part), heads, kv_heads, dim, dim ** -0.5, None)
         assert torch.equal(alone, got[row:row + 1])
     assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,window,keep", [(6, 2, 128, None, 0), (32, 1, 64, None, 0), (4, 2, 16, 50, 7), (8, 8, 256, None, 0)])
+def test_short_portions_have_the_bits_of_tiles(heads, kv_heads, dim, window, keep):
+    """Portions around 8 rows, 32 tokens and the end of the first segment, alone and beside one another, with a bound on the
+    positions that is exact and one that is not: the bits of a whole prompt in tiles."""
+    case, attend = _attention(torch.float32, heads, kv_heads, dim, 16, [(0, 300)], window, keep)
+    whole = attend(case["k_cache"], case["v_cache"])
+    parts = [(0, 1), (0, 3), (0, 9), (0, 32), (0, 33), (224, 32), (225, 32), (223, 33), (249, 7), (250, 7), (299, 1)]
+    for batch in [[part] for part in parts] + [parts, parts[:4] + parts[5:6]]:
+        rows = torch.cat([torch.arange(first, first + count, device=DEV) for first, count in batch])
+        ctx = _Ctx(dict(case, positions=rows.to(torch.int32), lens=batch, req_index=None,
+                        query_start=torch.tensor([0] + [n for _, n in batch], device=DEV).cumsum(0).to(torch.int32),
+                        context_lens=torch.tensor([c for c, _ in batch], dtype=torch.int32, device=DEV)))
+        for bound in (max(c + n for c, n in batch), 2000):
+            ctx.max_seq_len_bound = bound
+            got = K().paged_attention(case["qkv"][rows].contiguous(), case["k_cache"], case["v_cache"],
+                                      case["table"].repeat(len(batch), 1), ctx, heads, kv_heads, dim, dim ** -0.5, window,
+                                      keep_first=keep, force_general=True)
+            assert torch.equal(got, whole[rows]), (batch, bound)
+    assert K().read_status() == 0
