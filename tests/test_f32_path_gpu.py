@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,k", [(130, 257), (130, 260), (33, 16), (16, 5), (513, 129), (3072, 128)])
 def test_product_rows_have_the_same_bits_in_every_kernel(n, k):
-    """1 to 16 rows take the kernel of decode steps, more take tiles of 32, 64 or 128 rows; edges of all of them.
+    """1 to 16 rows take the kernel of decode steps, more take tiles of 32 or 64 rows (128: see below); edges of all of them.
     The error of a sum of k products, each addition rounded: below k/2 units of 2^-24 of the terms' magnitudes."""
     x, w = randn(700, k, dtype=torch.float32, seed=1), randn(n, k, dtype=torch.float32, seed=2)
     bias = randn(n, dtype=torch.float32, seed=3)
@@ -145,3 +145,19 @@ def test_short_portions_have_the_bits_of_tiles(heads, kv_heads, dim, window, kee
                                       keep_first=keep, force_general=True)
             assert torch.equal(got, whole[rows]), (batch, bound)
     assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,tile", [(600, 28673, 36, 128), (620, 28676, 33, 128), (700, 3072, 131, 64), (513, 3100, 260, 64),
+                                        (300, 515, 67, 32)])
+def test_product_rows_have_the_same_bits_in_every_tile(m, n, k, tile):
+    """Sizes that the rule sends to tiles of 128, 64 and 32 rows (rounds of 148 SMs; see kvb_gemm_f32), each with ragged
+    rows and columns, read in pieces of four and one by one: against the kernel of decode steps."""
+    rounds = lambda tm, tn: -(-(-(-m // tm) * -(-n // tn)) // K().api.sm_count(torch.device(DEV)))  # noqa: E731
+    cost = {128: 266.0 if rounds(128, 128) < 2 else 210.0 * rounds(128, 128), 64: 58.0 * max(2.2, rounds(64, 64)),
+            32: 38.0 * max(2.7, rounds(32, 64))}
+    assert min(cost, key=cost.get) == tile
+    x, w = randn(m, k, dtype=torch.float32, seed=1), randn(n, k, dtype=torch.float32, seed=2)
+    bias = randn(n, dtype=torch.float32, seed=3)
+    full = K().linear(x, w, bias)
+    for first in (0, 63, 127, 240, m - 16):
+        assert torch.equal(K().linear(x[first:first + 16].contiguous(), w, bias), full[first:first + 16]), first
