@@ -585,13 +585,16 @@ extern "C" int kvb_moe_gemm(void* out, const void* a, long long a_stride, int a_
   return 0;
 }
 
-// Decode-sized batches in bf16: one pass over each chosen expert's matrices.  grid (N / 32, pairs): the block of the
-// first pair that chose an expert works for all that did, two at a time (the others' blocks leave).  It holds the pairs'
-// input rows (weighted and rounded) in shared memory; each of its 8 warps owns 4 output columns (GATED: the 4 gate rows
-// and the 4 up rows) and walks K in 16-byte loads, lane-strided, two rounds of 256 columns in flight; a butterfly sums
-// the lanes.  No tile is padded with rows that are not there, so the kernel is bound by the weights it reads.
-// 16 experts of 2 x 4,096 x 2,048 and 2,048 x 4,096, 8 tokens of 2 (16 pairs, about 10 experts), the layer around them
-// included: 118 us; 123 before routing such a batch became one launch; a pass for every pair, a round in flight: 138.
+// Decode-sized batches in bf16: the chosen experts' matrices are read once for two pairs.  grid (N / 32, pairs): the pairs of
+// an expert, in their order, are taken two at a time (`hold`), the block of the first of the two works for both, that of
+// the second leaves; an expert that many chose has as many blocks side by side (its matrices come from the L2 cache for all
+// but one of them).  A block holds its pairs' input rows (weighted and rounded) in shared memory; each of its 8 warps owns
+// 4 output columns (GATED: the 4 gate rows and the 4 up rows) and walks K in 16-byte loads, lane-strided, two rounds of 256
+// columns in flight; a butterfly sums the lanes.  No tile is padded with rows that are not there, so the kernel is bound by
+// the weights it reads.
+// 16 experts of 2 x 4,096 x 2,048 and 2,048 x 4,096, both products of 8 tokens of 2 (B200, call by call): choices at random
+// 100 us, all tokens the same two experts 67, no expert twice 128 (one block taking an expert's pairs in turn: 107, 128 and
+// 137; a block and a pass for every pair, one round in flight: 125, 77 and 132).
 #define MOE_GEMV_COLS 32
 #define MOE_GEMV_PAIRS 2
 template <bool GATED>
@@ -602,15 +605,23 @@ moe_gemv_kernel(bf16* __restrict__ out, const bf16* __restrict__ a, long long a_
   KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_GEMM);
   extern __shared__ __align__(16) unsigned char gemv_smem[];
   bf16* xs = reinterpret_cast<bf16*>(gemv_smem);      // [hold][K], hold <= MOE_GEMV_PAIRS
-  __shared__ int mates[MOE_GEMV_PAIRS];
   const int pair = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int expert = ids[pair];
+  const int here = lane < pairs ? ids[lane] : -1, expert = ids[pair];          // (both asked for at once)
   if (expert < 0 || expert >= E) {                   // none, or one without tensors
     if (threadIdx.x == 0 && (expert < 0 || expert >= known)) atomicOr(status, KVB_STATUS_BAD_TOKEN);
     return;
   }
-  for (int i = 0; i < pair; i += 32)                  // every warp sees the same
-    if (__any_sync(0xffffffffu, i + lane < pair && ids[i + lane] == expert)) return;
+  int before = 0, mate = -1;                          // pairs of this expert in front of this one; the next behind it
+  for (int i = 0; i < pairs && mate < 0; i += 32) {   // every warp sees the same
+    const int choice = i == 0 ? here : i + lane < pairs ? ids[i + lane] : -1;
+    const unsigned same = __ballot_sync(0xffffffffu, choice == expert);
+    const unsigned front = pair >= i + 32 ? 0xffffffffu : pair <= i ? 0u : (1u << (pair - i)) - 1u;
+    before += __popc(same & front);
+    const unsigned behind = same & ~front & (pair >= i && pair < i + 32 ? ~(1u << (pair - i)) : 0xffffffffu);
+    if (behind != 0) mate = i + __ffs(behind) - 1;
+  }
+  if (before % hold != 0) return;
+  const int count = hold > 1 && mate >= 0 ? 2 : 1;
   const int n0 = blockIdx.x * MOE_GEMV_COLS + warp * 4;
   const bf16* we = w + (size_t)expert * (GATED ? 2 : 1) * N * K;
   constexpr int ROWS = GATED ? 8 : 4;
@@ -623,79 +634,72 @@ moe_gemv_kernel(bf16* __restrict__ out, const bf16* __restrict__ a, long long a_
     for (int r = 0; r < ROWS; ++r)
       if (k < K) to[r].load(rows[r & 3] + (r >= 4 ? (size_t)N * K : 0) + k);
   };
-  for (int next = pair;;) {
-    int count = 0;                                    // the next pairs of this expert
-    for (int i = next; i < pairs && count < hold; i += 32) {
-      unsigned found = __ballot_sync(0xffffffffu, i + lane < pairs && ids[i + lane] == expert);
-      for (; found != 0 && count < hold; found &= found - 1) {
-        const int mate = i + __ffs(found) - 1;
-        if (threadIdx.x == 0) mates[count] = mate;
-        next = mate + 1;
-        ++count;
-      }
-    }
-    if (count == 0) return;
-    fetch(wv[0], lane * 8);                           // on its way while the rows are staged
-    fetch(wv[1], lane * 8 + 256);
-    __syncthreads();
-    for (int p = 0; p < count; ++p) {
-      const bf16* row = a + (size_t)(mates[p] / a_row_div) * a_stride;
-      const float scale = pair_weight != nullptr ? pair_weight[mates[p]] : 1.0f;
-      for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {
-        Vec16<bf16> v;
-        v.load(row + k);
-        if (pair_weight != nullptr) {
+  fetch(wv[0], lane * 8);                             // on its way while the rows are staged
+  fetch(wv[1], lane * 8 + 256);
+  for (int p = 0; p < count; ++p) {
+    const int of = p == 0 ? pair : mate;
+    const bf16* row = a + (size_t)(of / a_row_div) * a_stride;
+    const float scale = pair_weight != nullptr ? pair_weight[of] : 1.0f;
+#pragma unroll 1
+    for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {
+      Vec16<bf16> v;
+      v.load(row + k);
+      if (pair_weight != nullptr) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v.set(j, v.get(j) * scale);
+        for (int j = 0; j < 8; ++j) v.set(j, v.get(j) * scale);
+      }
+      v.store(xs + (size_t)p * K + k);
+    }
+  }
+  __syncthreads();
+  float acc[MOE_GEMV_PAIRS][ROWS];
+#pragma unroll
+  for (int p = 0; p < MOE_GEMV_PAIRS; ++p)
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) acc[p][r] = 0.0f;
+  auto multiply = [&](const Vec16<bf16> (&from)[ROWS], int k) {
+    if (k >= K) return;
+    Vec16<bf16> x, y;
+    x.load(xs + k);
+    if (count > 1) {
+      y.load(xs + K + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const float wr = from[r].get(j);
+          acc[0][r] = fmaf(wr, x.get(j), acc[0][r]);
+          acc[1][r] = fmaf(wr, y.get(j), acc[1][r]);
         }
-        v.store(xs + (size_t)p * K + k);
-      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[0][r] = fmaf(from[r].get(j), x.get(j), acc[0][r]);
     }
-    __syncthreads();
-    float acc[MOE_GEMV_PAIRS][ROWS];
+  };
+#pragma unroll 1
+  for (int k = lane * 8; k < K; k += 512) {
+    multiply(wv[0], k);
+    fetch(wv[0], k + 512);
+    multiply(wv[1], k + 256);
+    fetch(wv[1], k + 768);
+  }
 #pragma unroll
-    for (int p = 0; p < MOE_GEMV_PAIRS; ++p)
+  for (int p = 0; p < MOE_GEMV_PAIRS; ++p) {
+    if (p >= count) continue;
 #pragma unroll
-      for (int r = 0; r < ROWS; ++r) acc[p][r] = 0.0f;
-    auto multiply = [&](const Vec16<bf16> (&from)[ROWS], int k) {
-      if (k >= K) return;
-#pragma unroll
-      for (int p = 0; p < MOE_GEMV_PAIRS; ++p) {
-        if (p < count) {
-          Vec16<bf16> x;
-          x.load(xs + (size_t)p * K + k);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xv = x.get(j);
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r) acc[p][r] = fmaf(from[r].get(j), xv, acc[p][r]);
-          }
-        }
+    for (int r = 0; r < ROWS; ++r) acc[p][r] = warp_sum(acc[p][r]);
+    if (lane < 4 && n0 + lane < N) {
+      float v = lane == 0 ? acc[p][0] : lane == 1 ? acc[p][1] : lane == 2 ? acc[p][2] : acc[p][3];
+      if (GATED) {
+        const float u = lane == 0 ? acc[p][4 % ROWS] : lane == 1 ? acc[p][5 % ROWS] : lane == 2 ? acc[p][6 % ROWS] : acc[p][7 % ROWS];
+        v = moe_join<bf16>(v, u, join);
+      } else {
+        v = moe_plain(v, join);
       }
-    };
-    for (int k = lane * 8; k < K; k += 512) {
-      multiply(wv[0], k);
-      fetch(wv[0], k + 512);
-      multiply(wv[1], k + 256);
-      fetch(wv[1], k + 768);
+      out[(size_t)(p == 0 ? pair : mate) * N + n0 + lane] = from_float<bf16>(v);
     }
-#pragma unroll
-    for (int p = 0; p < MOE_GEMV_PAIRS; ++p) {
-      if (p >= count) continue;
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) acc[p][r] = warp_sum(acc[p][r]);
-      if (lane < 4 && n0 + lane < N) {
-        float v = lane == 0 ? acc[p][0] : lane == 1 ? acc[p][1] : lane == 2 ? acc[p][2] : acc[p][3];
-        if (GATED) {
-          const float u = lane == 0 ? acc[p][4 % ROWS] : lane == 1 ? acc[p][5 % ROWS] : lane == 2 ? acc[p][6 % ROWS] : acc[p][7 % ROWS];
-          v = moe_join<bf16>(v, u, join);
-        } else {
-          v = moe_plain(v, join);
-        }
-        out[(size_t)mates[p] * N + n0 + lane] = from_float<bf16>(v);
-      }
-    }
-    __syncthreads();                                  // the rows and their numbers have been read
   }
 }
 
