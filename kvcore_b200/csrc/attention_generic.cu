@@ -536,21 +536,22 @@ static AttPlan att_plan(int reqs, int H, int KVH, int D, int max_query_len, int 
 
 template <typename T, int NJ>
 static int launch_attention(AttParams<T> p, const AttPlan& plan, int max_query_len, cudaStream_t stream) {
-  const int LK = ((p.D + 3) & ~3) + 4, DV = 64 * NJ;
+  constexpr int DV = 64 * NJ, MOST_LK = DV + 4;            // (what is allowed is the most that any D asks for: another
+  const int LK = ((p.D + 3) & ~3) + 4;                     // thread's launch may lie between the allowance and this one's)
+  auto tile_bytes = [](int lk) { return (int)sizeof(float) * (ATT_ROWS * lk + ATT_CHUNK * (lk + DV + ATT_LS)); };
+  auto few_bytes = [](int lk) { return (int)sizeof(float) * (ATT_FEW * lk + ATT_CHUNK * (lk + DV)); };
   const long long heads = (long long)p.reqs * p.KVH, most = (long long)max_query_len * (p.H / p.KVH);
   if (plan.tile) {
-    const int smem = (int)sizeof(float) * (ATT_ROWS * LK + ATT_CHUNK * (LK + DV + ATT_LS));
-    KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_tile_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_tile_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_bytes(MOST_LK)));
     KVB_CHECK_CUDA(kvb_launch((attention_tile_kernel<T, NJ>), dim3((unsigned)(heads * ((most + ATT_ROWS - 1) / ATT_ROWS))),
-                              dim3(ATT_THREADS), smem, stream, true, p));
+                              dim3(ATT_THREADS), tile_bytes(LK), stream, true, p));
   }
   if (plan.few) {
-    const int smem = (int)sizeof(float) * (ATT_FEW * LK + ATT_CHUNK * (LK + DV));
-    KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_few_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KVB_CHECK_CUDA(cudaFuncSetAttribute(attention_few_kernel<T, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, few_bytes(MOST_LK)));
     for (long long head0 = 0; head0 < heads; head0 += plan.lot) {    // one behind the other: the scratch is the same
       const unsigned here = (unsigned)(heads - head0 < plan.lot ? heads - head0 : plan.lot);
       p.head0 = (int)head0;
-      KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3(here * p.parts), dim3(ATT_THREADS), smem, stream, true, p));
+      KVB_CHECK_CUDA(kvb_launch((attention_few_kernel<T, NJ>), dim3(here * p.parts), dim3(ATT_THREADS), few_bytes(LK), stream, true, p));
       if (plan.fold)
         KVB_CHECK_CUDA(kvb_launch((attention_fold_kernel<T>), dim3(here), dim3(ATT_THREADS), 0, stream, true, p));
     }

@@ -32,6 +32,9 @@
 #define MOE_BM 16
 #define MOE_BN 64
 #define MOE_BK 16
+// Dynamic shared memory that a kernel of this file asks for at most, and what each that needs more than 48 KB is allowed: the
+// same whatever a launch needs, since another thread's launch may lie between the allowance and the launch.
+#define MOE_MOST_SMEM (200 * 1024)
 
 // Routing: a token's logits, then its choice.  Up to a token an SM one kernel does both; beyond, the logits [tokens, E + R]
 // go through memory, so that tokens share the router's rows (four tokens a block up to ROUTE_FEW_MAX, then eight) and a
@@ -318,8 +321,8 @@ template <typename T>
 static int launch_moe_logits(const RouteParams<T>& p, cudaStream_t stream) {
   // rows too long for shared memory take the few tokens' kernel at any number
   const size_t smem = (size_t)ROUTE_TOKENS * ((p.K + 127) / 128) * 128 * sizeof(T);
-  if (p.tokens > ROUTE_FEW_MAX && smem <= 200 * 1024) {
-    KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (p.tokens > ROUTE_FEW_MAX && smem <= MOE_MOST_SMEM) {
+    KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T>), cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_MOST_SMEM));
     KVB_CHECK_CUDA(kvb_launch((moe_logits_kernel<T>), dim3((p.tokens + ROUTE_TOKENS - 1) / ROUTE_TOKENS), dim3(128), smem, stream,
                               true, p));
     return 0;
@@ -343,7 +346,7 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
   if (score_mode == 2) renormalize = 1;
   KVB_REQUIRE((long long)E + R <= 65535, "moe_route: too many experts");
   size_t smem = (size_t)(2 * E + R + 2 * groups) * sizeof(float);
-  KVB_REQUIRE((size_t)K * (dtype == KVB_F32 ? sizeof(float) : sizeof(bf16)) + smem <= 200 * 1024,
+  KVB_REQUIRE((size_t)K * (dtype == KVB_F32 ? sizeof(float) : sizeof(bf16)) + smem <= MOE_MOST_SMEM,
               "moe_route: a token's row and scores do not fit in shared memory");
   const ChooseParams c = {ids_out, weights_out, gate_out, E, R, top, score_mode, renormalize, correction, groups, keep,
                           weight_scale, bias};
@@ -352,7 +355,7 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
   if (tokens <= kvb_moe_route_alone()) {
 #define KVB_ROUTE_TOKEN(T_, P_)                                                                                        \
     if (smem > 48 * 1024)                                                                                             \
-      KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_route_token_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+      KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_route_token_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_MOST_SMEM)); \
     KVB_CHECK_CUDA(kvb_launch((moe_route_token_kernel<T_>), dim3(tokens), dim3(1024), smem, stream, true, P_, c))
     if (dtype == KVB_F32) { KVB_ROUTE_TOKEN(float, in32); } else { KVB_ROUTE_TOKEN(bf16, in16); }
 #undef KVB_ROUTE_TOKEN
@@ -365,7 +368,7 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
   while (warps > 1 && warps * smem > 48 * 1024) warps /= 2;
   smem *= warps;
   if (smem > 48 * 1024)
-    KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_choose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_choose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_MOST_SMEM));
   KVB_CHECK_CUDA(kvb_launch((moe_choose_kernel), dim3((tokens + warps - 1) / warps), dim3(32 * warps), smem, stream, true,
                             (const float*)logits, tokens, c));
   KVB_CHECK_LAUNCH();
@@ -715,14 +718,14 @@ extern "C" int kvb_moe_gemv(void* out, const void* a, long long a_stride, int a_
   const size_t row_bytes = (size_t)K * sizeof(bf16), fit = 48 * 1024 / row_bytes;
   const int hold = fit < 1 ? 1 : fit > MOE_GEMV_PAIRS ? MOE_GEMV_PAIRS : (int)fit;
   const size_t smem = hold * row_bytes;
-  KVB_REQUIRE(smem <= 200 * 1024, "moe_gemv: an input row does not fit in shared memory");
+  KVB_REQUIRE(smem <= MOE_MOST_SMEM, "moe_gemv: an input row does not fit in shared memory");
   int* status = kvb_status_word();
   KVB_REQUIRE(status != nullptr, "moe_gemv: no status word");
   dim3 grid((N + MOE_GEMV_COLS - 1) / MOE_GEMV_COLS, pairs);
 #define KVB_MOE_GEMV(G_)                                                                                       \
   do {                                                                                                         \
     if (smem > 48 * 1024)                                                                                      \
-      KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_gemv_kernel<G_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+      KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_gemv_kernel<G_>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_MOST_SMEM)); \
     KVB_CHECK_CUDA(kvb_launch((moe_gemv_kernel<G_>), grid, dim3(256), smem, stream, true, (bf16*)out, (const bf16*)a, \
                               a_stride, a_row_div, pair_weight, (const bf16*)w, ids, pairs, hold, E, known, N, K, status, join)); \
   } while (0)

@@ -495,11 +495,11 @@ static int launch_state_scan(const ScanParams& p_in, int num_reqs, long long tok
 #define SCAN_CASE(DR, RS, CP, BRIEF)                                                                          \
   if (dreg == DR && rsplit == RS && cpt == CP && shape.brief == BRIEF) {                                      \
     constexpr int B = BRIEF ? 2 : DR * RS <= 128 ? 16 : 2048 / (DR * RS);                                     \
-    size_t smem = 2 * (size_t)B * ((MODE == 0 ? 3 : 2) * DR * RS + 4 + 2 * (SCAN_THREADS / RS * CP)) * sizeof(float); \
-    if (smem < alone) smem = alone;                                                                           \
-    if (smem > 48 * 1024)                                                                                     \
-      KVB_CHECK_CUDA(cudaFuncSetAttribute(state_scan_kernel<TV, MODE, DR, RS, CP, B>,                         \
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));           \
+    constexpr size_t need = 2 * (size_t)B * ((MODE == 0 ? 3 : 2) * DR * RS + 4 + 2 * (SCAN_THREADS / RS * CP)) * sizeof(float); \
+    const size_t smem = need < alone ? alone : need;                                                          \
+    if (smem > 48 * 1024)           /* the most that any launch asks for: another thread's may be in between */ \
+      KVB_CHECK_CUDA(cudaFuncSetAttribute(state_scan_kernel<TV, MODE, DR, RS, CP, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                          (int)(need < SCAN_SM_BYTES / 2 ? SCAN_SM_BYTES / 2 : need)));       \
     err = kvb_launch((state_scan_kernel<TV, MODE, DR, RS, CP, B>), grid, block, smem, stream, true, p);       \
   }
 #define SCAN_ROWS(DR, CP, BRIEF)                                                                              \

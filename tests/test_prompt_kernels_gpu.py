@@ -448,3 +448,30 @@ def test_batches_in_two_query_tiles_give_the_bits_of_their_requests_alone(seed):
                 assert torch.equal(got[at:at + new, cols], alone), (lens, group, page, window, form)
         at += new
     assert K().read_status() == 0
+
+
+def test_threads_that_launch_one_kernel_with_different_shared_memory():
+    """Two threads, each with a stream of its own, run the same scan with blocks that ask for different shares of an SM."""
+    import threading
+
+    failures = []
+
+    def work(heads):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                rows = randn(3, heads * 512, dtype=torch.bfloat16, seed=heads)
+                q, k, v = rows[:, :heads * 128], rows[:, heads * 128:heads * 256], rows[:, heads * 256:]
+                decay, batch = torch.full((heads,), 0.5, device=DEV), _Batch([(0, 3)])
+                state = torch.zeros(1, heads * 128 * 256, device=DEV)
+                for _ in range(600):
+                    K().lightning_scan(q, k, v, decay, state, batch, heads=heads, dim=128, value_dim=256)
+            stream.synchronize()
+        except Exception as error:  # noqa: BLE001 - whatever a thread meets fails the test
+            failures.append(error)
+    threads = [threading.Thread(target=work, args=(heads,)) for heads in (8, 16)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not failures, failures
