@@ -87,7 +87,8 @@ struct ScanParams {
 // holds those rows of CPT neighbouring columns (one load of q, k and the decays then serves CPT columns, and the
 // columns' chains of dependent instructions run interleaved); BATCH tokens a stage of shared memory.
 template <typename TV, int MODE, int DREG, int RSPLIT, int CPT, int BATCH>
-__global__ void __launch_bounds__(SCAN_THREADS, BATCH <= 2 ? 5 : 1)     // brief: every block's state in flight counts
+// (brief: every block's state in flight counts; keys of more than 256 entries: a column has 32 threads, and blocks are many)
+__global__ void __launch_bounds__(SCAN_THREADS, BATCH <= 2 ? 5 : BATCH == 4 ? 4 : 1)
 state_scan_kernel(ScanParams p) {
   KVB_KERNEL_PROLOGUE(MODE == 0 ? KVB_TAG_GLA_SCAN : MODE == 1 ? KVB_TAG_DELTA_SCAN
                                                    : MODE == 2 ? KVB_TAG_LIGHTNING_SCAN : KVB_TAG_SSM_SCAN);
@@ -440,7 +441,8 @@ state_scan_kernel(ScanParams p) {
 // 4,096 columns a request).  A step of single tokens moves every state once and does little else: 8 rows of four
 // columns, stages of two tokens (6 KB a block, so that many blocks share an SM).  A step with prompts in it is a
 // chain of dependent instructions per token, and the stages' hand-overs cost as much as their tokens: stages of
-// 16 tokens; 8 rows of four columns (one load of q, k and the decays serves four columns, the least work a row) once
+// 16 tokens.  The fewer rows a thread has the shorter its chain, so one column of as few rows as give every block an SM of
+// its own; beyond that 8 rows of four columns (one load of q, k and the decays serves four columns, the least work a row) once
 // they give the SMs two blocks each (one for the delta rule), else 4 rows of four columns; for the delta rule, whose
 // chain passes through a sum over the column's threads, 16 rows of one column (three shuffles in the chain, not five).
 // Microseconds, preparation included (B200, keys of 128): fixed decay, one prompt of 2,048, 16 heads of 256 values: 8 x 4
@@ -466,9 +468,11 @@ static ScanShape scan_shape(int mode, int D, long long heads_of_all, int V, bool
   if (c == 4) return {least, least <= 8 ? 4 : 1, brief && least == 8};
   if (c == 1) return {least, 1, false};
   if (brief) return least <= 8 ? ScanShape{8, 4, true} : ScanShape{16, 1, true};
+  for (int rows = least; rows <= (least <= 4 ? 8 : 16); rows *= 2)
+    if (scan_blocks(D, heads_of_all, V, rows, 1) <= sms) return {rows, 1, false};
   if (least <= 8 && scan_blocks(D, heads_of_all, V, 8, 4) >= (mode == 1 ? 1 : 2) * sms) return {8, 4, false};
-  if (mode == 1) return {16, 1, false};
-  if (least <= 4) return {4, 4, false};
+  if (mode == 1 && least <= 4) return {16, 1, false};
+  if (least <= 8) return {least, 4, false};
   return {least, 1, false};
 }
 
