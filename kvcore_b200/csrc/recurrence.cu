@@ -283,9 +283,13 @@ extern "C" int kvb_conv_prepare(float* out, const void* rows, long long row_stri
   const int slices = 2 * kv_heads + heads * ((V + 127) / 128), slice_blocks = (slices + CP_THREADS / 32 - 1) / (CP_THREADS / 32);
   // (the choice depends on the layer alone, so a token's bits do not depend on the batch)
   if (num_taps >= 2 && num_taps <= 4 && D <= 128 && D % 4 == 0 && V % 4 == 0 && row_stride % 4 == 0 && slice_blocks <= 65535 &&
-      (uintptr_t)rows % (4 * esize) == 0 && (uintptr_t)out % 8 == 0) {
-    // Runs as long as leave every SM a few blocks; single tokens of many requests read the state anyway.
-    const int run = tokens >= 512 && tokens > 2 * num_reqs ? 8 : tokens >= 64 && tokens > 2 * num_reqs ? 2 : 1;
+      (uintptr_t)rows % (4 * esize) == 0 && (uintptr_t)out % 8 == 0 && out_stride % 2 == 0) {
+    // Runs as long as leave the SMs about a wave of blocks (by the blocks an SM that runs of one would be); single tokens of
+    // many requests read the state anyway.  Microseconds for runs of 1, 2, 4, 8 (B200): 12 slices, 300 tokens (6 blocks an
+    // SM) 5.4, 5.8, 7.0, 9.5; 511 (10) 8.0, 6.1, 7.3, 9.8; 800 (16) 10.0, 9.1, 7.5, 10.1; 2,048 (42) 18.1, 13.8, 12.7,
+    // 11.7; 32 slices, 64 tokens (3) 5.7, 6.0, 7.0, 10.1; 300 (16) 13.5, 11.0, 8.4, 10.7; 800 (43) 26.6, 19.1, 15.3, 12.6.
+    const long long sms = kvb_sm_count() > 0 ? kvb_sm_count() : 148, blocks = (long long)tokens * slice_blocks;
+    const int run = tokens <= 2 * num_reqs || blocks <= 7 * sms ? 1 : blocks <= 14 * sms ? 2 : blocks <= 32 * sms ? 4 : 8;
     const dim3 grid((tokens + run - 1) / run, slice_blocks);
 #define KVB_CPR_LAUNCH(T_, N_)                                                                                       \
     KVB_CHECK_CUDA(kvb_launch((conv_prepare_runs_kernel<T_, N_>), grid, dim3(CP_THREADS), 0, stream, true, out, out_stride, \
