@@ -36,9 +36,9 @@
 // same whatever a launch needs, since another thread's launch may lie between the allowance and the launch.
 #define MOE_MOST_SMEM (200 * 1024)
 
-// Routing: a token's logits, then its choice.  Up to a token an SM one kernel does both; beyond, the logits [tokens, E + R]
-// go through memory, so that tokens share the router's rows (four tokens a block up to ROUTE_FEW_MAX, then eight) and a
-// warp a token chooses.  A logit is formed in the same order whichever kernel takes it: lane l adds the products
+// Routing: a token's logits, then its choice.  For few tokens one kernel does both (kvb_moe_route_alone); beyond, the logits
+// [tokens, E + R] go through memory, so that tokens share the router's rows (four tokens a block up to route_few_max, then
+// eight) and a warp a token chooses.  A logit is formed in the same order whichever kernel takes it: lane l adds the products
 // k = l, l + 32, ... into four partial sums by (k / 32) % 4, then ((p0 + p1) + (p2 + p3)), then the butterfly over the
 // lanes.
 template <typename T>
@@ -278,7 +278,7 @@ moe_choose_kernel(const float* __restrict__ logits, int tokens, ChooseParams c) 
   moe_choose(c, token, sc, lane);
 }
 
-// Up to a token an SM: a block a token, a warp an expert's row, and the choice behind them in the same launch.
+// A block a token, a warp an expert's row, and the choice behind them in the same launch.
 template <typename T>
 __global__ void __launch_bounds__(1024)
 moe_route_token_kernel(RouteParams<T> p, ChooseParams c) {
@@ -286,7 +286,7 @@ moe_route_token_kernel(RouteParams<T> p, ChooseParams c) {
   extern __shared__ __align__(16) float choose_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, token = blockIdx.x;
   const T* x = p.x + (size_t)token * p.x_stride;
-  for (int e = warp; e < p.E + p.R; e += 32) {
+  for (int e = warp; e < p.E + p.R; e += blockDim.x / 32) {
     const float* w = p.row(e);
     float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int k0 = lane; k0 < p.K; k0 += ROUTE_AHEAD * 32) {
@@ -308,20 +308,26 @@ moe_route_token_kernel(RouteParams<T> p, ChooseParams c) {
   if (warp == 0) moe_choose(c, token, choose_smem, lane);
 }
 
-// Where the kernels change, measured with 32 experts of 4,096 in bf16 (the whole routing, cold caches; before these: a
-// block of one token, then of eight, that read x from shared memory for each expert apart): 8 tokens 18.6 us by a block a
-// token, 25.6 and 44 by the others (34.8 before); 96: 19.5, 27.6, 46 (31.7); 150: 29.6, 27.6, 44 (31.7); 256: 30.8, 27.7,
-// 44 (91); 400: 41, 42, 44 (91); 600: 61, 50, 46 (91); 2,048: 161, 114, 58 (94).  64 experts of 2,048, 16 of 1,024 and 32-bit
-// rows change at the same places.
-#define ROUTE_FEW_MAX 400
-// Batches of up to so many tokens are routed by one kernel (and need no logits in memory), others by two.
-extern "C" int kvb_moe_route_alone() { return kvb_sm_count() > 0 ? kvb_sm_count() : 148; }
+// Where the kernels change.  Microseconds of the whole routing in bf16 (B200, call by call) by a block a token, by four tokens
+// a block, by eight:
+//   32 experts of 4,096: 64 tokens 10.6, 10.9, 26; 148: 11.0, 11.4, 26; 150: 19.5, 11.6, 26; 400: 29, 22.6, 26; 520: 38, 26.8,
+//   26.8; 700: 47, 32, 26.5.  256 of 7,168: 64 tokens 87, 46, 243; 148: 87, 84, 243; 150: 172, 86, 243; 520: 340, 250, 247.
+//   8 of 4,096: 148 tokens 7.4, 10.9, 18; 700: 31, 12.1, 18.  16 of 1,024: 400 tokens 12.4, 8.7, 8.6.
+// A block a token is one launch and reads the whole router for each token: up to a token an SM; two of 16 warps fit an SM, which
+// is enough for routers of at most 16 rows (16 of 4,096, 150 and 296 tokens: 10.5 and 11.2, with 32 warps 13.5 and 14.6, by
+// four 11.1 and 11.5; 8 of 1,024: 4.6, 7.8, 6.6; 32 of 4,096: 17.0 by 16 warps, 11.6 by four).
+#define ROUTE_ALONE_ROWS 16
+static int route_sms() { return kvb_sm_count() > 0 ? kvb_sm_count() : 148; }
+static int route_few_max(int rows, int K) { return (K >= 2048 ? 500 : 340) * (rows <= 8 ? 2 : 1); }
+// Batches of up to so many tokens are routed by one kernel (and need no logits in memory), others by two.  `rows`: experts and
+// gate rows.
+extern "C" int kvb_moe_route_alone(int rows) { return rows <= ROUTE_ALONE_ROWS ? 2 * route_sms() : route_sms(); }
 
 template <typename T>
 static int launch_moe_logits(const RouteParams<T>& p, cudaStream_t stream) {
   // rows too long for shared memory take the few tokens' kernel at any number
   const size_t smem = (size_t)ROUTE_TOKENS * ((p.K + 127) / 128) * 128 * sizeof(T);
-  if (p.tokens > ROUTE_FEW_MAX && smem <= MOE_MOST_SMEM) {
+  if (p.tokens > route_few_max(p.E + p.R, p.K) && smem <= MOE_MOST_SMEM) {
     KVB_CHECK_CUDA(cudaFuncSetAttribute((moe_logits_kernel<T>), cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_MOST_SMEM));
     KVB_CHECK_CUDA(kvb_launch((moe_logits_kernel<T>), dim3((p.tokens + ROUTE_TOKENS - 1) / ROUTE_TOKENS), dim3(128), smem, stream,
                               true, p));
@@ -332,7 +338,7 @@ static int launch_moe_logits(const RouteParams<T>& p, cudaStream_t stream) {
   return 0;
 }
 
-// logits: scratch, [tokens, E + R]; none for up to kvb_moe_route_alone() tokens.
+// logits: scratch, [tokens, E + R]; none for up to kvb_moe_route_alone(E + R) tokens.
 extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, float* logits, const void* x,
                              long long x_stride, const float* router, const float* gate_rows, int tokens, int E, int R, int K,
                              int top, int score_mode, int renormalize, const float* correction, int groups, int keep,
@@ -347,16 +353,17 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
   KVB_REQUIRE((long long)E + R <= 65535, "moe_route: too many experts");
   size_t smem = (size_t)(2 * E + R + 2 * groups) * sizeof(float);
   KVB_REQUIRE((size_t)K * (dtype == KVB_F32 ? sizeof(float) : sizeof(bf16)) + smem <= MOE_MOST_SMEM,
-              "moe_route: a token's row and scores do not fit in shared memory");
+              "moe_route: a token's row and scores are more than 200 KB");
   const ChooseParams c = {ids_out, weights_out, gate_out, E, R, top, score_mode, renormalize, correction, groups, keep,
                           weight_scale, bias};
   const RouteParams<float> in32 = {logits, (const float*)x, x_stride, router, gate_rows, tokens, E, R, K};
   const RouteParams<bf16> in16 = {logits, (const bf16*)x, x_stride, router, gate_rows, tokens, E, R, K};
-  if (tokens <= kvb_moe_route_alone()) {
+  if (tokens <= kvb_moe_route_alone(E + R)) {
+    const int threads = tokens <= route_sms() ? 1024 : 512;
 #define KVB_ROUTE_TOKEN(T_, P_)                                                                                        \
     if (smem > 48 * 1024)                                                                                             \
       KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_route_token_kernel<T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_MOST_SMEM)); \
-    KVB_CHECK_CUDA(kvb_launch((moe_route_token_kernel<T_>), dim3(tokens), dim3(1024), smem, stream, true, P_, c))
+    KVB_CHECK_CUDA(kvb_launch((moe_route_token_kernel<T_>), dim3(tokens), dim3(threads), smem, stream, true, P_, c))
     if (dtype == KVB_F32) { KVB_ROUTE_TOKEN(float, in32); } else { KVB_ROUTE_TOKEN(bf16, in16); }
 #undef KVB_ROUTE_TOKEN
     KVB_CHECK_LAUNCH();

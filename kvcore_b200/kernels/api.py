@@ -145,7 +145,7 @@ def ensure_built(verbose: bool = False) -> str:
     lib.kvb_paged_attention_launches.restype = _int
     lib.kvb_moe_tile_rows.argtypes = []
     lib.kvb_moe_tile_rows.restype = _int
-    lib.kvb_moe_route_alone.argtypes = []
+    lib.kvb_moe_route_alone.argtypes = [_int]
     lib.kvb_moe_route_alone.restype = _int
     _lib = lib
     return str(path)
@@ -2137,7 +2137,7 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, top: int, *, score: str = "
             or group_keep * (experts // group_count) < top):
         raise KernelError(f"moe_route: {group_keep} of {group_count} groups of {experts} experts must hold {top} experts")
     ensure_built()
-    alone = tokens <= _lib.kvb_moe_route_alone()
+    alone = tokens <= _lib.kvb_moe_route_alone(experts + extra)
     logits = None if alone else torch.empty((tokens, experts + extra), dtype=torch.float32, device=x.device)
     _call("kvb_moe_route", ids.data_ptr(), weights.data_ptr(), None if gates is None else gates.data_ptr(),
           None if alone else logits.data_ptr(), x.data_ptr(), x.stride(0), router.data_ptr(), None if gate_rows is None else gate_rows.data_ptr(),

@@ -475,3 +475,18 @@ def test_threads_that_launch_one_kernel_with_different_shared_memory():
     for thread in threads:
         thread.join()
     assert not failures, failures
+
+
+@pytest.mark.parametrize("experts,width", [(16, 2048), (17, 130), (8, 2048), (5, 13000)])
+def test_router_bits_at_the_edges_of_its_kernels(experts, width):
+    """A block a token (32 warps, 16 warps), four tokens, eight, and rows of which eight do not fit in shared memory."""
+    sms, few = K().api.sm_count(torch.device(DEV)), (500 if width >= 2048 else 340) * (2 if experts <= 8 else 1)
+    x = randn(few + 1, width, dtype=torch.bfloat16, seed=1)
+    router = randn(experts, width, dtype=torch.float32, seed=2, scale=0.1)
+    ids, weights, _ = K().moe_route(x, router, 4, score="sigmoid")
+    for count in (1, sms, sms + 1, 2 * sms, 2 * sms + 1, few):
+        some = K().moe_route(x[few + 1 - count:], router, 4, score="sigmoid")
+        assert torch.equal(some[0], ids[few + 1 - count:]) and torch.equal(some[1], weights[few + 1 - count:]), count
+    z = x.double() @ router.double().T
+    bound = float((x.double().abs() @ router.double().abs().T).amax() * width * 2.0 ** -24) + 1e-6     # see the router's test above
+    torch.testing.assert_close(weights.double(), torch.sigmoid(z.gather(1, ids.long())), rtol=0, atol=bound)
