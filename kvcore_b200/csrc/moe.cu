@@ -21,8 +21,8 @@
 //            out = g * sigmoid(alpha g) * (u + shift).  Ungated with SQUARE: out = max(sum, 0)^2.
 //   Experts without tensors (the ids from E on) hand their input on: align leaves their pairs out, no product sees
 //   them, and the sum over a token's slots adds weight * the token's own input row for them.
-//   gemv:    the same two products for a handful of pairs in bf16, bound by the bytes of the chosen
-//            experts' matrices (no padded tiles); for more pairs, a tile's pairs share one pass (stream_rows).
+//   gemv:    the same two products for a handful of pairs in bf16, two of an expert a pass, bound by the bytes of the
+//            chosen experts' matrices (no padded tiles); for more pairs, a tile's pairs share one pass (stream_rows).
 //   gather:  the pairs' input rows expert by expert at a common stride, for one batched library product
 //            over all experts.
 //   combine: y[token] = sum over slots of out[row of (token, slot)] (ascending slot, 32-bit)

@@ -17,8 +17,8 @@
 //         S <- g_t S + B_t (dt_t x_t)^T,                o_t = S^T C_t + D_h x_t
 //         with B_t, C_t (one of each for a group of heads), x_t, dt_t, g_t as `ssm_prepare` (state_space.cu) left them;
 //   S is kept column by column ([H, V, D] in the state row: a column's D rows lie together).  A column is shared
-//   by RSPLIT neighbouring lanes (4, 8 or 16 rows each, in registers, loaded and stored as 16-byte pieces); a
-//   thread holds those rows of one column or of four neighbouring ones; a block owns 128 / RSPLIT (times four)
+//   by RSPLIT lanes of a warp, 32 / RSPLIT apart (4, 8 or 16 rows each, in registers, loaded and stored as 16-byte
+//   pieces); a thread holds those rows of one column or of four neighbouring ones; a block owns 128 / RSPLIT (times four)
 //   columns of one (request, head).  The launch picks the shape (see scan_shape).
 //   Columns never exchange anything, and a sum over a column's rows is taken in one fixed order (four rows at a
 //   time, then a tree over those pieces) whatever the shape, so any cut of a request into steps and any batch it
@@ -449,6 +449,10 @@ state_scan_kernel(ScanParams p) {
 // 310, 4 x 4 286, 16 x 1 362, 4 x 1 710 (before two rows of the state shared an instruction and threads shared the sums'
 // exchanges: 4 x 4 726); 8 heads: 298, 203, 231, 489; state space, 4 prompts of 400, 32 heads of 64: 118, 126, 154, 267;
 // delta rule, one prompt of 2,048, 16 heads of 128: 658, 462, 318, 670; 4 prompts of 512: 201, 279, 237, 597.
+// Few columns, one prompt of 300, fixed decay, as many entries as values: 4 heads of 16: 4 x 1 16.5, 4 x 4 32.8; 4 of 32: 16.0,
+// 27.5; 16 of 64 (4 x 1 in 128 blocks): 18.4, 29.6; 8 of 256 (8 x 1 in 512 blocks): 8 x 1 168, 8 x 4 56.8; keys of 256 and 4
+// heads of 128 values, one prompt and three (128 and 384 blocks): 8 x 1 46 and 94, 8 x 4 56 and 58.  Keys of 512, delta rule, 4
+// heads of 512, three prompts: 682 with four blocks an SM, 866 with the two that more registers leave.
 struct ScanShape { int rows, cols; bool brief; };
 static long long scan_blocks(int D, long long heads_of_all, int V, int rows, int cols) {
   int rsplit = 1;

@@ -2150,7 +2150,8 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, top: int, *, score: str = "
 # bf16 batches of at most this many (token, expert) pairs take the kernel that streams each chosen expert's
 # matrices once; larger ones take library products over each expert's run of rows
 MOE_GEMV_MAX_PAIRS = int(os.environ.get("KVCORE_B200_MOE_GEMV_PAIRS", "512"))
-# up to this many pairs, each pair streams its expert alone; otherwise the pairs are grouped by expert first
+# up to this many pairs, blocks find the pairs of their expert themselves and stream it for two at a time; otherwise the
+# pairs are grouped by expert first
 MOE_GEMV_SINGLE_PAIRS = int(os.environ.get("KVCORE_B200_MOE_GEMV_SINGLE_PAIRS", "16"))
 
 
