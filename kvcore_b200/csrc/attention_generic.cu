@@ -362,7 +362,8 @@ attention_few_kernel(AttParams<T> p) {
   const AttRequest a = att_request(p, req);
   const int segment = a.few ? part_no * ATT_SEGMENT : 0, row0 = a.few ? 0 : part_no * ATT_FEW, begin = a.begin;
   if (!(a.few || a.portion) || row0 >= a.rows) return;
-  if (segment > a.last) return;            // a longer request's segment (the fold does not read what was not written)
+  // a longer request's segment (the fold does not read what was not written), or one beyond the bound on the positions
+  if (segment > a.last || (a.few && part_no >= p.segments)) return;
   const int r = threadIdx.x >> 5, lane = threadIdx.x & 31, rows = min(ATT_FEW, a.rows - row0);     // a warp a row
   const bool live = r < rows;
   // every warp looks the rows up for itself, a lane a row
