@@ -362,8 +362,8 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
       const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;   // (the scale is positive); -inf stays -inf
       const float new_max = fmaxf(row_max, tile_max);
       // The maximum is moved (and O rescaled) only when it would grow by more than 2^8; but always within the first four
-      // key tiles that the query tile sees: a row's largest probability is then exactly one, which counts while it is a large part of the row (33
-      // tokens behind 300 are 11 % further from their values in 64 bits without).
+      // key tiles that the query tile sees: a row's largest probability is then exactly one, which counts while it is a
+      // large part of the row (33 tokens behind 300 are 11 % further from their values in 64 bits without).
       const bool grows = new_max > row_max + (turn < 4 ? 0.0f : 8.0f);       // from -inf too
       const bool move = __any_sync(0xffffffffu, grows);
       float correction = 1.0f;
@@ -401,10 +401,12 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
       }
       // Values of rows outside [key_lo, key_hi): thread r clears row r, in the first tile that reads this key tile's
       // values (A where it sees the tile), whose product waits for all its threads and is issued ahead of the other's.
-      if (key0 + r < key_lo || key0 + r >= key_hi) {
+      // (A warp with such rows waits and goes on as a whole: the tensor memory's instructions behind are the whole warp's.)
+      const bool nobodys = key0 + r < key_lo || key0 + r >= key_hi;
+      if ((j < n_a) == (x == 0) && __any_sync(0xffffffffu, nobodys)) {
         const int vs = j % VS;
-        if ((j < n_a) == (x == 0)) {
-          if (!RT_WAIT(&v_full[vs], (j / VS) & 1)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, RT_WAIT(&v_full[vs], (j / VS) & 1))) { ok = false; break; }
+        if (nobodys) {
           unsigned char* row = v_smem + vs * V_BYTES + r * 128;
 #pragma unroll
           for (int c = 0; c < 8; ++c) {              // (lanes start at different pieces: no bank conflicts)
@@ -413,6 +415,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
           }
           kvb_fence_async_shared();                  // generic writes -> visible to the product's reads
         }
+        __syncwarp();
       }
       kvb_tc5_wait_st();
       kvb_tc5_fence_before();

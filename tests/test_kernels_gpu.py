@@ -296,8 +296,8 @@ def test_flash_paged_attention(heads, kv_heads, dim, page, lens, window, splits)
 def test_prompt_attention_on_tcgen05_random_batches(seed):
     """Batches drawn at random for the tcgen05 prompt kernel (head size 128): group sizes that divide 128
     (queries by TMA) and 3 (queries copied), every page size, windows, contexts that end anywhere in a key
-    tile, portions that leave the second query tile of a block empty, partly filled, or one key tile behind
-    the first.  Against the general kernel (itself checked against the plain statement), the first seeds
+    tile, portions of one query tile and of several.  These launches are small enough for blocks of one query tile;
+    blocks of two have batches of their own in test_prompt_kernels_gpu.py.  Against the general kernel (itself checked against the plain statement), the first seeds
     against the plain statement as well."""
     import random
 
