@@ -18,12 +18,18 @@
 // Rows that nobody in the block sees are another request's, or what a page's former owner left there: their scores are
 // masked, and their values, which a probability of zero would not undo if they were no numbers, are cleared in shared
 // memory ahead of the product (pages that hold nothing but such rows are not read at all).
+// Weights go in as two bf16, the second what the first rounding left: the products are exact to 2^-18 of a weight, the row
+// sum is taken in 32 bits, and the maximum may lag behind (see below).  With one bf16 and that lag, rows that a few large
+// weights decide were up to 1.6 times as far from their values in 64 bits as the mma.sync tiles of attention_flash_dims.cu
+// leave them, whose running maximum makes the largest weights exact: 2,048 tokens with scores up to 15, 9.8e-4 of the result
+// and 6.1e-4; now 5e-6.
 // What bounds it is the chain of products and softmax of each query tile (see attention_prefill_tc5.cu), not a unit.
-// One prompt of 2,048 tokens, call by call (B200; mma.sync tiles of attention_flash_dims.cu before): carried-up latents,
-// 32 heads of 192 / 128: 96 us (394); 16 heads of two maps, 128 / 256: 150 us (432); 32 heads over 8, 128 / 128, window
-// 1,024, a sink: 106 us (245), with slopes 116 (245).  Few rows as well: 40 tokens behind 2,000: 79 us (188).
+// One prompt of 2,048 tokens, call by call (B200; in brackets what the weights' second half costs of it, and the mma.sync
+// tiles): carried-up latents, 32 heads of 192 / 128: 111 us (15; 394); 16 heads of two maps, 128 / 256: 179 us (29; 432);
+// 32 heads over 8, 128 / 128, window 1,024, a sink: 118 us (12; 245), with slopes 135 (19; 245).  Few rows as well: 40 tokens
+// behind 2,000: 89 us (10; 188).
 //
-// Tensor memory: 512 columns = S_A | S_B | O_A | O_B of 128 each; P_X lies over the first 64 columns of S_X.
+// Tensor memory: 512 columns = S_A | S_B | O_A | O_B of 128 each; P_X lies over S_X, the second halves in the last 64 columns.
 // Every wait is bounded: on a time-out the thread sets the WAIT_TIMEOUT status bit, the block drains, frees its tensor
 // memory and returns.
 #include <cuda.h>
@@ -75,10 +81,13 @@ __device__ __forceinline__ void rt_add2(float& s0, float& s1, float a0, float a1
       " mov.b64 {%0, %1}, rd;}\n"
       : "+f"(s0), "+f"(s1) : "f"(a0), "f"(a1));
 }
-// (lo, hi) rounded to two bf16 in one register, the lower key in the lower half, and back.  The row sum is taken of the
-// rounded values, so that the weights of a row add up to one whatever the rounding did.  (attention_prefill_tc5.cu cuts
-// instead of rounding, an instruction less for two, and sums what it cut from; rows of few keys are then further from
-// their values in 64 bits than the mixers served here were before.)
+// (h0, h1) and what they are short of (e0, e1): exact, since h is e rounded
+__device__ __forceinline__ void rt_short_of(float& d0, float& d1, float e0, float e1, float h0, float h1) {
+  asm("{.reg .b64 rh, rm, re, rd;\n mov.b64 rh, {%4, %5};\n mov.b64 rm, {%6, %6};\n mov.b64 re, {%2, %3};\n"
+      " fma.rn.f32x2 rd, rh, rm, re;\n mov.b64 {%0, %1}, rd;}\n"
+      : "=f"(d0), "=f"(d1) : "f"(e0), "f"(e1), "f"(h0), "f"(h1), "f"(-1.0f));
+}
+// (lo, hi) rounded to two bf16 in one register, the lower key in the lower half, and back.
 __device__ __forceinline__ float rt_pack(float lo, float hi) {
   unsigned d;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
@@ -265,6 +274,7 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
       };
       auto issue_pv = [&](int x, int st, bool add) {
         kvb_tc5_mma8_ts<8, 128>(tmem_base + 256 + x * RT_V, tmem_base + x * RT_BN, v_desc[st], idesc_pv, add ? 1u : 0u);
+        kvb_tc5_mma8_ts<8, 128>(tmem_base + 256 + x * RT_V, tmem_base + x * RT_BN + 64, v_desc[st], idesc_pv, 1u);
         kvb_tc5_commit(&pv_done[x]);
       };
       if (p.q_by_tma && !RT_WAIT(q_full, 0)) ok = false;
@@ -361,10 +371,8 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
         for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = rt_max3(mx[(i >> 1) & 3], s[c][i], s[c][i + 1]);
       const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;   // (the scale is positive); -inf stays -inf
       const float new_max = fmaxf(row_max, tile_max);
-      // The maximum is moved (and O rescaled) only when it would grow by more than 2^8; but always within the first four
-      // key tiles that the query tile sees: a row's largest probability is then exactly one, which counts while it is a
-      // large part of the row (33 tokens behind 300 are 11 % further from their values in 64 bits without).
-      const bool grows = new_max > row_max + (turn < 4 ? 0.0f : 8.0f);       // from -inf too
+      // The maximum is moved (and O rescaled) only when it would grow by more than 2^8.
+      const bool grows = new_max > row_max + 8.0f;                       // from -inf too
       const bool move = __any_sync(0xffffffffu, grows);
       float correction = 1.0f;
       if (move) {
@@ -375,17 +383,20 @@ flash_rows_tc5_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
       float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        float packed[16];                            // 32 keys, two bf16 a register
+        float packed[16], rest[16];                  // 32 keys, two bf16 a register
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           float a0, a1, e0, e1;
           rt_fma2(a0, a1, s[c][i], s[c][i + 1], scale_log2, shift);      // masked entries stay -inf
           asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(a0));
           asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(a1));
+          rt_add2(sm[i & 2], sm[(i & 2) + 1], e0, e1);
           packed[i / 2] = rt_pack(e0, e1);
-          rt_add2(sm[i & 2], sm[(i & 2) + 1], rt_low(packed[i / 2]), rt_high(packed[i / 2]));
+          rt_short_of(a0, a1, e0, e1, rt_low(packed[i / 2]), rt_high(packed[i / 2]));
+          rest[i / 2] = rt_pack(a0, a1);
         }
         kvb_tc5_st16(s_addr + c * 16, packed);       // over S(j); S(j+1) comes after the tensor pipe has taken P(j)
+        kvb_tc5_st16(s_addr + 64 + c * 16, rest);
       }
       row_sum = row_sum * correction + ((sm[0] + sm[1]) + (sm[2] + sm[3]));
       if (move && turn > 0) {                        // P(j-1).V(j-1) has landed: it was issued before S(j)

@@ -1354,7 +1354,7 @@ def _flash_dims(out, q, keys, values, table, ctx, value_heads, group, maps, key_
                                                  value_strides, scale, softcap, rows_in_order)
     for run, run_table in runs:
         max_rows = run.max_query_len * group
-        if tc5 and max_rows > 32:            # beyond the few-row form, at any length (from 40 rows behind 2,000 keys: 79 us, 188)
+        if tc5 and max_rows > 32:            # beyond the few-row form, at any length (from 40 rows behind 2,000 keys: 89 us, 188)
             _call("kvb_flash_rows_tc5", out.data_ptr(), out.stride(0), out.stride(1), int(out.dtype == torch.float32),
                   q.data_ptr(), q.stride(0), q.stride(1), keys.data_ptr(), values.data_ptr(),
                   key_strides[0] if rows_in_order else key_strides[2], key_strides[1], value_strides[1],

@@ -490,3 +490,24 @@ def test_router_bits_at_the_edges_of_its_kernels(experts, width):
     z = x.double() @ router.double().T
     bound = float((x.double().abs() @ router.double().abs().T).amax() * width * 2.0 ** -24) + 1e-6     # see the router's test above
     torch.testing.assert_close(weights.double(), torch.sigmoid(z.gather(1, ids.long())), rtol=0, atol=bound)
+
+
+@pytest.mark.parametrize("lens", [[(0, 33)], [(0, 2047)], [(1500, 548), (0, 130)]])
+@pytest.mark.parametrize("turned,window,scale", [(64, None, 1.0), (64, None, 3.0), (0, None, 3.0), (64, 200, 3.0)])
+def test_rows_keep_32_bits_of_the_weights(lens, turned, window, scale):
+    """Flat rows and rows that a few large weights decide, of one key tile and of many, against 64 bits and the kernel of the
+    other shapes.  Weights go in as two bf16 (2^-18 of a weight at most), scores and sums are 32-bit (a score of up to 32
+    off by 2^-20 shifts its weight by as much): below 2^-15 in all."""
+    heads, dk = 4, 128 + turned
+    attend, carried, own = _rows_in_order(lens, heads, turned, window)
+    how = dict(scale=scale * dk ** -0.5, out_dtype=torch.float32)
+    keys, values = [], []
+    for (cached, n), rows in zip(lens, own):
+        seen = torch.zeros(cached + n, heads, 256 + turned, dtype=torch.bfloat16, device=DEV)
+        seen[cached + n - (rows.stop - rows.start):] = carried[rows].unflatten(1, (heads, 256 + turned))
+        keys.append(seen[..., :dk])
+        values.append(seen[..., dk:])
+    q = randn(sum(n for _, n in lens), heads, dk, dtype=torch.bfloat16, seed=2)
+    want = _attend(q, keys, values, lens, dict(group=1, maps=1, scale=how["scale"], window=window, sink=None, slopes=None))
+    got, other = (float((t.double() - want).norm() / want.norm()) for t in (attend(carried, **how), attend(carried, num_splits=1, **how)))
+    assert got <= min(other, 2.0 ** -15) and K().read_status() == 0, (got, other)
