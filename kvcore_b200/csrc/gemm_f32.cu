@@ -1,5 +1,6 @@
 // True 32-bit linear layer: out[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]), FMA on the CUDA
-// cores only, no tensor cores and no reduced-precision mode.
+// cores only, no tensor cores and no reduced-precision mode.  Matrices with K from 2,048 on take gemm_f32_tc5.cu, whatever
+// the rows.
 //
 // Every output element is one accumulator that takes its products in ascending k, so its value
 // does not depend on M, on the kernel or the tile it falls in, or on the rest of the batch: the

@@ -193,6 +193,33 @@ __device__ __forceinline__ void kvb_tc5_mma8_ts(unsigned tmem_d, unsigned tmem_a
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, q;\n}\n"
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(A_COLS), "n"(B_STEP) : "memory");
 }
+// One lane of a converged warp: the one that issues.  A whole warp that runs the issuing loop and leaves only the instructions
+// themselves to this lane lets the compiler keep descriptors in uniform registers, where tcgen05.mma takes them from; a loop
+// that one lane runs alone moves them there for every instruction (62 cycles an instruction, whatever its size).
+__device__ __forceinline__ unsigned kvb_elect() {
+  unsigned leader;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
+  return leader;
+}
+// Four products by the lane with `leader`, A in tensor memory: a k-range of 64.
+template <int A_COLS, int B_STEP>
+__device__ __forceinline__ void kvb_tc5_mma4_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc,
+                                                unsigned idesc, unsigned accumulate, unsigned leader) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    asm volatile(
+        "{\n.reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a + i * A_COLS), "l"(bdesc + (unsigned long long)(i * B_STEP)), "r"(idesc),
+          "r"(i == 0 ? accumulate : 1u), "r"(leader) : "memory");
+}
+// The barrier gets an arrival when every MMA that the lane with `leader` issued so far has finished.
+__device__ __forceinline__ void kvb_tc5_commit_by(unsigned long long* bar, unsigned leader) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n"
+               "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
+               ::"r"(kvb_smem(bar)), "r"(leader) : "memory");
+}
 // The barrier gets an arrival when every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void kvb_tc5_commit(unsigned long long* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(kvb_smem(bar)) : "memory");

@@ -72,6 +72,8 @@ def ensure_built(verbose: bool = False) -> str:
         "kvb_flash_prefill_tc5": [_vp, _ll, _vp, _ll, _vp, _vp, _vp, _int, _vp, _vp, _int, _int, _int, _int, _int,
                                   _int, _int, _int, _float, _int, _vp, _vp, _float, _vp],
         "kvb_gemm_f32": [_vp, _vp, _vp, _vp, _int, _int, _int, _ll, _ll, _vp],
+        "kvb_gemm_f32_split": [_vp, _vp, _vp, _vp, _int, _int, _int, _ll, _ll, _vp, _vp],
+        "kvb_gemm_f32_split_launches": [_int, _int, _int],
         "kvb_rms_norm_shift": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _float, _int, _int, _int, _vp],
         "kvb_stream_add_norm": [_vp, _vp, _vp, _vp, _int, _int, _float, _vp, _vp, _ll, _vp, _int, _vp, _int, _int, _vp],
         "kvb_attention_dims_rows": [_vp, _ll, _ll, _int, _vp, _ll, _ll, _vp, _ll, _ll, _ll, _vp, _ll, _ll, _ll, _vp,
@@ -134,6 +136,12 @@ def ensure_built(verbose: bool = False) -> str:
     # Kernels of this library overlap their start with the end of the kernel in front of them
     # (programmatic dependent launch); KVCORE_B200_SERIAL_LAUNCH=1 switches that off.
     lib.kvb_set_pdl(0 if os.environ.get("KVCORE_B200_SERIAL_LAUNCH") == "1" else 1)
+    lib.kvb_gemm_f32_split_min_k.argtypes = []
+    lib.kvb_gemm_f32_split_min_k.restype = _int
+    if lib.kvb_gemm_f32_split_min_k() != _F32_SPLIT_MIN_K:
+        raise KernelError("the library and this module disagree about where 32-bit products take the tensor cores")
+    lib.kvb_gemm_f32_split_scratch.argtypes = [_vp, _int, _int, _int]
+    lib.kvb_gemm_f32_split_scratch.restype = _ll
     lib.kvb_gemm_stream_scratch_floats.argtypes = [_int]
     lib.kvb_gemm_stream_scratch_floats.restype = _ll
     lib.kvb_gemm_stream_norm_max_k.argtypes = []
@@ -744,7 +752,7 @@ TRACE_TAGS = {27: "rms_norm_shift", 28: "stream_add_norm", 29: "attention_dims_r
               7: "flash_paged", 8: "flash_combine", 9: "flash_decode_tma", 10: "flash_decode_combine",
               11: "flash_prefill_tc5", 12: "gemm_f32", 13: "gemm_stream", 14: "sample", 16: "feed_tokens"}
 _TRACE_UNITS = ("elementwise", "attention_decode_tma", "attention_flash", "attention_generic",
-                "attention_prefill_tc5", "attention_rows_tc5", "gemm_f32", "sampling", "gemm_stream", "layer_norm", "qk_prepare", "moe", "attention_kept_first",
+                "attention_prefill_tc5", "attention_rows_tc5", "gemm_f32", "gemm_f32_tc5", "sampling", "gemm_stream", "layer_norm", "qk_prepare", "moe", "attention_kept_first",
                 "stream_norm", "attention_dims", "mixer_prepare", "attention_flash_dims", "recurrence", "turn_norm",
                 "state_space", "stream_rows", "fixed_decay", "attention_prepare")
 _trace_buffer: torch.Tensor | None = None
@@ -830,6 +838,29 @@ def linear_stream(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | No
     return out
 
 
+_F32_SPLIT_MIN_K = 2048       # K from which a 32-bit product may take the tensor cores (gemm_f32_tc5.cu; checked at load)
+
+
+def _linear_f32(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None) -> None:
+    """``out = x @ weight.T (+ bias)`` in float32; rows of ``x`` and ``out`` may lie apart.  Large weights take the
+    tensor cores in pieces of bf16 (``gemm_f32_tc5.cu``), small ones FMA: by ``weight`` alone, so that a row's bits do not
+    depend on the batch it is in."""
+    m, k = x.shape
+    n = weight.shape[0]
+    args = (out.data_ptr(), x.data_ptr(), weight.data_ptr(), None if bias is None else bias.data_ptr(), m, n, k,
+            x.stride(0), out.stride(0))
+    if k >= _F32_SPLIT_MIN_K:
+        if _lib is None:
+            ensure_built()
+        scratch_bytes = _lib.kvb_gemm_f32_split_scratch(weight.data_ptr(), m, n, k)
+        if scratch_bytes > 0:
+            scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=x.device)
+            _call("kvb_gemm_f32_split", *args, scratch.data_ptr(), _stream(),
+                  kernels=_lib.kvb_gemm_f32_split_launches(m, n, k))
+            return
+    _call("kvb_gemm_f32", *args, _stream())
+
+
 def linear(
     x: torch.Tensor,
     weight: torch.Tensor,
@@ -839,7 +870,7 @@ def linear(
 ) -> torch.Tensor:
     """``x @ weight.T (+ bias)`` for ``x [M, K]``, ``weight [N, K]``.
 
-    float32: this package's own FMA kernel (no tensor cores, fixed summation order).
+    float32: this package's own kernels (32-bit operands and sums, an order that depends on ``weight`` alone).
     bfloat16: the library matrix product with 32-bit accumulation.
     ``out_dtype=float32`` keeps the accumulator's precision in the result (the logits).
     """
@@ -854,8 +885,7 @@ def linear(
     n = weight.shape[0]
     if x.dtype == torch.float32:
         out = torch.empty((m, n), dtype=torch.float32, device=x.device)
-        _call("kvb_gemm_f32", out.data_ptr(), x.data_ptr(), weight.data_ptr(),
-              None if bias is None else bias.data_ptr(), m, n, k, x.stride(0), out.stride(0), _stream())
+        _linear_f32(out, x, weight, bias)
         return out
     # Decode-sized batches: the layer is one pass over the weights, which this library's own
     # streaming kernel does, overlapping its start with the kernels in front of it.
@@ -1538,7 +1568,7 @@ def sigmoid_gate_mul(o: torch.Tensor, gate: torch.Tensor, out: torch.Tensor | No
 
 def heads_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """A product per head: ``x [T, H, K]`` (a view; last stride 1) with ``weight [H, N, K]`` -> ``[T, H, N]``
-    (a view when the batched library product made it; into ``out``, a view with last stride 1, when given).  float32: this package's own FMA kernel, head by head; bfloat16: one batched library product."""
+    (a view when the batched library product made it; into ``out``, a view with last stride 1, when given).  float32: this package's own kernels, head by head; bfloat16: one batched library product."""
     _check(x, "x", contiguous=False)
     _check(weight, "weight", dtype=x.dtype)
     tokens, heads, k = x.shape
@@ -1551,8 +1581,7 @@ def heads_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None
         if tuple(out.shape) != (tokens, heads, n) or out.stride(2) != 1:
             raise KernelError(f"heads_linear: out {tuple(out.shape)} does not fit")
         for h in range(heads):
-            _call("kvb_gemm_f32", out[:, h].data_ptr(), x[:, h].data_ptr(), weight[h].data_ptr(), None, tokens, n, k,
-                  x.stride(0), out.stride(0), _stream())
+            _linear_f32(out[:, h], x[:, h], weight[h], None)
         return out
     if out is not None:                     # the library writes the rows where they belong
         if tuple(out.shape) != (tokens, heads, n) or out.stride(2) != 1:

@@ -161,3 +161,67 @@ def test_product_rows_have_the_same_bits_in_every_tile(m, n, k, tile):
     full = K().linear(x, w, bias)
     for first in (0, 63, 127, 240, m - 16):
         assert torch.equal(K().linear(x[first:first + 16].contiguous(), w, bias), full[first:first + 16]), first
+
+
+@pytest.mark.parametrize("n,k", [(128, 2048), (130, 2052), (515, 2108), (9601, 2048), (3072, 3072), (16390, 2064)])
+def test_product_in_pieces_has_the_same_bits_for_every_number_of_rows(n, k):
+    """Weights from K 2,048 on: tiles of 16 to 128 rows, ragged columns, k and last chunks, one stretch of K and several; rows
+    off 16-byte boundaries.  A float is three bf16 exactly and three of nine products are left out (2^-26 of a term each);
+    a chunk's accumulator may lose one unit of 2^-23 at each of 24 additions of up to its 64 terms, 2^-18.4 of them; and
+    k / 64 + 16 sums are rounded to nearest."""
+    x, w = randn(300, k, dtype=torch.float32, seed=1), randn(n, k, dtype=torch.float32, seed=2)
+    bias = randn(n, dtype=torch.float32, seed=3)
+    full = K().linear(x, w, bias)
+    terms = x.double().abs() @ w.double().abs().T + bias.double().abs()
+    error = (full.double() - (x.double() @ w.double().T + bias.double())).abs()
+    assert (error <= terms * (24 * 2.0 ** -23 + (k / 64 + 20) * 2.0 ** -24)).all()
+    by_fma = K().api
+    out = torch.empty_like(full)
+    by_fma._call("kvb_gemm_f32", out.data_ptr(), x.data_ptr(), w.data_ptr(), bias.data_ptr(), 300, n, k, k, n, by_fma._stream())
+    assert error.norm() <= (out.double() - (x.double() @ w.double().T + bias.double())).norm()
+    for rows in (1, 16, 17, 32, 33, 64, 65, 128, 129, 200):
+        assert torch.equal(K().linear(x[:rows].contiguous(), w, bias), full[:rows]), rows
+    wide = torch.zeros(20, k + 3, dtype=torch.float32, device=DEV)
+    wide[:, 3:] = x[:20]
+    assert torch.equal(K().linear(wide[:, 3:], w, bias), full[:20])
+    assert K().read_status() == 0
+
+
+def test_product_in_pieces_takes_many_rows_in_lots():
+    """More rows than the scratch for sums of stretches holds (2,048 at eight stretches of 2,048 columns)."""
+    x, w = randn(2200, 2048, dtype=torch.float32, seed=1), randn(2048, 2048, dtype=torch.float32, seed=2)
+    full = K().linear(x, w)
+    for first in (0, 1900, 2040, 2184):
+        assert torch.equal(K().linear(x[first:first + 16].contiguous(), w), full[first:first + 16]), first
+
+
+def test_product_in_pieces_of_numbers_that_are_not_finite_or_too_large_for_bf16():
+    """Infinities, NaN, numbers above the largest bf16 and sums that leave the range: as the product by FMA has them.  Numbers
+    down to 2^-110 keep their bits (all three pieces are above the smallest bf16)."""
+    x, w = randn(40, 2048, dtype=torch.float32, seed=1), randn(256, 2048, dtype=torch.float32, seed=2)
+    x[3, 5] = float("inf")
+    x[4, 7] = float("nan")
+    x[5, 64], x[5, 65] = float("inf"), float("-inf")
+    x[6, 0] = 3.4e38
+    w[9, 0] = 0.0
+    w[:, 5][17] = 0.0
+    w[20, 100] = float("-inf")
+    w[21, 2047] = float("nan")
+    x[30] *= 2.0 ** 126
+    w[30] *= 2.0 ** 126
+    x[31] *= 2.0 ** -100
+    got, api = K().linear(x, w), K().api
+    want = torch.empty_like(got)
+    api._call("kvb_gemm_f32", want.data_ptr(), x.data_ptr(), w.data_ptr(), None, 40, 256, 2048, 2048, 256, api._stream())
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    both = want.isfinite()
+    terms = (x.double().nan_to_num(0, 0, 0).abs() @ w.double().nan_to_num(0, 0, 0).abs().T)[both]
+    assert ((got - want)[both].double().abs() <= terms * 2049 * 2.0 ** -24).all()
+
+
+def test_heads_product_in_pieces():
+    x, w = randn(20, 3, 2048, dtype=torch.float32, seed=1), randn(3, 130, 2048, dtype=torch.float32, seed=2)
+    got = K().heads_linear(x, w)
+    for h in range(3):
+        assert torch.equal(got[:, h], K().linear(x[:, h].contiguous(), w[h]))
