@@ -383,14 +383,17 @@ extern "C" int kvb_moe_route(int* ids_out, float* weights_out, float* gate_out, 
 }
 
 // sorted [capacity] (capacity = MOE_BM * min(pairs, ceil((pairs + experts * (MOE_BM - 1)) / MOE_BM))),
-// tile_expert [capacity / MOE_BM], meta[0] = tiles used.
+// tile_expert [capacity / MOE_BM], meta[0] = tiles used.  row_tiles (or null): the runs cut into tiles of at most tile_rows rows
+// for kvb_moe_grouped, {expert, first row, rows | tiles of the expert << 12, the expert's first tile}, meta[1] of them (at most
+// the experts with pairs + capacity / tile_rows).
 // One block, bound by the latency of its reads and of the shared counters.  8,192 pairs of 32 experts (B200, cold caches):
 // 9.8 us; 17.4 with the choices read one after the other, twice, and the begins summed by one thread.
 #define ALIGN_AHEAD 8
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(int* __restrict__ sorted, int* __restrict__ tile_expert, int* __restrict__ meta,
                  int* __restrict__ row_of_pair, int* __restrict__ expert_begin,
-                 const int* __restrict__ ids, int pairs, int E, int known, int capacity, int* status) {
+                 const int* __restrict__ ids, int pairs, int E, int known, int capacity, int4* __restrict__ row_tiles, int tile_rows,
+                 int* status) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_ALIGN);
   extern __shared__ int ismem[];
   int* counts = ismem;        // [E]
@@ -421,7 +424,7 @@ moe_align_kernel(int* __restrict__ sorted, int* __restrict__ tile_expert, int* _
   }
   __syncthreads();
   if (threadIdx.x < 32) {                // the runs' begins: sums over the experts in front, a warp's worth at a time
-    int at = 0;
+    int at = 0, tiles_at = 0;
     for (int e0 = 0; e0 < E; e0 += 32) {
       const int e = e0 + threadIdx.x;
       const int rows = e < E ? (counts[e] + MOE_BM - 1) / MOE_BM * MOE_BM : 0;
@@ -438,10 +441,28 @@ moe_align_kernel(int* __restrict__ sorted, int* __restrict__ tile_expert, int* _
         counts[e] = 0;                   // becomes the fill cursor
         if (expert_begin != nullptr) expert_begin[e] = begin;   // where each expert's (padded) run of rows begins
       }
+      if (row_tiles != nullptr) {        // the run in as few tiles of tile_rows as hold it, equal but for MOE_BM rows
+        const int mine = (rows + tile_rows - 1) / tile_rows;
+        int tiles_upto = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+          const int below = __shfl_up_sync(0xffffffffu, tiles_upto, d);
+          if ((int)threadIdx.x >= d) tiles_upto += below;
+        }
+        const int first = tiles_at + tiles_upto - mine;
+        int row = at + upto - rows;
+        for (int t = 0; t < mine; ++t) {
+          const int units = rows / MOE_BM / mine + (t < rows / MOE_BM % mine ? 1 : 0);
+          row_tiles[first + t] = make_int4(e, row, units * MOE_BM | mine << 12, first);
+          row += units * MOE_BM;
+        }
+        tiles_at += __shfl_sync(0xffffffffu, tiles_upto, 31);
+      }
       at += __shfl_sync(0xffffffffu, upto, 31);
     }
     if (threadIdx.x == 0) {
       meta[0] = at / MOE_BM;
+      meta[1] = tiles_at;
       if (expert_begin != nullptr) expert_begin[E] = at;        // ... and the end of the last
     }
   }
@@ -466,8 +487,11 @@ moe_align_kernel(int* __restrict__ sorted, int* __restrict__ tile_expert, int* _
 }
 
 extern "C" int kvb_moe_align(int* sorted, int* tile_expert, int* meta, int* row_of_pair, int* expert_begin,
-                             const int* ids, int pairs, int E, int known, int capacity, cudaStream_t stream) {
+                             const int* ids, int pairs, int E, int known, int capacity, int* row_tiles, int tile_rows,
+                             cudaStream_t stream) {
   if (pairs == 0) return 0;
+  KVB_REQUIRE(row_tiles == nullptr || (aligned16(row_tiles) && tile_rows >= MOE_BM && tile_rows < 4096 && tile_rows % MOE_BM == 0),
+              "moe_align: the row tiles' table or size");
   KVB_REQUIRE(E > 0 && E <= 8192 && known >= E, "moe_align: between 1 and 8192 experts");
   // tiles used: one per started run of MOE_BM pairs of an expert, so at most one per pair
   const long long padded = (pairs + (long long)E * (MOE_BM - 1) + MOE_BM - 1) / MOE_BM;
@@ -476,7 +500,7 @@ extern "C" int kvb_moe_align(int* sorted, int* tile_expert, int* meta, int* row_
   int* status = kvb_status_word();
   KVB_REQUIRE(status != nullptr, "moe_align: no status word");
   KVB_CHECK_CUDA(kvb_launch((moe_align_kernel), dim3(1), dim3(1024), (size_t)2 * E * sizeof(int), stream, true,
-                            sorted, tile_expert, meta, row_of_pair, expert_begin, ids, pairs, E, known, capacity, status));
+                            sorted, tile_expert, meta, row_of_pair, expert_begin, ids, pairs, E, known, capacity, (int4*)row_tiles, tile_rows, status));
   KVB_CHECK_LAUNCH();
   return 0;
 }
@@ -884,15 +908,15 @@ extern "C" int kvb_moe_stream_rows(void* out, const void* a, long long a_stride,
 
 // Rows in the grouped order for batched library products: expert e owns rows [e * C, (e + 1) * C) of `out`;
 // row e * C + j holds weight(p) * a[p / a_row_div] for the j-th pair p of the expert (sorted[expert_begin[e] + j]),
-// zeros beyond the expert's pairs.  row_of_pair[p] is set to the row that pair p got.
+// zeros beyond the expert's pairs; without expert_begin (E is 1 then) the order of `sorted` itself.  row_of_pair[p] is set to the row that pair p got.
 template <typename T, bool VEC>
 __global__ void moe_gather_kernel(T* __restrict__ out, const T* __restrict__ a, long long a_stride, int a_row_div,
                                   const float* __restrict__ pair_weight, const int* __restrict__ sorted,
                                   const int* __restrict__ expert_begin, int C, int* __restrict__ row_of_pair, int K) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_GATHER);
   const int e = blockIdx.x / C, j = blockIdx.x % C;
-  const int at = expert_begin[e] + j;
-  const int pair = at < expert_begin[e + 1] ? sorted[at] : -1;
+  const int at = (expert_begin != nullptr ? expert_begin[e] : 0) + j;
+  const int pair = expert_begin == nullptr || at < expert_begin[e + 1] ? sorted[at] : -1;
   T* dst = out + (size_t)blockIdx.x * K;
   constexpr int N = VEC ? Vec16<T>::N : 1;
   if (pair < 0) {
@@ -924,7 +948,7 @@ extern "C" int kvb_moe_gather(void* out, const void* a, long long a_stride, int 
                               const int* sorted, const int* expert_begin, int E, int C, int* row_of_pair, int K,
                               int dtype, cudaStream_t stream) {
   if (E == 0 || C == 0) return 0;
-  KVB_REQUIRE(K > 0 && a_row_div > 0 && row_of_pair != nullptr, "moe_gather: empty rows");
+  KVB_REQUIRE(K > 0 && a_row_div > 0 && row_of_pair != nullptr && (E == 1 || expert_begin != nullptr), "moe_gather: empty rows");
   const int esize = dtype == KVB_F32 ? 4 : 2;
   const bool vec = ((size_t)K * esize) % 16 == 0 && ((size_t)a_stride * esize) % 16 == 0 && aligned16(out) && aligned16(a);
   const long long rows = (long long)E * C;

@@ -201,6 +201,15 @@ __device__ __forceinline__ unsigned kvb_elect() {
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
   return leader;
 }
+// D[tmem] (+)= A[smem] . B[smem], issued by the lane with `leader`.
+__device__ __forceinline__ void kvb_tc5_mma_by(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
+                                               unsigned idesc, unsigned accumulate, unsigned leader) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n"
+      "setp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
 // Four products by the lane with `leader`, A in tensor memory: a k-range of 64.
 template <int A_COLS, int B_STEP>
 __device__ __forceinline__ void kvb_tc5_mma4_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc,

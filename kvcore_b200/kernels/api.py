@@ -53,7 +53,9 @@ def ensure_built(verbose: bool = False) -> str:
         "kvb_glu_clamped": [_vp, _vp, _int, _int, _float, _float, _float, _int, _vp],
         "kvb_moe_route": [_vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _int, _int, _int, _int, _int, _int, _int, _vp, _int, _int,
                           _float, _vp, _int, _vp],
-        "kvb_moe_align": [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _vp],
+        "kvb_moe_align": [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _vp, _int, _vp],
+        "kvb_moe_grouped": [_vp, _vp, _vp, _vp, _vp, _ll, _int, _int, _int, _int, _int, _float, _float, _float, _vp],
+        "kvb_moe_grouped_rows": [_ll, _int],
         "kvb_moe_gemv": [_vp, _vp, _ll, _int, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _float, _float, _float, _vp],
         "kvb_moe_stream_rows": [_vp, _vp, _ll, _int, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _float, _float,
                                 _float, _vp],
@@ -752,7 +754,7 @@ TRACE_TAGS = {27: "rms_norm_shift", 28: "stream_add_norm", 29: "attention_dims_r
               7: "flash_paged", 8: "flash_combine", 9: "flash_decode_tma", 10: "flash_decode_combine",
               11: "flash_prefill_tc5", 12: "gemm_f32", 13: "gemm_stream", 14: "sample", 16: "feed_tokens"}
 _TRACE_UNITS = ("elementwise", "attention_decode_tma", "attention_flash", "attention_generic",
-                "attention_prefill_tc5", "attention_rows_tc5", "gemm_f32", "gemm_f32_tc5", "sampling", "gemm_stream", "layer_norm", "qk_prepare", "moe", "attention_kept_first",
+                "attention_prefill_tc5", "attention_rows_tc5", "gemm_f32", "gemm_f32_tc5", "sampling", "gemm_stream", "layer_norm", "qk_prepare", "moe", "moe_tc5", "attention_kept_first",
                 "stream_norm", "attention_dims", "mixer_prepare", "attention_flash_dims", "recurrence", "turn_norm",
                 "state_space", "stream_rows", "fixed_decay", "attention_prepare")
 _trace_buffer: torch.Tensor | None = None
@@ -2203,18 +2205,20 @@ class ExpertGrouping:
     counts on their way to the host: ``begins()`` waits for that copy alone, not for the stream."""
 
     __slots__ = ("sorted_pairs", "tile_expert", "meta", "row_of_pair", "expert_begin", "max_tiles", "capacity",
-                 "_host", "_ready")
+                 "row_tiles", "tile_rows", "_host", "_ready")
 
     def begins(self) -> list[int]:
         self._ready.synchronize()
         return self._host.tolist()
 
 
-def moe_group(ids: torch.Tensor, experts: int, *, for_library: bool, identity: int = 0) -> ExpertGrouping:
+def moe_group(ids: torch.Tensor, experts: int, *, for_library: bool, identity: int = 0,
+              for_grouped: bool = False) -> ExpertGrouping:
     """Group the pairs ``t * top + s`` of ``ids [T, top]`` by expert (the ``identity`` ids behind ``experts`` are left out).  ``for_library``: also the row of every
     pair and where each expert's run begins, the latter copied to pinned host memory behind an event, so that
     a caller who has other work to launch first (a layer whose mixer runs beside its feed-forward) finds the
-    counts there when it comes back, without draining the stream."""
+    counts there when it comes back, without draining the stream.  ``for_grouped``: the row of every pair, and the
+    runs cut into the row tiles of the grouped products; the host learns nothing of them."""
     _check(ids, "ids", dtype=torch.int32)
     pairs = ids.numel()
     tile = int(_lib.kvb_moe_tile_rows())
@@ -2224,13 +2228,17 @@ def moe_group(ids: torch.Tensor, experts: int, *, for_library: bool, identity: i
     g.sorted_pairs = torch.empty(g.capacity, dtype=torch.int32, device=ids.device)
     g.tile_expert = torch.empty(g.max_tiles, dtype=torch.int32, device=ids.device)
     g.meta = torch.empty(4, dtype=torch.int32, device=ids.device)
-    g.row_of_pair = torch.empty(pairs, dtype=torch.int32, device=ids.device) if for_library else None
+    g.row_of_pair = torch.empty(pairs, dtype=torch.int32, device=ids.device) if for_library or for_grouped else None
     g.expert_begin = torch.empty(experts + 1, dtype=torch.int32, device=ids.device) if for_library else None
-    g._host = g._ready = None
+    g._host = g._ready = g.row_tiles = None
+    g.tile_rows = 0
+    if for_grouped:
+        g.tile_rows = int(_lib.kvb_moe_grouped_rows(pairs, experts))
+        g.row_tiles = torch.empty((min(pairs, experts) + g.capacity // g.tile_rows, 4), dtype=torch.int32, device=ids.device)
     _call("kvb_moe_align", g.sorted_pairs.data_ptr(), g.tile_expert.data_ptr(), g.meta.data_ptr(),
           None if g.row_of_pair is None else g.row_of_pair.data_ptr(),
           None if g.expert_begin is None else g.expert_begin.data_ptr(), ids.data_ptr(), pairs, experts,
-          experts + int(identity), g.capacity,
+          experts + int(identity), g.capacity, None if g.row_tiles is None else g.row_tiles.data_ptr(), g.tile_rows,
           _stream())
     if for_library:
         g._host = torch.empty(experts + 1, dtype=torch.int32, pin_memory=True)
@@ -2247,23 +2255,15 @@ def _rounded_rows(rows: int) -> int:
     return -(-rows // unit) * unit
 
 
-_one_runs: dict[torch.device, torch.Tensor] = {}
-
-
-def _one_run(device: torch.device) -> torch.Tensor:
-    """Bounds of a single run of rows that begins at 0 and has no end (``moe_gather`` in the order of the grouping)."""
-    bounds = _one_runs.get(device)
-    if bounds is None:
-        bounds = _one_runs[device] = torch.tensor([0, 1 << 30], dtype=torch.int32, device=device)
-    return bounds
-
-
 def moe_path(x: torch.Tensor, pairs: int, ff: int) -> str:
     """Which way ``moe_experts`` takes for a batch of ``pairs`` (token, expert) pairs of ``x``'s type."""
     if x.dtype != torch.bfloat16:
         return "tiles"
-    if pairs <= MOE_GEMV_MAX_PAIRS and x.shape[1] % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0:
+    whole = x.shape[1] % 8 == 0 and ff % 8 == 0          # rows of 16-byte pieces
+    if pairs <= MOE_GEMV_MAX_PAIRS and whole and x.stride(0) % 8 == 0:
         return "stream"
+    if whole:
+        return "grouped"
     return "library" if not torch.cuda.is_current_stream_capturing() else "tiles"
 
 
@@ -2280,10 +2280,11 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, gate_
     [E, F, K]`` and ``down[e] @ max(up[e] @ a, 0)^2``.  ``identity``: that many ids behind ``E`` stand for experts whose
     output is their input; no product sees their pairs (see ``ExpertRows``).
 
-    Three ways, by ``path`` (default: by type and size).  "tiles": grouped products of this library, one
+    Four ways, by ``path`` (default: by type and size).  "tiles": grouped products of this library, one
     accumulator per output in ascending k (all of float32: bit-equal under any batching).  "stream": bf16,
-    a handful of pairs, one pass over each chosen expert's matrices.  "library": bf16 prompts, the pairs'
-    rows gathered expert by expert at a common stride and one batched library product per matrix over all
+    a handful of pairs, one pass over each chosen expert's matrices.  "grouped": bf16 prompts, the pairs' rows gathered
+    expert by expert and one launch a matrix on the tensor cores, the activation in the first (``moe_tc5.cu``).  "library":
+    bf16 prompts whose rows are not whole 16-byte pieces, the pairs' rows gathered expert by expert at a common stride and one batched library product per matrix over all
     experts (the experts' row counts are read back from the device once per call)."""
     _check(x, "x", contiguous=False)
     _check(ids, "ids", dtype=torch.int32)
@@ -2343,6 +2344,22 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, gate_
               None if weight_on_input else weights.data_ptr(), down.data_ptr(), ids.data_ptr(), pairs, experts,
               experts + identity, n, ff, 0, *joined, _stream())
         return ExpertRows(out, top=top, identity=own)
+    if path == "grouped" and x.dtype == torch.bfloat16 and k % 8 == 0 and ff % 8 == 0:
+        if grouping is None or grouping.row_tiles is None:
+            grouping = moe_group(ids, experts, for_library=False, identity=identity, for_grouped=True)
+        rows = grouping.capacity
+        gathered = torch.empty((rows, k), dtype=x.dtype, device=x.device)
+        hidden = torch.empty((rows, ff), dtype=x.dtype, device=x.device)
+        out = torch.empty((rows, n), dtype=x.dtype, device=x.device)
+        _call("kvb_moe_gather", gathered.data_ptr(), x.data_ptr(), x.stride(0), top,
+              weights.data_ptr() if weight_on_input else None, grouping.sorted_pairs.data_ptr(),
+              None, 1, rows, grouping.row_of_pair.data_ptr(), k, code, _stream())
+        table, how = (grouping.row_tiles.data_ptr(), grouping.meta.data_ptr(), rows, experts), 2 if activation else 0 if join is None else 1
+        _call("kvb_moe_grouped", hidden.data_ptr(), gathered.data_ptr(), gate_up.data_ptr(), *table, ff, k,
+              grouping.tile_rows, how, *joined, _stream())
+        _call("kvb_moe_grouped", out.data_ptr(), hidden.data_ptr(), down.data_ptr(), *table, n, ff,
+              grouping.tile_rows, 3, *joined, _stream())
+        return ExpertRows(out, grouping.row_of_pair, None if weight_on_input else weights.reshape(-1), top, own)
     library = path == "library"
     if grouping is None or (library and grouping.expert_begin is None):
         grouping = moe_group(ids, experts, for_library=library, identity=identity)
@@ -2378,7 +2395,7 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, gate_
             gathered = torch.empty((total + spare, k), dtype=x.dtype, device=x.device)
             _call("kvb_moe_gather", gathered.data_ptr(), x.data_ptr(), x.stride(0), top,
                   weights.data_ptr() if weight_on_input else None, sorted_pairs.data_ptr(),
-                  _one_run(x.device).data_ptr(), 1, total, row_of_pair.data_ptr(), k, code, _stream())
+                  None, 1, total, row_of_pair.data_ptr(), k, code, _stream())
             both = torch.empty((total + spare, two_ff), dtype=x.dtype, device=x.device)
             out = torch.empty((total + spare, n), dtype=x.dtype, device=x.device)
             spans = [(e, begins[e], begins[e] + counts[e]) for e in range(experts) if counts[e]]

@@ -132,8 +132,10 @@ class RoutedExperts(FeedForward):
                              correction=self.correction, group_count=self.group_count, group_keep=self.group_keep,
                              weight_scale=self.weight_scale, bias=self.router_bias)
         grouping = None
-        if K.moe_path(x, x.shape[0] * self.top_k, self.expert_size) == "library":
-            grouping = K.moe_group(routed[0], self.num_experts, for_library=True, identity=self.identity_experts)
+        path = K.moe_path(x, x.shape[0] * self.top_k, self.expert_size)
+        if path in ("grouped", "library"):
+            grouping = K.moe_group(routed[0], self.num_experts, for_library=path == "library", identity=self.identity_experts,
+                                   for_grouped=path == "grouped")
         return routed, grouping
 
     def _expert_rows(self, x: torch.Tensor, ctx, prepared):
