@@ -441,7 +441,7 @@ moe_align_kernel(int* __restrict__ sorted, int* __restrict__ tile_expert, int* _
         counts[e] = 0;                   // becomes the fill cursor
         if (expert_begin != nullptr) expert_begin[e] = begin;   // where each expert's (padded) run of rows begins
       }
-      if (row_tiles != nullptr) {        // the run in as few tiles of tile_rows as hold it, equal but for MOE_BM rows
+      if (row_tiles != nullptr) {        // the run in as few tiles of tile_rows as hold it, equal but for 32 rows
         const int mine = (rows + tile_rows - 1) / tile_rows;
         int tiles_upto = mine;
 #pragma unroll
@@ -452,9 +452,10 @@ moe_align_kernel(int* __restrict__ sorted, int* __restrict__ tile_expert, int* _
         const int first = tiles_at + tiles_upto - mine;
         int row = at + upto - rows;
         for (int t = 0; t < mine; ++t) {
-          const int units = rows / MOE_BM / mine + (t < rows / MOE_BM % mine ? 1 : 0);
-          row_tiles[first + t] = make_int4(e, row, units * MOE_BM | mine << 12, first);
-          row += units * MOE_BM;
+          const int all = (rows + 31) / 32, units = all / mine + (t < all % mine ? 1 : 0);
+          const int here = min(units * 32, at + upto - row);         // the run's last 32 may be 16
+          row_tiles[first + t] = make_int4(e, row, here | mine << 12, first);
+          row += here;
         }
         tiles_at += __shfl_sync(0xffffffffu, tiles_upto, 31);
       }

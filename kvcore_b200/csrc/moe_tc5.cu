@@ -5,22 +5,26 @@
 // in one launch each, the activation formed from the 32-bit sums.
 //
 // The experts' rows are few and uneven (256 on average where 2,048 tokens choose 4 of 32 experts), so they are the tensor
-// pipe's N, which may be any multiple of 16 up to 256, and the weights its M: a block multiplies two tiles of 128 weight
-// rows (a gate tile and the up tile beside it, or two neighbouring ones) with up to NT rows of one expert.  An expert's
-// rows are cut into equal tiles (moe_align's table), nothing is multiplied that is not there but a run's last few rows up to
-// 16, and the host need not know the experts' loads.
+// pipe's N, which may be any multiple of 32 up to 256, and the weights its M: two blocks on neighbouring SMs multiply 256
+// weight rows, 128 each (and, with gated units, the 256 rows of the other matrix beside them), with up to NT rows of one
+// expert, half of which lie in either block's shared memory.  An expert's rows are cut into equal tiles (moe_align's table),
+// nothing is multiplied that is not there but a run's last few rows up to 32, and the host need not know the experts' loads.
 //
-// One block an SM; the blocks take (expert, weight tile, row tile) in turn, the row tiles of a weight tile next to one another
-// so that weights come from memory once.  Warp 0 brings both weight tiles and the rows by TMA, 64 k a stage; warp 1 issues the
-// products (two accumulators of NT columns in tensor memory); warps 4 to 11 take the accumulators out, join and store them
-// (a lane owns a weight row, so a warp stores 64 neighbouring bytes of a row).  The ring runs on from item to item; with up to
-// 128 rows two pairs of accumulators alternate.
+// One pair of blocks a pair of SMs; the pairs take (expert, weight tile, row tile) in turn, the row tiles of a weight tile next
+// to one another so that weights come from memory once.  In each block warp 0 brings its weight rows and warp 2 its half of
+// the expert's rows by TMA, 64 k a stage, all of it reported to block 0; warp 1 of block 0 issues the products; the other 16 warps
+// take the block's accumulators out of tensor memory and join them (a lane owns a weight row), turn 16 rows of 32 results in
+// shared memory and store them in pieces of 16 bytes.  The ring runs on from item to item; where tensor memory holds them, two sets of accumulators
+// alternate.
 //
-// What bounds it: with many rows the shared memory, which takes 48 to 64 KB a stage in and gives every weight tile and all rows
-// to the products four times; with few the passes over the weights.  32 experts of 3,584 at width 4,096, 4 a token, whole
-// call with the choices given (B200, call after call): 2,048 tokens 763 us where two batched library products at a common
-// stride and an activation between them took 878 (the products 444 and 225 us for 494, 38 and 231); 1,000 tokens 550 and
-// 648; 130 tokens 458 and 532 (430 of bytes).  16 warps that take the accumulators out: the same.
+// What bounds it: with many rows the tensor pipe at the clock that the power limit leaves (75 % of its cycles; the rest is the
+// joining of gated units, 256 rows of which fill tensor memory, and pairs of blocks that have one item fewer); with few the
+// passes over the weights.  32 experts of 3,584 at width 4,096, 4 a token, whole call with the choices given (B200, call after
+// call, beside two batched library products at a common stride and an activation between): 2,048 tokens 706 us and 837; 1,000
+// tokens 516 and 628; 130 tokens 446 and 522 (430 of bytes); 16 experts of 4,096 at width 2,048, 2 a token: 2,048 tokens 236
+// and 287, 260 tokens 146 and 197.  Single blocks with tiles of 128 x 256 took 763 of 878; one lane alone asking for the copies
+// (90 cycles each) 850; results stored by lanes, two bytes each, by eight warps 766; items taken from a counter instead of in
+// turn 747 of 860.
 #include <cuda.h>
 #include <string.h>
 
@@ -28,8 +32,9 @@
 #include "sm100.cuh"
 
 #define MG_K 64
-#define MG_W_BYTES (128 * MG_K * 2)         // one weight tile of a stage
-#define MG_OUT_WARPS 8
+#define MG_W_BYTES (128 * MG_K * 2)         // a block's 128 weight rows of a stage
+#define MG_OUT_WARPS 16
+#define MG_OUT_BYTES 1024                   // a warp's 16 rows of 32 results on their way out
 #define MG_THREADS (128 + 32 * MG_OUT_WARPS)
 #define MG_SPIN_LIMIT (1u << 20)
 
@@ -43,17 +48,22 @@ struct GroupedParams {
   const int4* tiles;                        // {expert, first row, rows | row tiles of the expert << 12, the expert's first tile}
   const int* meta;                          // [1]: how many
   int width;                                // outputs of an expert
-  int weight_rows, second;                  // rows of an expert's matrix; the second tile's distance from the first
+  int weight_rows, second;                  // rows of an expert's matrix; the up rows' distance from the gate rows
   int weight_tiles, k_stages;
+  int out16;                                // rows of out are whole 16-byte pieces
   float alpha, limit, shift;
   int* status;
 };
 
-template <int NT> struct GroupedRing {
-  static constexpr int STAGE = 2 * MG_W_BYTES + NT * MG_K * 2;
-  static constexpr int STAGES = NT >= 256 ? 3 : NT >= 128 ? 4 : 5;
-  static constexpr int BUFFERS = NT >= 256 ? 1 : 2;          // pairs of accumulators
-  static constexpr int BYTES = STAGES * STAGE + 256;
+template <int NT, bool JOINED> struct GroupedRing {
+  static constexpr int WEIGHTS = JOINED ? 2 : 1;
+  static constexpr int BOX = NT / 2 < 64 ? NT / 2 : 64;               // rows of a copy of the experts' rows
+  static_assert(NT / 2 % BOX == 0, "a block's half of the rows is whole copies: none goes beyond its place");
+  static constexpr int STAGE = WEIGHTS * MG_W_BYTES + NT / 2 * MG_K * 2;
+  static constexpr int ROOM = 226 * 1024 - MG_OUT_WARPS * MG_OUT_BYTES;
+  static constexpr int STAGES = ROOM / STAGE < 8 ? ROOM / STAGE : 8;
+  static constexpr int BUFFERS = WEIGHTS * NT > 256 ? 1 : 2;          // sets of accumulators
+  static constexpr int BYTES = STAGES * STAGE + MG_OUT_WARPS * MG_OUT_BYTES + 256;
 };
 
 __device__ __forceinline__ void mg_ld16(unsigned taddr, float (&v)[16]) {
@@ -64,36 +74,34 @@ __device__ __forceinline__ void mg_ld16(unsigned taddr, float (&v)[16]) {
 }
 
 template <int NT, int MODE>
-__global__ void __launch_bounds__(MG_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
 moe_grouped_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map, const GroupedParams p) {
-  using Ring = GroupedRing<NT>;
-  constexpr int STAGES = Ring::STAGES, BUFFERS = Ring::BUFFERS;
   constexpr bool JOINED = MODE == MG_SILU || MODE == MG_CLAMPED;
-  constexpr int COVERS = JOINED ? 128 : 256;                 // outputs of an item
+  using Ring = GroupedRing<NT, JOINED>;
+  constexpr int STAGES = Ring::STAGES, BUFFERS = Ring::BUFFERS, WEIGHTS = Ring::WEIGHTS, BOX = Ring::BOX;
   KVB_KERNEL_PROLOGUE(KVB_TAG_MOE_GEMM);
   extern __shared__ __align__(1024) unsigned char mg_dyn[];
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(mg_dyn + STAGES * Ring::STAGE);
+  unsigned char* out_smem = mg_dyn + STAGES * Ring::STAGE;
+  unsigned long long* full = reinterpret_cast<unsigned long long*>(out_smem + MG_OUT_WARPS * MG_OUT_BYTES);   // block 0's counts
   unsigned long long* empty = full + STAGES;
   unsigned long long* acc_full = empty + STAGES;             // [BUFFERS]
-  unsigned long long* acc_empty = acc_full + BUFFERS;        // [BUFFERS] the warps that take them out
+  unsigned long long* acc_empty = acc_full + BUFFERS;        // [BUFFERS] block 0's: the warps of both that take them out
   unsigned long long* drain = acc_empty + BUFFERS;           // given up: products in flight
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(drain + 1);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  if (kvb_smem(mg_dyn) & 1023u) {                            // cannot happen with the alignment asked for; never run misaligned
-    if (threadIdx.x == 0) atomicOr(p.status, KVB_STATUS_WAIT_TIMEOUT);
-    return;
-  }
+  const unsigned rank = kvb_cluster_rank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { kvb_mbar_init(&full[s], 1); kvb_mbar_init(&empty[s], 1); }
-    for (int b = 0; b < BUFFERS; ++b) { kvb_mbar_init(&acc_full[b], 1); kvb_mbar_init(&acc_empty[b], MG_OUT_WARPS); }
+    for (int b = 0; b < BUFFERS; ++b) { kvb_mbar_init(&acc_full[b], 1); kvb_mbar_init(&acc_empty[b], 2 * MG_OUT_WARPS); }
     kvb_mbar_init(drain, 1);
-    *abort_flag = 0;
+    *abort_flag = (kvb_smem(mg_dyn) & 1023u) ? 1 : 0;        // cannot happen with the alignment asked for; never run misaligned
     kvb_mbar_init_fence();
   }
-  if (warp == 1) kvb_tc5_alloc(tmem_slot, 512u);
+  if (warp == 1) kvb_tc5_alloc_pair(tmem_slot, 512u);
   kvb_tc5_fence_before();
-  __syncthreads();
+  kvb_cluster_sync();                                        // both blocks' barriers stand
   kvb_tc5_fence_after();
   const unsigned tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   auto gave_up = [&] {
@@ -103,7 +111,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
   auto aborted = [&] { return *reinterpret_cast<volatile int*>(abort_flag) != 0; };
 
   const int items = p.meta[1] * p.weight_tiles;
-  struct Item { int expert, row0, rows, tile; bool both; };
+  struct Item { int expert, row0, rows, tile, half; };       // half: rows of the product that each block holds
   auto item = [&](int i) {
     Item it;
     const int4 any = p.tiles[i / p.weight_tiles];            // a row tile of the item's expert
@@ -113,121 +121,140 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
     it.expert = mine.x;
     it.row0 = mine.y;
     it.rows = mine.z & 0xfff;
-    it.both = JOINED || it.tile * COVERS + 128 < p.width;    // the second tile of the last two may lie beyond the matrix
+    it.half = (it.rows + 31) / 32 * 16;
     return it;
   };
 
-  if (warp == 0) {
-    // ================= weights and rows =================
-    if (lane == 0) {
-      int at = 0;                                            // stages asked for so far
-      bool ok = true;
-      for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
-        const Item it = item(i);
-        const int wrow = it.expert * p.weight_rows + it.tile * COVERS, boxes = (it.rows + 63) / 64;
-        const unsigned bytes = (it.both ? 2u : 1u) * MG_W_BYTES + boxes * 64 * MG_K * 2;
-        for (int k = 0; k < p.k_stages; ++k, ++at) {
-          const int s = at % STAGES;
-          if (at >= STAGES && !kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&empty[s], ((at / STAGES) - 1) & 1)) { gave_up(); ok = false; break; }
-          if (aborted()) { ok = false; break; }
-          unsigned char* to = mg_dyn + s * Ring::STAGE;
-          kvb_mbar_expect_tx(&full[s], bytes);
-          kvb_tma_2d(to, &w_map, k * MG_K, wrow, &full[s]);
-          if (it.both) kvb_tma_2d(to + MG_W_BYTES, &w_map, k * MG_K, wrow + p.second, &full[s]);
-          for (int b = 0; b < boxes; ++b)
-            kvb_tma_2d(to + 2 * MG_W_BYTES + b * 64 * MG_K * 2, &a_map, k * MG_K, it.row0 + 64 * b, &full[s]);
-        }
-      }
-      if (aborted())                                         // let the copies in flight land before the block may exit
-        for (int j = max(0, at - STAGES); j < at; ++j) kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&full[j % STAGES], (j / STAGES) & 1);
-    }
-  } else if (warp == 1) {
-    // ================= products: the whole warp, one lane issues =================
-    const unsigned leader = kvb_elect();
-    const unsigned long long base = kvb_tc5_desc(kvb_smem(mg_dyn), 16, 1024);
-    unsigned at = 0, n = 0;
+  if (warp == 0 || warp == 2) {
+    // ================= weights (warp 0) and rows (warp 2): whole warps, one lane issues =================
+    const unsigned leader = kvb_elect(), ring = kvb_smem(mg_dyn) + (warp == 0 ? 0 : WEIGHTS * MG_W_BYTES);
+    const unsigned bar0 = kvb_cluster_addr(full, 0), first = rank == 0 && warp == 0 ? leader : 0u;
+    unsigned at = 0;                                         // stages asked for so far
     bool ok = true;
-    for (int i = blockIdx.x; i < items && ok; i += gridDim.x, ++n) {
+    for (int i = pair; i < items && ok; i += pairs) {
       const Item it = item(i);
-      const int rows = __shfl_sync(0xffffffffu, it.rows, 0), both = __shfl_sync(0xffffffffu, (int)it.both, 0);
-      const unsigned idesc = kvb_tc5_idesc(128, rows, false);
-      const unsigned b = n % BUFFERS, acc = tmem + b * 2 * NT;
-      if (n >= BUFFERS) ok = __all_sync(0xffffffffu, kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&acc_empty[b], ((n / BUFFERS) - 1) & 1));
-      for (int k = 0; k < p.k_stages && ok; ++k, ++at) {
+      const int boxes = __shfl_sync(0xffffffffu, (it.half + BOX - 1) / BOX, 0);
+      const int row = __shfl_sync(0xffffffffu, warp == 0 ? it.expert * p.weight_rows + it.tile * 256 + (int)rank * 128
+                                                         : it.row0 + (int)rank * it.half, 0);
+      const unsigned bytes = WEIGHTS * MG_W_BYTES + boxes * BOX * MG_K * 2;
+      for (int k = 0; k < p.k_stages; ++k, ++at) {
         const unsigned s = at % STAGES;
-        ok = __all_sync(0xffffffffu, kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&full[s], (at / STAGES) & 1));
+        if (at >= STAGES) ok = __all_sync(0xffffffffu, kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&empty[s], ((at / STAGES) - 1) & 1));
         if (!ok) break;
-        kvb_tc5_fence_after();
-        const unsigned long long w = base + s * (Ring::STAGE / 16), a = w + 2 * MG_W_BYTES / 16;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {                        // 16 k: 32 bytes of a row of 128
-          kvb_tc5_mma_by(acc, w + 2 * j, a + 2 * j, idesc, k > 0 || j > 0 ? 1u : 0u, leader);
-          if (both) kvb_tc5_mma_by(acc + NT, w + MG_W_BYTES / 16 + 2 * j, a + 2 * j, idesc, k > 0 || j > 0 ? 1u : 0u, leader);
+        const unsigned to = ring + s * Ring::STAGE, bar = bar0 + s * 8;
+        if (warp == 0) {
+          if (first) kvb_mbar_expect_tx(&full[s], 2 * bytes);          // both blocks'
+          kvb_tma_2d_pair(to, &w_map, k * MG_K, row, bar, leader);
+          if (JOINED) kvb_tma_2d_pair(to + MG_W_BYTES, &w_map, k * MG_K, row + p.second, bar, leader);
+        } else {
+          for (int b = 0; b < boxes; ++b)
+            kvb_tma_2d_pair(to + b * BOX * MG_K * 2, &a_map, k * MG_K, row + BOX * b, bar, leader);
         }
-        kvb_tc5_commit_by(&empty[s], leader);
       }
-      if (ok) kvb_tc5_commit_by(&acc_full[b], leader);
     }
     if (!ok) {
       if (lane == 0) gave_up();
-      kvb_tc5_commit_by(drain, leader);                      // tensor memory is given back below: products in flight first
-      kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(drain, 0);
+      // the copies in flight land before the block may exit: block 0 sees them; block 1 gives them a millisecond
+      if (rank == 0)
+        for (unsigned j = at < STAGES ? 0 : at - STAGES; j < at; ++j) kvb_mbar_wait<MG_SPIN_LIMIT / 16, 4096>(&full[j % STAGES], (j / STAGES) & 1);
+      for (int j = 0; j < 1000; ++j) __nanosleep(1000);
     }
     __syncwarp();
+  } else if (warp == 1) {
+    // ================= products: block 0's whole warp, one lane issues =================
+    if (rank == 0) {
+      const unsigned leader = kvb_elect();
+      const unsigned long long base = kvb_tc5_desc(kvb_smem(mg_dyn), 16, 1024);
+      unsigned at = 0, n = 0;
+      bool ok = true;
+      for (int i = pair; i < items && ok; i += pairs, ++n) {
+        const int half = __shfl_sync(0xffffffffu, item(i).half, 0);
+        const unsigned idesc = kvb_tc5_idesc(256, 2 * half, false);
+        const unsigned b = n % BUFFERS, acc = tmem + b * WEIGHTS * NT;
+        if (n >= BUFFERS) ok = __all_sync(0xffffffffu, kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&acc_empty[b], ((n / BUFFERS) - 1) & 1));
+        for (int k = 0; k < p.k_stages && ok; ++k, ++at) {
+          const unsigned s = at % STAGES;
+          ok = __all_sync(0xffffffffu, kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&full[s], (at / STAGES) & 1)) && !aborted();
+          if (!ok) break;
+          kvb_tc5_fence_after();
+          const unsigned long long w = base + s * (Ring::STAGE / 16), a = w + WEIGHTS * MG_W_BYTES / 16;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {                      // 16 k: 32 bytes of a row of 128
+            kvb_tc5_mma_pair(acc, w + 2 * j, a + 2 * j, idesc, k > 0 || j > 0 ? 1u : 0u, leader);
+            if (JOINED) kvb_tc5_mma_pair(acc + NT, w + MG_W_BYTES / 16 + 2 * j, a + 2 * j, idesc, k > 0 || j > 0 ? 1u : 0u, leader);
+          }
+          kvb_tc5_commit_pair(&empty[s], leader);
+        }
+        if (ok) kvb_tc5_commit_pair(&acc_full[b], leader);
+      }
+      if (!ok) {
+        if (lane == 0) gave_up();
+        kvb_tc5_commit_pair(drain, leader);                  // tensor memory is given back below: products in flight first
+        kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(drain, 0);
+      }
+      __syncwarp();
+    }
   } else if (warp >= 4) {
-    // ================= results: 16 rows at a time, turn about between the two warps of a lane quarter =================
+    // ================= results: 16 rows at a time, turn about between the four warps of a lane quarter =================
     const int quarter = warp & 3, turn = (warp - 4) >> 2;
     const unsigned lanes = (unsigned)(quarter * 32) << 16;
     unsigned n = 0;
     bool ok = true;
-    for (int i = blockIdx.x; i < items; i += gridDim.x, ++n) {
+    for (int i = pair; i < items; i += pairs, ++n) {
       const Item it = item(i);
       const unsigned b = n % BUFFERS;
-      ok = __all_sync(0xffffffffu, kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&acc_full[b], (n / BUFFERS) & 1));
+      ok = __all_sync(0xffffffffu, kvb_mbar_wait<MG_SPIN_LIMIT, 4096>(&acc_full[b], (n / BUFFERS) & 1)) && !aborted();
       if (!ok) break;
       kvb_tc5_fence_after();
-      const unsigned acc = tmem + lanes + b * 2 * NT;
-      const int feature = it.tile * COVERS + quarter * 32 + lane;
-      bf16* const to = p.out + (long long)it.row0 * p.width + feature;
+      const unsigned acc = tmem + lanes + b * WEIGHTS * NT;
+      const int feature0 = it.tile * 256 + (int)rank * 128 + quarter * 32;
+      bf16* const mine = reinterpret_cast<bf16*>(out_smem + (warp - 4) * MG_OUT_BYTES);
       for (int c = turn * 16; c < it.rows; c += 4 * MG_OUT_WARPS) {
         float u[16], v[16];
         mg_ld16(acc + c, u);
-        if (it.both) mg_ld16(acc + NT + c, v);
+        if (JOINED) mg_ld16(acc + NT + c, v);
         kvb_tc5_wait_ld();
+        __syncwarp();                                        // the rows in front have left
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          bf16* const at = to + (long long)(c + j) * p.width;
-          if (JOINED) {
-            float r;
-            if (MODE == MG_SILU) {
-              r = kvb_silu_for_bf16(u[j]) * v[j];
-            } else {
-              const float g = fminf(u[j], p.limit);
-              r = __fdividef(g, 1.0f + __expf(-p.alpha * g)) * (fminf(fmaxf(v[j], -p.limit), p.limit) + p.shift);
-            }
-            if (feature < p.width) *at = __float2bfloat16_rn(r);
-          } else {
-            if (MODE == MG_SQUARED) {
-              const float r = fmaxf(u[j], 0.0f), q = fmaxf(v[j], 0.0f);
-              u[j] = r * r;
-              v[j] = q * q;
-            }
-            if (feature < p.width) *at = __float2bfloat16_rn(u[j]);
-            if (feature + 128 < p.width) at[128] = __float2bfloat16_rn(v[j]);
+          float r = u[j];
+          if (MODE == MG_SILU) {
+            r = kvb_silu_for_bf16(u[j]) * v[j];
+          } else if (MODE == MG_CLAMPED) {
+            const float g = fminf(u[j], p.limit);
+            r = __fdividef(g, 1.0f + __expf(-p.alpha * g)) * (fminf(fmaxf(v[j], -p.limit), p.limit) + p.shift);
+          } else if (MODE == MG_SQUARED) {
+            r = fmaxf(u[j], 0.0f);
+            r *= r;
           }
+          mine[j * 32 + lane] = __float2bfloat16_rn(r);
+        }
+        __syncwarp();
+        if (p.out16) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {                      // eight rows, four lanes a row
+            const int row = h * 8 + (lane >> 2), at = (lane & 3) * 8;
+            if (feature0 + at < p.width)
+              *reinterpret_cast<uint4*>(p.out + (long long)(it.row0 + c + row) * p.width + feature0 + at) =
+                  *reinterpret_cast<const uint4*>(mine + row * 32 + at);
+          }
+        } else if (feature0 + lane < p.width) {
+          for (int j = 0; j < 16; ++j) p.out[(long long)(it.row0 + c + j) * p.width + feature0 + lane] = mine[j * 32 + lane];
         }
       }
       kvb_tc5_fence_before();
       __syncwarp();
-      if (lane == 0) kvb_mbar_arrive(&acc_empty[b]);
+      if (lane == 0) kvb_cluster_arrive(kvb_cluster_addr(&acc_empty[b], 0));
     }
     if (!ok && lane == 0) gave_up();
+    __syncwarp();
   }
   kvb_tc5_fence_before();
   __syncthreads();
+  kvb_cluster_sync();                                        // nobody reads the other's shared memory or tensor memory any more
   if (warp == 1) {
     kvb_tc5_fence_after();
-    kvb_tc5_dealloc(tmem, 512u);
+    kvb_tc5_dealloc_pair(tmem, 512u);
   }
 }
 
@@ -246,6 +273,7 @@ extern "C" int kvb_moe_grouped(void* out, const void* a, const void* w, const in
   if (rows == 0 || E == 0) return 0;
   KVB_REQUIRE(width > 0 && K > 0 && K % 8 == 0 && aligned16(a) && aligned16(w) && aligned16(tiles), "moe_grouped: unsupported sizes or addresses");
   KVB_REQUIRE(mode >= 0 && mode <= 3, "moe_grouped: unknown mode");
+  KVB_REQUIRE(tile_rows == 64 || tile_rows == 128 || tile_rows == 256, "moe_grouped: tiles of 64, 128 or 256 rows");
   KVB_REQUIRE(rows < (1ll << 31) && (long long)E * 2 * width < (1ll << 31), "moe_grouped: too many rows");
   KvbEncodeTiledFn encode = kvb_encode_tiled_fn();
   KVB_REQUIRE(encode != nullptr, "moe_grouped: the driver does not export cuTensorMapEncodeTiled");
@@ -256,9 +284,10 @@ extern "C" int kvb_moe_grouped(void* out, const void* a, const void* w, const in
   p.meta = meta;
   p.width = width;
   p.weight_rows = joined ? 2 * width : width;
-  p.second = joined ? width : 128;
-  p.weight_tiles = joined ? (width + 127) / 128 : (width + 255) / 256;
+  p.second = width;
+  p.weight_tiles = (width + 255) / 256;
   p.k_stages = (K + MG_K - 1) / MG_K;
+  p.out16 = width % 8 == 0 && aligned16(out) ? 1 : 0;
   p.alpha = alpha; p.limit = limit; p.shift = shift;
   p.status = kvb_status_word();
   KVB_REQUIRE(p.status != nullptr, "moe_grouped: no status word");
@@ -267,7 +296,7 @@ extern "C" int kvb_moe_grouped(void* out, const void* a, const void* w, const in
   const cuuint32_t elem[2] = {1, 1};
   for (int i = 0; i < 2; ++i) {
     const cuuint64_t dims[2] = {(cuuint64_t)K, i == 0 ? (cuuint64_t)E * p.weight_rows : (cuuint64_t)rows};
-    const cuuint32_t box[2] = {MG_K, i == 0 ? 128u : 64u};
+    const cuuint32_t box[2] = {MG_K, i == 0 ? 128u : tile_rows / 2 < 64 ? (cuuint32_t)tile_rows / 2 : 64u};
     KVB_REQUIRE(encode(i == 0 ? &w_map : &a_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(i == 0 ? w : a), dims, strides, box,
                        elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS,
@@ -276,9 +305,9 @@ extern "C" int kvb_moe_grouped(void* out, const void* a, const void* w, const in
   const int sms = kvb_sm_count() > 0 ? kvb_sm_count() : 148;
 #define KVB_GROUPED(NT, MODE)                                                                                              \
   if (tile_rows == NT && mode == MODE) {                                                                                   \
-    KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_grouped_kernel<NT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
-                                        GroupedRing<NT>::BYTES));                                                          \
-    KVB_CHECK_CUDA(kvb_launch((moe_grouped_kernel<NT, MODE>), dim3(sms), dim3(MG_THREADS), GroupedRing<NT>::BYTES, stream, true, \
+    constexpr int bytes = GroupedRing<NT, MODE == MG_SILU || MODE == MG_CLAMPED>::BYTES;                                   \
+    KVB_CHECK_CUDA(cudaFuncSetAttribute(moe_grouped_kernel<NT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
+    KVB_CHECK_CUDA(kvb_launch((moe_grouped_kernel<NT, MODE>), dim3(sms / 2 * 2), dim3(MG_THREADS), bytes, stream, true,    \
                               w_map, a_map, p));                                                                           \
     KVB_CHECK_LAUNCH();                                                                                                    \
     return 0;                                                                                                              \

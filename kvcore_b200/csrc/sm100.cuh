@@ -201,15 +201,6 @@ __device__ __forceinline__ unsigned kvb_elect() {
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
   return leader;
 }
-// D[tmem] (+)= A[smem] . B[smem], issued by the lane with `leader`.
-__device__ __forceinline__ void kvb_tc5_mma_by(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
-                                               unsigned idesc, unsigned accumulate, unsigned leader) {
-  asm volatile(
-      "{\n.reg .pred p, q;\n"
-      "setp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
-}
 // Four products by the lane with `leader`, A in tensor memory: a k-range of 64.
 template <int A_COLS, int B_STEP>
 __device__ __forceinline__ void kvb_tc5_mma4_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc,
@@ -276,6 +267,57 @@ __device__ __forceinline__ void kvb_tc5_st16(unsigned taddr, const float (&v)[16
 }
 __device__ __forceinline__ void kvb_tc5_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void kvb_tc5_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+
+// ---- pairs of blocks (a cluster of two on neighbouring SMs) that multiply together --------------
+__device__ __forceinline__ unsigned kvb_cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+// All threads of both blocks meet; what they wrote before is seen behind it.
+__device__ __forceinline__ void kvb_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The address, for both blocks, of what lies where `p` lies in the shared memory of block `rank`.
+__device__ __forceinline__ unsigned kvb_cluster_addr(const void* p, unsigned rank) {
+  unsigned a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(kvb_smem(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void kvb_cluster_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// A tensor copy into this block's shared memory that reports to a barrier of either block, by the lane with `leader`.
+__device__ __forceinline__ void kvb_tma_2d_pair(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar, unsigned leader) {
+  asm volatile(
+      "{\n.reg .pred q;\nsetp.ne.b32 q, %5, 0;\n"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n"
+      ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(bar), "r"(leader) : "memory");
+}
+// Both blocks, a whole warp each.
+__device__ __forceinline__ void kvb_tc5_alloc_pair(unsigned* slot, unsigned columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(kvb_smem(slot)), "r"(columns));
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+}
+__device__ __forceinline__ void kvb_tc5_dealloc_pair(unsigned tmem_base, unsigned columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(columns));
+}
+// D (+)= A . B over both blocks, issued by one lane of block 0: A's first 128 rows and B's first half of rows lie in block
+// 0's shared memory, the others at the same place in block 1's; each block's tensor memory gets its rows' results.
+__device__ __forceinline__ void kvb_tc5_mma_pair(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
+                                                 unsigned idesc, unsigned accumulate, unsigned leader) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n"
+      "setp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+// The barrier at this place in both blocks gets an arrival when the products issued so far have finished.
+__device__ __forceinline__ void kvb_tc5_commit_pair(unsigned long long* bar, unsigned leader) {
+  asm volatile("{\n.reg .pred q;\n.reg .b16 both;\nsetp.ne.b32 q, %1, 0;\nmov.b16 both, 3;\n"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n}\n"
+               ::"r"(kvb_smem(bar)), "r"(leader) : "memory");
+}
 
 // ---- host side: tensor maps -------------------------------------------------------------------
 // cuTensorMapEncodeTiled through the runtime's driver entry point (the library does not link the
