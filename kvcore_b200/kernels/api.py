@@ -843,24 +843,22 @@ def linear_stream(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | No
 _F32_SPLIT_MIN_K = 2048       # K from which a 32-bit product may take the tensor cores (gemm_f32_tc5.cu; checked at load)
 
 
-def _linear_f32(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None) -> None:
-    """``out = x @ weight.T (+ bias)`` in float32; rows of ``x`` and ``out`` may lie apart.  Large weights take the
-    tensor cores in pieces of bf16 (``gemm_f32_tc5.cu``), small ones FMA: by ``weight`` alone, so that a row's bits do not
-    depend on the batch it is in."""
+def _linear_f32_pieces(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None) -> bool:
+    """``out = x @ weight.T (+ bias)`` in float32 on the tensor cores, in pieces of bf16 (``gemm_f32_tc5.cu``), if
+    ``weight`` takes that way: large ones do, by ``weight`` alone, so that a row's bits do not depend on the batch it is
+    in.  Rows of ``x`` and ``out`` may lie apart."""
+    if _lib is None:
+        ensure_built()
     m, k = x.shape
     n = weight.shape[0]
-    args = (out.data_ptr(), x.data_ptr(), weight.data_ptr(), None if bias is None else bias.data_ptr(), m, n, k,
-            x.stride(0), out.stride(0))
-    if k >= _F32_SPLIT_MIN_K:
-        if _lib is None:
-            ensure_built()
-        scratch_bytes = _lib.kvb_gemm_f32_split_scratch(weight.data_ptr(), m, n, k)
-        if scratch_bytes > 0:
-            scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=x.device)
-            _call("kvb_gemm_f32_split", *args, scratch.data_ptr(), _stream(),
-                  kernels=_lib.kvb_gemm_f32_split_launches(m, n, k))
-            return
-    _call("kvb_gemm_f32", *args, _stream())
+    scratch_bytes = _lib.kvb_gemm_f32_split_scratch(weight.data_ptr(), m, n, k)
+    if scratch_bytes == 0:
+        return False
+    scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=x.device)
+    _call("kvb_gemm_f32_split", out.data_ptr(), x.data_ptr(), weight.data_ptr(), None if bias is None else bias.data_ptr(),
+          m, n, k, x.stride(0), out.stride(0), scratch.data_ptr(), _stream(),
+          kernels=_lib.kvb_gemm_f32_split_launches(m, n, k))
+    return True
 
 
 def linear(
@@ -887,7 +885,10 @@ def linear(
     n = weight.shape[0]
     if x.dtype == torch.float32:
         out = torch.empty((m, n), dtype=torch.float32, device=x.device)
-        _linear_f32(out, x, weight, bias)
+        if k >= _F32_SPLIT_MIN_K and _linear_f32_pieces(out, x, weight, bias):
+            return out
+        _call("kvb_gemm_f32", out.data_ptr(), x.data_ptr(), weight.data_ptr(),
+              None if bias is None else bias.data_ptr(), m, n, k, x.stride(0), out.stride(0), _stream())
         return out
     # Decode-sized batches: the layer is one pass over the weights, which this library's own
     # streaming kernel does, overlapping its start with the kernels in front of it.
@@ -1583,7 +1584,10 @@ def heads_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None
         if tuple(out.shape) != (tokens, heads, n) or out.stride(2) != 1:
             raise KernelError(f"heads_linear: out {tuple(out.shape)} does not fit")
         for h in range(heads):
-            _linear_f32(out[:, h], x[:, h], weight[h], None)
+            if k >= _F32_SPLIT_MIN_K and _linear_f32_pieces(out[:, h], x[:, h], weight[h], None):
+                continue
+            _call("kvb_gemm_f32", out[:, h].data_ptr(), x[:, h].data_ptr(), weight[h].data_ptr(), None, tokens, n, k,
+                  x.stride(0), out.stride(0), _stream())
         return out
     if out is not None:                     # the library writes the rows where they belong
         if tuple(out.shape) != (tokens, heads, n) or out.stride(2) != 1:
