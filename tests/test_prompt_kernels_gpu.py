@@ -7,7 +7,7 @@ import torch
 
 import plain_kernels as P
 from test_dutivik_kernels_gpu import F32, _HostBatch, _states
-from test_kernels_gpu import DEV, DTYPES, K, _cache_case, randn
+from test_kernels_gpu import DEV, DTYPES, K, _cache_case, _Ctx, randn
 from test_pipesun_kernels_gpu import _Batch
 
 pytestmark = pytest.mark.gpu
@@ -511,3 +511,30 @@ def test_rows_keep_32_bits_of_the_weights(lens, turned, window, scale):
     want = _attend(q, keys, values, lens, dict(group=1, maps=1, scale=how["scale"], window=window, sink=None, slopes=None))
     got, other = (float((t.double() - want).norm() / want.norm()) for t in (attend(carried, **how), attend(carried, num_splits=1, **how)))
     assert got <= min(other, 2.0 ** -15) and K().read_status() == 0, (got, other)
+
+
+@pytest.mark.parametrize("lens", [[(700, 240), (700, 192)] + [(2999 - 20 * i, 1) for i in range(31)],
+                                  [(0, 2048), (63, 1)], [(0, 40), (0, 33)] + [(i * 17, 1) for i in range(200)],
+                                  [(5, 30)] + [(4000, 2)] * 3])
+def test_decoded_tokens_beside_prompt_portions_have_the_bits_of_one_behind_the_other(lens):
+    """The decode kernel does not wait for the prompt kernel in front of it: with the new keys written right in front of both,
+    and the rows read right behind them, the same bits as with kernels that wait for one another."""
+    case = _cache_case(torch.bfloat16, 24, 8, 128, 16, lens)
+    ctx = _Ctx(case)
+    ctx.host_query_lens, ctx.host_context_lens = [q for _, q in lens], [c for c, _ in lens]
+    cos_sin = torch.stack([torch.cos(case["positions"].float()[:, None] * 0.01 * torch.arange(64, device=DEV)),
+                           torch.sin(case["positions"].float()[:, None] * 0.01 * torch.arange(64, device=DEV))], -1).contiguous()
+
+    def run():
+        qkv, keys, values = case["qkv"].clone(), case["k_cache"].clone(), case["v_cache"].clone()
+        out = K().paged_attention(qkv, keys, values, case["table"], ctx, 24, 8, 128, 128 ** -0.5, None, cos_sin=cos_sin, write_kv=True)
+        return K().rmsnorm(out, torch.ones(24 * 128, dtype=torch.bfloat16, device=DEV), 1e-6), out
+
+    K().set_overlapped_launch(False)
+    want = run()
+    torch.cuda.synchronize()
+    K().set_overlapped_launch(True)
+    for _ in range(5):
+        got = run()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert K().read_status() == 0
