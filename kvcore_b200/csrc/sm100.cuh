@@ -201,6 +201,13 @@ __device__ __forceinline__ unsigned kvb_elect() {
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
   return leader;
 }
+// A tensor copy by the lane with `leader`.
+__device__ __forceinline__ void kvb_tma_2d_by(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar, unsigned leader) {
+  asm volatile(
+      "{\n.reg .pred q;\nsetp.ne.b32 q, %5, 0;\n"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n"
+      ::"r"(kvb_smem(dst)), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(kvb_smem(bar)), "r"(leader) : "memory");
+}
 // Four products by the lane with `leader`, A in tensor memory: a k-range of 64.
 template <int A_COLS, int B_STEP>
 __device__ __forceinline__ void kvb_tc5_mma4_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc,

@@ -538,3 +538,62 @@ def test_decoded_tokens_beside_prompt_portions_have_the_bits_of_one_behind_the_o
         got = run()
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("dim,vdim", [(16, 16), (32, 40), (64, 64), (128, 128), (256, 72), (24, 8), (72, 24), (136, 48), (128, 200)])
+@pytest.mark.parametrize("kind", ["decay", "delta", "lightning", "retention"])
+def test_scans_by_tma_give_the_bits_of_copies_by_the_threads(kind, dim, vdim, monkeypatch):
+    """Keys with and without threads beyond them, columns that fill no block, whole stages of 16 tokens and rests, requests of
+    no tokens, several blocks' worth of heads; every shape of either kernel, from a state that is not zero."""
+    heads, lens = 3, [(0, 16), (0, 0), (0, 1), (0, 47), (0, 64), (0, 7)]
+    batch = _Batch(lens, slots=[5, 1, 0, 3, 2, 4])
+    tokens, results = batch.num_tokens, []
+    dtype = torch.bfloat16 if kind == "retention" else torch.float32
+    rows = randn(tokens, 2 * heads * dim + heads * vdim, seed=31, dtype=dtype) * 0.3
+    q, k, v = rows[:, :heads * dim], rows[:, heads * dim:2 * heads * dim], rows[:, 2 * heads * dim:]
+    decay = torch.tensor([0.9, 0.99, 1.0], dtype=torch.float32, device=DEV)
+    sizes = dict(heads=heads, dim=dim, value_dim=vdim)
+    for shape in ((None, None), ("8", "1"), ("8", "2"), ("8", "4"), ("16", "1"), ("16", "2")):
+        for name, value in zip(("KVCORE_SCAN_ROWS", "KVCORE_SCAN_COLS"), shape):
+            monkeypatch.delenv(name, raising=False)
+            if value:
+                monkeypatch.setenv(name, value)
+        state, _ = _states(6, heads * dim * vdim, seed=21)
+        if kind == "decay":
+            z = randn(tokens, heads * dim, seed=33, dtype=dtype)
+            out = K().gla_scan(q, k, v, z, state, batch, q_scale=0.3, tau=4.0, **sizes)
+        elif kind == "delta":
+            prepared = randn(tokens, 2 * heads * dim + heads * vdim + 2 * heads, seed=34, dtype=torch.float32) * 0.2
+            prepared[:, -2 * heads:] = torch.sigmoid(prepared[:, -2 * heads:])
+            out = K().delta_scan(prepared, state, batch, kv_heads=heads, **sizes)
+        elif kind == "lightning":
+            out = K().lightning_scan(q, k, v, decay, state, batch, **sizes)
+        else:
+            out = K().retention_scan(q, k, v, None, decay, state, batch, k_scale=0.2, **sizes)
+        results.append((out, state))
+    for out, state in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(state, results[0][1])
+    assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [40, 500])
+def test_delta_scan_against_64_bits(tokens):
+    """Every step rounds the state twice and the sums over 128 keys a few times: with unit keys and decays below one the errors
+    of earlier steps shrink, below 2^-18 of the result in all."""
+    heads, dim = 2, 128
+    prepared = randn(tokens, 4 * heads * dim - heads * dim + 2 * heads, seed=41, dtype=torch.float32)
+    q, k, v = (prepared[:, i * heads * dim:(i + 1) * heads * dim].view(tokens, heads, dim) for i in range(3))
+    k /= k.norm(dim=-1, keepdim=True)
+    prepared[:, -2 * heads:] = 0.5 + 0.5 * torch.sigmoid(prepared[:, -2 * heads:])
+    beta, gate = prepared[:, -2 * heads:-heads].double(), prepared[:, -heads:].double()
+    state, _ = _states(1, heads * dim * dim, seed=42)
+    S = state[0].double().view(heads, dim, dim)
+    got = K().delta_scan(prepared, state, _Batch([(0, tokens)]), heads=heads, kv_heads=heads, dim=dim, value_dim=dim)
+    want = torch.empty(tokens, heads, dim, dtype=torch.float64, device=DEV)
+    for t in range(tokens):
+        S = S * gate[t][:, None, None]
+        u = beta[t][:, None] * (v[t].double() - (S @ k[t].double()[:, :, None])[..., 0])
+        S = S + u[:, :, None] * k[t].double()[:, None]
+        want[t] = (S @ q[t].double()[:, :, None])[..., 0]
+    assert (got.double() - want).norm() <= 2.0 ** -18 * want.norm()
+    assert (state[0].double().view(heads, dim, dim) - S).norm() <= 2.0 ** -18 * S.norm()
