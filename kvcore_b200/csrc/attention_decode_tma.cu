@@ -65,11 +65,6 @@ struct DecodeParams {
   // have seen the end; the last one puts both back to zero, where they must be before a launch).
   int total_items;
   int* work;
-  // The kernel in front is the prompt attention of the same step, which wrote nothing that is read here and waited for
-  // everything before it ahead of letting this one in: nothing is waited for but its end, ahead of this one's own, since what
-  // comes behind waits for this kernel alone.  A layer of 3,072 with 31 decoded tokens behind 2,300 to 3,000 beside two portions
-  // of 240 tokens (96 blocks): 211 us a pass for 217; one of 4,096 with 8 behind 8,192 beside 512 tokens: 342 for 366.
-  int beside;
 };
 
 __device__ __forceinline__ void td_ldmatrix_x4(unsigned (&r)[4], unsigned addr) {
@@ -191,7 +186,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
     // coalesced load), a batch ahead of their use, so no copy waits on a table lookup.  Lane 0 owns
     // the barriers and writes the headers; lanes 0..pages_per_tile-1 each issue one page's copies.
     const int ppt = TD_KEYS / p.page_size;            // pages per tile: 1, 2, 4 or 8
-    bool waited = p.beside != 0, reached_end = false;
+    bool waited = false, reached_end = false;
     int g = 0;                                        // stages pushed so far
     int item = blockIdx.x;
     while (true) {
@@ -281,7 +276,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
         item = __shfl_sync(0xffffffffu, next, 0);
       }
     }
-    if (!waited || p.beside) kvb_grid_wait();
+    if (!waited) kvb_grid_wait();
     // the last block to see the end of the work puts the counters back for the next launch
     if (p.work != nullptr && reached_end && lane == 0) {
       __threadfence();
@@ -310,7 +305,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
   bool row_valid[2] = {false, false};
   int req = 0, kvh = 0, split = 0, q_begin = 0, q_len = 0, context = 0, key_lo = 0, key_hi = 0, tile_begin = 0,
       rows_total = 0;
-  bool waited = p.beside != 0;
+  bool waited = false;
   const int wkey = warp * 16;
   auto begin_item = [&](const TdStageHeader& h) {
     // ---- a new item ----
@@ -709,7 +704,7 @@ extern "C" int kvb_flash_decode_tma(void* out, long long out_stride, const void*
                                     int num_reqs, int max_query_len, int H, int KVH, int D, int page_size,
                                     int num_pages, float scale, int window, int num_splits, float* scratch,
                                     const float* cos_sin, void* k_cache, void* v_cache, int* work, int max_blocks,
-                                    float* lse, const float* sink, float cap, int beside, cudaStream_t stream) {
+                                    float* lse, const float* sink, float cap, cudaStream_t stream) {
   if (num_reqs == 0) return 0;
   KVB_REQUIRE(D == 64 || D == 128, "decode attention (TMA): head_dim must be 64 or 128");
   KVB_REQUIRE((k_cache == nullptr) == (v_cache == nullptr), "decode attention (TMA): give both caches or none");
@@ -755,8 +750,6 @@ extern "C" int kvb_flash_decode_tma(void* out, long long out_stride, const void*
   p.total_items = num_reqs * KVH * p.num_splits;
   const bool shared = work != nullptr && max_blocks > 0 && p.total_items > max_blocks;
   p.work = shared ? work : nullptr;
-  KVB_REQUIRE(!beside || k_cache == nullptr, "decode attention (TMA): the cache is written in front of both");
-  p.beside = beside;
   const int blocks = shared ? max_blocks : p.total_items;
   if (sink != nullptr || cap > 0.0f)
     return D == 64 ? launch_decode_tma<64, true>(k_map, v_map, p, max_rows, blocks, stream)

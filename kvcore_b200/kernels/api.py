@@ -69,7 +69,7 @@ def ensure_built(verbose: bool = False) -> str:
                                  _int, _int, _float, _int, _int, _int, _vp],
         "kvb_make_kv_tensor_map": [_vp, _vp, _ll, _int, _int, _int],
         "kvb_flash_decode_tma": [_vp, _ll, _vp, _ll, _vp, _vp, _vp, _int, _vp, _vp, _int, _int, _int, _int,
-                                 _int, _int, _int, _float, _int, _int, _vp, _vp, _vp, _vp, _vp, _int, _vp, _vp, _float, _int, _vp],
+                                 _int, _int, _int, _float, _int, _int, _vp, _vp, _vp, _vp, _vp, _int, _vp, _vp, _float, _vp],
         "kvb_make_kv_half_tensor_map": [_vp, _vp, _ll, _int, _int, _int],
         "kvb_flash_prefill_tc5": [_vp, _ll, _vp, _ll, _vp, _vp, _vp, _int, _vp, _vp, _int, _int, _int, _int, _int,
                                   _int, _int, _int, _float, _int, _vp, _vp, _float, _vp],
@@ -636,11 +636,10 @@ def paged_attention(
                 and ctx.max_query_len * group > 16):
             long_count = sum(1 for n in lens if n * group > 16)
             if 0 < long_count < ctx.num_reqs and all(n * group > 16 for n in lens[:long_count]):
-                beside = False
                 for begin, end in ((0, long_count), (long_count, ctx.num_reqs)):
                     part = _RequestRun(ctx, begin, end)
-                    beside = _flash_attention_into(out, qkv, k_cache, v_cache, table[begin:end], part, geometry,
-                                                   None, use_tma, use_tc5, None, None, lse, *bounded, beside=beside)
+                    _flash_attention_into(out, qkv, k_cache, v_cache, table[begin:end], part, geometry,
+                                          None, use_tma, use_tc5, None, None, lse, *bounded)
                 add_kept_first()
                 return out
         _flash_attention_into(out, qkv, k_cache, v_cache, table, ctx, geometry, num_splits, use_tma, use_tc5,
@@ -681,11 +680,10 @@ class _RequestRun:
 
 
 def _flash_attention_into(out, qkv, k_cache, v_cache, table, ctx, geometry, num_splits, use_tma, use_tc5,
-                          cos_sin, write_kv, lse=None, sink=None, softcap=None, beside=False) -> bool:
+                          cos_sin, write_kv, lse=None, sink=None, softcap=None) -> None:
     """The tensor-core attention kernels on one batch (or one run of requests of a batch): the TMA
     decode kernel for at most 16 rows a kv head, the tcgen05 kernel for portions of prompts, the
-    ``mma.sync`` kernel for the shapes those two do not take.  Returns whether the tcgen05 kernel ran; ``beside``: it ran
-    right in front, on other requests of this step, and the decode kernel need not wait for it."""
+    ``mma.sync`` kernel for the shapes those two do not take."""
     num_heads, num_kv_heads, head_dim, scale, window = geometry
     num_pages, _, page_size, _ = k_cache.shape
     lse_ptr = None if lse is None else lse.data_ptr()    # [tokens, H] rows of the whole step, as ``out``
@@ -709,9 +707,9 @@ def _flash_attention_into(out, qkv, k_cache, v_cache, table, ctx, geometry, num_
               k_cache.data_ptr() if write_kv else None, v_cache.data_ptr() if write_kv else None,
               _decode_work(qkv.device).data_ptr() if TMA_DECODE_SHARED_WORK else None,
               sms * TMA_DECODE_BLOCKS_PER_SM, lse_ptr, None if sink is None else sink.data_ptr(), float(softcap or 0.0),
-              int(beside), _stream(),
+              _stream(),
               kernels=2 if splits > 1 else 1)   # the splits are merged by a second kernel
-        return False
+        return
     if (not split_mode and use_tc5 and tc5_prefill_supported(qkv.dtype, head_dim, page_size)
             and out.stride(0) % 8 == 0):
         k_map, v_map = _kv_tensor_map_pair(k_cache, v_cache, "half")
@@ -720,7 +718,7 @@ def _flash_attention_into(out, qkv, k_cache, v_cache, table, ctx, geometry, num_
               ctx.query_start.data_ptr(), ctx.context_lens.data_ptr(), ctx.num_reqs, ctx.max_query_len,
               qkv.shape[0], num_heads, num_kv_heads, head_dim, page_size, num_pages, scale, window,
               lse_ptr, None if sink is None else sink.data_ptr(), float(softcap or 0.0), _stream())
-        return True
+        return
     splits = 1
     if split_mode:
         splits = num_splits or decode_splits(ctx.num_reqs, num_kv_heads, bound, sm_count(qkv.device))
@@ -734,7 +732,6 @@ def _flash_attention_into(out, qkv, k_cache, v_cache, table, ctx, geometry, num_
           num_heads, num_kv_heads, head_dim, page_size, num_pages, scale, window,
           splits, None if scratch is None else scratch.data_ptr(), lse_ptr, _stream(),
           kernels=2 if splits > 1 else 1)
-    return False
 
 
 _mm_out_dtype_ok: bool | None = None

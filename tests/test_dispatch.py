@@ -1,6 +1,9 @@
 """Rules that send a call to one kernel or another, checked without a GPU."""
 from __future__ import annotations
 
+import re
+from pathlib import Path
+
 import torch
 
 from kvcore_b200.kernels import api
@@ -30,3 +33,11 @@ def test_which_calls_the_tcgen05_kernel_over_rows_takes():
     for change in (dict(page_size=16), dict(value_strides=(width + 8, 128, 0)), dict(key_strides=(0, 128, 0), value_strides=(0, 128, 0))):
         assert not takes(**dict(in_order, **change)), change
     assert takes(key_strides=(page * width, (1 << 28) - 8, width))
+
+
+def test_the_decode_attention_waits_for_the_kernel_in_front_of_it_always():
+    """What earlier kernels wrote is promised to be seen behind griddepcontrol.wait alone, and the counters that its blocks share
+    may be filled right in front of it: no launch may set out as one that has waited already."""
+    source = (Path(api.__file__).parent.parent / "csrc" / "attention_decode_tma.cu").read_text()
+    starts = re.findall(r"bool waited = ([^;,]+)[;,]", source)
+    assert starts == ["false", "false"] and len(re.findall(r"kvb_grid_wait\(\)", source)) >= 4

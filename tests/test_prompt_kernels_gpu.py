@@ -517,8 +517,8 @@ def test_rows_keep_32_bits_of_the_weights(lens, turned, window, scale):
                                   [(0, 2048), (63, 1)], [(0, 40), (0, 33)] + [(i * 17, 1) for i in range(200)],
                                   [(5, 30)] + [(4000, 2)] * 3])
 def test_decoded_tokens_beside_prompt_portions_have_the_bits_of_one_behind_the_other(lens):
-    """The decode kernel does not wait for the prompt kernel in front of it: with the new keys written right in front of both,
-    and the rows read right behind them, the same bits as with kernels that wait for one another."""
+    """With the new keys written right in front of both kernels, and the rows read right behind them: the same bits whether the
+    launches overlap or wait for one another."""
     case = _cache_case(torch.bfloat16, 24, 8, 128, 16, lens)
     ctx = _Ctx(case)
     ctx.host_query_lens, ctx.host_context_lens = [q for _, q in lens], [c for c, _ in lens]
