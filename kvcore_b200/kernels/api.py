@@ -2259,14 +2259,21 @@ def _rounded_rows(rows: int) -> int:
     return -(-rows // unit) * unit
 
 
-def moe_path(x: torch.Tensor, pairs: int, ff: int) -> str:
-    """Which way ``moe_experts`` takes for a batch of ``pairs`` (token, expert) pairs of ``x``'s type."""
+def _moe_grouped_takes(gate_up: torch.Tensor, down: torch.Tensor) -> bool:
+    """Whether tensor maps describe the experts' matrices: on 16-byte boundaries, rows that 31 bits count."""
+    experts, widest = gate_up.shape[0], max(gate_up.shape[1], 2 * down.shape[1])
+    return gate_up.data_ptr() % 16 == 0 and down.data_ptr() % 16 == 0 and experts * 2 * widest < 1 << 31
+
+
+def moe_path(x: torch.Tensor, pairs: int, ff: int, gate_up: torch.Tensor | None = None, down: torch.Tensor | None = None) -> str:
+    """Which way ``moe_experts`` takes for a batch of ``pairs`` (token, expert) pairs of ``x``'s type and the experts' matrices
+    (not given: such as an allocation of their own holds)."""
     if x.dtype != torch.bfloat16:
         return "tiles"
     whole = x.shape[1] % 8 == 0 and ff % 8 == 0          # rows of 16-byte pieces
     if pairs <= MOE_GEMV_MAX_PAIRS and whole and x.stride(0) % 8 == 0:
         return "stream"
-    if whole:
+    if whole and (gate_up is None or _moe_grouped_takes(gate_up, down)):
         return "grouped"
     return "library" if not torch.cuda.is_current_stream_capturing() else "tiles"
 
@@ -2288,8 +2295,9 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, gate_
     accumulator per output in ascending k (all of float32: bit-equal under any batching).  "stream": bf16,
     a handful of pairs, one pass over each chosen expert's matrices.  "grouped": bf16 prompts, the pairs' rows gathered
     expert by expert and one launch a matrix on the tensor cores, the activation in the first (``moe_tc5.cu``).  "library":
-    bf16 prompts whose rows are not whole 16-byte pieces, the pairs' rows gathered expert by expert at a common stride and one batched library product per matrix over all
-    experts (the experts' row counts are read back from the device once per call)."""
+    bf16 prompts whose rows are not whole 16-byte pieces or whose matrices lie off 16-byte boundaries, the pairs' rows gathered
+    expert by expert at a common stride and one batched library product per matrix over all experts (the experts' row counts are
+    read back from the device once per call)."""
     _check(x, "x", contiguous=False)
     _check(ids, "ids", dtype=torch.int32)
     _check(weights, "weights", dtype=torch.float32)
@@ -2325,7 +2333,7 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, gate_
         return glu_clamped(both, alpha=joined[0], limit=joined[1], shift=joined[2])
 
     if path is None:
-        path = moe_path(x, pairs, ff)
+        path = moe_path(x, pairs, ff, gate_up, down)
     if path == "stream" and pairs > MOE_GEMV_SINGLE_PAIRS:
         # some experts are shared: the pairs of an expert take one pass over its matrices together
         g = grouping if grouping is not None else moe_group(ids, experts, for_library=False, identity=identity)

@@ -41,3 +41,24 @@ def test_the_decode_attention_waits_for_the_kernel_in_front_of_it_always():
     source = (Path(api.__file__).parent.parent / "csrc" / "attention_decode_tma.cu").read_text()
     starts = re.findall(r"bool waited = ([^;,]+)[;,]", source)
     assert starts == ["false", "false"] and len(re.findall(r"kvb_grid_wait\(\)", source)) >= 4
+
+
+def test_which_experts_the_grouped_products_take(monkeypatch):
+    """Matrices that no tensor map describes go the way they went before there were grouped products."""
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    x, pairs = torch.empty(500, 64, dtype=torch.bfloat16), 1000
+
+    def matrix(*shape, offset=0):
+        room = torch.empty(torch.Size(shape).numel() + 8, dtype=torch.bfloat16)
+        return room[offset:offset + torch.Size(shape).numel()].view(shape)
+    up, down = matrix(4, 48, 64), matrix(4, 64, 24)
+    assert up.data_ptr() % 16 == 0 and down.data_ptr() % 16 == 0
+    assert api.moe_path(x, pairs, 24) == api.moe_path(x, pairs, 24, up, down) == "grouped"
+    for offset in (1, 2, 4):
+        assert api.moe_path(x, pairs, 24, matrix(4, 48, 64, offset=offset), down) == "library"
+        assert api.moe_path(x, pairs, 24, up, matrix(4, 64, 24, offset=offset)) == "library"
+    many = torch.empty(1, dtype=torch.bfloat16).expand(1 << 14, 1 << 17, 64)
+    assert api.moe_path(x, pairs, 1 << 16, many, down) == "library"
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert api.moe_path(x, pairs, 24, up, down) == "grouped"
+    assert api.moe_path(x, pairs, 24, matrix(4, 48, 64, offset=1), down) == "tiles"

@@ -94,3 +94,25 @@ def test_grouped_products_in_a_captured_graph():
         graph.replay()
         assert torch.equal(out, run())
     assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("of", ["up", "down"])
+def test_experts_off_16_byte_boundaries_are_still_taken(of):
+    """Views of a larger allocation that begin 2 bytes behind a boundary: the results of the same numbers on one (results of two
+    ways, each of three roundings to bf16: 2^-7 of the sums)."""
+    tokens, experts, width, ff = 300, 6, 128, 64
+    x = randn(tokens, width, dtype=torch.bfloat16, seed=2)
+    up = randn(experts, 2 * ff, width, dtype=torch.bfloat16, seed=3, scale=0.08)
+    down = randn(experts, width, ff, dtype=torch.bfloat16, seed=4, scale=0.1)
+    weights = torch.ones(tokens, 2, device=DEV)
+    ids = torch.stack([torch.randperm(experts, generator=torch.Generator().manual_seed(i))[:2] for i in range(tokens)]).to(DEV, torch.int32)
+
+    def off(t):
+        room = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        room[1:] = t.flatten()
+        return room[1:].view(t.shape)
+    want = K().moe_combine(K().moe_experts(x, ids, weights, up, down, weight_on_input=False), tokens, 2).double()
+    rows = K().moe_experts(x, ids, weights, off(up) if of == "up" else up, off(down) if of == "down" else down, weight_on_input=False)
+    got = K().moe_combine(rows, tokens, 2).double()
+    assert (got - want).norm() <= want.norm() * 2.0 ** -7
+    assert K().read_status() == 0
