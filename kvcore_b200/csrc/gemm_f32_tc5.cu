@@ -1,13 +1,16 @@
 // 32-bit linear layer on the 5th-generation tensor cores without giving up 32-bit operands:
 // out[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]), float in and out.
 //
-// A float is the sum of three bf16 numbers, exactly: the number rounded to bf16, what that left rounded to bf16, and the
-// rest (8 + 8 + 8 bits; a rest below 2^-133 is lost).  Six of the nine products of such pieces are taken (bf16 x bf16 is
-// exact in 32 bits); the three left out are below 2^-26 of the product they belong to.  What limits the result is then how
-// sums are taken.  The tensor pipe adds into its accumulator without rounding to nearest, so an accumulator holds 64 k
-// only, small products first, and is then added to the sum proper in a register, rounded to nearest.  Error against 64 bits
-// relative to the result, random inputs: 1.1e-7 to 1.5e-7 at K 2048 to 8192 where one accumulator in ascending k
-// (gemm_f32.cu) has 8.1e-7 to 1.6e-6.
+// A float is three bf16 numbers, exactly: the number rounded to bf16, what that left, times 2^8, rounded to bf16, and the rest, times
+// 2^16 (8 + 8 + 8 bits; the factors keep the smallest float, 2^-149, above the smallest bf16, 2^-133.  In the pipe a number below
+// 2^-126 stands as high as 2^-126: sums of such numbers only are off by up to half of 2^-149 of one a term).  Six of the nine products
+// of such pieces are taken (bf16 x bf16 is exact in 32 bits); the three left out are below 2^-25, 2^-25 and 2^-34 of the
+// product they belong to.  What limits the result is then how sums are taken.  The tensor pipe adds into its accumulator without
+// rounding to nearest, so an accumulator holds 64 k only, small products first, and is then added to the sum proper in a
+// register, rounded to nearest.  Error against 64 bits relative to the result, random inputs: 1.1e-7 to 1.5e-7 at K 2048 to
+// 8192 where one accumulator in ascending k (gemm_f32.cu) has 8.1e-7 to 1.6e-6.  Sums of up to about 16 terms that are not zero
+// are further off than there, by a unit in the last place: largest error in 2^-24 of the terms, this kernel and that one, one
+// term 2.3 and 1.0, four 3.8 and 2.9, eight 3.2 and 4.0, 64 1.8 and 6.1, 2048 0.4 and 5.4.
 //
 // The order of the sums depends on N and K only: 64 k at a time in ascending order, within `segments` equal stretches of K
 // (they give the SMs work where N has few tiles) whose sums are added in order.  Every number of rows takes this kernel
@@ -49,17 +52,30 @@ struct SplitParams {
   int* status;
 };
 
-// Two floats as three pairs of bf16 (the lower one in the lower half), exactly.
+// Two floats at once, each rounded as a scalar instruction rounds it.
+__device__ __forceinline__ float2 fs_fma2(float2 a, float b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, z;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %4};\nmov.b64 z, {%5, %6};\n"
+      "fma.rn.f32x2 x, x, y, z;\nmov.b64 {%0, %1}, x;\n}\n"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 fs_times2(float2 a, float b) {
+  float2 d;
+  asm("{\n.reg .b64 x, y;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %4};\nmul.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}\n"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b));
+  return d;
+}
+// Two floats as three pairs of bf16 (the lower one in the lower half), exactly: hi + mid / 2^8 + lo / 2^16.
 __device__ __forceinline__ void fs_cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  float2 v = make_float2(a, b);
+  __nv_bfloat162 h = __float22bfloat162_rn(v);
   hi = *reinterpret_cast<unsigned*>(&h);
-  a -= __uint_as_float(hi << 16);
-  b -= __uint_as_float(hi & 0xffff0000u);
-  __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+  v = fs_times2(fs_fma2(make_float2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)), -1.0f, v), 256.0f);
+  __nv_bfloat162 m = __float22bfloat162_rn(v);
   mid = *reinterpret_cast<unsigned*>(&m);
-  a -= __uint_as_float(mid << 16);
-  b -= __uint_as_float(mid & 0xffff0000u);
-  __nv_bfloat162 l = __floats2bfloat162_rn(a, b);
+  v = fs_times2(fs_fma2(make_float2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u)), -1.0f, v), 256.0f);
+  __nv_bfloat162 l = __float22bfloat162_rn(v);
   lo = *reinterpret_cast<unsigned*>(&l);
 }
 
@@ -252,13 +268,14 @@ f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
       const unsigned acc = tmem + b * 128, a = tmem + FS_TMEM_W + b * 96;
       const unsigned long long x0 = x_desc + b * (X_BYTES / 16);
       constexpr int PIECE = NT * FS_K * 2 / 16;            // a piece of the rows, in the descriptor's units of 16 bytes
-      // pieces (weight, row), 0 the largest: small products first
+      // Pieces (weight, row), 0 the largest: small products first.  What the pieces' factors of 2^8 and 2^16 made of them is taken
+      // back from sum to sum: the three smallest stand 2^16 too high, the next two 2^8.
       kvb_tc5_mma4_ts<8, 2>(acc, a + 64, x0, idesc, 0u, leader);
       kvb_tc5_mma4_ts<8, 2>(acc, a, x0 + 2 * PIECE, idesc, 1u, leader);
       kvb_tc5_mma4_ts<8, 2>(acc, a + 32, x0 + PIECE, idesc, 1u, leader);
-      kvb_tc5_mma4_ts<8, 2>(acc, a + 32, x0, idesc, 1u, leader);
+      kvb_tc5_mma4_ts<8, 2, 8>(acc, a + 32, x0, idesc, 1u, leader);
       kvb_tc5_mma4_ts<8, 2>(acc, a, x0 + PIECE, idesc, 1u, leader);
-      kvb_tc5_mma4_ts<8, 2>(acc, a, x0, idesc, 1u, leader);
+      kvb_tc5_mma4_ts<8, 2, 8>(acc, a, x0, idesc, 1u, leader);
       kvb_tc5_commit_by(&done[b], leader);
       issued = c + 1;
     }

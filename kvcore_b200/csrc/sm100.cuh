@@ -208,18 +208,26 @@ __device__ __forceinline__ void kvb_tma_2d_by(void* dst, const CUtensorMap* map,
       "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n"
       ::"r"(kvb_smem(dst)), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(kvb_smem(bar)), "r"(leader) : "memory");
 }
-// Four products by the lane with `leader`, A in tensor memory: a k-range of 64.
-template <int A_COLS, int B_STEP>
+// Four products by the lane with `leader`, A in tensor memory: a k-range of 64.  The first one takes what the accumulator holds
+// times 2^-DOWN.
+template <int A_COLS, int B_STEP, int DOWN = 0>
 __device__ __forceinline__ void kvb_tc5_mma4_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc,
                                                 unsigned idesc, unsigned accumulate, unsigned leader) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    asm volatile(
-        "{\n.reg .pred p, q;\n"
-        "setp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "r"(tmem_a + i * A_COLS), "l"(bdesc + (unsigned long long)(i * B_STEP)), "r"(idesc),
-          "r"(i == 0 ? accumulate : 1u), "r"(leader) : "memory");
+    if (DOWN != 0 && i == 0)
+      asm volatile(
+          "{\n.reg .pred p, q;\n"
+          "setp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+          "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%6, %6, %6, %6}, p, %7;\n}\n"
+          ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader), "r"(0u), "n"(DOWN) : "memory");
+    else
+      asm volatile(
+          "{\n.reg .pred p, q;\n"
+          "setp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+          "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+          ::"r"(tmem_d), "r"(tmem_a + i * A_COLS), "l"(bdesc + (unsigned long long)(i * B_STEP)), "r"(idesc),
+            "r"(i == 0 ? accumulate : 1u), "r"(leader) : "memory");
 }
 // The barrier gets an arrival when every MMA that the lane with `leader` issued so far has finished.
 __device__ __forceinline__ void kvb_tc5_commit_by(unsigned long long* bar, unsigned leader) {

@@ -166,7 +166,7 @@ def test_product_rows_have_the_same_bits_in_every_tile(m, n, k, tile):
 @pytest.mark.parametrize("n,k", [(128, 2048), (130, 2052), (515, 2108), (9601, 2048), (3072, 3072), (16390, 2064)])
 def test_product_in_pieces_has_the_same_bits_for_every_number_of_rows(n, k):
     """Weights from K 2,048 on: tiles of 16 to 128 rows, ragged columns, k and last chunks, one stretch of K and several; rows
-    off 16-byte boundaries.  A float is three bf16 exactly and three of nine products are left out (2^-26 of a term each);
+    off 16-byte boundaries.  A float is three bf16 exactly and three of nine products are left out (2^-24 of a term in all);
     a chunk's accumulator may lose one unit of 2^-23 at each of 24 additions of up to its 64 terms, 2^-18.4 of them; and
     k / 64 + 16 sums are rounded to nearest."""
     x, w = randn(300, k, dtype=torch.float32, seed=1), randn(n, k, dtype=torch.float32, seed=2)
@@ -196,8 +196,7 @@ def test_product_in_pieces_takes_many_rows_in_lots():
 
 
 def test_product_in_pieces_of_numbers_that_are_not_finite_or_too_large_for_bf16():
-    """Infinities, NaN, numbers above the largest bf16 and sums that leave the range: as the product by FMA has them.  Numbers
-    down to 2^-110 keep their bits (all three pieces are above the smallest bf16)."""
+    """Infinities, NaN, numbers above the largest bf16 and sums that leave the range: as the product by FMA has them."""
     x, w = randn(40, 2048, dtype=torch.float32, seed=1), randn(256, 2048, dtype=torch.float32, seed=2)
     x[3, 5] = float("inf")
     x[4, 7] = float("nan")
@@ -218,6 +217,53 @@ def test_product_in_pieces_of_numbers_that_are_not_finite_or_too_large_for_bf16(
     both = want.isfinite()
     terms = (x.double().nan_to_num(0, 0, 0).abs() @ w.double().nan_to_num(0, 0, 0).abs().T)[both]
     assert ((got - want)[both].double().abs() <= terms * 2049 * 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("down,up", [(60, 0), (100, 0), (110, 20), (114, 40), (118, 60), (123, 60)])
+@pytest.mark.parametrize("n,k", [(130, 2052), (3072, 2048)])
+def test_product_in_pieces_of_small_numbers_keeps_their_bits(n, k, down, up):
+    """Numbers between 2^-3 and 2^3, times an exact power of two that leaves them floats of 24 bits: the result of the unscaled
+    ones times that power, whichever side is small.  Down to 2^-117 bit for bit; below, pieces that are no normal numbers stand
+    lower in the pipe than the others, which may turn a rounding: as far from 64 bits as the unscaled ones, but for a quarter
+    (without the third piece it would be ten times as far)."""
+    apart = lambda t: t + torch.copysign(torch.full_like(t, 0.125), t)  # noqa: E731
+    x, w = (apart(randn(20, k, dtype=torch.float32, seed=1).clamp(-7, 7)), apart(randn(n, k, dtype=torch.float32, seed=2).clamp(-7, 7)))
+    assert torch.equal(x * 2.0 ** -down * 2.0 ** down, x)
+    plain, exact, back = K().linear(x, w).double(), x.double() @ w.double().T, 2.0 ** (down - up)
+    assert ((plain.float() / back).abs() > 2.0 ** -120).float().mean() > 0.99
+    for got in (K().linear(x * 2.0 ** -down, w * 2.0 ** up), K().linear(x * 2.0 ** up, w * 2.0 ** -down)):
+        if down <= 114:
+            assert torch.equal(got, (plain / back).float())
+        assert (got.double() * back - exact).norm() <= 1.25 * (plain - exact).norm()
+    assert K().read_status() == 0
+
+
+def test_product_in_pieces_of_numbers_below_the_smallest_normal_float():
+    """Whole multiples of 2^-149 are three bf16 exactly too; in the pipe a number below 2^-126 stands as high as 2^-126: the bound
+    of ordinary numbers for these, half of 2^-149 of a number a term."""
+    k = 2048
+    x = torch.randint(-(1 << 23), 1 << 23, (20, k), generator=torch.Generator().manual_seed(1)).to(DEV)
+    x[10:] >>= 12
+    x, w = (x.double() * 2.0 ** -149).float(), randn(200, k, dtype=torch.float32, seed=2) * 2.0 ** 100
+    error = (K().linear(x, w).double() - x.double() @ w.double().T).abs()
+    assert (error <= 2.0 ** -126 * w.double().abs().sum(1) * (24 * 2.0 ** -23 + (k / 64 + 20) * 2.0 ** -24)).all()
+
+
+@pytest.mark.parametrize("terms", [1, 2, 3, 5, 16])
+@pytest.mark.parametrize("numbers", ["random", "worst"])
+def test_product_in_pieces_of_few_terms(terms, numbers):
+    """Sums of few terms that are not zero, also of numbers whose pieces left out are the largest (2^-24 of a term in all, all of
+    one sign): each term may cost the accumulator one unit of 2^-23 and, but for the first, the sum proper 2^-24; the sums of
+    smaller pieces may lose 0.3 of 2^-24 at most."""
+    x, w = torch.zeros(32, 2048, device=DEV), randn(256, 2048, dtype=torch.float32, seed=2)
+    values = randn(32, terms, dtype=torch.float32, seed=3)
+    if numbers == "worst":
+        worst = 1 + 2.0 ** -8 - 2.0 ** -16 + 2.0 ** -17 - 2.0 ** -23
+        values, w = torch.full_like(values, worst), torch.full_like(w, worst)
+    for r in range(32):
+        x[r, torch.randperm(2048, generator=torch.Generator().manual_seed(r))[:terms].to(DEV)] = values[r]
+    error = (K().linear(x, w).double() - x.double() @ w.double().T).abs()
+    assert (error <= (x.double().abs() @ w.double().abs().T) * (3 * terms + 0.3) * 2.0 ** -24).all()
 
 
 def test_heads_product_in_pieces():
