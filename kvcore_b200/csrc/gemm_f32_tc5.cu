@@ -30,7 +30,8 @@
 // 283, N 3072, K 8192 77 and 424; 32 rows, N 16384, K 3072 54 and 174; 4 rows 52 and 74.
 //
 // Where the result is not finite the output is taken again in plain FMA (infinities would otherwise meet the zeros among
-// the pieces and numbers above 3.39e38 would round to one): such outputs are as gemm_f32.cu has them.
+// the pieces and numbers above 3.39e38 would round to one): such outputs are as gemm_f32.cu has them, and cost a multiple of the
+// finite ones (fs_by_fma).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -46,7 +47,7 @@
 struct SplitParams {
   float* out; long long ldo;               // where a block's sums go: the result, or [segments][rows][N] of scratch
   const float* bias;                       // with the result only
-  const float* x; long long ldx; const float* w;   // for outputs that are not finite
+  const float* x; long long ldx; const float* w; int x16;   // for outputs that are not finite (x16: rows of x on 16-byte boundaries)
   int M, N, K;
   int tiles_m, tiles_n, segments, seg_chunks, chunks;
   int* status;
@@ -79,11 +80,48 @@ __device__ __forceinline__ void fs_cut(float a, float b, unsigned& hi, unsigned&
   lo = *reinterpret_cast<unsigned*>(&l);
 }
 
-// An output that is not finite, again: one accumulator in ascending k, as gemm_f32.cu takes it.
-__device__ __noinline__ float fs_by_fma(const float* xr, const float* wr, int K) {
-  float acc = 0.0f;
-  for (int k = 0; k < K && acc == acc; ++k) acc = fmaf(xr[k], wr[k], acc);     // a NaN stays one
-  return acc;
+// Outputs that are not finite, again, FS_AGAIN at a time that share a row (of x or of w): one accumulator each in ascending k, as
+// gemm_f32.cu takes it.  Bound by the latency of the loads, eight k at a time.  Whole products of which some is infinite, now, with
+// one output after the other four bytes at a time, and by gemm_f32.cu, microseconds: 256 rows, N 5120, K 3072: a row of x 511,
+// 1,850, 289; a column of weights (every output) 6,250, 27,300, 288; N 16384: a row of weights 3,030, 13,300, 623; a column
+// 8,500, 81,600, 624; finite 124.
+#define FS_AGAIN 4
+#define FS_AGAIN_QUADS 2
+__device__ __forceinline__ float4 fs_load4(const float* p, bool vec) {
+  return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __noinline__ void fs_by_fma(float (&out)[FS_AGAIN], const float* one, bool one16, const float* const (&others)[FS_AGAIN],
+                                       bool others16, int K) {
+  float acc[FS_AGAIN];
+  const float* row[FS_AGAIN];
+#pragma unroll
+  for (int r = 0; r < FS_AGAIN; ++r) { acc[r] = 0.0f; row[r] = others[r]; }
+  bool any = true;
+  for (int k = 0; k < K && any; k += 4 * FS_AGAIN_QUADS) {         // K is a multiple of four
+    float4 a[FS_AGAIN_QUADS], b[FS_AGAIN_QUADS][FS_AGAIN];
+#pragma unroll
+    for (int i = 0; i < FS_AGAIN_QUADS; ++i) {
+      const int at = min(k + 4 * i, K - 4);
+      a[i] = fs_load4(one + at, one16);
+#pragma unroll
+      for (int r = 0; r < FS_AGAIN; ++r) b[i][r] = fs_load4(row[r] + at, others16);
+    }
+#pragma unroll
+    for (int i = 0; i < FS_AGAIN_QUADS; ++i)
+      if (k + 4 * i < K)
+#pragma unroll
+        for (int r = 0; r < FS_AGAIN; ++r) {
+          acc[r] = fmaf(b[i][r].x, a[i].x, acc[r]);
+          acc[r] = fmaf(b[i][r].y, a[i].y, acc[r]);
+          acc[r] = fmaf(b[i][r].z, a[i].z, acc[r]);
+          acc[r] = fmaf(b[i][r].w, a[i].w, acc[r]);
+        }
+    any = false;                                                   // a NaN stays one
+#pragma unroll
+    for (int r = 0; r < FS_AGAIN; ++r) any |= acc[r] == acc[r];
+  }
+#pragma unroll
+  for (int r = 0; r < FS_AGAIN; ++r) out[r] = acc[r];
 }
 
 // x [M, K] -> pieces [3][M][Kp] bf16.  Four neighbouring k a thread (K is a multiple of four).
@@ -109,7 +147,7 @@ __global__ void __launch_bounds__(256) f32_pieces_kernel(bf16* pieces, const flo
 
 // out = sum of the stretches' sums in order (+ bias).
 template <int V>
-__global__ void __launch_bounds__(256) f32_fold_kernel(const SplitParams p, const float* partial) {
+__global__ void __launch_bounds__(256, 4) f32_fold_kernel(const SplitParams p, const float* partial) {
   KVB_KERNEL_PROLOGUE(KVB_TAG_GEMM_F32);
   const int pieces = p.N / V;
   const long long total = (long long)p.M * pieces, plane = (long long)p.M * p.N;
@@ -130,11 +168,22 @@ __global__ void __launch_bounds__(256) f32_fold_kernel(const SplitParams p, cons
         sum[0] += from[s * plane];
       }
     }
+    bool finite = true;
 #pragma unroll
-    for (int c = 0; c < V; ++c) {
-      if (!isfinite(sum[c])) sum[c] = fs_by_fma(p.x + m * p.ldx, p.w + (long long)(n + c) * p.K, p.K);
-      if (p.bias != nullptr) sum[c] += p.bias[n + c];
+    for (int c = 0; c < V; ++c) finite = finite && isfinite(sum[c]);
+    if (!finite) {
+      const float* rows[FS_AGAIN];
+      float again[FS_AGAIN];
+#pragma unroll
+      for (int c = 0; c < FS_AGAIN; ++c) rows[c] = p.w + (long long)(n + (c < V ? c : 0)) * p.K;
+      fs_by_fma(again, p.x + m * p.ldx, p.x16 != 0, rows, true, p.K);
+#pragma unroll
+      for (int c = 0; c < V; ++c)
+        if (!isfinite(sum[c])) sum[c] = again[c];
     }
+#pragma unroll
+    for (int c = 0; c < V; ++c)
+      if (p.bias != nullptr) sum[c] += p.bias[n + c];
     if (V == 4 && out16) {
       *reinterpret_cast<float4*>(to) = make_float4(sum[0], sum[1 % V], sum[2 % V], sum[3 % V]);
     } else {
@@ -370,9 +419,18 @@ f32_split_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         }
         if (p.segments > 1) again = 0;                     // the kernel that adds the stretches looks after these
         while (again) {
-          const int m = m0 + half * CW + __ffsll((long long)again) - 1;
-          again &= again - 1;
-          to[(long long)m * p.ldo] = fs_by_fma(p.x + m * p.ldx, p.w + (long long)n * p.K, p.K) + bias;
+          int m[FS_AGAIN];
+          const float* rows[FS_AGAIN];
+          float value[FS_AGAIN];
+#pragma unroll
+          for (int r = 0; r < FS_AGAIN; ++r) {             // the last of them again where there are fewer
+            m[r] = again ? m0 + half * CW + __ffsll((long long)again) - 1 : m[r > 0 ? r - 1 : 0];
+            again &= again - 1;
+            rows[r] = p.x + m[r] * p.ldx;
+          }
+          fs_by_fma(value, p.w + (long long)n * p.K, true, rows, p.x16 != 0, p.K);
+#pragma unroll
+          for (int r = 0; r < FS_AGAIN; ++r) to[(long long)m[r] * p.ldo] = value[r] + bias;
         }
       }
     } else if (lane == 0) {
@@ -486,10 +544,10 @@ extern "C" int kvb_gemm_f32_split(float* out, const float* x, const float* w, co
     p.x = x + (long long)first * ldx;
     p.out = p.segments > 1 ? partial : out + (long long)first * ldo;
     p.ldo = p.segments > 1 ? N : ldo;
-    const int vec = ldx % 4 == 0 && aligned16(p.x) ? 1 : 0;
+    p.x16 = ldx % 4 == 0 && aligned16(p.x) ? 1 : 0;
     const long long cut = ((long long)rows * (K / 4) + 255) / 256;
     KVB_CHECK_CUDA(kvb_launch(f32_pieces_kernel, dim3((unsigned)(cut < fill ? cut : fill)), dim3(256), 0, stream, true, pieces, p.x, rows, K,
-                              Kp, ldx, vec));
+                              Kp, ldx, p.x16));
     // tiles of 64 rows where 128 would hold many rows that are not there (a chunk of 64 rows costs half)
     const int nt = rows <= 16 ? 16 : rows <= 32 ? 32 : (rows + 63) / 64 * 64 < (rows + 127) / 128 * 128 ? 64 : 128;
     p.tiles_m = (rows + nt - 1) / nt;

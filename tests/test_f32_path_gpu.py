@@ -219,6 +219,53 @@ def test_product_in_pieces_of_numbers_that_are_not_finite_or_too_large_for_bf16(
     assert ((got - want)[both].double().abs() <= terms * 2049 * 2.0 ** -24).all()
 
 
+@pytest.mark.parametrize("m,n,k", [(150, 300, 2052), (33, 515, 2048), (5, 16390, 2064), (130, 19000, 2048)])
+def test_product_in_pieces_whose_rows_or_columns_are_not_finite(m, n, k):
+    """Infinities through a whole column of weights, a row of weights, a row of x and NaN behind them, one stretch of K and
+    several, rows of x on 16-byte boundaries and off them: every output is what the product by FMA has for it, or finite in both."""
+    api, room = K().api, torch.zeros(m, k + 1, dtype=torch.float32, device=DEV)
+    for where in ("column", "row", "x", "all"):
+        x, w = randn(m, k, dtype=torch.float32, seed=1), randn(n, k, dtype=torch.float32, seed=2)
+        if where in ("column", "all"):
+            w[:, 5] = float("inf")
+        if where in ("row", "all"):
+            w[n - 1, k - 1] = float("-inf")
+        if where in ("x", "all"):
+            x[m - 1, 70], x[1, k - 2], x[2] = float("inf"), float("nan"), 3e38
+        room[:, 1:] = x
+        want = torch.empty(m, n, dtype=torch.float32, device=DEV)
+        api._call("kvb_gemm_f32", want.data_ptr(), x.data_ptr(), w.data_ptr(), None, m, n, k, k, n, api._stream())
+        assert not want.isfinite().all()
+        for rows in (x, room[:, 1:]):
+            got = K().linear(rows, w)
+            assert torch.equal(got.isnan(), want.isnan()), where
+            assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()]), where
+    assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("most", [45, 4])
+def test_product_in_pieces_that_is_not_finite_does_not_stall(most):
+    """An infinite column of weights makes every output infinite, an infinite number of x a row: below 45 and 4 times the product
+    by FMA (22 and 1.8 as measured; 94 and 6.4 with one output behind the other)."""
+    api, (m, n, k) = K().api, (256, 5120, 3072)
+    x, w = randn(m, k, dtype=torch.float32, seed=1), randn(n, k, dtype=torch.float32, seed=2)
+    where = w[:, 5] if most == 45 else x[0, 5:6]
+    where.fill_(float("inf"))
+    out, times = torch.empty(m, n, dtype=torch.float32, device=DEV), []
+    for call in (lambda: api._call("kvb_gemm_f32", out.data_ptr(), x.data_ptr(), w.data_ptr(), None, m, n, k, k, n, api._stream()),
+                 lambda: K().linear(x, w)):
+        taken = []
+        for _ in range(4):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            call()
+            end.record()
+            torch.cuda.synchronize()
+            taken.append(begin.elapsed_time(end))
+        times.append(min(taken))
+    assert times[1] < most * times[0], times
+
+
 @pytest.mark.parametrize("down,up", [(60, 0), (100, 0), (110, 20), (114, 40), (118, 60), (123, 60)])
 @pytest.mark.parametrize("n,k", [(130, 2052), (3072, 2048)])
 def test_product_in_pieces_of_small_numbers_keeps_their_bits(n, k, down, up):
