@@ -8,7 +8,7 @@
 //   * the cached positions fall into chunks of 64 (from position 0 on);
 //   * a score is one accumulator in ascending d, times the scale; a chunk has its own maximum and sum of exponentials
 //     (lanes hold keys n and n + 32, then a butterfly), and an output entry one accumulator over its keys in ascending order;
-//   * chunks are added to the row's result one after the other (`Folded`).
+//   * chunks are added to the row's result one after the other (`Folded`); one without weight for the row is passed over.
 // A key the row does not see has no part in any of it, whatever its value holds (a later token's may be no number): in
 // chunks that not every row sees whole, an entry's sum passes over the keys that its row does not see.
 //
@@ -222,7 +222,7 @@ attention_tile_kernel(AttParams<T> p) {
   float* const vs = ks + ATT_CHUNK * LK;                             // [ATT_CHUNK][DV]
   float* const ss = vs + ATT_CHUNK * DV;                             // [ATT_CHUNK][LS]: scores, then probabilities
   __shared__ long long offset[ATT_CHUNK];
-  __shared__ int pos[ROWS], ends[5];
+  __shared__ int pos[ROWS], ends[5], by_row;                         // by_row: some row has no weight for any key of the chunk
   __shared__ float old_factor[ROWS], new_factor[ROWS], row_sum[ROWS];
   AttBlock<T> b{p, req, kvh, G, begin, min(ROWS, all_rows - row0), row0, 0, 0, 0, 0, 0,
                 (long long)kvh * p.page_size * p.D, (long long)p.KVH * p.page_size * p.D};
@@ -244,6 +244,7 @@ attention_tile_kernel(AttParams<T> p) {
     if (!b.chunk_wanted(base)) continue;
     __syncthreads();                                                 // the chunk in front has been read
     if (threadIdx.x < ATT_CHUNK) offset[threadIdx.x] = b.find(base + threadIdx.x);
+    if (threadIdx.x == 0) by_row = 0;
     __syncthreads();
     const int keys = b.keys_of(base);
     b.template fetch<THREADS>(ks, LK, DK, p.k_cache, offset, keys);
@@ -290,8 +291,13 @@ attention_tile_kernel(AttParams<T> p) {
       att_softmax(s0, s1, m, l);
       ss[lane * LS + r] = s0;
       ss[(lane + 32) * LS + r] = s1;
-      // a row that sees nothing of the chunk keeps what it has: factors of one and zero (its chunk's sums are zeros)
-      if (l != 0.0f) total[n].fold(m, l);
+      // a row for which the chunk has no weight (none of it seen, or every score -infinity) keeps what it has
+      if (l != 0.0f) {
+        total[n].fold(m, l);
+      } else if (r < b.rows) {
+        ss[lane * LS + r] = ss[(lane + 32) * LS + r] = ATT_UNSEEN;
+        if (lane == 0) by_row = 1;
+      }
       __syncwarp();
       if (lane == 0) { old_factor[r] = l != 0.0f ? total[n].a_factor : 1.0f; new_factor[r] = l != 0.0f ? total[n].s_factor : 0.0f; }
     }
@@ -324,7 +330,7 @@ attention_tile_kernel(AttParams<T> p) {
         }
       }
     };
-    if (ragged) {
+    if (ragged || by_row) {
 #pragma unroll 4
       for (int key = 0; key < keys; ++key) add_key(key, true);
     } else {

@@ -646,9 +646,9 @@ def paged_attention(
                               cos_sin, write_kv, lse, *bounded)
         add_kept_first()
         return out
-    # Requests of at most 8 rows a kv head (decoded tokens) have the segments of their cached tokens read by different
+    # Requests of at most 8 rows a kv head (decoded tokens) have the chunks of their cached tokens read by different
     # blocks and folded behind them (sized by the bound that the batch's shape gives, which a captured step keeps), in lots
-    # whose scratch stays below 64 MB.
+    # whose scratch stays below 64 MB (one request and kv head alone may ask for more, from half a million positions on).
     ensure_built()
     bound = getattr(ctx, "max_seq_len_bound", 0) or getattr(ctx, "max_seq_len", 0) or table.shape[1] * page_size
     sizes = (ctx.num_reqs, num_heads, num_kv_heads, head_dim, ctx.max_query_len, tokens, bound)

@@ -92,6 +92,35 @@ def test_values_a_row_does_not_see_do_not_count(dtype, value, window, keep):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim", [40, 128])
+def test_a_chunk_without_weight_does_not_count_however_the_rows_are_cut(dtype, dim):
+    """Every score of 64 positions is -infinity and their values are infinite: rows of a prompt's tiles, decoded tokens with one
+    block and with one a chunk have the bits that they have where those values are zero."""
+    heads, kv_heads, page, total = 6, 2, 16, 300
+    case, attend = _attention(dtype, heads, kv_heads, dim, page, [(0, total)])
+    qkv, planes = case["qkv"].clone(), [case["k_cache"].clone(), case["v_cache"].clone()]
+    qkv[:, : heads * dim : dim] = qkv[:, : heads * dim : dim].abs() + 0.5
+    for at in range(64, 128):
+        planes[0][int(case["table"][0, at // page]), :, at % page, 0] = float("-inf")
+        planes[1][int(case["table"][0, at // page]), :, at % page] = 0.0
+    want = attend(*planes, qkv)
+    for at in range(64, 128):
+        planes[1][int(case["table"][0, at // page]), :, at % page] = float("inf")
+    assert want.isfinite().all() and torch.equal(attend(*planes, qkv), want)
+    for at in (63, 64, 100, 127, 128, 255, 299):
+        one = dict(case, positions=case["positions"][at:at + 1], lens=[(at, 1)], req_index=case["req_index"][:1],
+                   query_start=torch.tensor([0, 1], dtype=torch.int32, device=DEV),
+                   context_lens=torch.tensor([at], dtype=torch.int32, device=DEV))
+        ctx = _Ctx(one)
+        for bound in (at + 1, 2000):
+            ctx.max_seq_len_bound = bound
+            got = K().paged_attention(qkv[at:at + 1], *planes, case["table"], ctx, heads, kv_heads, dim, dim ** -0.5, None,
+                                      force_general=True)
+            assert torch.equal(got, want[at:at + 1]), (at, bound)
+    assert K().read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_a_query_that_is_no_number_is_not_hidden(dtype):
     """All of a row's scores are NaN, in one segment or several: so is its result, as that of plain attention."""
     for lens in ([(0, 70)], [(0, 300)], [(700, 1)], [(100, 1)]):
