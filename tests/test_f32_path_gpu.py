@@ -216,12 +216,21 @@ def test_product_in_pieces_has_the_same_bits_for_every_number_of_rows(n, k):
     assert K().read_status() == 0
 
 
-def test_product_in_pieces_takes_many_rows_in_lots():
-    """More rows than the scratch for sums of stretches holds (2,048 at eight stretches of 2,048 columns)."""
-    x, w = randn(2200, 2048, dtype=torch.float32, seed=1), randn(2048, 2048, dtype=torch.float32, seed=2)
-    full = K().linear(x, w)
-    for first in (0, 1900, 2040, 2184):
-        assert torch.equal(K().linear(x[first:first + 16].contiguous(), w), full[first:first + 16]), first
+@pytest.mark.parametrize("rows,n,k", [(4300, 2048, 2048), (2101, 6144, 3072)])
+def test_product_in_pieces_takes_many_rows_in_lots(rows, n, k):
+    """More rows than the scratch for sums of stretches holds: the pieces, the sums and the rows' map are the next lot's while the
+    lot in front is being added up.  Rows on both sides of every lot's end, of x whose rows lie apart, into rows that lie apart."""
+    x, w = randn(rows, 2, k, dtype=torch.float32, seed=1), randn(2, n, k, dtype=torch.float32, seed=2)
+    K().api.ensure_built()
+    launches = lambda m: K().api._lib.kvb_gemm_f32_split_launches(m, n, k)  # noqa: E731
+    lot = next(m for m in range(128, rows, 128) if launches(m + 1) > launches(m))
+    assert launches(rows) == -(-rows // lot) * launches(1) and launches(1) == 3
+    got = K().heads_linear(x, w)
+    for h in range(2):
+        for first in [0, rows - 16] + [end - 9 for end in range(lot, rows, lot)]:
+            assert torch.equal(K().linear(x[first:first + 16, h].contiguous(), w[h]), got[first:first + 16, h]), (h, first)
+        assert ((got[:, h].double() - x[:, h].double() @ w[h].double().T).norm() <= 2.0 ** -21 * got[:, h].double().norm())
+    assert K().read_status() == 0
 
 
 def test_product_in_pieces_of_numbers_that_are_not_finite_or_too_large_for_bf16():
