@@ -662,13 +662,24 @@ static ScanShape scan_shape(int mode, int D, long long heads_of_all, int V, bool
   if ((r == 8 || r == 16) && r >= least) return {r, c == 4 ? (r == 8 ? 4 : 2) : c == 2 ? 2 : 1, false};
   if (c == 4) return {least, least == 8 ? 4 : 2, brief && least == 8};
   if (c == 1) return {least, 1, false};
-  if (brief) return least <= 8 ? ScanShape{8, 4, true} : ScanShape{16, 1, true};
+  // Single tokens with keys of 512, 16 heads of 512 values: 16 x 2 147 us, 16 x 1 167 (165 as four rows at a time); 64 heads 564 and 669 (636).
+  if (brief) return least <= 8 ? ScanShape{8, 4, true} : ScanShape{16, 2, false};
   if (least > 8) return {least, 1, false};
-  if ((D & (D - 1)) != 0 && D % 8 == 0) return {8, 2, false};     // the one shape by TMA for threads without rows
+  // Keys that leave threads without rows come by TMA in the shape 8 x 2 alone.  Beyond 128 entries a stage of them takes the room
+  // of 256, one block fits an SM (three vectors a token) or two, and with more blocks than that 8 x 4 by copies is sooner done.
+  // 64 heads of 128 values, 4 prompts of 100, keys of 192: gated linear 8 x 2 388, 8 x 4 271, lightning 249 and 214; 4 heads, one
+  // prompt of 300: 44 and 69, 36 and 56; keys of 96 with 96 values, 64 heads, 32 prompts of 33: 286 and 302, 214 and 250.
+  const bool spare = (D & (D - 1)) != 0 && D % 8 == 0;
+  if (spare && mode != 1)
+    return D <= 128 || scan_blocks(D, heads_of_all, V, 8, 2) <= (mode == 0 ? 1 : 2) * sms ? ScanShape{8, 2, false} : ScanShape{8, 4, false};
+  // Delta rule, keys of 256 (two blocks of 16 x 2 an SM by their stages): 16 heads of 128 values, 32 prompts of 33: 8 x 4 by copies
+  // 232, 16 x 2 260; one prompt of 300: 92 and 74.
+  if (mode == 1 && D == 256 && scan_blocks(D, heads_of_all, V, 16, 2) > 3 * sms) return {8, 4, false};
   struct { int rows, cols; double cost; } const fixed[] = {{8, 1, 0.5}, {8, 2, 0.6}, {8, 4, 1.0}}, delta[] = {{8, 1, 0.72}, {8, 2, 0.79}, {16, 2, 1.0}};
   ScanShape best = {8, 1, false};
   double least_cost = 0.0;
   for (const auto& o : mode == 1 ? delta : fixed) {
+    if (spare && o.cols == 1) continue;               // 16 heads of 128 values, 32 prompts of 33, keys of 192: 8 x 1 628, 8 x 2 382, 16 x 2 210
     const double cost = (double)((scan_blocks(D, heads_of_all, V, o.rows, o.cols) + sms - 1) / sms) * o.cost;
     if (least_cost > 0.0 && cost >= least_cost) continue;
     least_cost = cost;
