@@ -442,7 +442,7 @@ state_scan_kernel(ScanParams p) {
   }
 }
 
-// The same scan of prompts whose vectors and values a tensor map can describe (keys of 16 to 256 entries, a multiple of eight,
+// The same scan of prompts whose vectors and values a tensor map can describe (keys of 16 to 256 entries, a multiple of four,
 // rows and pointers on 16-byte boundaries): a warp of its own brings a stage's vectors, one box of [16 tokens] x [D] each, and values,
 // [16 tokens] x [columns], through a ring of SCAN_DEPTH stages, and the warps that compute meet nobody.  Copies by those warps
 // themselves cost more than their instructions, since whatever they load waits for the copies asked for in front of it.
@@ -528,7 +528,7 @@ state_scan_tma_kernel(const __grid_constant__ ScanMaps maps, const ScanParams p)
 #pragma unroll
     for (int j = 0; j < J; ++j) {
       ulonglong2 s4 = make_ulonglong2(0, 0);
-      if (col + cc < V && (WHOLE || part * DREG < D)) s4 = *reinterpret_cast<const ulonglong2*>(S_head + (size_t)(col + cc) * D + part * DREG + 4 * j);
+      if (col + cc < V && (WHOLE || part * DREG + 4 * j < D)) s4 = *reinterpret_cast<const ulonglong2*>(S_head + (size_t)(col + cc) * D + part * DREG + 4 * j);
       S[cc][2 * j] = s4.x;
       S[cc][2 * j + 1] = s4.y;
     }
@@ -539,14 +539,14 @@ state_scan_tma_kernel(const __grid_constant__ ScanMaps maps, const ScanParams p)
     return to_float(reinterpret_cast<const TV*>(at + Ring::VECTORS)[tt * COLS + c + cc]);
   };
   auto take = [&](Vectors& n, const unsigned char* at, int tt) {
-    const bool live = WHOLE || part * DREG < D;
-    const float* q = live ? reinterpret_cast<const float*>(at) + tt * pitch + part * DREG : zeros;
-    const int next = live ? SCAN_STAGE * pitch : 0;
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-      n.q4[j] = *reinterpret_cast<const ulonglong2*>(q + 4 * j);
-      n.k4[j] = *reinterpret_cast<const ulonglong2*>(q + next + 4 * j);
-      if (MODE == 0) n.a4[j] = *reinterpret_cast<const ulonglong2*>(q + 2 * next + 4 * j);
+      const bool live = WHOLE || part * DREG + 4 * j < D;
+      const float* q = live ? reinterpret_cast<const float*>(at) + tt * pitch + part * DREG + 4 * j : zeros;
+      const int next = live ? SCAN_STAGE * pitch : 0;
+      n.q4[j] = *reinterpret_cast<const ulonglong2*>(q);
+      n.k4[j] = *reinterpret_cast<const ulonglong2*>(q + next);
+      if (MODE == 0) n.a4[j] = *reinterpret_cast<const ulonglong2*>(q + 2 * next);
     }
     if constexpr (CPT == 4 && sizeof(TV) == 4) {
       const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const TV*>(at + Ring::VECTORS) + tt * COLS + c);
@@ -627,7 +627,7 @@ state_scan_tma_kernel(const __grid_constant__ ScanMaps maps, const ScanParams p)
   for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
     for (int j = 0; j < J; ++j)
-      if (col + cc < V && (WHOLE || part * DREG < D))
+      if (col + cc < V && (WHOLE || part * DREG + 4 * j < D))
         *reinterpret_cast<ulonglong2*>(S_head + (size_t)(col + cc) * D + part * DREG + 4 * j) =
             make_ulonglong2(S[cc][2 * j], S[cc][2 * j + 1]);
 }
@@ -651,7 +651,8 @@ static long long scan_blocks(int D, long long heads_of_all, int V, int rows, int
   const int owned = SCAN_THREADS / rsplit * cols;
   return heads_of_all * ((V + owned - 1) / owned);
 }
-static ScanShape scan_shape(int mode, int D, long long heads_of_all, int V, bool brief) {
+// tma: vectors and values may come by TMA.
+static ScanShape scan_shape(int mode, int D, long long heads_of_all, int V, bool brief, bool tma) {
   const long long sms = kvb_sm_count() > 0 ? kvb_sm_count() : 148;
   int least = 8;                                      // 32 threads a column at most
   while (least * 32 < D) least *= 2;
@@ -669,7 +670,9 @@ static ScanShape scan_shape(int mode, int D, long long heads_of_all, int V, bool
   // of 256, one block fits an SM (three vectors a token) or two, and with more blocks than that 8 x 4 by copies is sooner done.
   // 64 heads of 128 values, 4 prompts of 100, keys of 192: gated linear 8 x 2 388, 8 x 4 271, lightning 249 and 214; 4 heads, one
   // prompt of 300: 44 and 69, 36 and 56; keys of 96 with 96 values, 64 heads, 32 prompts of 33: 286 and 302, 214 and 250.
-  const bool spare = (D & (D - 1)) != 0 && D % 8 == 0;
+  // (Values that no map describes leave the choice to the costs below: gated linear, keys and values of 100, 64 heads, 32 prompts of
+  // 33: 8 x 4 by copies 388, 8 x 2 by copies 505.)
+  const bool spare = tma && (D & (D - 1)) != 0;
   if (spare && mode != 1)
     return D <= 128 || scan_blocks(D, heads_of_all, V, 8, 2) <= (mode == 0 ? 1 : 2) * sms ? ScanShape{8, 2, false} : ScanShape{8, 4, false};
   // Delta rule, keys of 256 (two blocks of 16 x 2 an SM by their stages): 16 heads of 128 values, 32 prompts of 33: 8 x 4 by copies
@@ -688,13 +691,16 @@ static ScanShape scan_shape(int mode, int D, long long heads_of_all, int V, bool
   return best;
 }
 
-// Whether a tensor map describes the vectors and values of a launch, and the maps.
+// Whether tensor maps describe the vectors and values of a launch, but for the width of its blocks, and the maps.
+static bool scan_by_tma(const ScanParams& p, size_t e, long long tokens) {
+  return p.D % 4 == 0 && p.D <= 256 && p.D >= 16 && p.vec16 && p.state16 && tokens < (1ll << 31) && p.V * e % 16 == 0 &&
+         (size_t)p.v_token * e % 16 == 0 && aligned16(p.v) && (size_t)p.vec_token * 4 % 16 == 0 &&
+         (long long)p.heads * p.V < (1ll << 31) && (long long)p.heads * p.D < (1ll << 31);
+}
 template <typename TV>
-static bool scan_maps(ScanMaps* maps, const ScanParams& p, int mode, int dreg, int cols, long long tokens) {
-  if (p.D % dreg != 0 || p.D > 256 || p.D < 16 || !p.vec16 || !p.state16 || cols > 256 || tokens >= (1ll << 31)) return false;
+static bool scan_maps(ScanMaps* maps, const ScanParams& p, int mode, int cols, long long tokens) {
   const size_t e = sizeof(TV);
-  if (p.V * e % 16 || cols * e % 16 || (size_t)p.v_token * e % 16 || !aligned16(p.v) || (size_t)p.vec_token * 4 % 16) return false;
-  if ((long long)p.heads * p.V >= (1ll << 31) || (long long)p.heads * p.D >= (1ll << 31)) return false;
+  if (!scan_by_tma(p, e, tokens) || cols > 256 || cols * e % 16) return false;
   KvbEncodeTiledFn encode = kvb_encode_tiled_fn();
   if (encode == nullptr) return false;
   const cuuint32_t elem[2] = {1, 1};
@@ -716,13 +722,14 @@ template <typename TV, int MODE>
 static int launch_state_scan(const ScanParams& p_in, int num_reqs, long long tokens, cudaStream_t stream) {
   ScanParams p = p_in;
   KVB_REQUIRE(p.D <= 512, "state_scan: keys wider than 512 entries");
-  const ScanShape shape = scan_shape(MODE, p.D, (long long)num_reqs * p.heads, p.V, tokens <= 2LL * num_reqs);
-  const int dreg = shape.rows, cpt = shape.cols;
-  int rsplit = 1;
-  while (dreg * rsplit < p.D) rsplit *= 2;
   p.vec16 = (p.D % 4 == 0 && p.vec_token % 4 == 0 &&
              ((uintptr_t)p.q | (uintptr_t)p.k | (MODE == 2 ? 0 : (uintptr_t)p.a)) % 16 == 0) ? 1 : 0;
   p.state16 = (p.D % 4 == 0 && p.state_stride % 4 == 0 && p.state_offset % 4 == 0 && (uintptr_t)p.state % 16 == 0) ? 1 : 0;
+  const ScanShape shape = scan_shape(MODE, p.D, (long long)num_reqs * p.heads, p.V, tokens <= 2LL * num_reqs,
+                                     scan_by_tma(p, sizeof(TV), tokens));
+  const int dreg = shape.rows, cpt = shape.cols;
+  int rsplit = 1;
+  while (dreg * rsplit < p.D) rsplit *= 2;
   const int cols = SCAN_THREADS / rsplit * cpt;
   const dim3 grid(num_reqs, p.heads, (p.V + cols - 1) / cols), block(SCAN_THREADS);
   cudaError_t err = cudaErrorInvalidValue;
@@ -748,7 +755,7 @@ static int launch_state_scan(const ScanParams& p_in, int num_reqs, long long tok
   ScanMaps maps = {};
   p.status = kvb_status_word();
   KVB_REQUIRE(p.status != nullptr, "state_scan: no status word");
-  if (!shape.brief && scan_maps<TV>(&maps, p, MODE, dreg, cols, tokens)) {
+  if (!shape.brief && scan_maps<TV>(&maps, p, MODE, cols, tokens)) {
 #define SCAN_TMA(DR, RS, CP, WHOLE)                                                                           \
     if (dreg == DR && rsplit == RS && cpt == CP && (p.D == DR * RS) == WHOLE) {                               \
       using Ring = ScanRing<TV, MODE, DR, RS, CP>;                                                            \

@@ -540,7 +540,8 @@ def test_decoded_tokens_beside_prompt_portions_have_the_bits_of_one_behind_the_o
     assert K().read_status() == 0
 
 
-@pytest.mark.parametrize("dim,vdim", [(16, 16), (32, 40), (64, 64), (128, 128), (256, 72), (24, 8), (72, 24), (136, 48), (128, 200)])
+@pytest.mark.parametrize("dim,vdim", [(16, 16), (32, 40), (64, 64), (128, 128), (256, 72), (24, 8), (72, 24), (136, 48), (128, 200), (20, 8),
+                                      (36, 24), (100, 48), (252, 16)])
 @pytest.mark.parametrize("kind", ["decay", "delta", "lightning", "retention"])
 def test_scans_by_tma_give_the_bits_of_copies_by_the_threads(kind, dim, vdim, monkeypatch):
     """Keys with and without threads beyond them, columns that fill no block, whole stages of 16 tokens and rests, requests of
@@ -601,7 +602,8 @@ def test_delta_scan_against_64_bits(tokens):
 
 @pytest.mark.parametrize("kind,dim,vdim,heads,lens", [
     ("delta", 192, 128, 16, [(0, 33)] * 32), ("delta", 96, 96, 64, [(0, 100)] * 4), ("delta", 48, 48, 64, [(0, 33)] * 32),
-    ("delta", 256, 128, 16, [(0, 33)] * 32), ("decay", 224, 128, 64, [(0, 100)] * 4), ("lightning", 160, 160, 64, [(0, 33)] * 32),
+    ("delta", 256, 128, 16, [(0, 33)] * 32), ("decay", 96, 100, 64, [(0, 33)] * 32), ("lightning", 100, 100, 64, [(0, 100)] * 4),
+    ("decay", 224, 128, 64, [(0, 100)] * 4), ("lightning", 160, 160, 64, [(0, 33)] * 32),
     ("lightning", 512, 512, 16, [(5, 1)] * 16)])
 def test_the_shape_of_a_scan_is_near_the_best_for_other_keys_than_128(kind, dim, vdim, heads, lens, monkeypatch):
     """The launch's own choice against every shape asked for: within a tenth of the best (from an eighth to three quarters slower
