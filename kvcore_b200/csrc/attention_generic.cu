@@ -284,23 +284,30 @@ attention_tile_kernel(AttParams<T> p) {
       }
     }
     __syncthreads();
+    // all rows' softmaxes before any is folded, so that their shuffles overlap: 24 heads of 128 over 8 in bf16, 1,000 tokens, 431 us for
+    // 452
+    float m[8], l[8];
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       const int r = warp * 8 + n;
-      float s0 = ss[lane * LS + r], s1 = ss[(lane + 32) * LS + r], m, l;
-      att_softmax(s0, s1, m, l);
+      float s0 = ss[lane * LS + r], s1 = ss[(lane + 32) * LS + r];
+      att_softmax(s0, s1, m[n], l[n]);
       ss[lane * LS + r] = s0;
       ss[(lane + 32) * LS + r] = s1;
+    }
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const int r = warp * 8 + n;
       // a row for which the chunk has no weight (none of it seen, or every score -infinity) keeps what it has
-      if (l != 0.0f) {
-        total[n].fold(m, l);
+      if (l[n] != 0.0f) {
+        total[n].fold(m[n], l[n]);
       } else if (r < b.rows) {
         ss[lane * LS + r] = ss[(lane + 32) * LS + r] = ATT_UNSEEN;
         if (lane == 0) by_row = 1;
       }
-      __syncwarp();
-      if (lane == 0) { old_factor[r] = l != 0.0f ? total[n].a_factor : 1.0f; new_factor[r] = l != 0.0f ? total[n].s_factor : 0.0f; }
+      if (lane == 0) { old_factor[r] = l[n] != 0.0f ? total[n].a_factor : 1.0f; new_factor[r] = l[n] != 0.0f ? total[n].s_factor : 0.0f; }
     }
+    __syncwarp();
     const bool ragged = b.ragged(base);
     if (ragged)
       for (int n = 0; n < 8; ++n) {
@@ -606,9 +613,11 @@ static int launch_attention(AttParams<T> p, const AttPlan& plan, int max_query_l
     KVB_CHECK_CUDA(kvb_launch((attention_tile_kernel<T, NJ, ROWS_>), dim3((unsigned)(heads * ((most + ROWS_ - 1) / ROWS_))),  \
                               dim3(4 * ROWS_), tile_bytes(LK, ROWS_), stream, true, p))
     // Blocks of 64 rows that do not fill the GPU twice take as long as the longest of them: half of them is done sooner.
-    // 24 heads of 128 over 8: 250 tokens 64 us for 86; 3 portions of 100 behind 700: 202 for 256.
+    // 24 heads of 128 over 8: 250 tokens 64 us for 86; 3 portions of 100 behind 700: 202 for 256.  Where keys and values do not go
+    // on their own (bf16, rows off 16 bytes) half the threads take longer to bring a chunk: 6 heads of 40 over 2 in bf16, 4 portions
+    // of 3 behind 4,000: 64 rows 720 us, 32 rows 820.
     const long long sms = kvb_sm_count() > 0 ? kvb_sm_count() : 148;
-    if (heads * ((most + 63) / 64) <= 2 * sms) { KVB_ATT_TILE(32); } else { KVB_ATT_TILE(64); }
+    if (sizeof(T) == 4 && p.vec && heads * ((most + 63) / 64) <= 2 * sms) { KVB_ATT_TILE(32); } else { KVB_ATT_TILE(64); }
 #undef KVB_ATT_TILE
   }
   if (plan.few) {
