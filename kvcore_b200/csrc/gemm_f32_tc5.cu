@@ -465,11 +465,14 @@ static void split_segments(int N, int K, int* segments, int* seg_chunks) {
     }
   }
 }
-// Whether w [N, K] takes this kernel, whatever the rows.  The line by K: a single row, the other kernel's best case (microseconds,
-// this one and gemm_f32.cu): N 2048: K 512 15 and 10, K 1024 15.4 and 14.4, K 1280 15.4 and 16.4, K 2048 17 and 22; N 4096:
-// K 1280 19.5 and 16.4, K 2048 21.5 and 23.4; N 8192, K 2048 27.6 and 24.6; N 16384: K 2048 42 and 43, K 3072 52 and 59.
-// With more rows this kernel is the faster one from K 512 on (64 rows, N 2048: K 512 15 and 32, K 2048 21 and 108), but the
-// rule must not ask for them.
+// Whether w [N, K] takes this kernel, whatever the rows: the order of the sums may not depend on them.  Microseconds, this one and
+// gemm_f32.cu, in a captured run of calls on different weights.  One row: K 2048: N 128 8.4 and 15.3, N 1024 9.6 and 15.4, N 2048
+// 12.5 and 15.6, N 3072 14.9 and 16.1, N 5120 16.0 and 18.4, N 16384 31.4 and 36.9; K 3072: N 128 9.0 and 22.4, N 3072 15.2 and
+// 23.6, N 16384 42.2 and 53.7; below K 2048 with launches of their own: N 2048: K 512 15 and 10, K 1024 15.4 and 14.4, K 1280 15.4
+// and 16.4; N 4096, K 1280 19.5 and 16.4.  A single row loses where the other kernel's blocks of 16 columns just fill a round
+// of the GPU (9,472 columns, four blocks an SM): K 2048: N 6400 19.5 and 18.5, N 8192 20.3 and 19.1, N 9472 22.5 and 19.2; K 2560: N
+// 6912 26.1 and 22.7; K 3072: N 6912 29.2 and 27.2; K 2048, N 26624 55.8 and 53.9.  With more rows it does not: N 8192, K 2048: 2
+// rows 20.4 and 21.1, 8 rows 21.6 and 38, 64 rows 25 and 102, 256 rows 54 and 242; N 6912, K 2560: 8 rows 27 and 44.
 static bool split_takes(const void* w, int N, int K) {
   return K % 4 == 0 && aligned16(w) && K >= FS_MIN_K && N >= FS_MIN_N;
 }

@@ -17,7 +17,7 @@
 // shared memory and store them in pieces of 16 bytes.  The ring runs on from item to item; where tensor memory holds them, two sets of accumulators
 // alternate.
 //
-// What bounds it: with many rows the tensor pipe at the clock that the power limit leaves (75 % of its cycles; the rest is the
+// What bounds it: with many rows the tensor pipe at the clock that the power limit leaves (72 to 78 % of its cycles; the rest is the
 // joining of gated units, 256 rows of which fill tensor memory, and pairs of blocks that have one item fewer); with few the
 // passes over the weights.  32 experts of 3,584 at width 4,096, 4 a token, whole call with the choices given (B200, call after
 // call, beside two batched library products at a common stride and an activation between): 2,048 tokens 706 us and 837; 1,000
@@ -259,7 +259,10 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
 }
 
 // Rows of a tile for a batch: `pairs` of `experts`.  Also what moe_align cuts runs by.  Smaller tiles leave room for more stages,
-// which keep more of the weights in flight where the rows are few.
+// which keep more of the weights in flight where the rows are few; larger ones pass over the weights less often.  Microseconds
+// with tiles of 64, 128 and 256 rows, 32 experts of 3,584 at width 4,096: 24 rows an expert 461, 460, 481; 48: 472, 473, 497; 64:
+// 514, 479, 525; 100: 655, 521, 551; 128: 832, 613, 579; 192: 982, 717, 646; 256: 1337, 799, 831; 384: 1563, 1013, 1413 (a second
+// tile of few rows an expert); 16 of 4,096 at 2,048: 48: 183, 183, 196; 100: 180, 166, 172; 160: 252, 206, 195; 384: 435, 298, 294.
 extern "C" int kvb_moe_grouped_rows(long long pairs, int experts) {
   const long long mean = experts > 0 ? pairs / experts : pairs;
   return mean <= 48 ? 64 : mean <= 100 ? 128 : 256;
